@@ -836,7 +836,7 @@ extern "C" void lumi_session_free(lumi_session* s) {
     for (auto& g : s->graphs) if (g.second.exec) cudaGraphExecDestroy(g.second.exec);
     void* dev[] = {s->score_logits, s->gemm_counters, s->gemm_scratch, s->h, s->xprev, s->bprev, s->cum, s->kv_pool, s->page_table, s->kv_pos, s->x, s->proj, s->y32, s->logits,
                    s->act_hi, s->act_lo, s->tok_cur, s->finished, s->out_len, s->ctl, s->gen_out, s->prompt_dev, s->gen_dump,
-                   s->pf_x, s->pf_proj, s->pf_rb, s->pf_rc, s->pf_hi, s->pf_lo, s->slot_buf, s->xn_hi, s->xn_lo, s->ssq, s->attn_part, s->attn_part_count, s->amax_val, s->amax_idx, s->row_len, s->xlast,
+                   s->pf_x, s->pf_proj, s->pf_rb, s->pf_rc, s->pf_hi, s->pf_lo, s->pf_y, s->slot_buf, s->xn_hi, s->xn_lo, s->ssq, s->attn_part, s->attn_part_count, s->amax_val, s->amax_idx, s->row_len, s->xlast,
                    s->b1_layers, s->b1_grid_ctl, s->b1_amax_val, s->b1_amax_idx, s->b1_timing, s->b1_tagged};
     for (void* p : dev) if (p) cudaFree(p);
     s->dec.x = nullptr;                                   // the session's x, freed above
@@ -2038,7 +2038,7 @@ int32_t grow(T*& p, size_t& cap, size_t need_elems) {
     return LUMI_OK;
 }
 
-bool use_chunked_prefill(const lumi_session* s, int batch, int T) {
+bool use_chunked_scan(const lumi_session* s, int T) {
     if (s->m->cfg.stacked()) return s->opt_chunked_prefill > 0 && T >= 2;       // any element type, windows included: the ring holds a slice more
     if (!(s->opt_chunked_prefill > 0 && T >= s->opt_chunked_prefill && s->m->wdtype == LUMI_DTYPE_BF16 && s->opt_gemm != 1 &&
           prefill_ssd_supported(s->m->cfg) && (s->m->cfg.d_model % 64) == 0 && (s->m->cfg.d_inner() % 64) == 0))
@@ -2052,10 +2052,28 @@ bool use_chunked_prefill(const lumi_session* s, int batch, int T) {
     return true;
 }
 
+// Prompts a layer at a time with the recurrence in token order: what the chunked scan does not take (fp32 weights, prompts under its
+// minimum, head shapes other than its own).  The weights are read once per pass instead of once per token.  Where the line lies, on
+// the 48-layer base model (pass against decode steps): bf16, one sequence, 3 tokens about 2.2 against 1.84 ms, 4 tokens 2.22 against
+// 2.47, 32 tokens 2.85 against 19.5; fp32, one sequence, 6 tokens 3.66 against 3.26 ms, 8 tokens 3.57 against 4.32, 32 tokens 3.72
+// against 16.7; four sequences of 4 tokens 3.18 against 4.99.  fp32 passes cost their K splits and tiles of 32 rows however few the rows are.
+bool use_rows_prefill(const lumi_session* s, int batch, int T) {
+    const Config& c = s->m->cfg;
+    if (c.stacked() || s->opt_chunked_prefill <= 0 || T < 4 || s->m->n_mamba == 0 || !ssm_rows_supported(c.head_dim(), c.d_state)) return false;
+    if (s->m->wdtype == LUMI_DTYPE_F32 && T < 8 && (long)batch * T < 12) return false;
+    if (s->m->wdtype == LUMI_DTYPE_F32) return s->m->n_attn == 0 && row_gemm_supported(c.d_model) && row_gemm_supported(c.d_inner());
+    if (s->opt_gemm == 1 || !use_tc(s, 9)) return false;
+    for (const Layer& L : s->m->layers) if (L.is_attn && L.window > 0) return false;       // as for the chunked scan below
+    return true;
+}
+
 // Head over a slice's rows, a block of rows at a time, then the log-probability of each row's target (shared by the slice loops).
 int score_block_rows(int V) {
     return (int)std::min<size_t>(4096, std::max<size_t>(128, ((size_t)256 << 20) / ((size_t)V * sizeof(float)) / 128 * 128));
 }
+
+// Prompts that prefill_chunked takes, in either form.
+bool use_chunked_prefill(const lumi_session* s, int batch, int T) { return use_chunked_scan(s, T) || use_rows_prefill(s, batch, T); }
 
 // The slice loop for designs that list their layers: slices of up to slice_max tokens per sequence, each through every layer
 // with the caches and states carried from slice to slice.  Arguments as for prefill_chunked.
@@ -2169,7 +2187,7 @@ int32_t prefill_chunked(lumi_session* s, int batch, int T, bool with_head, float
     const Config& c = s->m->cfg;
     if (c.stacked()) return prefill_listed(s, batch, T, with_head, score_out, lens, slot0, want, want_out);
     const int D = c.d_model, DI = c.d_inner(), R = c.in_proj_out();
-    const bool hybrid = s->m->n_attn > 0;
+    const bool hybrid = s->m->n_attn > 0, f32 = s->m->wdtype == LUMI_DTYPE_F32, scan = use_chunked_scan(s, T);
     const int KVD = hybrid ? c.kv_dim() : 0, Q = D + 2 * KVD, MLP = hybrid ? c.mlp_dim() : 0;
     const size_t wproj = std::max<size_t>({(size_t)R, (size_t)Q, (size_t)2 * MLP});       // widest fp32 row of a projection
     const size_t wact = std::max<size_t>({(size_t)DI, (size_t)D, (size_t)MLP});           // widest bf16 operand row
@@ -2178,25 +2196,48 @@ int32_t prefill_chunked(lumi_session* s, int batch, int T, bool with_head, float
     if (TS > T) TS = T;
     const size_t rows_max = (size_t)nb_max * TS;
     if (rows_max > s->pf_rows) {
-        void* olds[] = {s->pf_x, s->pf_proj, s->pf_rb, s->pf_rc, s->pf_hi, s->pf_lo};
+        void* olds[] = {s->pf_x, s->pf_proj, s->pf_rb, s->pf_rc, s->pf_hi, s->pf_lo, s->pf_y};
         for (void* q : olds) if (q) LUMI_CUDA(cudaFree(q));
-        s->pf_x = s->pf_proj = s->pf_rb = s->pf_rc = nullptr; s->pf_hi = s->pf_lo = nullptr; s->pf_rows = 0;
+        s->pf_x = s->pf_proj = s->pf_rb = s->pf_rc = s->pf_y = nullptr; s->pf_hi = s->pf_lo = nullptr; s->pf_rows = 0;
         const size_t rp = (rows_max + 127) / 128 * 128;
         LUMI_CUDA(cudaMalloc(&s->pf_x, sizeof(float) * rp * D));
         LUMI_CUDA(cudaMalloc(&s->pf_proj, sizeof(float) * rp * wproj));
         LUMI_CUDA(cudaMalloc(&s->pf_rb, sizeof(float) * rp));
         LUMI_CUDA(cudaMalloc(&s->pf_rc, sizeof(float) * rp));
-        LUMI_CUDA(cudaMalloc(&s->pf_hi, sizeof(__nv_bfloat16) * rp * wact));
-        LUMI_CUDA(cudaMalloc(&s->pf_lo, sizeof(__nv_bfloat16) * rp * wact));
+        if (f32) {
+            LUMI_CUDA(cudaMalloc(&s->pf_y, sizeof(float) * rp * wact));
+        } else {
+            LUMI_CUDA(cudaMalloc(&s->pf_hi, sizeof(__nv_bfloat16) * rp * wact));
+            LUMI_CUDA(cudaMalloc(&s->pf_lo, sizeof(__nv_bfloat16) * rp * wact));
+        }
         // rows that a launch skips (padding behind a shorter prompt) keep what they held: make that finite from the start
         LUMI_CUDA(cudaMemsetAsync(s->pf_x, 0, sizeof(float) * rp * D, s->stream));
         LUMI_CUDA(cudaMemsetAsync(s->pf_proj, 0, sizeof(float) * rp * wproj, s->stream));
-        LUMI_CUDA(cudaMemsetAsync(s->pf_hi, 0, sizeof(__nv_bfloat16) * rp * wact, s->stream));
-        LUMI_CUDA(cudaMemsetAsync(s->pf_lo, 0, sizeof(__nv_bfloat16) * rp * wact, s->stream));
+        if (f32) {
+            LUMI_CUDA(cudaMemsetAsync(s->pf_y, 0, sizeof(float) * rp * wact, s->stream));
+        } else {
+            LUMI_CUDA(cudaMemsetAsync(s->pf_hi, 0, sizeof(__nv_bfloat16) * rp * wact, s->stream));
+            LUMI_CUDA(cudaMemsetAsync(s->pf_lo, 0, sizeof(__nv_bfloat16) * rp * wact, s->stream));
+        }
         s->pf_rows = rows_max;
     }
     const size_t B = s->max_batch;
     __nv_bfloat16* lo = s->opt_split ? s->pf_lo : nullptr;
+    // bf16 models: a product of rows given as halves.  Few rows of short prompts split K over CTAs, which needs the session's counters;
+    // the chunked scan's products add in one order whatever the rows, so that a sequence gets the same angles alone and among others
+    auto product_tc = [&](const __nv_bfloat16* hi, const __nv_bfloat16* lo_, int K, const DevTensor& W, float* out, int rows, int N, int accumulate) {
+        GemmArgs g{hi, lo_, (const __nv_bfloat16*)W.p, out, N, rows, N, K, accumulate, &s->ctl->status, scan ? nullptr : s->gemm_counters, kGemmCounters,
+                   s->gemm_scratch, kGemmScratchFloats};
+        return launch_gemm_tcgen05(g, s->stream);
+    };
+    // fp32 models: the norm of `rows` rows of x into pf_y, and products of rows with fp32 weights
+    auto norm_rows = [&](const float* x, const float* gamma, int rows) {
+        return launch_row_norm(RowNormArgs{const_cast<float*>(x), nullptr, gamma, s->pf_y, nullptr, nullptr, nullptr, rows, D, D, c.eps, nullptr}, s->stream);
+    };
+    auto product_f32 = [&](const float* in, int K, const DevTensor& W, float* out, int rows, int N, int accumulate) {
+        return launch_row_gemm(RowGemmArgs{in, K, (const float*)W.p, out, N, rows, N, K, accumulate, s->gemm_counters, kGemmCounters, s->gemm_scratch,
+                                           2 * kGemmScratchFloats}, s->stream);
+    };
     for (int b0 = 0; b0 < batch; b0 += nb_max) {
         const int nb = std::min(nb_max, batch - b0);
         for (int t0 = 0; t0 < T; t0 += TS) {
@@ -2211,8 +2252,7 @@ int32_t prefill_chunked(lumi_session* s, int batch, int T, bool with_head, float
                     // AttentionBlock over all rows of the slice (model.rs:562-611 in forward_window's terms): q|k|v for every
                     // row, the slice's K/V appended to the cache, then every row attends to the cache up to its own position
                     LUMI_CUDA(launch_norm_split(s->pf_x, L.a.attn_norm_g, s->pf_hi, lo, M, D, c.eps, s->stream));
-                    GemmArgs gq{s->pf_hi, lo, (const __nv_bfloat16*)L.a.qkv.p, s->pf_proj, Q, M, Q, D, 0, &s->ctl->status};
-                    LUMI_TRY(launch_gemm_tcgen05(gq, s->stream));
+                    LUMI_TRY(product_tc(s->pf_hi, lo, D, L.a.qkv, s->pf_proj, M, Q, 0));
                     AttnArgs a{};
                     a.qkv = s->pf_proj; a.ldq = Q;
                     a.pool = (char*)s->kv_pool + l * s->kv_layer_bytes;
@@ -2233,21 +2273,22 @@ int32_t prefill_chunked(lumi_session* s, int batch, int T, bool with_head, float
                         if (e == cudaErrorInvalidValue) return fail(LUMI_E_UNSUPPORTED, "attention head_dim %d with %d query heads per kv head is not built", a.head_dim, a.n_heads / a.kv_heads);
                         LUMI_CUDA(e);
                     }
-                    GemmArgs go{s->pf_hi, lo, (const __nv_bfloat16*)L.a.o.p, s->pf_x, D, M, D, D, 1, &s->ctl->status};
-                    LUMI_TRY(launch_gemm_tcgen05(go, s->stream));
+                    LUMI_TRY(product_tc(s->pf_hi, lo, D, L.a.o, s->pf_x, M, D, 1));
                     // sigmoid-gated MLP (model.rs:546-555)
                     LUMI_CUDA(launch_norm_split(s->pf_x, L.a.mlp_norm_g, s->pf_hi, lo, M, D, c.eps, s->stream));
-                    GemmArgs gu{s->pf_hi, lo, (const __nv_bfloat16*)L.a.gate_up.p, s->pf_proj, 2 * MLP, M, 2 * MLP, D, 0, &s->ctl->status};
-                    LUMI_TRY(launch_gemm_tcgen05(gu, s->stream));
+                    LUMI_TRY(product_tc(s->pf_hi, lo, D, L.a.gate_up, s->pf_proj, M, 2 * MLP, 0));
                     LUMI_CUDA(launch_gate_mul(s->pf_proj, 2 * MLP, nullptr, s->pf_hi, lo, M, MLP, s->stream));
-                    GemmArgs gd{s->pf_hi, lo, (const __nv_bfloat16*)L.a.down.p, s->pf_x, D, M, D, MLP, 1, &s->ctl->status};
-                    LUMI_TRY(launch_gemm_tcgen05(gd, s->stream));
+                    LUMI_TRY(product_tc(s->pf_hi, lo, MLP, L.a.down, s->pf_x, M, D, 1));
                     s->launches += 10;
                     continue;
                 }
-                LUMI_CUDA(launch_norm_split(s->pf_x, L.m.norm_g, s->pf_hi, lo, M, D, c.eps, s->stream));
-                GemmArgs g1{s->pf_hi, lo, (const __nv_bfloat16*)L.m.in_proj.p, s->pf_proj, R, M, R, D, 0, &s->ctl->status};
-                LUMI_TRY(launch_gemm_tcgen05(g1, s->stream));
+                if (f32) {
+                    LUMI_CUDA(norm_rows(s->pf_x, L.m.norm_g, M));
+                    LUMI_CUDA(product_f32(s->pf_y, D, L.m.in_proj, s->pf_proj, M, R, 0));
+                } else {
+                    LUMI_CUDA(launch_norm_split(s->pf_x, L.m.norm_g, s->pf_hi, lo, M, D, c.eps, s->stream));
+                    LUMI_TRY(product_tc(s->pf_hi, lo, D, L.m.in_proj, s->pf_proj, M, R, 0));
+                }
                 PrefillArgs a{};
                 a.proj = s->pf_proj; a.ldp = R;
                 a.bg = L.m.b_gamma; a.cg = L.m.c_gamma; a.bb = L.m.b_bias; a.cb = L.m.c_bias; a.dskip = L.m.d_skip; a.dtb = L.m.dt_bias;
@@ -2260,9 +2301,13 @@ int32_t prefill_chunked(lumi_session* s, int batch, int T, bool with_head, float
                 a.H = c.n_heads; a.G = c.n_groups; a.ts = ts; a.nb = nb; a.b0 = b0; a.eps = c.eps;
                 a.status = &s->ctl->status;
                 a.lens = lens; a.t_abs0 = t0;
-                LUMI_CUDA(launch_prefill_scan(a, s->stream));
-                GemmArgs g2{s->pf_hi, lo, (const __nv_bfloat16*)L.m.out_proj.p, s->pf_x, D, M, D, DI, 1, &s->ctl->status};
-                LUMI_TRY(launch_gemm_tcgen05(g2, s->stream));
+                if (scan) LUMI_CUDA(launch_prefill_scan(a, s->stream));
+                else LUMI_CUDA(launch_ssm_rows(a, c.head_dim(), c.d_state, s->pf_y, s->stream));
+                if (f32) {
+                    LUMI_CUDA(product_f32(s->pf_y, DI, L.m.out_proj, s->pf_x, M, D, 1));
+                } else {
+                    LUMI_TRY(product_tc(s->pf_hi, lo, DI, L.m.out_proj, s->pf_x, M, D, 1));
+                }
                 s->launches += 5;
             }
             if (hybrid) {
@@ -2274,12 +2319,12 @@ int32_t prefill_chunked(lumi_session* s, int batch, int T, bool with_head, float
                 const int V = c.vocab;
                 const int SR = score_block_rows(V);
                 LUMI_TRY(grow(s->score_logits, s->score_logits_cap, (size_t)SR * V));
-                LUMI_CUDA(launch_norm_split(s->pf_x, s->m->final_norm_g, s->pf_hi, lo, M, D, c.eps, s->stream));
+                if (f32) LUMI_CUDA(norm_rows(s->pf_x, s->m->final_norm_g, M));
+                else LUMI_CUDA(launch_norm_split(s->pf_x, s->m->final_norm_g, s->pf_hi, lo, M, D, c.eps, s->stream));
                 for (int r0 = 0; r0 < M; r0 += SR) {
                     const int nr = std::min(SR, M - r0);
-                    GemmArgs gh{s->pf_hi + (size_t)r0 * D, lo ? lo + (size_t)r0 * D : nullptr, (const __nv_bfloat16*)s->m->embedding.p,
-                                s->score_logits, V, nr, V, D, 0, &s->ctl->status};
-                    LUMI_TRY(launch_gemm_tcgen05(gh, s->stream));
+                    if (f32) LUMI_CUDA(product_f32(s->pf_y + (size_t)r0 * D, D, s->m->embedding, s->score_logits, nr, V, 0));
+                    else LUMI_TRY(product_tc(s->pf_hi + (size_t)r0 * D, lo ? lo + (size_t)r0 * D : nullptr, D, s->m->embedding, s->score_logits, nr, V, 0));
                     LUMI_CUDA(launch_logprob_rows(s->score_logits, nr, V, s->prompt_dev, batch, T, ts, t0, b0, r0, score_out, s->stream));
                     s->launches += 2;
                 }
@@ -2292,9 +2337,9 @@ int32_t prefill_chunked(lumi_session* s, int batch, int T, bool with_head, float
         }
     }
     if (with_head) {
-        StepPlan p{s, batch, true};
+        StepPlan p{s, batch, !f32};
         p.st_hi = p.st_lo = s->stream;
-        LUMI_CUDA(launch_norm_split(s->x, s->m->final_norm_g, s->act_hi, s->opt_split ? s->act_lo : nullptr, batch, D, c.eps, s->stream));
+        if (!f32) LUMI_CUDA(launch_norm_split(s->x, s->m->final_norm_g, s->act_hi, s->opt_split ? s->act_lo : nullptr, batch, D, c.eps, s->stream));
         p.fam = FAM_HEAD;
         LUMI_TRY(linear(p, s->m->embedding, s->x, D, s->logits, c.vocab, nullptr, s->m->final_norm_g, 0, c.vocab));
         LUMI_CUDA(launch_sample(s->logits, batch, c.vocab, s->ctl, s->tok_cur, s->finished, s->out_len, s->stream));

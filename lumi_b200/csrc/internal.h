@@ -293,6 +293,7 @@ struct lumi_session {
     // chunked-prefill workspace (grow-only): residual rows, in_proj output, bf16 halves, BCNorm scales
     float *pf_x = nullptr, *pf_proj = nullptr, *pf_rb = nullptr, *pf_rc = nullptr;
     __nv_bfloat16 *pf_hi = nullptr, *pf_lo = nullptr;
+    float* pf_y = nullptr;            // fp32 models: normalised rows, then the state's read-outs
     size_t pf_rows = 0;
     // options
     int opt_gemm = 0, opt_split = 1, opt_graph = 1, opt_pdl = 1, opt_mega = 0;
@@ -592,6 +593,24 @@ cudaError_t launch_prefill_embed(const void* emb, int dtype, const uint32_t* pro
                                  int t_abs0, int b_abs0, int batch_total, StepCtl* ctl, cudaStream_t st, const int32_t* lens = nullptr,
                                  const EmbedPost& post = EmbedPost());
 cudaError_t launch_prefill_scan(const PrefillArgs& a, cudaStream_t st);
+cudaError_t launch_bc_stats(const PrefillArgs& a, int P, int N, cudaStream_t st);      // fills a.rb / a.rc
+// The recurrence in token order over the same rows, in the decode step's arithmetic (prefill_rows.cu): any element type and
+// prompt length.  y32 (may be null): [nb * ts][heads * P] fp32 beside or in place of yhi / ylo.
+bool ssm_rows_supported(int P, int N);
+cudaError_t launch_ssm_rows(const PrefillArgs& a, int P, int N, float* y32, cudaStream_t st);
+// D[M][N] (+)= A[M][K] W[N][K]^T in fp32 on the CUDA cores, for many rows (prefill_rows.cu).  K % 16 == 0, lda % 4 == 0.  counters (zeroed
+// ints, left zeroed) and scratch serve the split of K.
+struct RowGemmArgs {
+    const float* A; int lda;
+    const float* W;
+    float* D; int ldd;
+    int M, N, K;
+    int accumulate;
+    int32_t* counters; int n_counters;
+    float* scratch; size_t scratch_floats;
+};
+bool row_gemm_supported(int K);
+cudaError_t launch_row_gemm(const RowGemmArgs& g, cudaStream_t st);
 cudaError_t launch_gather_last(const float* xr, float* x, int D, int ts, int nb, int b0, cudaStream_t st, const int32_t* lens = nullptr, int t_abs0 = 0);
 
 // ---- listed layers: norm of a sublayer's output into the residual stream (sublayer.cu) --------------------

@@ -665,6 +665,12 @@ cudaError_t launch_prefill_embed(const void* emb, int dtype, const uint32_t* pro
     return cudaGetLastError();
 }
 
+cudaError_t launch_bc_stats(const PrefillArgs& a, int P, int N, cudaStream_t st) {
+    const int rows = a.nb * a.ts;
+    bc_stats_kernel<<<(rows + 7) / 8, 256, 0, st>>>(a.proj, a.ldp, 2 * a.H * P, a.G * N, a.eps, a.rb, a.rc, rows);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_prefill_scan(const PrefillArgs& a, cudaStream_t st) {
     const size_t smem = sizeof(PfSmem) + 1024;
     static bool set = false;
@@ -679,8 +685,7 @@ cudaError_t launch_prefill_scan(const PrefillArgs& a, cudaStream_t st) {
     if (make_f32_map_2d(&m32, a.proj, (uint64_t)rows, (uint64_t)a.ldp, (uint64_t)a.ldp * 4, 32, LCH) != LUMI_OK ||
         make_f32_map_2d(&m64, a.proj, (uint64_t)rows, (uint64_t)a.ldp, (uint64_t)a.ldp * 4, 64, LCH) != LUMI_OK)
         return cudaErrorInvalidValue;
-    bc_stats_kernel<<<(rows * 32 + 255) / 256, 256, 0, st>>>(a.proj, a.ldp, 2 * a.H * 32, a.G * 64, a.eps, a.rb, a.rc, rows);
-    cudaError_t e = cudaGetLastError();
+    cudaError_t e = launch_bc_stats(a, 32, 64, st);
     if (e != cudaSuccess) return e;
     ssd_prefill_kernel<<<dim3(a.H, a.nb), 128, smem, st>>>(m32, m64, a);
     return cudaGetLastError();

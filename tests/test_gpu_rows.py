@@ -1,0 +1,89 @@
+"""Prompts taken a layer at a time with the recurrence in token order (fp32 weights, short prompts, other head shapes) against
+the same prompt token by token, and against the oracle."""
+import numpy as np
+import pytest
+
+import lumi_b200
+from lumi_b200 import synth
+from oracle import cpu_oracle
+
+pytestmark = pytest.mark.gpu
+
+
+def rel(a, b):
+    return float(np.abs(a - b).max() / np.abs(b).max())
+
+
+def pair(cfg, dtype, batch, seed=3):
+    tens = list(synth.iter_tensors(cfg, seed=seed, weights_dtype=dtype, perturb_ones=0.1))
+    model = lumi_b200.NmModel.from_tensors(cfg, tens)
+    rows, steps = model.init_states(batch, 256), model.init_states(batch, 256)
+    steps.set_option("chunked_prefill", 0)
+    return tens, model, rows, steps
+
+
+def same_state(rows, steps, b, layer, tol):
+    for x, y, what in zip(rows.read_state(b, layer), steps.read_state(b, layer), ("h", "x_prev", "b_prev", "angle")):
+        if what == "angle":
+            x = y + np.mod(x - y + np.pi, 2 * np.pi) - np.pi
+        assert np.abs(x - y).max() <= tol * max(1.0, np.abs(y).max()), (b, layer, what)
+
+
+# Sums of at most 512 products in two orders: 512 * 2^-24 = 3e-5 of the sum of magnitudes at the very worst, a tenth of it in practice;
+# bf16 models add the products' bf16 halves (2^-17 per factor) on one side only, because few rows take fp32 activations.
+TOL = {"f32": 3e-5, "bf16": 2e-4}
+
+
+# tokens around the sixteen that are taken at a time, rows around the tiles of 32 and 64, K split and not
+@pytest.mark.parametrize("dtype", ["f32", "bf16"])
+@pytest.mark.parametrize("batch,T", [(1, 4), (1, 15), (1, 16), (1, 17), (1, 33), (2, 32), (3, 22), (5, 65), (13, 5), (20, 33)])
+def test_rows_equal_steps(dtype, batch, T):
+    cfg = synth.tiny_config(n_layers=3)
+    tens, _, rows, steps = pair(cfg, dtype, batch)
+    prompts = synth.random_prompts(batch, T, cfg.vocab_size, seed=T)
+    assert rel(rows.prefill(prompts), steps.prefill(prompts)) < TOL[dtype]
+    for layer in range(cfg.n_layers):
+        same_state(rows, steps, batch - 1, layer, 10 * TOL[dtype])
+    # a second prompt behind the first starts from the handed-over state, and the oracle agrees with both
+    more = synth.random_prompts(batch, 5, cfg.vocab_size, seed=T + 1)
+    a, b = rows.prefill(more), steps.prefill(more)
+    assert rel(a, b) < TOL[dtype]
+    st = cpu_oracle.OracleModel(cfg, tens).init_states()
+    for tok in np.concatenate([prompts[-1], more[-1]]):
+        ref = st.forward_step(int(tok))
+    assert rel(a[-1], ref) < TOL[dtype]
+
+
+@pytest.mark.parametrize("heads,d_state", [(8, 32), (8, 64), (8, 128), (16, 32), (16, 64), (16, 128), (4, 16), (4, 32), (4, 64), (4, 128), (16, 16)])
+def test_rows_of_every_head_shape(heads, d_state):
+    """Head widths 64, 32 and 16 (16 x 16 is the one that stays with the steps)."""
+    cfg = synth.tiny_config(n_layers=2, n_heads=heads, d_state=d_state)
+    _, _, rows, steps = pair(cfg, "f32", 3)
+    prompts = synth.random_prompts(3, 37, cfg.vocab_size, seed=heads + d_state)
+    assert rel(rows.prefill(prompts), steps.prefill(prompts)) < TOL["f32"]
+    for layer in range(2):
+        same_state(rows, steps, 1, layer, 10 * TOL["f32"])
+
+
+@pytest.mark.parametrize("dtype", ["f32", "bf16"])
+def test_rows_of_different_lengths_and_scores(dtype):
+    cfg = synth.tiny_config(n_layers=3)
+    _, _, rows, steps = pair(cfg, dtype, 4)
+    prompts = synth.random_prompts(4, 40, cfg.vocab_size, seed=8)
+    lengths = np.array([40, 1, 16, 33], dtype=np.int32)
+    assert rel(rows.prefill_ragged(prompts, lengths), steps.prefill_ragged(prompts, lengths)) < TOL[dtype]
+    for b in range(4):
+        same_state(rows, steps, b, 1, 10 * TOL[dtype])
+    rows.reset(), steps.reset()
+    a, b = rows.score(prompts), steps.score(prompts)
+    assert np.abs(a - b).max() < 10 * TOL[dtype] * np.abs(b).max()
+    assert np.array_equal(rows.forward_step(prompts[:, 0])[1], steps.forward_step(prompts[:, 0])[1])
+
+
+@pytest.mark.parametrize("T", [5, 30])
+def test_short_prompts_with_attention_layers(T):
+    cfg = synth.tiny_config(attention_interval=2, attn_rope_base=10000.0)
+    _, _, rows, steps = pair(cfg, "bf16", 2)
+    prompts = synth.random_prompts(2, T, cfg.vocab_size, seed=T)
+    assert rel(rows.prefill(prompts), steps.prefill(prompts)) < 2e-3          # the two sides round their keys and values to bf16 on their own
+    assert rel(rows.forward_step(prompts[:, 0])[0], steps.forward_step(prompts[:, 0])[0]) < 2e-3
