@@ -241,16 +241,16 @@ int32_t lumi_k_gemm_bf16_tcgen05(uint64_t a_hi, uint64_t a_lo, uint64_t w, uint6
 
 /* Failure-path test hook for the bounded device-side waits (no counterpart in the reference, whose kernels never wait
  * on one another): runs the same GEMM with activations a_hi only, every device-side wait limited to wait_limit_ns, and
- * the producer stopping before work unit `skip_unit` (units are 128-row x tile-width output tiles in launch order;
- * -1 = none), so that the waits of the consumers run out.  status_word: a zeroed device int32.  Returns LUMI_E_TIMEOUT
+ * the producer stopping before work unit `skip_unit` (units are 128-row x tile-width output tiles in launch order, CTAs
+ * up to 64 rows; -1 = none), so that the waits of the consumers run out.  status_word: a zeroed device int32.  Returns LUMI_E_TIMEOUT
  * when a wait gave up — the kernel has then returned cleanly (copies drained, tensor memory freed) and further calls
  * work — or LUMI_OK when nothing was skipped.  Synchronises the default stream. */
 int32_t lumi_debug_gemm_wait_timeout(uint64_t a_hi, uint64_t w, uint64_t d, int32_t M, int32_t N, int32_t K,
                                      uint64_t wait_limit_ns, int32_t skip_unit, uint64_t status_word);
 
 /* Host-side only (no device is touched, nothing is launched; no counterpart in the reference): the output-tile width and
- * the number of CTAs K is split over that lumi_k_gemm_bf16_tcgen05 and the decode / prefill steps take for a product of
- * this shape.  two_planes: activations as bf16 hi + lo halves; producer: the epilogue also leaves the next RMSNorm's
+ * the number of CTAs K is split over that the persistent kernel of lumi_k_gemm_bf16_tcgen05 and the decode / prefill steps
+ * takes for a product of this shape (products of few rows have a kernel of their own: gemm_few_rows.cu).  two_planes: activations as bf16 hi + lo halves; producer: the epilogue also leaves the next RMSNorm's
  * input (tile widths are then multiples of 32).  For tests of the choice and for reading profiles. */
 int32_t lumi_debug_gemm_plan(int32_t M, int32_t N, int32_t K, int32_t two_planes, int32_t producer, int32_t* width,
                              int32_t* splits);
