@@ -157,18 +157,29 @@ struct PfSmem {
     float rC[LCH][64];                 // raw C (group)    -> C~: same layout
     float rz[LCH][32];                 // raw z            -> gate silu(z)
     uint8_t St[2 * 32 * 128];          // augmented state S^: [plane hi | lo][p = 32 rows][n, 128 bytes]
-    float ell[LCH], eli[LCH], lam[LCH + 4], kap[LCH], wj[LCH], dtp[LCH], rbs[LCH], rcs[LCH];
-    float seg[5][32];                  // angle prefix sums at the boundaries of the four 16-token segments
-    float cum[32];
+    struct Scalars {                   // per token; the next chunk's are prepared under this one
+        float ell[LCH], eli[LCH], lam[LCH], kap[LCH], wj[LCH], dtp[LCH], rbs[LCH], rcs[LCH];
+    } sc[2];
+    float seg[4][32];                  // angle sums of the four 16-token segments
     float gam[4][64];                  // this group's BCNorm weights: b gamma, b bias, c gamma, c bias
     unsigned long long bar;
-    int ok;
 };
 
 // byte offset of bf16 element (row, col) inside a tile whose rows are `pitch` bytes apart and hold 64 bf16 (128 bytes)
 // with the 16-byte chunks XOR-ed by row % 8
 __device__ __forceinline__ int swz(int row, int col, int pitch) {
     return row * pitch + ((((col >> 3) ^ (row & 7)) << 4) | ((col & 7) << 1));
+}
+
+// fmodf(x, y) for y > 0 in a few instructions: the remainder of the nearest smaller multiple is exact in one fused multiply-add, and a
+// quotient that rounding carried over a multiple is put back and the multiply-add repeated.
+__device__ __forceinline__ float fmod_near(float x, float y, float inv_y) {
+    if (!(fabsf(x) < 1e6f)) return fmodf(x, y);
+    const float q = truncf(x * inv_y);
+    float r = fmaf(-q, y, x);
+    if (r != 0.f && (r < 0.f) != (x < 0.f)) r = fmaf(-(q - copysignf(1.f, x)), y, x);
+    else if (fabsf(r) >= y) r = fmaf(-(q + copysignf(1.f, x)), y, x);
+    return r;
 }
 
 constexpr uint32_t kChunkTxBytes = 3 * LCH * 32 * 4 + 2 * LCH * 64 * 4;
@@ -245,7 +256,6 @@ ssd_prefill_kernel(const __grid_constant__ CUtensorMap map32, const __grid_const
     if (ts == 0) return;
     const int grp = h / (H / a.G);
     const size_t bh = (size_t)(a.b0 + b) * H + h;
-    const float* prow0 = a.proj + (size_t)b * tsl * R;     // first token row of this sequence
     const int off_b = 2 * DI, off_c = off_b + BC, off_dt = off_c + BC;
     const float PI_F = 3.14159265358979323846f;
     const float TWO_PI = 6.28318530717958647692f;
@@ -260,7 +270,7 @@ ssd_prefill_kernel(const __grid_constant__ CUtensorMap map32, const __grid_const
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(bar)));
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (tid < HN) sm.cum[tid] = a.cum[bh * HN + tid];
+    float cum = a.cum[bh * HN + lane];                     // running angle of pair `lane`, kept by every warp
     if (tid < 64) {
         const int c = grp * N + tid;
         sm.gam[0][tid] = a.bg[c]; sm.gam[1][tid] = a.bb[c]; sm.gam[2][tid] = a.cg[c]; sm.gam[3][tid] = a.cb[c];
@@ -280,21 +290,57 @@ ssd_prefill_kernel(const __grid_constant__ CUtensorMap map32, const __grid_const
     uint8_t* const tC = reinterpret_cast<uint8_t*>(&sm.rC[0][0]);     // C~ tile (in place)
     uint8_t* const tX = reinterpret_cast<uint8_t*>(&sm.rx[0][0]);     // X^T tile (in place): pitch 128, lo plane at +4096
     uint8_t* const tS = sm.St;                                        // S^ tile: pitch 128, lo plane at +4096
-    // per-token scalars of a chunk, requested into registers one chunk ahead (threads 0..63: own token; thread 64:
-    // lambda of the token after the chunk)
-    float n_dt = 0.f, n_lam = 0.f, n_a = 0.f, n_rb = 0.f, n_rc = 0.f;
-    auto request_scalars = [&](int t0) {
-        if (tid < LCH && t0 + tid < ts) {
-            const float* pr = prow0 + (size_t)(t0 + tid) * R;
-            const size_t row = (size_t)b * tsl + t0 + tid;
-            n_dt = pr[off_dt + h]; n_lam = pr[off_dt + H + h]; n_a = pr[off_dt + 2 * H + h];
-            n_rb = a.rb[row]; n_rc = a.rc[row];
-        } else if (tid == LCH && t0 + LCH < ts) {
-            n_lam = prow0[(size_t)(t0 + LCH) * R + off_dt + H + h];
+    // Per-token scalars of a chunk (model.rs:307, 314-317), by warp 0 alone: lane l takes tokens 2 l and 2 l + 1, the last lane also lambda
+    // of the token behind the chunk.  Done for the next chunk while the other warps, which have more of the causal products, are still at theirs.
+    auto prepare_scalars = [&](int t0, PfSmem::Scalars& q) {
+        const int nv = min(LCH, ts - t0);
+        float n_dt[2] = {0.f, 0.f}, n_lam[2] = {0.f, 0.f}, n_a[2] = {0.f, 0.f}, n_rb[2] = {0.f, 0.f}, n_rc[2] = {0.f, 0.f}, n_after = 0.f;
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+            if (2 * lane + e < nv) {
+                const size_t row = (size_t)b * tsl + t0 + 2 * lane + e;
+                const float* pr = a.proj + row * R + off_dt + h;
+                n_dt[e] = pr[0]; n_lam[e] = pr[H]; n_a[e] = pr[2 * H];
+                n_rb[e] = a.rb[row]; n_rc[e] = a.rc[row];
+            }
+        if (lane == 31 && t0 + LCH < ts) n_after = a.proj[((size_t)b * tsl + t0 + LCH) * R + off_dt + H + h];
+        float dtpv[2] = {0.f, 0.f}, gl[2] = {0.f, 0.f}, lm[2] = {0.f, 0.f};
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+            if (2 * lane + e < nv) {
+                dtpv[e] = softplus_ref(__fadd_rn(n_dt[e], dtb));
+                float av = -softplus_ref(n_a[e]);
+                av = fminf(fmaxf(av, -1e6f), -1e-4f);
+                gl[e] = __fmul_rn(av, dtpv[e]);           // log a_t
+                lm[e] = sigmoid_ref(n_lam[e]);
+            }
+        const float after = t0 + LCH < ts ? sigmoid_ref(n_after) : -1.0f;      // < 0: no next token in this launch
+        const float sum = gl[0] + gl[1];                   // inclusive prefix of log a over the chunk
+        float incl = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) { const float n = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= o) incl += n; }
+        const float excl = incl - sum;
+        const float l[2] = {excl + gl[0], excl + sum};
+        const float tot = __shfl_sync(0xffffffffu, l[1], 31), down = __shfl_down_sync(0xffffffffu, lm[0], 1);
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const int i = 2 * lane + e;
+            float k = 0.f;
+            if (i < nv) {
+                // lambda of the next token: this lane's second one, the next lane's first, or the one behind the chunk
+                float ln = -1.0f;
+                if (i + 1 < nv) ln = e == 0 ? lm[1] : down;
+                else if (nv == LCH) ln = after;                  // lane 31's last token only
+                k = ln < 0.f ? lm[e] : __fadd_rn(lm[e], __fsub_rn(1.0f, ln));
+            }
+            q.dtp[i] = dtpv[e]; q.ell[i] = l[e]; q.lam[i] = lm[e]; q.rbs[i] = n_rb[e]; q.rcs[i] = n_rc[e];
+            q.kap[i] = k;
+            q.wj[i] = __expf(tot - l[e]) * k;
+            q.eli[i] = __expf(l[e]);
         }
     };
     if (tid == 0) issue_chunk(0);
-    request_scalars(0);
+    if (warp == 0) prepare_scalars(0, sm.sc[0]);
 
     // state S^ of this warp: rows p0 + {g4, g4 + 8}, columns n0 + 8 nt + 2 t4 + {0, 1}
     const int p0 = 16 * (warp & 1), n0 = 32 * (warp >> 1);
@@ -308,6 +354,8 @@ ssd_prefill_kernel(const __grid_constant__ CUtensorMap map32, const __grid_const
             S[nt][0] = v0.x; S[nt][1] = v0.y; S[nt][2] = v1.x; S[nt][3] = v1.y;
         }
     }
+
+    __syncthreads();                                       // the first chunk's scalars are there
 
     // this warp's block of S^ as bf16 hi + lo into the shared tile (B operand of C~ S^T in the next chunk)
     auto store_state_tile = [&]() {
@@ -331,50 +379,13 @@ ssd_prefill_kernel(const __grid_constant__ CUtensorMap map32, const __grid_const
         const int nv = FULL ? LCH : min(LCH, ts - t0);     // valid tokens in this chunk
         auto valid = [&](int i) { return FULL || i < nv; };
         const bool last_chunk = t0 + LCH >= ts;
-        // ---- 0. the chunk's raw rows have landed (one thread waits, bounded; everyone follows its verdict)
-        if (tid == 0) sm.ok = mbar_wait(bar, phase, kScanWaitLimitNs) ? 1 : 0;
-        // ---- 1. per-token scalars (model.rs:307, 314-317) from the registers requested a chunk earlier
-        if (tid < LCH) {
-            float dtpv = 0.f, gl = 0.f, lm = 0.f;
-            if (valid(tid)) {
-                dtpv = softplus_ref(__fadd_rn(n_dt, dtb));
-                float av = -softplus_ref(n_a);
-                av = fminf(fmaxf(av, -1e6f), -1e-4f);
-                gl = __fmul_rn(av, dtpv);                 // log a_t
-                lm = sigmoid_ref(n_lam);
-            }
-            sm.dtp[tid] = dtpv; sm.ell[tid] = gl; sm.lam[tid] = lm;
-            sm.rbs[tid] = n_rb; sm.rcs[tid] = n_rc;
-        }
-        if (tid == LCH) sm.lam[LCH] = (t0 + LCH < ts) ? sigmoid_ref(n_lam) : -1.0f;      // < 0: no next token in this launch
-        __syncthreads();
-        if (!sm.ok) return false;
+        PfSmem::Scalars& sc = sm.sc[chunk & 1];
+        // ---- 0. the chunk's raw rows have landed (every thread waits, bounded; the next barrier makes one verdict of it)
+        const bool landed = mbar_wait(bar, phase, kScanWaitLimitNs);
         phase ^= 1;
-        if (!last_chunk) request_scalars(t0 + LCH);        // the next chunk's scalars travel while this chunk is computed
-        if (tid < 32) {                                    // inclusive prefix of log a over the chunk
-            float v0 = sm.ell[2 * lane], v1 = sm.ell[2 * lane + 1];
-            float s = v0 + v1, incl = s;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) { float n = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= o) incl += n; }
-            const float excl = incl - s;
-            sm.ell[2 * lane] = excl + v0;
-            sm.ell[2 * lane + 1] = excl + s;
-        }
-        __syncthreads();
-        if (tid < LCH) {
-            const int i = tid;
-            float k = 0.f;
-            if (valid(i)) {
-                const float ln = valid(i + 1) && i + 1 < LCH ? sm.lam[i + 1] : ((nv == LCH) ? sm.lam[LCH] : -1.0f);
-                k = (ln < 0.f) ? sm.lam[i] : __fadd_rn(sm.lam[i], __fsub_rn(1.0f, ln));
-            }
-            sm.kap[i] = k;
-            sm.wj[i] = __expf(sm.ell[LCH - 1] - sm.ell[i]) * k;
-            sm.eli[i] = __expf(sm.ell[i]);
-        }
         if (chunk == 0) {
             // S^_in = S + (1 - lam_first) x_prev (x) B~_prev   (prev_bx of the decode state, model.rs:359)
-            const float oml = __fadd_rn(__fmul_rn(sm.lam[0], -1.0f), 1.0f);
+            const float oml = __fadd_rn(__fmul_rn(sc.lam[0], -1.0f), 1.0f);
             const float xp0 = a.xprev[bh * P + p0 + g4] * oml, xp1 = a.xprev[bh * P + p0 + g4 + 8] * oml;
 #pragma unroll
             for (int nt = 0; nt < 4; ++nt) {
@@ -392,11 +403,11 @@ ssd_prefill_kernel(const __grid_constant__ CUtensorMap map32, const __grid_const
             float loc[16], run = 0.f;
 #pragma unroll
             for (int ii = 0; ii < 16; ++ii) {
-                const float d = sm.dtp[i0 + ii] * (tanh_fast(sm.rth[i0 + ii][k]) * PI_F);      // model.rs:341-342; dtp = 0 past the end
+                const float d = sc.dtp[i0 + ii] * (tanh_fast(sm.rth[i0 + ii][k]) * PI_F);      // model.rs:341-342; dtp = 0 past the end
                 run += d;
                 loc[ii] = run;
             }
-            sm.seg[warp + 1][k] = run;
+            sm.seg[warp][k] = run;
             // x -> silu (registers; the tile is written after every warp has read its raw x) ; z -> gate in place
             const int p = lane;
             float xs[16];
@@ -405,15 +416,18 @@ ssd_prefill_kernel(const __grid_constant__ CUtensorMap map32, const __grid_const
                 const int i = i0 + ii;
                 xs[ii] = valid(i) ? silu_fast(sm.rx[i][p]) : 0.f;                              // model.rs:310
                 sm.rz[i][p] = valid(i) ? silu_fast(sm.rz[i][p]) : 0.f;                         // model.rs:370
-                if (last_chunk && i == nv - 1) a.xprev[bh * P + p] = xs[ii];                   // hand-over: x of the launch's last token
             }
-            __syncthreads();
-            if (tid < 32) {
-                float off = sm.cum[tid];
-                sm.seg[0][tid] = off;
-                // reduced mod 2 pi at every segment boundary, so sums stay small and keep their low bits
-                for (int s2 = 1; s2 <= 4; ++s2) { off = fmodf(off + sm.seg[s2][tid], TWO_PI); sm.seg[s2][tid] = off; }
-                sm.cum[tid] = off;                         // angle after the chunk's last valid token
+            if (!__syncthreads_and(landed)) return false;
+            // reduced mod 2 pi at every segment boundary, so sums stay small and keep their low bits
+            float base = cum;
+#pragma unroll
+            for (int s2 = 0; s2 < 4; ++s2) {
+                if (s2 == warp) base = cum;
+                cum = fmod_near(cum + sm.seg[s2][k], TWO_PI, INV_TWO_PI);
+            }
+            if (last_chunk) {                              // hand-over: x of the launch's last token (every warp has read the old one)
+#pragma unroll
+                for (int ii = 0; ii < 16; ++ii) if (i0 + ii == nv - 1) a.xprev[bh * P + p] = xs[ii];
             }
             // X^T tile over the raw x rows: row p, tokens i0 .. i0 + 15 (two per 32-bit word)
 #pragma unroll
@@ -423,8 +437,6 @@ ssd_prefill_kernel(const __grid_constant__ CUtensorMap map32, const __grid_const
                 *reinterpret_cast<uint32_t*>(tX + swz(p, i0 + ii, 128)) = hi;
                 *reinterpret_cast<uint32_t*>(tX + 4096 + swz(p, i0 + ii, 128)) = lo;
             }
-            __syncthreads();
-            const float base = sm.seg[warp][k];
             const float bgm0 = sm.gam[0][2 * k], bgm1 = sm.gam[0][2 * k + 1], bbs0 = sm.gam[1][2 * k], bbs1 = sm.gam[1][2 * k + 1];
             const float cgm0 = sm.gam[2][2 * k], cgm1 = sm.gam[2][2 * k + 1], cbs0 = sm.gam[3][2 * k], cbs1 = sm.gam[3][2 * k + 1];
 #pragma unroll
@@ -443,7 +455,7 @@ ssd_prefill_kernel(const __grid_constant__ CUtensorMap map32, const __grid_const
                     ang -= TWO_PI * rintf(ang * INV_TWO_PI);                 // into [-pi, pi] for the fast sin / cos
                     float b0 = 0.f, b1 = 0.f, c0 = 0.f, c1 = 0.f;
                     if (valid(i)) {
-                        const float rb = sm.rbs[i], rc = sm.rcs[i];
+                        const float rb = sc.rbs[i], rc = sc.rcs[i];
                         const float nb0 = fmaf(rawb[q].x * rb, bgm0, bbs0), nb1 = fmaf(rawb[q].y * rb, bgm1, bbs1);      // model.rs:311-313
                         const float nc0 = fmaf(rawc[q].x * rc, cgm0, cbs0), nc1 = fmaf(rawc[q].y * rc, cgm1, cbs1);
                         float sa, ca;
@@ -500,7 +512,7 @@ ssd_prefill_kernel(const __grid_constant__ CUtensorMap map32, const __grid_const
                 mma3x4(y2[0], y2[1], y2[2], y2[3], Ch[ks], Cl[ks], sh0, sl0, sh1, sl1);
             }
             const int ia = 16 * warp + g4, ib = ia + 8;
-            const float ella = sm.ell[ia], ellb = sm.ell[ib];
+            const float ella = sc.ell[ia], ellb = sc.ell[ib];
             for (int jp = 0; jp <= warp; ++jp) {           // token columns 16 jp .. 16 jp + 15
                 // six independent accumulation chains (hi*hi, hi*lo, lo*hi of the two 8-column tiles), added at the end
                 float g0[4] = {0.f, 0.f, 0.f, 0.f}, g1[4] = {0.f, 0.f, 0.f, 0.f};
@@ -529,8 +541,8 @@ ssd_prefill_kernel(const __grid_constant__ CUtensorMap map32, const __grid_const
                         const int i = (e < 2) ? ia : ib, j = 16 * jp + 8 * q + 2 * t4 + (e & 1);
                         const float gv = q == 0 ? g0[e] : g1[e];
                         float w = 0.f;
-                        if (j < i) w = gv * __expf(((e < 2) ? ella : ellb) - sm.ell[j]) * sm.kap[j];
-                        else if (j == i) w = fmaf(gv, sm.lam[i], dskip);          // lam_i (C~_i . B~_i) x_i + D x_i
+                        if (j < i) w = gv * __expf(((e < 2) ? ella : ellb) - sc.ell[j]) * sc.kap[j];
+                        else if (j == i) w = fmaf(gv, sc.lam[i], dskip);          // lam_i (C~_i . B~_i) x_i + D x_i
                         wv[q][e] = w;
                     }
                 uint32_t wh[4], wl[4];
@@ -549,7 +561,7 @@ ssd_prefill_kernel(const __grid_constant__ CUtensorMap map32, const __grid_const
                 }
             }
             // y = Y1 + e^{l_i} Y2, gated; four lanes of a quad exchange words so that each stores 16 bytes of a row
-            const float ela = sm.eli[ia], elb = sm.eli[ib];
+            const float ela = sc.eli[ia], elb = sc.eli[ib];
             uint32_t oh[2][4], ol[2][4];                   // [row a / b][p tile]
 #pragma unroll
             for (int nt = 0; nt < 4; ++nt) {
@@ -582,10 +594,10 @@ ssd_prefill_kernel(const __grid_constant__ CUtensorMap map32, const __grid_const
                 }
             }
         }
-        __syncthreads();                                   // every warp has read S^_in's tile
+        if (warp == 0 && !last_chunk) prepare_scalars(t0 + LCH, sm.sc[(chunk + 1) & 1]);
         // ---- 4. S^_out = e^{l_last} S^_in + (w x)^T B~  for this warp's 16 x 32 block; new S^ tile for the next chunk
         {
-            const float el = __expf(sm.ell[LCH - 1]);
+            const float el = __expf(sc.ell[LCH - 1]);
 #pragma unroll
             for (int nt = 0; nt < 4; ++nt)
 #pragma unroll
@@ -599,7 +611,7 @@ ssd_prefill_kernel(const __grid_constant__ CUtensorMap map32, const __grid_const
                     const int p = p0 + g4 + 8 * (e & 1), j = 16 * ks + 2 * t4 + 8 * (e >> 1);
                     const float2 xh = unpack2(*reinterpret_cast<const uint32_t*>(tX + swz(p, j, 128)));
                     const float2 xl = unpack2(*reinterpret_cast<const uint32_t*>(tX + 4096 + swz(p, j, 128)));
-                    split2((xh.x + xl.x) * sm.wj[j], (xh.y + xl.y) * sm.wj[j + 1], ah[e], al[e]);
+                    split2((xh.x + xl.x) * sc.wj[j], (xh.y + xl.y) * sc.wj[j + 1], ah[e], al[e]);
                 }
                 {
                     uint32_t bh0[4], bl0[4], bh1[4], bl1[4];   // state columns n0 .. n0 + 15 and n0 + 16 .. n0 + 31
@@ -611,12 +623,14 @@ ssd_prefill_kernel(const __grid_constant__ CUtensorMap map32, const __grid_const
                     mma3x4(S[0], S[1], S[2], S[3], ah, al, bh0, bl0, bh1, bl1);
                 }
             }
-            if (!last_chunk) store_state_tile();
         }
         // every operand tile and raw row of this chunk has been consumed: order these generic-proxy accesses before the copies
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncthreads();
-        if (!last_chunk && tid == 0) issue_chunk(t0 + LCH);
+        if (!last_chunk) {
+            if (tid == 0) issue_chunk(t0 + LCH);
+            store_state_tile();                            // every warp has read S^_in's tile
+        }
         return true;
     };
     bool failed = false;
@@ -631,7 +645,7 @@ ssd_prefill_kernel(const __grid_constant__ CUtensorMap map32, const __grid_const
         // the wait gave up: report, let this CTA's copies land (bounded) so nothing writes into shared memory after exit
         if (tid == 0) {
             if (a.status != nullptr) atomicOr(a.status, STATUS_TIMEOUT);
-            mbar_wait(bar, phase, kScanWaitLimitNs);
+            mbar_wait(bar, phase ^ 1, kScanWaitLimitNs);      // the chunk that did not land: its phase has been turned already
         }
         __syncthreads();
         return;
@@ -645,7 +659,7 @@ ssd_prefill_kernel(const __grid_constant__ CUtensorMap map32, const __grid_const
             *reinterpret_cast<float2*>(hp + (p0 + g4 + 8) * N + n0 + 8 * nt + 2 * t4) = make_float2(S[nt][2], S[nt][3]);
         }
     }
-    if (tid < HN) a.cum[bh * HN + tid] = sm.cum[tid];
+    if (warp == 0) a.cum[bh * HN + lane] = cum;
 }
 
 }  // namespace
