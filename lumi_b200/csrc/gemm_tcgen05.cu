@@ -28,13 +28,15 @@ namespace {
 constexpr int BM = 128;
 constexpr int kSmemBudget = 196608;          // bytes of pipeline stages
 constexpr int kMaxSplits = 4;                // K split over at most this many CTAs
+constexpr int kPairMinRows = 4096;           // from this many rows on: pairs of CTAs
+constexpr int kBlockRows = 4096;             // rows of A that are taken through all columns together
 
 // OCC = CTAs meant to share an SM: with 2, each gets half the stage budget and the epilogue of one
 // tile runs under the main loop of the other.
-template <int BN, bool SPLIT, int OCC>
+template <int BN, bool SPLIT, int OCC, bool PAIR = false>
 struct Tile {
     static constexpr int A_BYTES = BM * BK * 2;                 // 16 KiB
-    static constexpr int B_BYTES = BN * BK * 2;
+    static constexpr int B_BYTES = BN * BK * 2 / (PAIR ? 2 : 1);
     static constexpr int STAGE = A_BYTES * (SPLIT ? 2 : 1) + B_BYTES;
     static constexpr int STAGES = (kSmemBudget / OCC) / STAGE;
     static constexpr int SMEM = STAGES * STAGE + 1024 /* alignment slack */ + 256 /* barriers */;
@@ -253,14 +255,18 @@ __device__ __forceinline__ void ext_strip(const uint32_t (&r)[32], float rs, int
     }
 }
 
-template <int BN, bool SPLIT, bool EXT>
+// PAIR: two CTAs of a cluster (two SMs) work on one tile of 256 rows (cta_group::2).  Each stages its 128 rows of A and half of the weight
+// tile, the first one issues the MMAs for both, each finishes its own rows: 48 KiB of operands per CTA and k-block of a 256-wide tile
+// instead of 64, and half as many bytes of W read from shared memory per MMA.  Operands are copied without multicast.
+template <int BN, bool SPLIT, bool EXT, bool PAIR>
 __global__ void __launch_bounds__(192, 1)
 gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_ahi, const __grid_constant__ CUtensorMap map_alo,
                        const __grid_constant__ CUtensorMap map_w, float* D, int ldd, int M, int N, int K,
                        int accumulate, int tiles_m, int ntiles, int splits, int32_t* tile_counters, float* scratch, int32_t* status,
                        uint64_t wait_ns, int skip_unit, NormFuse nf, GemmExt ex) {
-    using T = Tile<BN, SPLIT, 1>;
+    using T = Tile<BN, SPLIT, 1, PAIR>;
     constexpr int S = T::STAGES;
+    const int rank = PAIR ? (int)(blockIdx.x & 1) : 0, unit0 = PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x, units_at_once = PAIR ? (int)(gridDim.x >> 1) : (int)gridDim.x;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     uint64_t* full_bar = reinterpret_cast<uint64_t*>(base + S * T::STAGE);
@@ -276,22 +282,31 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_ahi, const __grid
     // A successor launched with programmatic dependent launch may become resident now and run the part of its
     // prologue that does not depend on this kernel (the state step requests its state tiles there).
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    if (status != nullptr && (*reinterpret_cast<volatile int32_t*>(status) & STATUS_TIMEOUT)) return;
+    if (status != nullptr && (*reinterpret_cast<volatile int32_t*>(status) & STATUS_TIMEOUT)) {
+        if constexpr (PAIR) ntiles = 0;           // no work, but the cluster's barriers are taken
+        else return;
+    }
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < S; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
-        for (int i = 0; i < 2; ++i) { mbar_init(&tmem_full[i], 1); mbar_init(&tmem_empty[i], 4); }
+        for (int i = 0; i < 2; ++i) { mbar_init(&tmem_full[i], 1); mbar_init(&tmem_empty[i], PAIR ? 8 : 4); }
         mbar_init(drain_bar, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
     constexpr uint32_t ACC_COLS = BN > 128 ? 256u : (BN > 64 ? 128u : 64u);      // TMEM columns per accumulator (allocation is a power of two)
     if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(2u * ACC_COLS) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        if constexpr (PAIR) {
+            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(2u * ACC_COLS) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+        } else {
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(2u * ACC_COLS) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        }
     }
     tc_fence_before();
-    __syncthreads();
+    if constexpr (PAIR) { __syncwarp(); cluster_arrive(); cluster_wait(); }      // the other CTA's barriers exist, its TMEM is allocated
+    else __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(tmem_slot);
     // Launched with programmatic dependent launch (small batches), this CTA may have become resident and done all of the
@@ -304,22 +319,35 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_ahi, const __grid
     // the rows of A behind it
     struct Place { int m0, n0, k0, group, n, m_end; };
     const int tiles_pg = EXT ? (ex.group_rows + BN - 1) / BN : 0;       // column tiles per group
+    // Tiles are numbered by blocks of kBlockRows rows, column by column within a block: a block's rows of A are read from memory once and, with
+    // the weights, stay in L2 for all columns.  By columns alone, 32768 rows of 1024 as two planes, 134 MB, came from memory once per column
+    // tile: 32768 x 7360 x 1024 960 -> 771 us with single CTAs, 894 -> 735 us with pairs.
+    // (splits > 1: one row tile)
+    constexpr int kTileRows = PAIR ? 2 * BM : BM, kBlockTiles = kBlockRows / kTileRows;
+    const int tiles_all = tiles_m > 0 ? ntiles / tiles_m : 0;      // column tiles
+    auto row_tile = [&](int t, int& col) {
+        if (tiles_m <= kBlockTiles) { col = t / tiles_m; return t - col * tiles_m; }
+        const int blk = t / (kBlockTiles * tiles_all), r = t - blk * kBlockTiles * tiles_all, rows = min(kBlockTiles, tiles_m - blk * kBlockTiles);
+        col = r / rows;
+        return blk * kBlockTiles + r - col * rows;
+    };
     auto place = [&](int t) {
         Place p;
         if constexpr (!EXT) {
-            p.m0 = (t % tiles_m) * BM; p.n0 = (t / tiles_m) * BN; p.k0 = 0; p.group = 0; p.n = p.n0; p.m_end = M;
+            int col;
+            p.m0 = row_tile(t, col) * kTileRows + rank * BM; p.n0 = col * BN; p.k0 = 0; p.group = 0; p.n = p.n0; p.m_end = M;
         } else if (ex.tiles != nullptr) {
             const int4 rt = __ldg(ex.tiles + t / tiles_pg);
             p.m0 = rt.x; p.m_end = rt.x + rt.y; p.group = rt.z; p.n = (t % tiles_pg) * BN; p.n0 = p.group * ex.group_rows + p.n; p.k0 = 0;
         } else {
-            const int tn = t / tiles_m;
-            p.m0 = (t % tiles_m) * BM; p.m_end = M; p.group = tn / tiles_pg; p.n = (tn % tiles_pg) * BN; p.n0 = p.group * ex.group_rows + p.n;
+            int tn;
+            p.m0 = row_tile(t, tn) * kTileRows + rank * BM; p.m_end = M; p.group = tn / tiles_pg; p.n = (tn % tiles_pg) * BN; p.n0 = p.group * ex.group_rows + p.n;
             p.k0 = p.group * K;
         }
         return p;
     };
     const bool by_rows = EXT && ex.tiles != nullptr;      // the tiles are known only behind the dependency wait
-    if (!by_rows && warp == 0 && lane == 0 && (int)blockIdx.x < ntiles * splits && (int)blockIdx.x != skip_unit) {
+    if (!PAIR && !by_rows && warp == 0 && lane == 0 && (int)blockIdx.x < ntiles * splits && (int)blockIdx.x != skip_unit) {
         const int t = blockIdx.x / splits, sp = blockIdx.x - t * splits;
         const int n0 = place(t).n0;
         const int kb0 = sp * num_kb / splits, kb1 = (sp + 1) * num_kb / splits;
@@ -336,7 +364,7 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_ahi, const __grid
     if (warp == 0) {
         if (lane == 0) {
             uint32_t kbg = 0;                    // k-blocks issued so far, over all tiles of this CTA
-            for (int u = blockIdx.x; u < ntiles * splits && !timed_out; u += gridDim.x) {
+            for (int u = unit0; u < ntiles * splits && !timed_out; u += units_at_once) {
                 if (u == skip_unit) break;       // test hook: this unit's operands never arrive, so the waits below it run out
                 const int t = u / splits, sp = u - t * splits;
                 const Place pl = place(t);
@@ -347,22 +375,38 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_ahi, const __grid
                     const uint32_t ph = (kbg / S) & 1u;
                     if (!mbar_wait(&empty_bar[s], ph ^ 1u, wait_ns)) { timed_out = true; break; }
                     uint8_t* st = base + s * T::STAGE;
+                    if constexpr (PAIR) {        // both CTAs' copies complete on the first one's barrier
+                        const uint32_t bar = map_to_rank(smem_u32(&full_bar[s]), 0);
+                        if (rank == 0) mbar_expect_tx(&full_bar[s], 2u * (uint32_t)T::STAGE);
+                        tma_load_2d_pair(st, &map_ahi, bar, pl.k0 + kb * BK, m0);
+                        if (SPLIT) tma_load_2d_pair(st + T::A_BYTES, &map_alo, bar, pl.k0 + kb * BK, m0);
+                        tma_load_2d_pair(st + T::A_BYTES * (SPLIT ? 2 : 1), &map_w, bar, kb * BK, n0 + rank * (BN / 2));
+                        continue;
+                    }
                     if (kbg >= pre) mbar_expect_tx(&full_bar[s], (uint32_t)T::STAGE);
                     tma_load_2d(st, &map_ahi, &full_bar[s], pl.k0 + kb * BK, m0);
                     if (SPLIT) tma_load_2d(st + T::A_BYTES, &map_alo, &full_bar[s], pl.k0 + kb * BK, m0);
                     if (kbg >= pre) tma_load_2d(st + T::A_BYTES * (SPLIT ? 2 : 1), &map_w, &full_bar[s], kb * BK, n0);
                 }
             }
-            if (timed_out) {
+            if (timed_out && rank == 0) {
                 // drain: wait (bounded) for the copies this thread issued and nobody may consume
                 for (uint32_t k = kbg > (uint32_t)S ? kbg - S : 0; k < kbg; ++k) mbar_wait(&full_bar[k % S], (k / S) & 1u, wait_ns);
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+        if (lane == 0 && rank == 0) {
+            constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)((PAIR ? 2 * BM : BM) >> 4) << 24);
+            auto mma = [&](uint32_t d, uint64_t da, uint64_t db, uint32_t add) {
+                if constexpr (PAIR) umma_bf16_pair(d, da, db, idesc, add);
+                else umma_bf16(d, da, db, idesc, add);
+            };
+            auto commit = [&](uint64_t* bar) {
+                if constexpr (PAIR) umma_commit_pair(bar);
+                else umma_commit(bar);
+            };
             uint32_t kbg = 0, it = 0;
-            for (int u = blockIdx.x; u < ntiles * splits && !timed_out; u += gridDim.x, ++it) {
+            for (int u = unit0; u < ntiles * splits && !timed_out; u += units_at_once, ++it) {
                 const uint32_t as = it & 1u, aph = (it >> 1) & 1u;
                 if (!mbar_wait(&tmem_empty[as], aph ^ 1u, wait_ns)) { timed_out = true; break; }     // the epilogue has drained this accumulator
                 tc_fence_after();
@@ -378,19 +422,19 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_ahi, const __grid
                     const uint32_t b_addr = a_hi + T::A_BYTES * (SPLIT ? 2 : 1);
 #pragma unroll
                     for (int k = 0; k < BK / 16; ++k)
-                        umma_bf16(acc, make_smem_desc(a_hi + k * 32), make_smem_desc(b_addr + k * 32), idesc, (kb > kb0 || k > 0) ? 1u : 0u);
+                        mma(acc, make_smem_desc(a_hi + k * 32), make_smem_desc(b_addr + k * 32), (kb > kb0 || k > 0) ? 1u : 0u);
                     if (SPLIT) {
 #pragma unroll
                         for (int k = 0; k < BK / 16; ++k)
-                            umma_bf16(acc, make_smem_desc(a_hi + T::A_BYTES + k * 32), make_smem_desc(b_addr + k * 32), idesc, 1u);
+                            mma(acc, make_smem_desc(a_hi + T::A_BYTES + k * 32), make_smem_desc(b_addr + k * 32), 1u);
                     }
-                    umma_commit(&empty_bar[s]);
+                    commit(&empty_bar[s]);
                 }
                 if (timed_out) break;
-                umma_commit(&tmem_full[as]);
+                commit(&tmem_full[as]);
             }
             if (timed_out) {                     // let every MMA issued so far finish before TMEM is freed
-                umma_commit(drain_bar);
+                commit(drain_bar);
                 mbar_wait(drain_bar, 0, wait_ns);         // bounded
             }
         }
@@ -398,7 +442,7 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_ahi, const __grid
         const int q = warp & 3;                  // TMEM lane quarter this warp may read
         const bool vec_ok = (ldd & 3) == 0;
         uint32_t it = 0;
-        for (int u = blockIdx.x; u < ntiles * splits; u += gridDim.x, ++it) {
+        for (int u = unit0; u < ntiles * splits; u += units_at_once, ++it) {
             const uint32_t as = it & 1u, aph = (it >> 1) & 1u;
             const int t = u / splits, sp = u - t * splits;
             const Place pl = place(t);
@@ -619,16 +663,20 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_ahi, const __grid
             }
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&tmem_empty[as]);          // this warp has read its quarter of the accumulator
-
+            if (lane == 0) {                                      // this warp has read its quarter of the accumulator
+                if constexpr (PAIR) mbar_arrive_at(map_to_rank(smem_u32(&tmem_empty[as]), 0));
+                else mbar_arrive(&tmem_empty[as]);
+            }
         }
     }
     if (timed_out && status != nullptr) atomicOr(status, STATUS_TIMEOUT);
     tc_fence_before();
-    __syncthreads();
+    if constexpr (PAIR) { __syncwarp(); cluster_arrive(); cluster_wait(); }      // neither CTA's memory goes away under the other's MMAs and arrivals
+    else __syncthreads();
     if (warp == 1) {
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(2u * ACC_COLS) : "memory");
+        if constexpr (PAIR) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(2u * ACC_COLS) : "memory");
+        else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(2u * ACC_COLS) : "memory");
     }
 }
 
@@ -675,31 +723,36 @@ int sm_count_gemm() {
     return n;
 }
 
-template <int BN, bool SPLIT, bool EXT = false>
+template <int BN, bool SPLIT, bool EXT = false, bool PAIR = false>
 int32_t launch_persistent(const GemmArgs& a, int splits, cudaStream_t st) {
-    using T = Tile<BN, SPLIT, 1>;
+    using T = Tile<BN, SPLIT, 1, PAIR>;
     CUtensorMap mh, ml, mw;
     const int lda = EXT ? a.ext->lda : a.K;
     LUMI_TRY(make_map(&mh, a.a_hi, a.M, lda, BM));
     LUMI_TRY(make_map(&ml, SPLIT ? a.a_lo : a.a_hi, a.M, lda, BM));
-    LUMI_TRY(make_map(&mw, a.w, a.N, a.K, BN));
-    auto kern = gemm_persistent_kernel<BN, SPLIT, EXT>;
+    LUMI_TRY(make_map(&mw, a.w, a.N, a.K, PAIR ? BN / 2 : BN));
+    auto kern = gemm_persistent_kernel<BN, SPLIT, EXT, PAIR>;
     LUMI_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, T::SMEM));
-    const int tiles_m = (a.M + BM - 1) / BM;
+    const int tiles_m = (a.M + (PAIR ? 2 * BM : BM) - 1) / (PAIR ? 2 * BM : BM);
     const int tiles_n = EXT ? (a.ext->group_rows + BN - 1) / BN * (a.ext->tiles != nullptr ? 1 : a.ext->groups) : (a.N + BN - 1) / BN;
     const int ntiles = (EXT && a.ext->tiles != nullptr ? a.ext->max_tiles : tiles_m) * tiles_n;      // by rows: as many as there can be
     const int units = ntiles * splits;
-    const int grid = units < sm_count_gemm() ? units : sm_count_gemm();
+    const int grid = PAIR ? 2 * std::min(units, sm_count_gemm() / 2) : std::min(units, sm_count_gemm());
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(192);
     cfg.dynamicSmemBytes = T::SMEM;
     cfg.stream = st;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = launch_pdl_gemm_on() ? 1 : 0;   // the set-up overlaps the predecessor's tail
+    if (PAIR) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+        attr[cfg.numAttrs].val.clusterDim.x = 2; attr[cfg.numAttrs].val.clusterDim.y = 1; attr[cfg.numAttrs].val.clusterDim.z = 1;
+        ++cfg.numAttrs;
+    }
     LUMI_CUDA(cudaLaunchKernelEx(&cfg, kern, mh, ml, mw, a.d, a.ldd, a.M, a.N, a.K, a.accumulate, tiles_m, ntiles, splits, a.tile_counters,
                                  a.scratch, a.status_word, a.wait_limit_ns ? a.wait_limit_ns : kWaitLimitNs, a.debug_skip_unit, a.nf, EXT ? *a.ext : GemmExt()));
     return LUMI_OK;
@@ -831,6 +884,24 @@ static int32_t launch_ext(const GemmArgs& a, cudaStream_t st) {
     return LUMI_OK;
 }
 
+// Tile width for pairs of CTAs (256-row tiles, half as many workers), or 0 where single CTAs take the product.  Widths whose half is a multiple
+// of 32: 208 was 15 % slower than single CTAs of that width.  Measured with blocked tiles, pair / single, microseconds: 4096 rows 7360 x 1024
+// 104.5 / 115.6, 1024 x 2048 33.5 / 33.7, 6208 x 1024 89 / 101; 32768 rows 735 / 771, 173 / 189, 625 / 720, 8192 x 2048 1403 / 1497; below 4096 rows
+// half as many, twice as high tiles leave more of the last round idle (2048 rows 1024 x 2048 23.6 / 22.1).  The sums differ in their last
+// bits from those of one CTA.
+static int pair_width(const GemmArgs& a) {
+    static const bool on = !(getenv("LUMI_GEMM_PAIR") && atoi(getenv("LUMI_GEMM_PAIR")) == 0);      // 0: tuning aid
+    if (!on || a.one_order || a.a_lo == nullptr || a.M < kPairMinRows) return 0;
+    const long tiles_m = (a.M + 2 * BM - 1) / (2 * BM), workers = sm_count_gemm() / 2;
+    int best = 0;
+    long best_cost = -1;
+    for (int w : {256, 192, 128}) {
+        const long tiles = tiles_m * ((a.N + w - 1) / w), cost = (tiles + workers - 1) / workers * (w + 32);
+        if (best_cost < 0 || cost < best_cost) { best = w; best_cost = cost; }
+    }
+    return best;
+}
+
 int32_t launch_gemm_tcgen05(const GemmArgs& a, cudaStream_t st) {
     if (a.M <= 0 || a.N <= 0 || a.K <= 0 || (a.K % BK) != 0)
         return fail(LUMI_E_UNSUPPORTED, "tcgen05 GEMM needs K %% 64 == 0 (M %d N %d K %d)", a.M, a.N, a.K);
@@ -857,6 +928,12 @@ int32_t launch_gemm_tcgen05(const GemmArgs& a, cudaStream_t st) {
     const long tiles256 = (long)((a.N + 255) / 256) * ((a.M + BM - 1) / BM);
     static const int persist = getenv("LUMI_GEMM_PERSIST") ? atoi(getenv("LUMI_GEMM_PERSIST")) : 1;     // 0: tuning aid
     if (persist || fused) {
+        switch (pair_width(a)) {
+            case 256: return launch_persistent<256, true, false, true>(a, 1, st);
+            case 192: return launch_persistent<192, true, false, true>(a, 1, st);
+            case 128: return launch_persistent<128, true, false, true>(a, 1, st);
+            default: break;
+        }
         int best = 256, best_splits = 1;
         pick_tile(a, &best, &best_splits);
 #define LUMI_PERSIST_CASE(W) if (best == W) return split ? launch_persistent<W, true>(a, best_splits, st) : launch_persistent<W, false>(a, best_splits, st);

@@ -541,7 +541,7 @@ struct GemmArgs {
     int debug_skip_unit = -1;           // test hook: the producer stops before this work unit, so the consumers' waits run out
     NormFuse nf;                        // RMSNorm folded around the product (persistent kernel only)
     const GemmExt* ext = nullptr;       // products in groups, gated results
-    bool one_order = false;             // sums in one order whatever the rows: nothing but the persistent kernel
+    bool one_order = false;             // sums in one order whatever the rows: nothing but the persistent kernel's single CTAs
 };
 int32_t launch_gemm_tcgen05(const GemmArgs& a, cudaStream_t st);   // returns LUMI_* status
 constexpr int kFewRowsMax = 1024;                                   // rows up to which gemm_few_rows.cu may take a product
