@@ -7,6 +7,8 @@
 // products use FMA with a fixed summation order (per-lane strided partials, xor-shuffle tree), so
 // results are bit-stable from run to run.
 #include "internal.h"
+
+#include <algorithm>
 #include "embed_post.cuh"
 #include <type_traits>
 
@@ -215,22 +217,26 @@ __global__ void __launch_bounds__(256) gemv_kernel(const float* A, int lda, cons
     const int K4 = K >> 2, KC = K / E;
     const int gpc = 8 / KS;                             // row groups per CTA
     const int g = warp / KS, seg = warp - g * KS;
-    const int row0 = (blockIdx.x * gpc + g) * RPW;
+    const int ngrp = (N + gpc * RPW - 1) / (gpc * RPW); // groups of rows; a CTA takes every gridDim.x-th, so that staging and norm are paid once for all of them
+    int row0 = (blockIdx.x * gpc + g) * RPW;
     const int c0 = seg * 32 * U + lane;                 // this lane's first 16-byte chunk
 
     pdl_launch_dependents();
     // the weights do not depend on the previous kernel: all loads go out before waiting for it
     uint4 wreg[NR][U];
+    auto load_rows = [&]() {
 #pragma unroll
-    for (int r = 0; r < NR; ++r) {
-        const int row = weight_row(min(row0 + (r % RPW), N - 1), r >= RPW);
-        const WT* wp = W + (size_t)row * K;
+        for (int r = 0; r < NR; ++r) {
+            const int row = weight_row(min(row0 + (r % RPW), N - 1), r >= RPW);
+            const WT* wp = W + (size_t)row * K;
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const int c = c0 + 32 * u;
-            wreg[r][u] = (c < KC && row0 < N) ? __ldg(reinterpret_cast<const uint4*>(wp + (size_t)c * E)) : make_uint4(0u, 0u, 0u, 0u);
+            for (int u = 0; u < U; ++u) {
+                const int c = c0 + 32 * u;
+                wreg[r][u] = (c < KC && row0 < N) ? __ldg(reinterpret_cast<const uint4*>(wp + (size_t)c * E)) : make_uint4(0u, 0u, 0u, 0u);
+            }
         }
-    }
+    };
+    load_rows();
     pdl_wait();
 
     for (int i = threadIdx.x; i < NB * K4; i += 256) {
@@ -292,83 +298,90 @@ __global__ void __launch_bounds__(256) gemv_kernel(const float* A, int lda, cons
         }
         __syncthreads();
     }
-    float acc[NR][NB];
-#pragma unroll
-    for (int r = 0; r < NR; ++r)
-#pragma unroll
-        for (int b = 0; b < NB; ++b) acc[r][b] = 0.f;
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-        const int c = c0 + 32 * u;
-        if (c < KC) {
-            float w[NR][E];
-#pragma unroll
-            for (int r = 0; r < NR; ++r) WRaw<WT>::cvt(wreg[r][u], w[r]);
-#pragma unroll
-            for (int b = 0; b < NB; ++b) {
-                float xv[E];
-#pragma unroll
-                for (int q = 0; q < E / 4; ++q) {
-                    float4 v = *reinterpret_cast<const float4*>(xs + b * K + c * E + 4 * q);
-                    xv[4 * q] = v.x; xv[4 * q + 1] = v.y; xv[4 * q + 2] = v.z; xv[4 * q + 3] = v.w;
-                }
-#pragma unroll
-                for (int r = 0; r < NR; ++r)
-#pragma unroll
-                    for (int e = 0; e < E; ++e) acc[r][b] = fmaf(w[r][e], xv[e], acc[r][b]);
-            }
-        }
-    }
-#pragma unroll
-    for (int r = 0; r < NR; ++r)
-#pragma unroll
-        for (int b = 0; b < NB; ++b) acc[r][b] = warp_sum(acc[r][b]);
-    if (KS > 1) {
-        if (lane == 0) {
-#pragma unroll
-            for (int r = 0; r < NR; ++r)
-#pragma unroll
-                for (int b = 0; b < NB; ++b) part[warp][r][b] = acc[r][b];
-        }
-        __syncthreads();
-        if (seg == 0) {
-#pragma unroll
-            for (int r = 0; r < NR; ++r)
-#pragma unroll
-                for (int b = 0; b < NB; ++b) {
-                    float t = part[warp][r][b];
-                    for (int sg = 1; sg < KS; ++sg) t += part[warp + sg][r][b];
-                    acc[r][b] = t;
-                }
-        }
-    }
     // greedy head: this warp's best (value, lowest row on ties) per batch row, for the per-CTA partial below
     float bestv[NB];
     int besti[NB];
 #pragma unroll
     for (int b = 0; b < NB; ++b) { bestv[b] = -INFINITY; besti[b] = 0x7fffffff; }
-    if (seg == 0 && lane == 0 && row0 < N) {
+    for (int grp = blockIdx.x;;) {
+        float acc[NR][NB];
 #pragma unroll
-        for (int r = 0; r < RPW; ++r) {
-            int row = row0 + r;
-            if (row >= N) break;
+        for (int r = 0; r < NR; ++r)
 #pragma unroll
-            for (int b = 0; b < NB; ++b) {
-                if (b >= nb) break;
-                float v = acc[r][b];
-                if (bias != nullptr) v += bias[weight_row(row, false)];
-                if constexpr (ACT == ACT_SIGMOID_GATE) v = __fmul_rn(sigmoid_ref(v), acc[RPW + r][b]);     // model.rs:550-552
-                if constexpr (ACT == ACT_RELU_GATE || ACT == ACT_SILU_GATE) {
-                    const float up = acc[RPW + r][b] + (bias != nullptr ? bias[weight_row(row, true)] : 0.f);
-                    v = __fmul_rn(ACT == ACT_RELU_GATE ? fmaxf(v, 0.f) : silu_ref(v), up);
+            for (int b = 0; b < NB; ++b) acc[r][b] = 0.f;
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int c = c0 + 32 * u;
+            if (c < KC) {
+                float w[NR][E];
+#pragma unroll
+                for (int r = 0; r < NR; ++r) WRaw<WT>::cvt(wreg[r][u], w[r]);
+#pragma unroll
+                for (int b = 0; b < NB; ++b) {
+                    float xv[E];
+#pragma unroll
+                    for (int q = 0; q < E / 4; ++q) {
+                        float4 v = *reinterpret_cast<const float4*>(xs + b * K + c * E + 4 * q);
+                        xv[4 * q] = v.x; xv[4 * q + 1] = v.y; xv[4 * q + 2] = v.z; xv[4 * q + 3] = v.w;
+                    }
+#pragma unroll
+                    for (int r = 0; r < NR; ++r)
+#pragma unroll
+                        for (int e = 0; e < E; ++e) acc[r][b] = fmaf(w[r][e], xv[e], acc[r][b]);
                 }
-                if constexpr (ACT == ACT_RELU2) { v = fmaxf(v, 0.f); v = __fmul_rn(v, v); }
-                size_t o = (size_t)(m0 + b) * ldd + row;
-                if (R != nullptr) v = __fadd_rn(v, R[o]);
-                if (D != nullptr) D[o] = v;
-                if (v > bestv[b] || (v == bestv[b] && row < besti[b])) { bestv[b] = v; besti[b] = row; }
             }
         }
+#pragma unroll
+        for (int r = 0; r < NR; ++r)
+#pragma unroll
+            for (int b = 0; b < NB; ++b) acc[r][b] = warp_sum(acc[r][b]);
+        if (KS > 1) {
+            if (lane == 0) {
+#pragma unroll
+                for (int r = 0; r < NR; ++r)
+#pragma unroll
+                    for (int b = 0; b < NB; ++b) part[warp][r][b] = acc[r][b];
+            }
+            __syncthreads();
+            if (seg == 0) {
+#pragma unroll
+                for (int r = 0; r < NR; ++r)
+#pragma unroll
+                    for (int b = 0; b < NB; ++b) {
+                        float t = part[warp][r][b];
+                        for (int sg = 1; sg < KS; ++sg) t += part[warp + sg][r][b];
+                        acc[r][b] = t;
+                    }
+            }
+        }
+        if (seg == 0 && lane == 0 && row0 < N) {
+#pragma unroll
+            for (int r = 0; r < RPW; ++r) {
+                int row = row0 + r;
+                if (row >= N) break;
+#pragma unroll
+                for (int b = 0; b < NB; ++b) {
+                    if (b >= nb) break;
+                    float v = acc[r][b];
+                    if (bias != nullptr) v += bias[weight_row(row, false)];
+                    if constexpr (ACT == ACT_SIGMOID_GATE) v = __fmul_rn(sigmoid_ref(v), acc[RPW + r][b]);     // model.rs:550-552
+                    if constexpr (ACT == ACT_RELU_GATE || ACT == ACT_SILU_GATE) {
+                        const float up = acc[RPW + r][b] + (bias != nullptr ? bias[weight_row(row, true)] : 0.f);
+                        v = __fmul_rn(ACT == ACT_RELU_GATE ? fmaxf(v, 0.f) : silu_ref(v), up);
+                    }
+                    if constexpr (ACT == ACT_RELU2) { v = fmaxf(v, 0.f); v = __fmul_rn(v, v); }
+                    size_t o = (size_t)(m0 + b) * ldd + row;
+                    if (R != nullptr) v = __fadd_rn(v, R[o]);
+                    if (D != nullptr) D[o] = v;
+                    if (v > bestv[b] || (v == bestv[b] && row < besti[b])) { bestv[b] = v; besti[b] = row; }
+                }
+            }
+        }
+        grp += gridDim.x;
+        if (grp >= ngrp) break;
+        if (KS > 1) __syncthreads();                    // the segments' sums have been read
+        row0 = (grp * gpc + g) * RPW;
+        load_rows();
     }
     if (amax_val != nullptr) {
         // argmax fused behind the product (replaces the host-side argmax of inference/src/main.rs:142-143): one
@@ -1423,8 +1436,13 @@ static cudaError_t gemv_launch(const GemvArgs& a, int KS, cudaStream_t st) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
     }
-    const int rows_per_cta = (8 / KS) * RPW;
-    dim3 grid((a.N + rows_per_cta - 1) / rows_per_cta, (a.M + NB - 1) / NB);
+    // as many CTAs as are resident together, each with several groups of rows: eight staged and normed rows cost a CTA more than
+    // a group's weights.  Without overlap, us: 8 bf16 rows x 7360 x 1024 41.1 -> 23.9, x 32000 x 1024 141 -> 56 (two weight rows per warp now as well);
+    // one row x 32000 x 1024 24.6 -> 19.1; at most four CTAs of eight staged rows per SM instead of two 30.6 and 69
+    const int rows_per_cta = (8 / KS) * RPW, groups = (a.N + rows_per_cta - 1) / rows_per_cta;
+    const int resident = sm_count() * std::max(1, std::min(NB == 8 ? 2 : 4, (int)((200 * 1024) / smem)));
+    const int turns = (groups + resident - 1) / resident;
+    dim3 grid((groups + turns - 1) / turns, (a.M + NB - 1) / NB);
     if (a.amax_val != nullptr) {
         if ((int)grid.x > a.amax_stride) return cudaErrorInvalidValue;
         if (a.amax_parts != nullptr) *a.amax_parts = (int)grid.x;
@@ -1441,7 +1459,7 @@ static cudaError_t gemv_dispatch(const GemvArgs& a, cudaStream_t st) {
     while (KS < 8 && KS * kseg < a.K) KS *= 2;
     if (KS * kseg < a.K) return cudaErrorInvalidValue;          // K beyond 8 segments per row
     // two rows per warp only when that still leaves at least two CTAs per SM
-    if (ACT == 0 && NB <= 4 && (long)a.N / ((8 / KS) * 2) >= 296) return gemv_launch<WT, NB, 2, ACT>(a, KS, st);
+    if (ACT == 0 && (long)a.N / ((8 / KS) * 2) >= 296) return gemv_launch<WT, NB, 2, ACT>(a, KS, st);
     return gemv_launch<WT, NB, 1, ACT>(a, KS, st);
 }
 
@@ -1479,16 +1497,6 @@ static cudaError_t gemv_by_batch(const GemvArgs& a, cudaStream_t st) {
 }
 
 // ---- the preloading single-wave variant: when it applies and how it is launched ----
-static int sm_count() {
-    static int n = 0;
-    if (n == 0) {
-        int dev = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0)
-            n = 148;
-    }
-    return n;
-}
-
 // LUMI_GEMV_PRE=0 keeps every small-batch product on the multi-wave kernel (tuning aid).
 static bool gemv_pre_enabled() {
     static int v = -1;
