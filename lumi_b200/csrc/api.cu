@@ -1812,9 +1812,12 @@ int32_t enqueue_step(lumi_session* s, int B, bool with_head, int64_t* launches,
     StepPlan p{s, B, use_tc(s, B)};
     p.prof = prof;
     p.row_len = row_len;
+    // five to eight rows of bf16 weights: early CTAs of the next kernels take registers and shared memory from the staging CTAs (8 sequences, 64 tokens
+    // of the 48-layer base model: 140 ms with dependent launch, 127 without; fp32, 6 sequences: 122 and 126)
+    const bool staged_rows = !c.stacked() && s->m->wdtype == LUMI_DTYPE_BF16 && B > 4;
     // dependent launch overlaps each kernel's prologue (weight prefetch) with its predecessor; it is
     // used on the weight-streaming path, where launch gaps are the same order as the kernels
-    struct PdlScope { PdlScope(bool on) { set_launch_pdl(on); } ~PdlScope() { set_launch_pdl(false); } } pdl_scope(s->opt_pdl && prof == nullptr && (!p.tc || (pdl_tc_max() > 0 && B <= pdl_tc_max())));
+    struct PdlScope { PdlScope(bool on) { set_launch_pdl(on); } ~PdlScope() { set_launch_pdl(false); } } pdl_scope(s->opt_pdl && prof == nullptr && (p.tc ? pdl_tc_max() > 0 && B <= pdl_tc_max() : !staged_rows));
     // the tensor-core GEMMs themselves: dependent launch up to LUMI_PDL_GEMM rows (their barrier / TMEM set-up then runs under the
     // tail of the state step; unlike an early state step this takes nothing from a running GEMM)
     struct PdlGemmScope { PdlGemmScope(bool on) { set_launch_pdl_gemm(on); } ~PdlGemmScope() { set_launch_pdl_gemm(false); } } pdl_gemm_scope(s->opt_pdl && prof == nullptr && p.tc && B <= pdl_gemm_max());
