@@ -2281,7 +2281,7 @@ int32_t prefill_chunked(lumi_session* s, int batch, int T, bool with_head, float
                     a.rope_base = c.attn_rope_base;
                     a.ctl = s->ctl;
                     a.rows_per_seq = ts; a.b0 = b0;
-                    a.row_len = lens;
+                    a.row_len = lens; a.t_abs0 = t0;
                     for (int phase = 1; phase <= 2; ++phase) {
                         a.phase = phase;
                         cudaError_t e = launch_attention_decode(a, s->stream);

@@ -108,7 +108,7 @@ __global__ void __launch_bounds__(128) attn_decode_kernel(AttnArgs a, KT* pool) 
         if (a.phase == 0) {
             const int pp = a.ctl->prompt_pos;
             if (pp < a.ctl->prompt_len && pp >= a.row_len[b]) return;
-        } else if (a.pos[b] + r % a.rows_per_seq >= a.row_len[b]) {
+        } else if (a.t_abs0 + r % a.rows_per_seq >= a.row_len[b]) {
             // a row of a prompt slice behind a shorter prompt: nothing to attend to; its output row is zero, so that
             // whatever follows it through the layers stays finite
             for (int i = tid; i < HPK * HD; i += 128) {
@@ -420,7 +420,7 @@ __global__ void __launch_bounds__(256) kv_append_kernel(AttnArgs a, KT* pool, lo
     const int pr = (int)(i % half), kvh = (int)((i / half) % a.kv_heads), r = (int)(i / ((long)half * a.kv_heads));
     const int b = a.b0 + r / a.rows_per_seq;
     const int pos = a.pos[b] + r % a.rows_per_seq;
-    if (a.row_len != nullptr && pos >= a.row_len[b]) return;          // padding behind a shorter prompt
+    if (a.row_len != nullptr && a.t_abs0 + r % a.rows_per_seq >= a.row_len[b]) return;          // padding behind a shorter prompt
     const int cap = a.window > 0 ? min(a.window, a.max_tokens) : a.max_tokens;
     const int slot = (a.window > 0 && a.window <= a.max_tokens) ? pos % a.window : pos;
     if (pos < 0 || slot >= cap) {
@@ -510,7 +510,7 @@ __global__ void __launch_bounds__(128) attn_mma_kernel(AttnArgs a, const __grid_
             const int pp = a.ctl->prompt_pos;
             if (pp < a.ctl->prompt_len && pp >= a.row_len[b]) return;
         } else {
-            nvalid = max(0, min(nrow, a.row_len[b] - pos0));
+            nvalid = max(0, min(nrow, a.row_len[b] - a.t_abs0 - i0));
         }
     }
     if (nvalid < nrow) {

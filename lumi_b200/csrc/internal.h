@@ -477,7 +477,8 @@ struct AttnArgs {
     int32_t* part_count = nullptr;
     int max_ctx_hint = 0;
     const int32_t* row_len = nullptr;    // prompts of different lengths: rows at or past their sequence's prompt length are skipped (decode form: by the
-                                         // step's prompt position; prompt slices: by the row's own position, and their output rows are zero)
+                                         // step's prompt position; prompt slices: by the row's place in the prompt, and their output rows are zero)
+    int t_abs0 = 0;                      // prompt slices: place in the prompt of a sequence's first row (its position is larger behind earlier tokens)
     size_t pool_bytes = 0;               // size of this layer's page pool (bounds the tensor map of the tensor-core kernel); 0: not given
 };
 constexpr int kAttnPartSlices = 16;

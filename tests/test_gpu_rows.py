@@ -87,3 +87,23 @@ def test_short_prompts_with_attention_layers(T):
     prompts = synth.random_prompts(2, T, cfg.vocab_size, seed=T)
     assert rel(rows.prefill(prompts), steps.prefill(prompts)) < 2e-3          # the two sides round their keys and values to bf16 on their own
     assert rel(rows.forward_step(prompts[:, 0])[0], steps.forward_step(prompts[:, 0])[0]) < 2e-3
+
+
+# a slice's rows count from the prompt's first token, the cache from the sequence's: first prompts of different lengths, so that the two differ by
+# another amount in every sequence; lengths of one token, of the longest, around a slice of 64; tensor-core and CUDA-core attention
+@pytest.mark.parametrize("kv_heads,heads", [(4, 16), (8, 32)])
+@pytest.mark.parametrize("T", [30, 140])
+def test_ragged_prompts_behind_earlier_tokens(T, kv_heads, heads):
+    cfg = synth.base_config(n_layers=3, vocab_size=700, attention_layers=[1], attn_mlp_dim=256, attn_rope_base=10000.0, attn_n_heads=heads, attn_kv_heads=kv_heads)
+    _, _, rows, steps = pair(cfg, "bf16", 4)
+    rows.set_option("prefill_rows", 256)
+    first = synth.random_prompts(4, 40, cfg.vocab_size, seed=1)
+    second = synth.random_prompts(4, T, cfg.vocab_size, seed=2)
+    lengths = np.array([T, 1, min(T, 64), min(T, 65)], dtype=np.int32)
+    for prompts, lens in ((first, np.array([40, 7, 33, 40], dtype=np.int32)), (second, lengths)):
+        a, b = rows.prefill_ragged(prompts, lens), steps.prefill_ragged(prompts, lens)
+        assert rel(a, b) < 2e-3                            # keys and values are rounded to bf16 on each side
+    for i in range(3):
+        a, b = (s.forward_step(second[:, i], step=i)[0] for s in (rows, steps))
+        for j in range(4):
+            assert rel(a[j], b[j]) < 2e-3, (i, j)
