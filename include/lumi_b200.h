@@ -260,6 +260,11 @@ int32_t lumi_debug_gemm_plan(int32_t M, int32_t N, int32_t K, int32_t two_planes
 int32_t lumi_k_gemv(uint64_t a_f32, uint64_t w, int32_t w_dtype, uint64_t d, uint64_t residual,
                     uint64_t norm_gamma, int32_t M, int32_t N, int32_t K, uint64_t stream);
 
+/* The same product for many rows (prompts a layer at a time): D[M][N] (+)= A[M][K] * W[N][K]^T on CUDA cores, fp32 throughout,
+ * K % 16 == 0, rows of A 16-byte aligned.  The order of a sum depends on K alone, so a row's results are the same bits alone and among others. */
+int32_t lumi_k_row_gemm(uint64_t a_f32, uint64_t w, int32_t w_dtype, uint64_t d, int32_t M, int32_t N, int32_t K,
+                        int32_t accumulate, uint64_t stream);
+
 /* The fused Mamba-3 state step alone (inference/src/model.rs:301-370 after in_proj, before
  * out_proj): proj[B][ldp] holds in_proj's output rows; h[B][H][P][N], x_prev[B][H][P],
  * b_prev[B][H][N], cum_angle[B][H][N/2] are updated in place; y[B][H*P] receives the gated output. */

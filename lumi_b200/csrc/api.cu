@@ -2896,27 +2896,34 @@ extern "C" int32_t lumi_debug_run_block(lumi_session* s, int32_t layer, float* x
 }
 
 // ---- single kernels over caller-owned device pointers ---------------------------------------------------
-extern "C" int32_t lumi_k_gemm_bf16_tcgen05(uint64_t a_hi, uint64_t a_lo, uint64_t w, uint64_t d, int32_t M, int32_t N, int32_t K,
-                                            int32_t ldd, int32_t accumulate, uint64_t stream) {
-    if (!a_hi || !w || !d) return fail(LUMI_E_INVALID, "null device pointer");
-    // split-K needs zeroed counters: one small buffer per device for this test entry, made on first use
+namespace {
+// Splits of K need zeroed counters and room for partial sums: one small buffer per device for these entries, made on first use.
+struct KernelScratch { int32_t* counters = nullptr; int n_counters = 0; float* scratch = nullptr; size_t floats = 0; };
+int32_t kernel_scratch(KernelScratch* out) {
     static std::mutex mu;
     static int32_t* counters[64] = {nullptr};
     static float* scratch[64] = {nullptr};
     int dev = 0;
     LUMI_CUDA(cudaGetDevice(&dev));
-    int32_t* cnt = nullptr;
-    if (dev >= 0 && dev < 64) {
-        std::lock_guard<std::mutex> lock(mu);
-        if (counters[dev] == nullptr) {
-            LUMI_CUDA(cudaMalloc(&counters[dev], sizeof(int32_t) * kGemmCounters));
-            LUMI_CUDA(cudaMemset(counters[dev], 0, sizeof(int32_t) * kGemmCounters));
-            LUMI_CUDA(cudaMalloc(&scratch[dev], sizeof(float) * kGemmScratchFloats));
-        }
-        cnt = counters[dev];
+    if (dev < 0 || dev >= 64) return LUMI_OK;
+    std::lock_guard<std::mutex> lock(mu);
+    if (counters[dev] == nullptr) {
+        LUMI_CUDA(cudaMalloc(&counters[dev], sizeof(int32_t) * kGemmCounters));
+        LUMI_CUDA(cudaMemset(counters[dev], 0, sizeof(int32_t) * kGemmCounters));
+        LUMI_CUDA(cudaMalloc(&scratch[dev], sizeof(float) * kGemmScratchFloats));
     }
+    *out = KernelScratch{counters[dev], kGemmCounters, scratch[dev], kGemmScratchFloats};
+    return LUMI_OK;
+}
+}  // namespace
+
+extern "C" int32_t lumi_k_gemm_bf16_tcgen05(uint64_t a_hi, uint64_t a_lo, uint64_t w, uint64_t d, int32_t M, int32_t N, int32_t K,
+                                            int32_t ldd, int32_t accumulate, uint64_t stream) {
+    if (!a_hi || !w || !d) return fail(LUMI_E_INVALID, "null device pointer");
+    KernelScratch ks;
+    LUMI_TRY(kernel_scratch(&ks));
     GemmArgs g{(const __nv_bfloat16*)a_hi, (const __nv_bfloat16*)a_lo, (const __nv_bfloat16*)w, (float*)d, ldd, M, N, K, accumulate, nullptr,
-               cnt, cnt ? kGemmCounters : 0, cnt ? scratch[dev] : nullptr, cnt ? kGemmScratchFloats : 0};
+               ks.counters, ks.n_counters, ks.scratch, ks.floats};
     return launch_gemm_tcgen05(g, (cudaStream_t)stream);
 }
 
@@ -2957,6 +2964,17 @@ extern "C" int32_t lumi_debug_gemm_wait_timeout(uint64_t a_hi, uint64_t w, uint6
     int32_t st = 0;
     LUMI_CUDA(cudaMemcpy(&st, (const void*)status_word, sizeof(st), cudaMemcpyDeviceToHost));
     if (st & STATUS_TIMEOUT) return fail(LUMI_E_TIMEOUT, "a bounded device-side wait expired in the tensor-core GEMM (limit %llu ns)", (unsigned long long)wait_limit_ns);
+    return LUMI_OK;
+}
+
+extern "C" int32_t lumi_k_row_gemm(uint64_t a_f32, uint64_t w, int32_t w_dtype, uint64_t d, int32_t M, int32_t N, int32_t K, int32_t accumulate,
+                                   uint64_t stream) {
+    if (!a_f32 || !w || !d || M <= 0 || N <= 0 || K <= 0 || ((a_f32 | w) & 15)) return fail(LUMI_E_INVALID, "bad argument to lumi_k_row_gemm");
+    if (!row_gemm_supported(K) || w_dtype != LUMI_DTYPE_F32) return fail(LUMI_E_UNSUPPORTED, "a product of rows needs fp32 weights and K %% 16 == 0");
+    KernelScratch ks;
+    LUMI_TRY(kernel_scratch(&ks));
+    LUMI_CUDA(launch_row_gemm(RowGemmArgs{(const float*)a_f32, K, (const float*)w, (float*)d, N, M, N, K, accumulate, ks.counters, ks.n_counters, ks.scratch,
+                                          ks.floats}, (cudaStream_t)stream));
     return LUMI_OK;
 }
 

@@ -13,112 +13,138 @@ namespace lumi {
 namespace {
 
 // ---- fp32 product over rows ---------------------------------------------------------------------------------
-// D[M][N] (+)= A[M][K] W[N][K]^T on the CUDA cores, fp32 throughout.  A CTA of 64 threads owns BM x 64 results and, with K split
-// over blockIdx.z, part of the sum; a thread owns TM x 8 of them, rows and columns eight apart, so that the eight columns that a
-// quarter warp reads lie in eight different bank groups (rows of 16 + 4 padding floats).  Even and odd k are summed apart in
+// D[M][N] (+)= A[M][K] W[N][K]^T on the CUDA cores, fp32 throughout.  A CTA of 128 threads owns BM x 64 results and, with K split
+// over blockIdx.z, part of the sum; a thread owns TM x 8 of them, rows sixteen and columns eight apart, so that the eight columns that a
+// quarter warp reads lie in eight different bank groups (rows of 32 + 4 padding floats).  Even and odd k are summed apart in
 // the two halves of packed multiply-adds (fma.rn.f32x2): operands come as 16-byte loads along K as they are stored, with no
-// transposition, and one instruction does two multiply-adds.  Every 128 of K the sums go to a total in shared memory: one running
-// sum over all of K was 2e-7 off in log-probabilities where the decode step's sums by lanes are 0.9e-7 off.  What bounds it: the FMA pipe at many rows (64 packed
-// multiply-adds per eight 16-byte shared loads), the stream of the weights at few.  Small CTAs, four to seven per SM, so that
-// copies of one run under the arithmetic of the others and the last wave is short.  Measured: 384 x 32000 x 1024 in 597 us (0.58 of the
-// FMA pipe's 36 T/s), 384 x 7360 x 1024 in 184 us, 384 x 1024 x 2048 in 68 us, 32 x 7360 x 1024 in 22 us (its arithmetic takes 6.6 us, its
-// bytes 4.7 us).
-constexpr int kBK = 16, kPad = kBK + 4, kStages = 3, kBN = 64, kFlush = 8;
+// transposition, and one instruction does two multiply-adds.
+// The order of a sum is fixed by K alone: chains of 16 products (32 of K, even and odd apart), four of them added up to a unit of 128 of K,
+// four units to a group, the groups in order, wherever K is split and however many rows there are; a row's results are the same bits alone
+// and among others.  With one running sum per half for 128 of K at a time prompts were further from 64 bits than token by token (48-layer base
+// model, logits of a 9-token prompt 2.2e-6 against 1.6e-6, scores of 8 x 120 tokens 1.0e-7 against 0.86e-7); this order comes to 1.6e-6 and 0.82e-7.
+// What bounds it: shared-memory reads at many rows (a 16-byte load for five packed multiply-adds), the stream of the weights at few.  Measured: 384 x
+// 32000 x 1024 in 697 us (half of the FMA pipe's 36 T/s), 384 x 7360 x 1024 in 178 us, 384 x 1024 x 2048 in 71 us.  A thread's tile of 8 x 8 with the unit's
+// sums in registers spills (225 us for the second), with them in shared memory its copies cost as much (220 us).
+constexpr int kBK = 32, kPad = kBK + 4, kBN = 64, kUnit = 4, kGroup = 4, kStages = 2;      // kUnit: blocks of kBK; kGroup: units
 
 __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
     uint64_t d;
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
     return d;
 }
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
 __device__ __forceinline__ float halves_sum(uint64_t v) { return __uint_as_float((uint32_t)v) + __uint_as_float((uint32_t)(v >> 32)); }
-__device__ __forceinline__ void copy16(void* dst, const void* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+__device__ __forceinline__ float4 add4(float4 a, float4 b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
+__device__ __forceinline__ void copy16(void* dst, const void* src, int bytes) {      // bytes 0: zeros
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(bytes) : "memory");
 }
 
 template <int TM>
-__global__ void __launch_bounds__(64) row_gemm_kernel(RowGemmArgs g, int blocks_per_split) {
-    constexpr int BM = 8 * TM, ROWS = BM + kBN, CPT = ROWS * 4 / 64;       // 16-byte copies per thread and stage
-    extern __shared__ __align__(16) float sm[];                            // [stage][A rows, then W rows][kPad], then the totals
+constexpr int row_gemm_smem() { return (kStages * (16 * TM + kBN) * kPad + 2 * 16 * TM * kBN) * (int)sizeof(float); }      // TM 4: 68 KiB, three CTAs per SM
+
+template <int TM>
+__global__ void __launch_bounds__(128, TM == 4 ? 3 : 4) row_gemm_kernel(RowGemmArgs g, int units_per_split) {
+    constexpr int BM = 16 * TM, ROWS = BM + kBN, TILE4 = BM * kBN / 4;
+    extern __shared__ __align__(16) float sm[];                            // [stage][A rows, then W rows][kPad], the group's sums, the sums of the groups before
     const int tid = threadIdx.x, tn = tid & 7, tm = tid >> 3;
     const int n0 = blockIdx.x * kBN, m0 = blockIdx.y * BM;
-    const int kb0 = blockIdx.z * blocks_per_split, kb1 = min(g.K / kBK, kb0 + blocks_per_split);
-    const float* src[CPT];
-    int dst[CPT];
-#pragma unroll
-    for (int c = 0; c < CPT; ++c) {
-        const int row = (tid + 64 * c) >> 2, q = tid & 3;                  // rows past the end read the last one: never stored
-        src[c] = (row < BM ? g.A + (size_t)min(m0 + row, g.M - 1) * g.lda : g.W + (size_t)min(n0 + row - BM, g.N - 1) * g.K) + (size_t)kb0 * kBK + 4 * q;
-        dst[c] = row * kPad + 4 * q;
-    }
+    const int blocks = (g.K + kBK - 1) / kBK, units = (blocks + kUnit - 1) / kUnit;
+    const int kb0 = blockIdx.z * units_per_split * kUnit, kb1 = min(blocks, kb0 + units_per_split * kUnit);
+    const bool split = gridDim.z > 1;
+    // this thread copies 16 bytes at column cq of every sixteenth row; rows past the end read the last one: never stored
+    const int cq = 4 * (tid & 7), crow = tid >> 3, a_end = g.M - 1 - m0, w_end = g.N - 1 - n0;
+    const float *const a0 = g.A + (size_t)m0 * g.lda + cq, *const w0 = g.W + (size_t)n0 * g.K + cq;
     auto stage = [&](int kb) {
         if (kb < kb1) {
-            float* s = sm + ((kb - kb0) % kStages) * ROWS * kPad;
+            float* s = sm + (kb & 1) * ROWS * kPad + crow * kPad + cq;
+            const bool in = kb * kBK + cq < g.K;                           // K is a multiple of 16: the last block may be half zeros
+            const int k = in ? kb * kBK : 0, bytes = in ? 16 : 0;
 #pragma unroll
-            for (int c = 0; c < CPT; ++c) { copy16(s + dst[c], src[c]); src[c] += kBK; }
+            for (int c = 0; c < ROWS / 16; ++c) {
+                const int row = crow + 16 * c;
+                copy16(s + 16 * c * kPad, 16 * c < BM ? a0 + min(row, a_end) * g.lda + k : w0 + min(row - BM, w_end) * g.K + k, bytes);
+            }
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    uint64_t acc[TM][8];
+    uint64_t mid[TM][8];                                                   // the unit's chains so far
 #pragma unroll
     for (int i = 0; i < TM; ++i)
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = 0ull;
-    float* const total = sm + kStages * ROWS * kPad + tid;                 // this thread's sums of the blocks before the last flush
-    bool flushed = false;
-    auto result = [&](int i, int j) { return flushed ? total[(i * 8 + j) * 64] + halves_sum(acc[i][j]) : halves_sum(acc[i][j]); };
-    for (int s = 0; s < kStages - 1; ++s) stage(kb0 + s);
+        for (int j = 0; j < 8; ++j) mid[i][j] = 0ull;
+    float4* const group_sum = reinterpret_cast<float4*>(sm + kStages * ROWS * kPad) + tid;      // this thread's results four by four, 128 apart
+    float4* const total = group_sum + TILE4;
+    const int tile = blockIdx.y * gridDim.x + blockIdx.x;
+    float4* const parts = reinterpret_cast<float4*>(g.scratch) + (size_t)tile * units * TILE4 + tid;      // K split: the units' sums
+    stage(kb0);
     for (int kb = kb0; kb < kb1; ++kb) {
-        asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 2) : "memory");
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncthreads();                                                   // the block has landed, and the one before it is no longer read
-        stage(kb + kStages - 1);
-        const float* s = sm + ((kb - kb0) % kStages) * ROWS * kPad;
+        stage(kb + 1);
+        const float* s = sm + (kb & 1) * ROWS * kPad;
+        uint64_t acc[TM][8];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
+        for (int q = 0; q < kBK / 4; ++q) {
             ulonglong2 a[TM];
 #pragma unroll
-            for (int i = 0; i < TM; ++i) a[i] = *reinterpret_cast<const ulonglong2*>(s + (tm + 8 * i) * kPad + 4 * q);
+            for (int i = 0; i < TM; ++i) a[i] = *reinterpret_cast<const ulonglong2*>(s + (tm + 16 * i) * kPad + 4 * q);
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
                 const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(s + (BM + tn + 8 * j) * kPad + 4 * q);
 #pragma unroll
-                for (int i = 0; i < TM; ++i) acc[i][j] = fma2(a[i].y, w.y, fma2(a[i].x, w.x, acc[i][j]));
+                for (int i = 0; i < TM; ++i) acc[i][j] = fma2(a[i].y, w.y, q == 0 ? mul2(a[i].x, w.x) : fma2(a[i].x, w.x, acc[i][j]));
             }
         }
-        if ((kb - kb0) % kFlush == kFlush - 1 && kb + 1 < kb1) {
-#pragma unroll
-            for (int i = 0; i < TM; ++i)
-#pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    total[(i * 8 + j) * 64] = result(i, j);
-                    acc[i][j] = 0ull;
-                }
-            flushed = true;
-        }
-    }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    auto put = [&](int i, int j, float v) {
-        const int m = m0 + tm + 8 * i, n = n0 + tn + 8 * j;
-        if (m < g.M && n < g.N) {
-            float* d = g.D + (size_t)m * g.ldd + n;
-            *d = g.accumulate ? *d + v : v;
-        }
-    };
-    if (gridDim.z == 1) {
 #pragma unroll
         for (int i = 0; i < TM; ++i)
 #pragma unroll
-            for (int j = 0; j < 8; ++j) put(i, j, result(i, j));
+            for (int j = 0; j < 8; ++j) mid[i][j] = add2(mid[i][j], acc[i][j]);
+        if (kb % kUnit != kUnit - 1 && kb + 1 != blocks) continue;
+        const int u = kb / kUnit;
+#pragma unroll
+        for (int i = 0; i < TM; ++i)
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                const int at = (2 * i + q) * 128;
+                float4 v = make_float4(halves_sum(mid[i][4 * q]), halves_sum(mid[i][4 * q + 1]), halves_sum(mid[i][4 * q + 2]), halves_sum(mid[i][4 * q + 3]));
+#pragma unroll
+                for (int j = 0; j < 4; ++j) mid[i][4 * q + j] = 0ull;
+                if (split) { parts[(size_t)u * TILE4 + at] = v; continue; }
+                if (u % kGroup != 0) v = add4(group_sum[at], v);
+                if (u % kGroup != kGroup - 1 && u + 1 != units) group_sum[at] = v;
+                else total[at] = u < kGroup ? v : add4(total[at], v);
+            }
+    }
+    auto put4 = [&](int i, int q, float4 v) {
+        const float* e = &v.x;
+        const int m = m0 + tm + 16 * i;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int n = n0 + tn + 8 * (4 * q + j);
+            if (m < g.M && n < g.N) {
+                float* d = g.D + (size_t)m * g.ldd + n;
+                *d = g.accumulate ? *d + e[j] : e[j];
+            }
+        }
+    };
+    if (!split) {
+#pragma unroll
+        for (int i = 0; i < TM; ++i)
+#pragma unroll
+            for (int q = 0; q < 2; ++q) put4(i, q, total[(2 * i + q) * 128]);
         return;
     }
-    // K split: partial tiles to scratch, the last CTA of the tile to arrive adds them in the order of the splits
+    // the last CTA of the tile to arrive adds the units as above
     __shared__ int last;
-    const int tile = blockIdx.y * gridDim.x + blockIdx.x;
-    float* part = g.scratch + (size_t)tile * gridDim.z * (BM * kBN);
-    float* own = part + (size_t)blockIdx.z * (BM * kBN);
-#pragma unroll
-    for (int i = 0; i < TM; ++i)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) own[(i * 8 + j) * 64 + tid] = result(i, j);
     __threadfence();
     __syncthreads();
     if (tid == 0) {
@@ -128,20 +154,29 @@ __global__ void __launch_bounds__(64) row_gemm_kernel(RowGemmArgs g, int blocks_
     __syncthreads();
     if (!last) return;
     __threadfence();
-    float sum[TM][8];
+    float4 sum[TM][2];
+    for (int u0 = 0; u0 < units; u0 += kGroup) {
+        float4 grp[TM][2];
 #pragma unroll
-    for (int i = 0; i < TM; ++i)
+        for (int z = 0; z < kGroup; ++z) {
+            if (u0 + z >= units) break;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) sum[i][j] = 0.f;
-    for (int z = 0; z < (int)gridDim.z; ++z, part += BM * kBN)             // a split's values are all requested before any is added
+            for (int i = 0; i < TM; ++i)
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    const float4 v = __ldcg(parts + (size_t)(u0 + z) * TILE4 + (2 * i + q) * 128);
+                    grp[i][q] = z == 0 ? v : add4(grp[i][q], v);
+                }
+        }
 #pragma unroll
         for (int i = 0; i < TM; ++i)
 #pragma unroll
-            for (int j = 0; j < 8; ++j) sum[i][j] += __ldcg(part + (i * 8 + j) * 64 + tid);
+            for (int q = 0; q < 2; ++q) sum[i][q] = u0 == 0 ? grp[i][q] : add4(sum[i][q], grp[i][q]);
+    }
 #pragma unroll
     for (int i = 0; i < TM; ++i)
 #pragma unroll
-        for (int j = 0; j < 8; ++j) put(i, j, sum[i][j]);
+        for (int q = 0; q < 2; ++q) put4(i, q, sum[i][q]);
 }
 
 // ---- the recurrence over prompt rows --------------------------------------------------------------------------
@@ -290,29 +325,27 @@ __global__ void __launch_bounds__(128) ssm_rows_kernel(PrefillArgs a, float* y32
 
 template <int TM>
 cudaError_t row_gemm_launch(const RowGemmArgs& g, int splits, cudaStream_t st) {
-    const size_t smem = (size_t)(kStages * (8 * TM + kBN) * kPad + 8 * TM * kBN) * sizeof(float);      // at most 46 KiB
-    const int blocks = g.K / kBK, per = (blocks + splits - 1) / splits;
-    dim3 grid((g.N + kBN - 1) / kBN, (g.M + 8 * TM - 1) / (8 * TM), (blocks + per - 1) / per);
-    row_gemm_kernel<TM><<<grid, 64, smem, st>>>(g, per);
+    const cudaError_t e = cudaFuncSetAttribute(row_gemm_kernel<TM>, cudaFuncAttributeMaxDynamicSharedMemorySize, row_gemm_smem<TM>());
+    if (e != cudaSuccess) return e;
+    const int units = (g.K + kBK * kUnit - 1) / (kBK * kUnit), per = (units + splits - 1) / splits;
+    dim3 grid((g.N + kBN - 1) / kBN, (g.M + 16 * TM - 1) / (16 * TM), (units + per - 1) / per);
+    row_gemm_kernel<TM><<<grid, 128, row_gemm_smem<TM>(), st>>>(g, per);
     return cudaGetLastError();
 }
 
 }  // namespace
 
-bool row_gemm_supported(int K) { return K >= kBK && K % kBK == 0; }
+bool row_gemm_supported(int K) { return K >= 16 && K % 16 == 0; }
 
 cudaError_t launch_row_gemm(const RowGemmArgs& g, cudaStream_t st) {
     if (!row_gemm_supported(g.K) || g.lda % 4 != 0) return cudaErrorInvalidValue;
-    // 32-row tiles while they waste less than 64-row ones; K split until every SM has about four CTAs, each with at least
-    // 128 elements of K
+    // 32-row tiles while they waste less than 64-row ones; K split, unit by unit, until every SM has as many CTAs as fit it
     const bool narrow = g.M <= 32 || (g.M > 64 && g.M <= 96);
     const int bm = narrow ? 32 : 64;
-    const long tiles = (long)((g.M + bm - 1) / bm) * ((g.N + kBN - 1) / kBN);
-    long splits = std::min<long>(g.K / 128, 4 * 148 / tiles);
-    if (tiles > g.n_counters) splits = 1;
-    while (splits > 1 && (size_t)(tiles * splits) * bm * kBN > g.scratch_floats) --splits;
-    splits = std::max<long>(splits, 1);
-    return narrow ? row_gemm_launch<4>(g, (int)splits, st) : row_gemm_launch<8>(g, (int)splits, st);
+    const long tiles = (long)((g.M + bm - 1) / bm) * ((g.N + kBN - 1) / kBN), units = (g.K + kBK * kUnit - 1) / (kBK * kUnit);
+    long splits = std::max<long>(1, std::min<long>(units, (narrow ? 4 : 3) * 148 / tiles));
+    if (tiles > g.n_counters || (size_t)(tiles * units) * bm * kBN > g.scratch_floats) splits = 1;
+    return narrow ? row_gemm_launch<2>(g, (int)splits, st) : row_gemm_launch<4>(g, (int)splits, st);
 }
 
 #define LUMI_ROWS_SHAPES(X) X(32, 64) X(32, 16) X(32, 32) X(32, 128) X(16, 32) X(16, 64) X(16, 128) X(64, 16) X(64, 32) X(64, 64) X(64, 128)
