@@ -2076,6 +2076,7 @@ bool use_rows_prefill(const lumi_session* s, int batch, int T) {
     const Config& c = s->m->cfg;
     if (c.stacked() || s->opt_chunked_prefill <= 0 || T < 4 || s->m->n_mamba == 0 || !ssm_rows_supported(c.head_dim(), c.d_state)) return false;
     if (s->m->wdtype == LUMI_DTYPE_F32 && T < 8 && (long)batch * T < 12) return false;
+    if (s->m->wdtype == LUMI_DTYPE_BF16 && !use_tc(s, batch) && T < 6 && (long)batch * T < 10) return false;
     if (s->m->wdtype == LUMI_DTYPE_F32) return s->m->n_attn == 0 && row_gemm_supported(c.d_model) && row_gemm_supported(c.d_inner());
     if (s->opt_gemm == 1 || !use_tc(s, 9)) return false;
     for (const Layer& L : s->m->layers) if (L.is_attn && L.window > 0) return false;       // as for the chunked scan below
@@ -2202,56 +2203,63 @@ int32_t prefill_chunked(lumi_session* s, int batch, int T, bool with_head, float
     const Config& c = s->m->cfg;
     if (c.stacked()) return prefill_listed(s, batch, T, with_head, score_out, lens, slot0, want, want_out);
     const int D = c.d_model, DI = c.d_inner(), R = c.in_proj_out();
-    const bool hybrid = s->m->n_attn > 0, f32 = s->m->wdtype == LUMI_DTYPE_F32, scan = use_chunked_scan(s, T);
+    const bool hybrid = s->m->n_attn > 0, scan = use_chunked_scan(s, T);
+    // activations as bf16 halves on the tensor cores, or as they are: the scan takes halves, prompts in token order what the same sequences' steps take
+    const bool tc = scan || use_tc(s, batch);
     const int KVD = hybrid ? c.kv_dim() : 0, Q = D + 2 * KVD, MLP = hybrid ? c.mlp_dim() : 0;
     const size_t wproj = std::max<size_t>({(size_t)R, (size_t)Q, (size_t)2 * MLP});       // widest fp32 row of a projection
-    const size_t wact = std::max<size_t>({(size_t)DI, (size_t)D, (size_t)MLP});           // widest bf16 operand row
+    const size_t wact = std::max<size_t>({(size_t)DI, (size_t)D, (size_t)MLP});           // widest operand row
     const int nb_max = std::min(batch, 2048);
     int TS = std::max(64, (std::max(64, s->opt_prefill_rows) / nb_max) / 64 * 64);
     if (TS > T) TS = T;
     const size_t rows_max = (size_t)nb_max * TS;
+    const size_t rp = (rows_max + 127) / 128 * 128;
     if (rows_max > s->pf_rows) {
-        void* olds[] = {s->pf_x, s->pf_proj, s->pf_rb, s->pf_rc, s->pf_hi, s->pf_lo, s->pf_y};
+        void* olds[] = {s->pf_x, s->pf_proj, s->pf_rb, s->pf_rc};
         for (void* q : olds) if (q) LUMI_CUDA(cudaFree(q));
-        s->pf_x = s->pf_proj = s->pf_rb = s->pf_rc = s->pf_y = nullptr; s->pf_hi = s->pf_lo = nullptr; s->pf_rows = 0;
-        const size_t rp = (rows_max + 127) / 128 * 128;
+        s->pf_x = s->pf_proj = s->pf_rb = s->pf_rc = nullptr; s->pf_rows = 0;
         LUMI_CUDA(cudaMalloc(&s->pf_x, sizeof(float) * rp * D));
         LUMI_CUDA(cudaMalloc(&s->pf_proj, sizeof(float) * rp * wproj));
         LUMI_CUDA(cudaMalloc(&s->pf_rb, sizeof(float) * rp));
         LUMI_CUDA(cudaMalloc(&s->pf_rc, sizeof(float) * rp));
-        if (f32) {
-            LUMI_CUDA(cudaMalloc(&s->pf_y, sizeof(float) * rp * wact));
-        } else {
-            LUMI_CUDA(cudaMalloc(&s->pf_hi, sizeof(__nv_bfloat16) * rp * wact));
-            LUMI_CUDA(cudaMalloc(&s->pf_lo, sizeof(__nv_bfloat16) * rp * wact));
-        }
         // rows that a launch skips (padding behind a shorter prompt) keep what they held: make that finite from the start
         LUMI_CUDA(cudaMemsetAsync(s->pf_x, 0, sizeof(float) * rp * D, s->stream));
         LUMI_CUDA(cudaMemsetAsync(s->pf_proj, 0, sizeof(float) * rp * wproj, s->stream));
-        if (f32) {
-            LUMI_CUDA(cudaMemsetAsync(s->pf_y, 0, sizeof(float) * rp * wact, s->stream));
-        } else {
-            LUMI_CUDA(cudaMemsetAsync(s->pf_hi, 0, sizeof(__nv_bfloat16) * rp * wact, s->stream));
-            LUMI_CUDA(cudaMemsetAsync(s->pf_lo, 0, sizeof(__nv_bfloat16) * rp * wact, s->stream));
-        }
         s->pf_rows = rows_max;
     }
+    if (tc && rp * wact > s->pf_half_cap) {
+        if (s->pf_hi) LUMI_CUDA(cudaFree(s->pf_hi));
+        if (s->pf_lo) LUMI_CUDA(cudaFree(s->pf_lo));
+        s->pf_hi = s->pf_lo = nullptr; s->pf_half_cap = 0;
+        LUMI_CUDA(cudaMalloc(&s->pf_hi, sizeof(__nv_bfloat16) * rp * wact));
+        LUMI_CUDA(cudaMalloc(&s->pf_lo, sizeof(__nv_bfloat16) * rp * wact));
+        LUMI_CUDA(cudaMemsetAsync(s->pf_hi, 0, sizeof(__nv_bfloat16) * rp * wact, s->stream));
+        LUMI_CUDA(cudaMemsetAsync(s->pf_lo, 0, sizeof(__nv_bfloat16) * rp * wact, s->stream));
+        s->pf_half_cap = rp * wact;
+    }
+    if (!tc && rp * wact > s->pf_y_cap) {
+        LUMI_TRY(grow(s->pf_y, s->pf_y_cap, rp * wact));
+        LUMI_CUDA(cudaMemsetAsync(s->pf_y, 0, sizeof(float) * rp * wact, s->stream));
+    }
     const size_t B = s->max_batch;
-    __nv_bfloat16* lo = s->opt_split ? s->pf_lo : nullptr;
-    // bf16 models: a product of rows given as halves.  Few rows of short prompts split K over CTAs, which needs the session's counters;
+    __nv_bfloat16* const hi = tc ? s->pf_hi : nullptr;
+    __nv_bfloat16* const lo = tc && s->opt_split ? s->pf_lo : nullptr;
+    float* const y = tc ? nullptr : s->pf_y;
+    // the norm of `rows` rows of x, and the product of `rows` operand rows of width K from row r0 on.  Tensor cores: few rows of short prompts split K over CTAs, which needs the session's counters;
     // the chunked scan's products add in one order whatever the rows, so that a sequence gets the same angles alone and among others
-    auto product_tc = [&](const __nv_bfloat16* hi, const __nv_bfloat16* lo_, int K, const DevTensor& W, float* out, int rows, int N, int accumulate) {
-        GemmArgs g{hi, lo_, (const __nv_bfloat16*)W.p, out, N, rows, N, K, accumulate, &s->ctl->status, scan ? nullptr : s->gemm_counters, kGemmCounters,
-                   s->gemm_scratch, kGemmScratchFloats};
+    auto norm = [&](const float* gamma, int rows) {
+        if (tc) return launch_norm_split(s->pf_x, gamma, hi, lo, rows, D, c.eps, s->stream);
+        return launch_row_norm(RowNormArgs{s->pf_x, nullptr, gamma, y, nullptr, nullptr, nullptr, rows, D, D, c.eps, nullptr}, s->stream);
+    };
+    auto product = [&](int K, const DevTensor& W, float* out, int rows, int N, int accumulate, size_t r0 = 0) -> int32_t {
+        if (!tc) {
+            LUMI_CUDA(launch_row_gemm(RowGemmArgs{y + r0 * K, K, W.p, W.dtype, out, N, rows, N, K, accumulate, s->gemm_counters, kGemmCounters, s->gemm_scratch,
+                                                  2 * kGemmScratchFloats}, s->stream));
+            return LUMI_OK;
+        }
+        GemmArgs g{hi + r0 * K, lo ? lo + r0 * K : nullptr, (const __nv_bfloat16*)W.p, out, N, rows, N, K, accumulate, &s->ctl->status,
+                   scan ? nullptr : s->gemm_counters, kGemmCounters, s->gemm_scratch, kGemmScratchFloats};
         return launch_gemm_tcgen05(g, s->stream);
-    };
-    // fp32 models: the norm of `rows` rows of x into pf_y, and products of rows with fp32 weights
-    auto norm_rows = [&](const float* x, const float* gamma, int rows) {
-        return launch_row_norm(RowNormArgs{const_cast<float*>(x), nullptr, gamma, s->pf_y, nullptr, nullptr, nullptr, rows, D, D, c.eps, nullptr}, s->stream);
-    };
-    auto product_f32 = [&](const float* in, int K, const DevTensor& W, float* out, int rows, int N, int accumulate) {
-        return launch_row_gemm(RowGemmArgs{in, K, (const float*)W.p, out, N, rows, N, K, accumulate, s->gemm_counters, kGemmCounters, s->gemm_scratch,
-                                           2 * kGemmScratchFloats}, s->stream);
     };
     for (int b0 = 0; b0 < batch; b0 += nb_max) {
         const int nb = std::min(nb_max, batch - b0);
@@ -2266,8 +2274,8 @@ int32_t prefill_chunked(lumi_session* s, int batch, int T, bool with_head, float
                 if (L.is_attn) {
                     // AttentionBlock over all rows of the slice (model.rs:562-611 in forward_window's terms): q|k|v for every
                     // row, the slice's K/V appended to the cache, then every row attends to the cache up to its own position
-                    LUMI_CUDA(launch_norm_split(s->pf_x, L.a.attn_norm_g, s->pf_hi, lo, M, D, c.eps, s->stream));
-                    LUMI_TRY(product_tc(s->pf_hi, lo, D, L.a.qkv, s->pf_proj, M, Q, 0));
+                    LUMI_CUDA(norm(L.a.attn_norm_g, M));
+                    LUMI_TRY(product(D, L.a.qkv, s->pf_proj, M, Q, 0));
                     AttnArgs a{};
                     a.qkv = s->pf_proj; a.ldq = Q;
                     a.pool = (char*)s->kv_pool + l * s->kv_layer_bytes;
@@ -2275,7 +2283,7 @@ int32_t prefill_chunked(lumi_session* s, int batch, int T, bool with_head, float
                     a.kv_is_f32 = 0;
                     a.page_table = s->page_table; a.pages_per_seq = s->pages_per_seq;
                     a.pos = s->kv_pos;
-                    a.ctx32 = nullptr; a.chi = s->pf_hi; a.clo = lo;
+                    a.ctx32 = y; a.chi = hi; a.clo = lo;
                     a.B = M; a.n_heads = c.attn_n_heads; a.kv_heads = c.attn_kv_heads; a.head_dim = c.attn_head_dim();
                     a.window = 0; a.max_tokens = std::min(s->pages_per_seq * kPageTokens, s->max_tokens_kv);
                     a.rope_base = c.attn_rope_base;
@@ -2288,22 +2296,17 @@ int32_t prefill_chunked(lumi_session* s, int batch, int T, bool with_head, float
                         if (e == cudaErrorInvalidValue) return fail(LUMI_E_UNSUPPORTED, "attention head_dim %d with %d query heads per kv head is not built", a.head_dim, a.n_heads / a.kv_heads);
                         LUMI_CUDA(e);
                     }
-                    LUMI_TRY(product_tc(s->pf_hi, lo, D, L.a.o, s->pf_x, M, D, 1));
+                    LUMI_TRY(product(D, L.a.o, s->pf_x, M, D, 1));
                     // sigmoid-gated MLP (model.rs:546-555)
-                    LUMI_CUDA(launch_norm_split(s->pf_x, L.a.mlp_norm_g, s->pf_hi, lo, M, D, c.eps, s->stream));
-                    LUMI_TRY(product_tc(s->pf_hi, lo, D, L.a.gate_up, s->pf_proj, M, 2 * MLP, 0));
-                    LUMI_CUDA(launch_gate_mul(s->pf_proj, 2 * MLP, nullptr, s->pf_hi, lo, M, MLP, s->stream));
-                    LUMI_TRY(product_tc(s->pf_hi, lo, MLP, L.a.down, s->pf_x, M, D, 1));
+                    LUMI_CUDA(norm(L.a.mlp_norm_g, M));
+                    LUMI_TRY(product(D, L.a.gate_up, s->pf_proj, M, 2 * MLP, 0));
+                    LUMI_CUDA(launch_gate_mul(s->pf_proj, 2 * MLP, y, hi, lo, M, MLP, s->stream));
+                    LUMI_TRY(product(MLP, L.a.down, s->pf_x, M, D, 1));
                     s->launches += 10;
                     continue;
                 }
-                if (f32) {
-                    LUMI_CUDA(norm_rows(s->pf_x, L.m.norm_g, M));
-                    LUMI_CUDA(product_f32(s->pf_y, D, L.m.in_proj, s->pf_proj, M, R, 0));
-                } else {
-                    LUMI_CUDA(launch_norm_split(s->pf_x, L.m.norm_g, s->pf_hi, lo, M, D, c.eps, s->stream));
-                    LUMI_TRY(product_tc(s->pf_hi, lo, D, L.m.in_proj, s->pf_proj, M, R, 0));
-                }
+                LUMI_CUDA(norm(L.m.norm_g, M));
+                LUMI_TRY(product(D, L.m.in_proj, s->pf_proj, M, R, 0));
                 PrefillArgs a{};
                 a.proj = s->pf_proj; a.ldp = R;
                 a.bg = L.m.b_gamma; a.cg = L.m.c_gamma; a.bb = L.m.b_bias; a.cb = L.m.c_bias; a.dskip = L.m.d_skip; a.dtb = L.m.dt_bias;
@@ -2312,17 +2315,13 @@ int32_t prefill_chunked(lumi_session* s, int batch, int T, bool with_head, float
                 a.bprev = s->bprev + l * B * c.n_heads * c.d_state;
                 a.cum = s->cum + l * B * c.n_heads * (c.d_state / 2);
                 a.rb = s->pf_rb; a.rc = s->pf_rc;
-                a.yhi = s->pf_hi; a.ylo = lo;
+                a.yhi = hi; a.ylo = lo;
                 a.H = c.n_heads; a.G = c.n_groups; a.ts = ts; a.nb = nb; a.b0 = b0; a.eps = c.eps;
                 a.status = &s->ctl->status;
                 a.lens = lens; a.t_abs0 = t0;
                 if (scan) LUMI_CUDA(launch_prefill_scan(a, s->stream));
-                else LUMI_CUDA(launch_ssm_rows(a, c.head_dim(), c.d_state, s->pf_y, s->stream));
-                if (f32) {
-                    LUMI_CUDA(product_f32(s->pf_y, DI, L.m.out_proj, s->pf_x, M, D, 1));
-                } else {
-                    LUMI_TRY(product_tc(s->pf_hi, lo, DI, L.m.out_proj, s->pf_x, M, D, 1));
-                }
+                else LUMI_CUDA(launch_ssm_rows(a, c.head_dim(), c.d_state, y, s->stream));
+                LUMI_TRY(product(DI, L.m.out_proj, s->pf_x, M, D, 1));
                 s->launches += 5;
             }
             if (hybrid) {
@@ -2334,12 +2333,10 @@ int32_t prefill_chunked(lumi_session* s, int batch, int T, bool with_head, float
                 const int V = c.vocab;
                 const int SR = score_block_rows(V);
                 LUMI_TRY(grow(s->score_logits, s->score_logits_cap, (size_t)SR * V));
-                if (f32) LUMI_CUDA(norm_rows(s->pf_x, s->m->final_norm_g, M));
-                else LUMI_CUDA(launch_norm_split(s->pf_x, s->m->final_norm_g, s->pf_hi, lo, M, D, c.eps, s->stream));
+                LUMI_CUDA(norm(s->m->final_norm_g, M));
                 for (int r0 = 0; r0 < M; r0 += SR) {
                     const int nr = std::min(SR, M - r0);
-                    if (f32) LUMI_CUDA(product_f32(s->pf_y + (size_t)r0 * D, D, s->m->embedding, s->score_logits, nr, V, 0));
-                    else LUMI_TRY(product_tc(s->pf_hi + (size_t)r0 * D, lo ? lo + (size_t)r0 * D : nullptr, D, s->m->embedding, s->score_logits, nr, V, 0));
+                    LUMI_TRY(product(D, s->m->embedding, s->score_logits, nr, V, 0, (size_t)r0));
                     LUMI_CUDA(launch_logprob_rows(s->score_logits, nr, V, s->prompt_dev, batch, T, ts, t0, b0, r0, score_out, s->stream));
                     s->launches += 2;
                 }
@@ -2352,9 +2349,9 @@ int32_t prefill_chunked(lumi_session* s, int batch, int T, bool with_head, float
         }
     }
     if (with_head) {
-        StepPlan p{s, batch, !f32};
+        StepPlan p{s, batch, tc};
         p.st_hi = p.st_lo = s->stream;
-        if (!f32) LUMI_CUDA(launch_norm_split(s->x, s->m->final_norm_g, s->act_hi, s->opt_split ? s->act_lo : nullptr, batch, D, c.eps, s->stream));
+        if (tc) LUMI_CUDA(launch_norm_split(s->x, s->m->final_norm_g, s->act_hi, s->opt_split ? s->act_lo : nullptr, batch, D, c.eps, s->stream));
         p.fam = FAM_HEAD;
         LUMI_TRY(linear(p, s->m->embedding, s->x, D, s->logits, c.vocab, nullptr, s->m->final_norm_g, 0, c.vocab));
         LUMI_CUDA(launch_sample(s->logits, batch, c.vocab, s->ctl, s->tok_cur, s->finished, s->out_len, s->stream));
@@ -2970,10 +2967,10 @@ extern "C" int32_t lumi_debug_gemm_wait_timeout(uint64_t a_hi, uint64_t w, uint6
 extern "C" int32_t lumi_k_row_gemm(uint64_t a_f32, uint64_t w, int32_t w_dtype, uint64_t d, int32_t M, int32_t N, int32_t K, int32_t accumulate,
                                    uint64_t stream) {
     if (!a_f32 || !w || !d || M <= 0 || N <= 0 || K <= 0 || ((a_f32 | w) & 15)) return fail(LUMI_E_INVALID, "bad argument to lumi_k_row_gemm");
-    if (!row_gemm_supported(K) || w_dtype != LUMI_DTYPE_F32) return fail(LUMI_E_UNSUPPORTED, "a product of rows needs fp32 weights and K %% 16 == 0");
+    if (!row_gemm_supported(K)) return fail(LUMI_E_UNSUPPORTED, "a product of rows needs K %% 16 == 0");
     KernelScratch ks;
     LUMI_TRY(kernel_scratch(&ks));
-    LUMI_CUDA(launch_row_gemm(RowGemmArgs{(const float*)a_f32, K, (const float*)w, (float*)d, N, M, N, K, accumulate, ks.counters, ks.n_counters, ks.scratch,
+    LUMI_CUDA(launch_row_gemm(RowGemmArgs{(const float*)a_f32, K, (const void*)w, w_dtype, (float*)d, N, M, N, K, accumulate, ks.counters, ks.n_counters, ks.scratch,
                                           ks.floats}, (cudaStream_t)stream));
     return LUMI_OK;
 }

@@ -293,8 +293,8 @@ struct lumi_session {
     // chunked-prefill workspace (grow-only): residual rows, in_proj output, bf16 halves, BCNorm scales
     float *pf_x = nullptr, *pf_proj = nullptr, *pf_rb = nullptr, *pf_rc = nullptr;
     __nv_bfloat16 *pf_hi = nullptr, *pf_lo = nullptr;
-    float* pf_y = nullptr;            // fp32 models: normalised rows, then the state's read-outs
-    size_t pf_rows = 0;
+    float* pf_y = nullptr;            // products of fp32 rows: normalised rows, then the state's read-outs
+    size_t pf_rows = 0, pf_half_cap = 0, pf_y_cap = 0;       // rows of the arrays above, elements of the halves and of pf_y
     // options
     int opt_gemm = 0, opt_split = 1, opt_graph = 1, opt_pdl = 1, opt_mega = 0;
     // greedy head with the argmax fused behind the lm_head GEMV (batch <= 8): set by the caller of a step that wants
@@ -603,11 +603,11 @@ cudaError_t launch_bc_stats(const PrefillArgs& a, int P, int N, cudaStream_t st)
 // prompt length.  y32 (may be null): [nb * ts][heads * P] fp32 beside or in place of yhi / ylo.
 bool ssm_rows_supported(int P, int N);
 cudaError_t launch_ssm_rows(const PrefillArgs& a, int P, int N, float* y32, cudaStream_t st);
-// D[M][N] (+)= A[M][K] W[N][K]^T in fp32 on the CUDA cores, for many rows (prefill_rows.cu).  K % 16 == 0, lda % 4 == 0.  counters (zeroed
+// D[M][N] (+)= A[M][K] W[N][K]^T in fp32 on the CUDA cores, for many rows (prefill_rows.cu).  K % 16 == 0, lda % 4 == 0, 16-byte aligned operands.  counters (zeroed
 // ints, left zeroed) and scratch serve the split of K.
 struct RowGemmArgs {
     const float* A; int lda;
-    const float* W;
+    const void* W; int w_dtype;          // LUMI_DTYPE_*
     float* D; int ldd;
     int M, N, K;
     int accumulate;

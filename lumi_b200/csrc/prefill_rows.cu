@@ -12,8 +12,8 @@
 namespace lumi {
 namespace {
 
-// ---- fp32 product over rows ---------------------------------------------------------------------------------
-// D[M][N] (+)= A[M][K] W[N][K]^T on the CUDA cores, fp32 throughout.  A CTA of 128 threads owns BM x 64 results and, with K split
+// ---- product over rows with fp32 activations ---------------------------------------------------------------
+// D[M][N] (+)= A[M][K] W[N][K]^T on the CUDA cores, fp32 throughout (bf16 weights are widened).  A CTA of 128 threads owns BM x 64 results and, with K split
 // over blockIdx.z, part of the sum; a thread owns TM x 8 of them, rows sixteen and columns eight apart, so that the eight columns that a
 // quarter warp reads lie in eight different bank groups (rows of 32 + 4 padding floats).  Even and odd k are summed apart in
 // the two halves of packed multiply-adds (fma.rn.f32x2): operands come as 16-byte loads along K as they are stored, with no
@@ -48,13 +48,26 @@ __device__ __forceinline__ void copy16(void* dst, const void* src, int bytes) { 
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(bytes) : "memory");
 }
 
-template <int TM>
-constexpr int row_gemm_smem() { return (kStages * (16 * TM + kBN) * kPad + 2 * 16 * TM * kBN) * (int)sizeof(float); }      // TM 4: 68 KiB, three CTAs per SM
+// four consecutive weights of a staged row as two packed pairs
+__device__ __forceinline__ ulonglong2 weights4(const float* w) { return *reinterpret_cast<const ulonglong2*>(w); }
+__device__ __forceinline__ ulonglong2 weights4(const __nv_bfloat16* w) {
+    const uint2 v = *reinterpret_cast<const uint2*>(w);
+    auto pair = [](uint32_t two) { return (uint64_t)(two & 0xffff0000u) << 32 | (uint64_t)(two << 16); };
+    return make_ulonglong2(pair(v.x), pair(v.y));
+}
 
-template <int TM>
+template <int TM, typename WT>
+struct RowTile {
+    static constexpr int BM = 16 * TM, E = 16 / (int)sizeof(WT), W_PITCH = kBK + E;      // rows of weights: 32 and one 16-byte piece
+    static constexpr int A_BYTES = BM * kPad * 4, STAGE = A_BYTES + kBN * W_PITCH * (int)sizeof(WT);
+    static constexpr int SMEM = kStages * STAGE + 2 * BM * kBN * 4;        // TM 4: 68 KiB, with bf16 weights 60: three CTAs per SM
+};
+
+template <int TM, typename WT>
 __global__ void __launch_bounds__(128, TM == 4 ? 3 : 4) row_gemm_kernel(RowGemmArgs g, int units_per_split) {
-    constexpr int BM = 16 * TM, ROWS = BM + kBN, TILE4 = BM * kBN / 4;
-    extern __shared__ __align__(16) float sm[];                            // [stage][A rows, then W rows][kPad], the group's sums, the sums of the groups before
+    using T = RowTile<TM, WT>;
+    constexpr int BM = T::BM, E = T::E, TILE4 = BM * kBN / 4;
+    extern __shared__ __align__(16) unsigned char sm[];                    // [stage][A rows, then W rows], the group's sums, the sums of the groups before
     const int tid = threadIdx.x, tn = tid & 7, tm = tid >> 3;
     const int n0 = blockIdx.x * kBN, m0 = blockIdx.y * BM;
     const int blocks = (g.K + kBK - 1) / kBK, units = (blocks + kUnit - 1) / kUnit;
@@ -62,17 +75,21 @@ __global__ void __launch_bounds__(128, TM == 4 ? 3 : 4) row_gemm_kernel(RowGemmA
     const bool split = gridDim.z > 1;
     // this thread copies 16 bytes at column cq of every sixteenth row; rows past the end read the last one: never stored
     const int cq = 4 * (tid & 7), crow = tid >> 3, a_end = g.M - 1 - m0, w_end = g.N - 1 - n0;
-    const float *const a0 = g.A + (size_t)m0 * g.lda + cq, *const w0 = g.W + (size_t)n0 * g.K + cq;
+    constexpr int WQ = kBK / E, WSTEP = 128 / WQ;                          // the same for the weights: pieces per row, rows per turn
+    const int wq = E * (tid % WQ), wrow = tid / WQ;
+    const float* const a0 = g.A + (size_t)m0 * g.lda + cq;
+    const WT* const w0 = static_cast<const WT*>(g.W) + (size_t)n0 * g.K + wq;
     auto stage = [&](int kb) {
         if (kb < kb1) {
-            float* s = sm + (kb & 1) * ROWS * kPad + crow * kPad + cq;
-            const bool in = kb * kBK + cq < g.K;                           // K is a multiple of 16: the last block may be half zeros
-            const int k = in ? kb * kBK : 0, bytes = in ? 16 : 0;
+            unsigned char* s = sm + (kb & 1) * T::STAGE;
+            float* sa = reinterpret_cast<float*>(s) + crow * kPad + cq;
+            WT* sw = reinterpret_cast<WT*>(s + T::A_BYTES) + wrow * T::W_PITCH + wq;
+            const bool ain = kb * kBK + cq < g.K, win = kb * kBK + wq < g.K;      // K is a multiple of 16: the last block may be half zeros
 #pragma unroll
-            for (int c = 0; c < ROWS / 16; ++c) {
-                const int row = crow + 16 * c;
-                copy16(s + 16 * c * kPad, 16 * c < BM ? a0 + min(row, a_end) * g.lda + k : w0 + min(row - BM, w_end) * g.K + k, bytes);
-            }
+            for (int c = 0; c < BM / 16; ++c) copy16(sa + 16 * c * kPad, a0 + min(crow + 16 * c, a_end) * g.lda + (ain ? kb * kBK : 0), ain ? 16 : 0);
+#pragma unroll
+            for (int c = 0; c < kBN / WSTEP; ++c)
+                copy16(sw + WSTEP * c * T::W_PITCH, w0 + min(wrow + WSTEP * c, w_end) * g.K + (win ? kb * kBK : 0), win ? 16 : 0);
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
@@ -81,7 +98,7 @@ __global__ void __launch_bounds__(128, TM == 4 ? 3 : 4) row_gemm_kernel(RowGemmA
     for (int i = 0; i < TM; ++i)
 #pragma unroll
         for (int j = 0; j < 8; ++j) mid[i][j] = 0ull;
-    float4* const group_sum = reinterpret_cast<float4*>(sm + kStages * ROWS * kPad) + tid;      // this thread's results four by four, 128 apart
+    float4* const group_sum = reinterpret_cast<float4*>(sm + kStages * T::STAGE) + tid;      // this thread's results four by four, 128 apart
     float4* const total = group_sum + TILE4;
     const int tile = blockIdx.y * gridDim.x + blockIdx.x;
     float4* const parts = reinterpret_cast<float4*>(g.scratch) + (size_t)tile * units * TILE4 + tid;      // K split: the units' sums
@@ -90,16 +107,17 @@ __global__ void __launch_bounds__(128, TM == 4 ? 3 : 4) row_gemm_kernel(RowGemmA
         asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncthreads();                                                   // the block has landed, and the one before it is no longer read
         stage(kb + 1);
-        const float* s = sm + (kb & 1) * ROWS * kPad;
+        const float* sa = reinterpret_cast<const float*>(sm + (kb & 1) * T::STAGE) + tm * kPad;
+        const WT* sw = reinterpret_cast<const WT*>(sm + (kb & 1) * T::STAGE + T::A_BYTES) + tn * T::W_PITCH;
         uint64_t acc[TM][8];
 #pragma unroll
         for (int q = 0; q < kBK / 4; ++q) {
             ulonglong2 a[TM];
 #pragma unroll
-            for (int i = 0; i < TM; ++i) a[i] = *reinterpret_cast<const ulonglong2*>(s + (tm + 16 * i) * kPad + 4 * q);
+            for (int i = 0; i < TM; ++i) a[i] = *reinterpret_cast<const ulonglong2*>(sa + 16 * i * kPad + 4 * q);
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
-                const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(s + (BM + tn + 8 * j) * kPad + 4 * q);
+                const ulonglong2 w = weights4(sw + 8 * j * T::W_PITCH + 4 * q);
 #pragma unroll
                 for (int i = 0; i < TM; ++i) acc[i][j] = fma2(a[i].y, w.y, q == 0 ? mul2(a[i].x, w.x) : fma2(a[i].x, w.x, acc[i][j]));
             }
@@ -323,13 +341,14 @@ __global__ void __launch_bounds__(128) ssm_rows_kernel(PrefillArgs a, float* y32
     if (tid < HN) a.cum[bh * HN + tid] = cu;
 }
 
-template <int TM>
+template <int TM, typename WT>
 cudaError_t row_gemm_launch(const RowGemmArgs& g, int splits, cudaStream_t st) {
-    const cudaError_t e = cudaFuncSetAttribute(row_gemm_kernel<TM>, cudaFuncAttributeMaxDynamicSharedMemorySize, row_gemm_smem<TM>());
+    using T = RowTile<TM, WT>;
+    const cudaError_t e = cudaFuncSetAttribute(row_gemm_kernel<TM, WT>, cudaFuncAttributeMaxDynamicSharedMemorySize, T::SMEM);
     if (e != cudaSuccess) return e;
     const int units = (g.K + kBK * kUnit - 1) / (kBK * kUnit), per = (units + splits - 1) / splits;
     dim3 grid((g.N + kBN - 1) / kBN, (g.M + 16 * TM - 1) / (16 * TM), (units + per - 1) / per);
-    row_gemm_kernel<TM><<<grid, 128, row_gemm_smem<TM>(), st>>>(g, per);
+    row_gemm_kernel<TM, WT><<<grid, 128, T::SMEM, st>>>(g, per);
     return cudaGetLastError();
 }
 
@@ -345,7 +364,8 @@ cudaError_t launch_row_gemm(const RowGemmArgs& g, cudaStream_t st) {
     const long tiles = (long)((g.M + bm - 1) / bm) * ((g.N + kBN - 1) / kBN), units = (g.K + kBK * kUnit - 1) / (kBK * kUnit);
     long splits = std::max<long>(1, std::min<long>(units, (narrow ? 4 : 3) * 148 / tiles));
     if (tiles > g.n_counters || (size_t)(tiles * units) * bm * kBN > g.scratch_floats) splits = 1;
-    return narrow ? row_gemm_launch<2>(g, (int)splits, st) : row_gemm_launch<4>(g, (int)splits, st);
+    if (g.w_dtype == LUMI_DTYPE_BF16) return narrow ? row_gemm_launch<2, __nv_bfloat16>(g, (int)splits, st) : row_gemm_launch<4, __nv_bfloat16>(g, (int)splits, st);
+    return narrow ? row_gemm_launch<2, float>(g, (int)splits, st) : row_gemm_launch<4, float>(g, (int)splits, st);
 }
 
 #define LUMI_ROWS_SHAPES(X) X(32, 64) X(32, 16) X(32, 32) X(32, 128) X(16, 32) X(16, 64) X(16, 128) X(64, 16) X(64, 32) X(64, 64) X(64, 128)

@@ -23,7 +23,7 @@ def operands(M, N, K, wdt="f32"):
     return torch.randn((M, K), generator=g, device="cuda"), w.to(torch.bfloat16) if wdt == "bf16" else w
 
 
-WEIGHTS = ["f32"]
+WEIGHTS = ["f32", "bf16"]
 
 
 # edges: tiles of 32 and 64 rows and 64 columns; K of one block, of an odd count, of less than a unit of 128, of a short last unit; K split and in one piece

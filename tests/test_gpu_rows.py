@@ -89,6 +89,23 @@ def test_short_prompts_with_attention_layers(T):
     assert rel(rows.forward_step(prompts[:, 0])[0], steps.forward_step(prompts[:, 0])[0]) < 2e-3
 
 
+# up to eight bf16 sequences take fp32 activations token by token, and have to as prompts: two bf16 halves (2^-17 of each factor, 8e-6) would show
+# against sums in another order (at most 512 products, 512 * 2^-24 = 3e-5 at the very worst, a tenth of it in practice)
+@pytest.mark.parametrize("batch,T", [(1, 6), (1, 90), (3, 33), (8, 20)])
+@pytest.mark.parametrize("split", [1, 0])
+def test_few_bf16_sequences_keep_fp32_activations(batch, T, split):
+    cfg = synth.tiny_config(n_layers=3)
+    _, _, rows, steps = pair(cfg, "bf16", batch)
+    for s in (rows, steps):
+        s.set_option("split_activations", split)
+    prompts = synth.random_prompts(batch, T, cfg.vocab_size, seed=T)
+    a, b = rows.prefill(prompts), steps.prefill(prompts)
+    assert rel(a, b) < 3e-6
+    rows.reset(), steps.reset()
+    a, b = rows.score(prompts), steps.score(prompts)
+    assert np.abs(a - b).max() < 3e-6 * np.abs(b).max()
+
+
 # a slice's rows count from the prompt's first token, the cache from the sequence's: first prompts of different lengths, so that the two differ by
 # another amount in every sequence; lengths of one token, of the longest, around a slice of 64; tensor-core and CUDA-core attention
 @pytest.mark.parametrize("kv_heads,heads", [(4, 16), (8, 32)])
