@@ -205,7 +205,7 @@ __device__ __forceinline__ float silu_ref(float x) { return __fdiv_rn(x, __fadd_
 
 constexpr int kTok = 16;             // tokens taken through the pointwise part at a time
 template <int P, int N>
-struct RowsSmem {
+struct alignas(16) RowsSmem {          // B~ and C~ are read sixteen bytes at a time
     float bt[kTok][N], ct[kTok][N], xa[kTok][P], gate[kTok][P], yo[kTok][P], ang[kTok][N / 2];
     float dtp[kTok], abar[kTok], lam[kTok], c2[kTok], rb[kTok], rc[kTok];
 };

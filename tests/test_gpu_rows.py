@@ -34,6 +34,21 @@ def same_state(rows, steps, b, layer, tol):
 TOL = {"f32": 3e-5, "bf16": 2e-4}
 
 
+# Without this the comparisons below could hold steps against steps.  A step is at least four launches per layer and token, a pass five per layer.
+@pytest.mark.parametrize("dtype,batch,T,kw,taken", [
+    ("f32", 1, 4, {}, False), ("f32", 1, 8, {}, True), ("f32", 3, 4, {}, True), ("f32", 13, 5, {}, True), ("f32", 4, 40, dict(n_heads=16, d_state=16), False),
+    ("f32", 4, 40, dict(n_heads=16, d_state=32), True), ("f32", 4, 40, dict(n_heads=4, d_state=128), True), ("f32", 4, 40, dict(attention_interval=2), False),
+    ("bf16", 1, 4, {}, False), ("bf16", 1, 6, {}, True), ("bf16", 3, 4, {}, True), ("bf16", 13, 4, {}, True), ("bf16", 13, 3, {}, False),
+    ("bf16", 2, 5, dict(attention_interval=2, attn_rope_base=10000.0), True)])
+def test_which_prompts_go_a_layer_at_a_time(dtype, batch, T, kw, taken):
+    cfg = synth.tiny_config(**{**dict(n_layers=3), **kw})
+    _, _, rows, steps = pair(cfg, dtype, batch)
+    prompts = synth.random_prompts(batch, T, cfg.vocab_size, seed=T)
+    launches = [s.generate(prompts, 1, ignore_eos=True)[3].kernel_launches for s in (rows, steps)]
+    assert (launches[0] < launches[1]) == taken, launches
+    assert taken or launches[0] == launches[1]
+
+
 # tokens around the sixteen that are taken at a time, rows around the tiles of 32 and 64, K split and not
 @pytest.mark.parametrize("dtype", ["f32", "bf16"])
 @pytest.mark.parametrize("batch,T", [(1, 4), (1, 15), (1, 16), (1, 17), (1, 33), (2, 32), (3, 22), (5, 65), (13, 5), (20, 33)])
