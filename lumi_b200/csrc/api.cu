@@ -2088,8 +2088,78 @@ int score_block_rows(int V) {
     return (int)std::min<size_t>(4096, std::max<size_t>(128, ((size_t)256 << 20) / ((size_t)V * sizeof(float)) / 128 * 128));
 }
 
+// A pass of prefill_chunked: its sequences and tokens per sequence, and whether activations go as bf16 halves on the tensor cores or as they are (the
+// scan takes halves, prompts in token order what the same sequences' steps take).
+struct PrefillPass { int nb, ts; bool scan, tc; size_t rows() const { return (size_t)nb * ts; } };
+PrefillPass prefill_pass(const lumi_session* s, int batch, int T, int rows_per_pass) {
+    const bool scan = use_chunked_scan(s, T);
+    if (scan) {
+        const int nb = std::min(batch, 2048);
+        return {nb, std::min(T, std::max(64, (std::max(64, rows_per_pass) / nb) / 64 * 64)), true, true};
+    }
+    const int ts = std::min(T, rows_per_pass);                          // whole prompts of as many sequences as fit
+    return {std::min(batch, std::max(1, rows_per_pass / ts)), ts, false, use_tc(s, batch)};
+}
+
+// Room for the passes of prefill_chunked (grow-only); `scored`: for the logits of a block of rows as well.
+int32_t prefill_workspace(lumi_session* s, const PrefillPass& ps, bool scored) {
+    const Config& c = s->m->cfg;
+    const size_t D = c.d_model, DI = c.d_inner();
+    const bool hybrid = s->m->n_attn > 0;
+    const size_t wproj = std::max<size_t>({(size_t)c.in_proj_out(), hybrid ? D + 2 * c.kv_dim() : 0, hybrid ? (size_t)2 * c.mlp_dim() : 0});       // widest fp32 row of a projection
+    const size_t wact = std::max<size_t>({DI, D, hybrid ? (size_t)c.mlp_dim() : 0});                                                    // widest operand row
+    const size_t rp = (ps.rows() + 127) / 128 * 128;
+    if (ps.rows() > s->pf_rows) {
+        void* olds[] = {s->pf_x, s->pf_proj, s->pf_rb, s->pf_rc};
+        s->pf_x = s->pf_proj = s->pf_rb = s->pf_rc = nullptr; s->pf_rows = 0;
+        for (void* q : olds) if (q) LUMI_CUDA(cudaFree(q));
+        LUMI_CUDA(cudaMalloc(&s->pf_x, sizeof(float) * rp * D));
+        LUMI_CUDA(cudaMalloc(&s->pf_proj, sizeof(float) * rp * wproj));
+        LUMI_CUDA(cudaMalloc(&s->pf_rb, sizeof(float) * rp));
+        LUMI_CUDA(cudaMalloc(&s->pf_rc, sizeof(float) * rp));
+        // rows that a launch skips (padding behind a shorter prompt) keep what they held: make that finite from the start
+        LUMI_CUDA(cudaMemsetAsync(s->pf_x, 0, sizeof(float) * rp * D, s->stream));
+        LUMI_CUDA(cudaMemsetAsync(s->pf_proj, 0, sizeof(float) * rp * wproj, s->stream));
+        s->pf_rows = ps.rows();
+    }
+    if (ps.tc && rp * wact > s->pf_half_cap) {
+        void* olds[] = {s->pf_hi, s->pf_lo};
+        s->pf_hi = s->pf_lo = nullptr; s->pf_half_cap = 0;
+        for (void* q : olds) if (q) LUMI_CUDA(cudaFree(q));
+        LUMI_CUDA(cudaMalloc(&s->pf_hi, sizeof(__nv_bfloat16) * rp * wact));
+        LUMI_CUDA(cudaMalloc(&s->pf_lo, sizeof(__nv_bfloat16) * rp * wact));
+        LUMI_CUDA(cudaMemsetAsync(s->pf_hi, 0, sizeof(__nv_bfloat16) * rp * wact, s->stream));
+        LUMI_CUDA(cudaMemsetAsync(s->pf_lo, 0, sizeof(__nv_bfloat16) * rp * wact, s->stream));
+        s->pf_half_cap = rp * wact;
+    }
+    if (!ps.tc && rp * wact > s->pf_y_cap) {
+        LUMI_TRY(grow(s->pf_y, s->pf_y_cap, rp * wact));
+        LUMI_CUDA(cudaMemsetAsync(s->pf_y, 0, sizeof(float) * rp * wact, s->stream));
+    }
+    if (scored) LUMI_TRY(grow(s->score_logits, s->score_logits_cap, std::min<size_t>(score_block_rows(c.vocab), rp) * c.vocab));
+    return LUMI_OK;
+}
+
+// Prompts in token order need no workspace as steps, and must not fail for want of it: their passes are of 16384 rows at most (41 KB each for the
+// base model), take half as many rows while there is no room for them, and without room for 512 the prompt goes token by token.  Where the
+// bound lies: 160 hybrid sequences of 100 tokens 91.2 ms in one pass, 95.0 in two of 8192 rows; 256 of 40 73.4 and 74.5.
+constexpr int kRowsPass = 16384, kRowsPassMin = 512;
+bool rows_workspace(lumi_session* s, int batch, int T, bool scored) {
+    for (int rows = std::min(kRowsPass, std::max(64, s->opt_prefill_rows));; rows /= 2) {
+        if (prefill_workspace(s, prefill_pass(s, batch, T, rows), scored) == LUMI_OK) {
+            s->pf_pass = rows;
+            return true;
+        }
+        cudaGetLastError();                                             // no room: not this call's error
+        if (rows / 2 < kRowsPassMin) return false;
+    }
+}
+
 // Prompts that prefill_chunked takes, in either form.
-bool use_chunked_prefill(const lumi_session* s, int batch, int T) { return use_chunked_scan(s, T) || use_rows_prefill(s, batch, T); }
+bool use_chunked_prefill(lumi_session* s, int batch, int T, bool scored = false) {
+    if (use_chunked_scan(s, T)) { s->pf_pass = s->opt_prefill_rows; return true; }
+    return use_rows_prefill(s, batch, T) && rows_workspace(s, batch, T, scored);
+}
 
 // The slice loop for designs that list their layers: slices of up to slice_max tokens per sequence, each through every layer
 // with the caches and states carried from slice to slice.  Arguments as for prefill_chunked.
@@ -2203,44 +2273,12 @@ int32_t prefill_chunked(lumi_session* s, int batch, int T, bool with_head, float
     const Config& c = s->m->cfg;
     if (c.stacked()) return prefill_listed(s, batch, T, with_head, score_out, lens, slot0, want, want_out);
     const int D = c.d_model, DI = c.d_inner(), R = c.in_proj_out();
-    const bool hybrid = s->m->n_attn > 0, scan = use_chunked_scan(s, T);
-    // activations as bf16 halves on the tensor cores, or as they are: the scan takes halves, prompts in token order what the same sequences' steps take
-    const bool tc = scan || use_tc(s, batch);
+    const bool hybrid = s->m->n_attn > 0;
+    const PrefillPass ps = prefill_pass(s, batch, T, s->pf_pass);
+    const bool scan = ps.scan, tc = ps.tc;
     const int KVD = hybrid ? c.kv_dim() : 0, Q = D + 2 * KVD, MLP = hybrid ? c.mlp_dim() : 0;
-    const size_t wproj = std::max<size_t>({(size_t)R, (size_t)Q, (size_t)2 * MLP});       // widest fp32 row of a projection
-    const size_t wact = std::max<size_t>({(size_t)DI, (size_t)D, (size_t)MLP});           // widest operand row
-    const int nb_max = std::min(batch, 2048);
-    int TS = std::max(64, (std::max(64, s->opt_prefill_rows) / nb_max) / 64 * 64);
-    if (TS > T) TS = T;
-    const size_t rows_max = (size_t)nb_max * TS;
-    const size_t rp = (rows_max + 127) / 128 * 128;
-    if (rows_max > s->pf_rows) {
-        void* olds[] = {s->pf_x, s->pf_proj, s->pf_rb, s->pf_rc};
-        for (void* q : olds) if (q) LUMI_CUDA(cudaFree(q));
-        s->pf_x = s->pf_proj = s->pf_rb = s->pf_rc = nullptr; s->pf_rows = 0;
-        LUMI_CUDA(cudaMalloc(&s->pf_x, sizeof(float) * rp * D));
-        LUMI_CUDA(cudaMalloc(&s->pf_proj, sizeof(float) * rp * wproj));
-        LUMI_CUDA(cudaMalloc(&s->pf_rb, sizeof(float) * rp));
-        LUMI_CUDA(cudaMalloc(&s->pf_rc, sizeof(float) * rp));
-        // rows that a launch skips (padding behind a shorter prompt) keep what they held: make that finite from the start
-        LUMI_CUDA(cudaMemsetAsync(s->pf_x, 0, sizeof(float) * rp * D, s->stream));
-        LUMI_CUDA(cudaMemsetAsync(s->pf_proj, 0, sizeof(float) * rp * wproj, s->stream));
-        s->pf_rows = rows_max;
-    }
-    if (tc && rp * wact > s->pf_half_cap) {
-        if (s->pf_hi) LUMI_CUDA(cudaFree(s->pf_hi));
-        if (s->pf_lo) LUMI_CUDA(cudaFree(s->pf_lo));
-        s->pf_hi = s->pf_lo = nullptr; s->pf_half_cap = 0;
-        LUMI_CUDA(cudaMalloc(&s->pf_hi, sizeof(__nv_bfloat16) * rp * wact));
-        LUMI_CUDA(cudaMalloc(&s->pf_lo, sizeof(__nv_bfloat16) * rp * wact));
-        LUMI_CUDA(cudaMemsetAsync(s->pf_hi, 0, sizeof(__nv_bfloat16) * rp * wact, s->stream));
-        LUMI_CUDA(cudaMemsetAsync(s->pf_lo, 0, sizeof(__nv_bfloat16) * rp * wact, s->stream));
-        s->pf_half_cap = rp * wact;
-    }
-    if (!tc && rp * wact > s->pf_y_cap) {
-        LUMI_TRY(grow(s->pf_y, s->pf_y_cap, rp * wact));
-        LUMI_CUDA(cudaMemsetAsync(s->pf_y, 0, sizeof(float) * rp * wact, s->stream));
-    }
+    const int nb_max = ps.nb, TS = ps.ts;
+    LUMI_TRY(prefill_workspace(s, ps, score_out != nullptr));
     const size_t B = s->max_batch;
     __nv_bfloat16* const hi = tc ? s->pf_hi : nullptr;
     __nv_bfloat16* const lo = tc && s->opt_split ? s->pf_lo : nullptr;
@@ -2332,7 +2370,6 @@ int32_t prefill_chunked(lumi_session* s, int batch, int T, bool with_head, float
                 // final norm + tied head over the rows of the slice, a block of rows at a time, then log-softmax at the target
                 const int V = c.vocab;
                 const int SR = score_block_rows(V);
-                LUMI_TRY(grow(s->score_logits, s->score_logits_cap, (size_t)SR * V));
                 LUMI_CUDA(norm(s->m->final_norm_g, M));
                 for (int r0 = 0; r0 < M; r0 += SR) {
                     const int nr = std::min(SR, M - r0);
@@ -2546,7 +2583,7 @@ extern "C" int32_t lumi_score(lumi_session* s, const uint32_t* tokens, int32_t b
     s->ctl_host->prompt = s->prompt_dev;
     s->ctl_host->prompt_len = T;
     s->ctl_host->ignore_eos = 1;
-    const bool chunked = use_chunked_prefill(s, batch, T);
+    const bool chunked = use_chunked_prefill(s, batch, T, true);
     if (chunked) s->ctl_host->prompt_pos = T;          // the batched path consumes the whole prompt itself
     LUMI_TRY(push_ctl(s));
     if (chunked) {

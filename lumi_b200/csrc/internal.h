@@ -294,6 +294,7 @@ struct lumi_session {
     float *pf_x = nullptr, *pf_proj = nullptr, *pf_rb = nullptr, *pf_rc = nullptr;
     __nv_bfloat16 *pf_hi = nullptr, *pf_lo = nullptr;
     float* pf_y = nullptr;            // products of fp32 rows: normalised rows, then the state's read-outs
+    int pf_pass = 0;                  // rows per pass, as far as there was room
     size_t pf_rows = 0, pf_half_cap = 0, pf_y_cap = 0;       // rows of the arrays above, elements of the halves and of pf_y
     // options
     int opt_gemm = 0, opt_split = 1, opt_graph = 1, opt_pdl = 1, opt_mega = 0;

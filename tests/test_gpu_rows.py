@@ -139,3 +139,36 @@ def test_ragged_prompts_behind_earlier_tokens(T, kv_heads, heads):
         a, b = (s.forward_step(second[:, i], step=i)[0] for s in (rows, steps))
         for j in range(4):
             assert rel(a[j], b[j]) < 2e-3, (i, j)
+
+
+# 16 x 160 rows of 41 KB: in one pass with room for it, in smaller passes, and token by token without room for the smallest (512 rows, 21 MB)
+@pytest.mark.parametrize("op", ["prefill", "score"])
+@pytest.mark.parametrize("left_mb,fits", [(None, True), (64, True), (12, False)])
+def test_prompts_where_there_is_little_memory(op, left_mb, fits):
+    import torch
+    cfg = synth.base_config(n_layers=2, vocab_size=500)
+    tens = list(synth.iter_tensors(cfg, seed=3, weights_dtype="f32", perturb_ones=0.1))
+    model = lumi_b200.NmModel.from_tensors(cfg, tens)
+    warm, rows, steps = (model.init_states(16, 256) for _ in range(3))
+    steps.set_option("chunked_prefill", 0)
+    rows.set_option("graph", 0)                              # captured graphs take memory of their own
+    prompts = synth.random_prompts(16, 160, cfg.vocab_size, seed=5)
+    want = getattr(steps, op)(prompts)
+    getattr(warm, op)(prompts)                               # every kernel is loaded
+    warm.close()
+    hold = []
+    try:
+        if left_mb is not None:                              # blocks of 32 MB and more come straight from the device
+            spare = torch.cuda.mem_get_info()[0] - (left_mb << 20)
+            hold = [torch.empty(1 << 30, dtype=torch.uint8, device="cuda") for _ in range((spare >> 30) - 1)]
+            spare = torch.cuda.mem_get_info()[0] - (left_mb << 20)
+            hold.append(torch.empty(spare >> 21 << 21, dtype=torch.uint8, device="cuda"))
+        got = getattr(rows, op)(prompts)
+    finally:
+        del hold
+        torch.cuda.empty_cache()
+    if fits:
+        assert rel(got, want) < TOL["f32"] * (10 if op == "score" else 1)
+    else:
+        assert np.array_equal(got, want)
+    assert rel(rows.forward_step(prompts[:, 0])[0], steps.forward_step(prompts[:, 0])[0]) < TOL["f32"]
