@@ -1144,6 +1144,7 @@ int32_t linear(StepPlan& p, const DevTensor& W, const float* in32, int K, float*
         g.nf.gamma_next = gamma_next; g.nf.out_hi = s->xn_hi + xoff; g.nf.out_lo = s->opt_split ? s->xn_lo + xoff : nullptr;
         g.nf.ssq_out = s->ssq + soff; g.nf.ssq_stride = s->ssq_stride;
     }
+    g.few_rows = true;
     mark(p);
     LUMI_TRY(launch_gemm_tcgen05(g, p.st_hi));
     if (gamma_next != nullptr) { p.xn_ready = true; p.ssq_parts = (N + 31) / 32; }      // one partial sum per 32 columns, whatever the tile width
@@ -1298,10 +1299,11 @@ EmbedPost embed_post_of(const lumi_session* s, const RowBufs& b, int slot0, bool
     return e;
 }
 
-// Models with experts keep the order of their sums: a router that meets a near tie falls the other way when the last bits move, and a
-// whole expert with it.  (128 sequences, 16 steps, 32 experts: sums in another order changed one sequence's logits by up to 0.06 of their
-// root mean square; everything else moved by 1e-4.)
-bool one_order(const lumi_session* s) {
+// Models with experts keep the persistent kernel's single CTAs, K split by the rows up to 128 of them: a router that meets a near tie falls the
+// other way when the last bits move, and a whole expert with it.  (128 sequences, 16 steps, 32 experts: with the sums of the kernel for few
+// rows one sequence's logits moved by 0.06 of their root mean square, everything else by 1e-4; the distance from 64 bits was the same,
+// 9e-4.)  Pairs of CTAs give the same bits and could be let in; these models have not been measured with them.
+bool has_experts(const lumi_session* s) {
     for (const LayerSpec& L : s->m->cfg.specs) if (L.ff.experts > 0) return true;
     return false;
 }
@@ -1326,7 +1328,7 @@ int32_t product(StepPlan& p, int rows, const DevTensor& W, const float* in32, co
     g.nf.act = act;
     g.nf.out_hi = out_hi;
     g.nf.out_lo = s->opt_split ? out_lo : nullptr;
-    g.one_order = one_order(s);
+    g.few_rows = g.pairs = !has_experts(s);
     return launch_gemm_tcgen05(g, p.st_hi);
 }
 
@@ -1464,7 +1466,7 @@ int32_t norm_product(StepPlan& p, RowPass& r, const DevTensor& W, const float* g
         g.ext = &ex;
     }
     mark(p);
-    g.one_order = one_order(s);
+    g.few_rows = g.pairs = !has_experts(s);
     return launch_gemm_tcgen05(g, p.st_hi);
 }
 
@@ -1487,7 +1489,7 @@ int32_t residual_product(StepPlan& p, RowPass& r, const DevTensor& W, const floa
     g.nf.bias = bias;
     g.nf.gamma_next = gamma_next; g.nf.out_hi = b.xh; g.nf.out_lo = s->opt_split ? b.xl : nullptr;
     g.nf.ssq_out = b.ssq; g.nf.ssq_stride = b.ssq_stride;
-    g.one_order = one_order(s);
+    g.few_rows = g.pairs = !has_experts(s);
     LUMI_TRY(launch_gemm_tcgen05(g, p.st_hi));
     r.gamma_ready = gamma_next;
     r.ssq_parts = (N + 31) / 32;
@@ -1521,7 +1523,7 @@ int32_t grouped_product(StepPlan& p, int rows, const GroupedProduct& q) {
     g.nf.out_hi = q.oh;
     g.nf.out_lo = s->opt_split ? q.ol : nullptr;
     g.ext = &ex;
-    g.one_order = one_order(s);
+    g.few_rows = g.pairs = !has_experts(s);
     return launch_gemm_tcgen05(g, p.st_hi);
 }
 
@@ -2283,8 +2285,9 @@ int32_t prefill_chunked(lumi_session* s, int batch, int T, bool with_head, float
     __nv_bfloat16* const hi = tc ? s->pf_hi : nullptr;
     __nv_bfloat16* const lo = tc && s->opt_split ? s->pf_lo : nullptr;
     float* const y = tc ? nullptr : s->pf_y;
-    // the norm of `rows` rows of x, and the product of `rows` operand rows of width K from row r0 on.  Tensor cores: few rows of short prompts split K over CTAs, which needs the session's counters;
-    // the chunked scan's products add in one order whatever the rows, so that a sequence gets the same angles alone and among others
+    // the norm of `rows` rows of x, and the product of `rows` operand rows of width K from row r0 on.  Tensor cores: few rows of short prompts
+    // share K between CTAs; the chunked scan's products add in one order whatever the rows (no shares, no splits of K), so that a sequence
+    // gets the same state alone and among others
     auto norm = [&](const float* gamma, int rows) {
         if (tc) return launch_norm_split(s->pf_x, gamma, hi, lo, rows, D, c.eps, s->stream);
         return launch_row_norm(RowNormArgs{s->pf_x, nullptr, gamma, y, nullptr, nullptr, nullptr, rows, D, D, c.eps, nullptr}, s->stream);
@@ -2297,6 +2300,7 @@ int32_t prefill_chunked(lumi_session* s, int batch, int T, bool with_head, float
         }
         GemmArgs g{hi + r0 * K, lo ? lo + r0 * K : nullptr, (const __nv_bfloat16*)W.p, out, N, rows, N, K, accumulate, &s->ctl->status,
                    scan ? nullptr : s->gemm_counters, kGemmCounters, s->gemm_scratch, kGemmScratchFloats};
+        g.few_rows = !scan;
         return launch_gemm_tcgen05(g, s->stream);
     };
     for (int b0 = 0; b0 < batch; b0 += nb_max) {
@@ -2958,6 +2962,7 @@ extern "C" int32_t lumi_k_gemm_bf16_tcgen05(uint64_t a_hi, uint64_t a_lo, uint64
     LUMI_TRY(kernel_scratch(&ks));
     GemmArgs g{(const __nv_bfloat16*)a_hi, (const __nv_bfloat16*)a_lo, (const __nv_bfloat16*)w, (float*)d, ldd, M, N, K, accumulate, nullptr,
                ks.counters, ks.n_counters, ks.scratch, ks.floats};
+    g.few_rows = true;
     return launch_gemm_tcgen05(g, (cudaStream_t)stream);
 }
 
@@ -2989,8 +2994,7 @@ extern "C" int32_t lumi_debug_gemm_wait_timeout(uint64_t a_hi, uint64_t w, uint6
                                                 int32_t skip_unit, uint64_t status_word) {
     if (!a_hi || !w || !d || !status_word) return fail(LUMI_E_INVALID, "null device pointer");
     GemmArgs g{(const __nv_bfloat16*)a_hi, nullptr, (const __nv_bfloat16*)w, (float*)d, N, M, N, K, 0, (int32_t*)status_word};
-    int32_t few = 0;
-    if (M <= 64) g.tile_counters = &few;                  // as a step's products of few rows, whose kernel needs no counters
+    g.few_rows = M <= 64;                                 // as a step's products; above, the persistent kernel
     g.wait_limit_ns = wait_limit_ns;
     g.debug_skip_unit = skip_unit;
     LUMI_TRY(launch_gemm_tcgen05(g, nullptr));

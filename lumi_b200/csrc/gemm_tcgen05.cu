@@ -855,7 +855,7 @@ void gemm_tcgen05_plan(const GemmArgs& a, int* width, int* splits) { pick_tile(a
 // Products that gemm_few_rows.cu takes.
 static bool few_rows(const GemmArgs& a) {
     static const bool on = !(getenv("LUMI_FEW_ROWS") && atoi(getenv("LUMI_FEW_ROWS")) == 0);      // 0: tuning aid
-    return on && !a.one_order && (a.ext != nullptr ? a.ext->tiles == nullptr : a.tile_counters != nullptr) && gemm_few_rows_takes(a);
+    return on && a.few_rows && (a.ext == nullptr || a.ext->tiles == nullptr) && gemm_few_rows_takes(a);
 }
 
 // Products in groups and gated results.
@@ -887,11 +887,11 @@ static int32_t launch_ext(const GemmArgs& a, cudaStream_t st) {
 // Tile width for pairs of CTAs (256-row tiles, half as many workers), or 0 where single CTAs take the product.  Widths whose half is a multiple
 // of 32: 208 was 15 % slower than single CTAs of that width.  Measured with blocked tiles, pair / single, microseconds: 4096 rows 7360 x 1024
 // 104.5 / 115.6, 1024 x 2048 33.5 / 33.7, 6208 x 1024 89 / 101; 32768 rows 735 / 771, 173 / 189, 625 / 720, 8192 x 2048 1403 / 1497; below 4096 rows
-// half as many, twice as high tiles leave more of the last round idle (2048 rows 1024 x 2048 23.6 / 22.1).  The sums differ in their last
-// bits from those of one CTA.
+// half as many, twice as high tiles leave more of the last round idle (2048 rows 1024 x 2048 23.6 / 22.1).  The results are the same bits as
+// single CTAs', at every width of either.
 static int pair_width(const GemmArgs& a) {
     static const bool on = !(getenv("LUMI_GEMM_PAIR") && atoi(getenv("LUMI_GEMM_PAIR")) == 0);      // 0: tuning aid
-    if (!on || a.one_order || a.a_lo == nullptr || a.M < kPairMinRows) return 0;
+    if (!on || !a.pairs || a.a_lo == nullptr || a.M < kPairMinRows) return 0;
     const long tiles_m = (a.M + 2 * BM - 1) / (2 * BM), workers = sm_count_gemm() / 2;
     int best = 0;
     long best_cost = -1;

@@ -543,7 +543,10 @@ struct GemmArgs {
     int debug_skip_unit = -1;           // test hook: the producer stops before this work unit, so the consumers' waits run out
     NormFuse nf;                        // RMSNorm folded around the product (persistent kernel only)
     const GemmExt* ext = nullptr;       // products in groups, gated results
-    bool one_order = false;             // sums in one order whatever the rows: nothing but the persistent kernel's single CTAs
+    // Besides the persistent kernel's single CTAs, which kernels may take the product.  few_rows: gemm_few_rows.cu, whose K shares, and with them the
+    // order of the sums, depend on the rows (as the persistent kernel's do where it is given counters, up to 128 rows).  pairs: pairs of CTAs, whose
+    // results are the same bits as single ones'.
+    bool few_rows = false, pairs = true;
 };
 int32_t launch_gemm_tcgen05(const GemmArgs& a, cudaStream_t st);   // returns LUMI_* status
 constexpr int kFewRowsMax = 1024;                                   // rows up to which gemm_few_rows.cu may take a product

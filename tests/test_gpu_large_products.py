@@ -50,3 +50,20 @@ def test_streaming_ctas_with_several_groups_of_rows(wdt, M, N, K):
     ref = x @ w.double().T + res.double()
     # fp32 throughout: lanes add K / 32 products each, then a tree; 2e-6 of the largest result as for the shorter products
     assert (d.double() - ref).abs().max() < 2e-6 * ref.abs().max()
+
+
+def test_a_long_prompt_has_the_same_state_alone_and_among_others():
+    """Alone its products have 1024 rows (single CTAs), among 31 others 32768 (pairs of CTAs, blocks of row tiles): the sums run in one order."""
+    import numpy as np
+    from lumi_b200 import synth
+    cfg = synth.base_config(n_layers=3, vocab_size=500, attention_layers=[1], attn_mlp_dim=256, attn_rope_base=10000.0)
+    model = lumi_b200.NmModel.from_tensors(cfg, list(synth.iter_tensors(cfg, seed=29, weights_dtype="bf16", perturb_ones=0.05)))
+    prompts = synth.random_prompts(32, 1024, cfg.vocab_size, seed=31)
+    many, one = model.init_states(32, 1030), model.init_states(1, 1030)
+    many.prefill(prompts, want_logits=False)
+    for b in (0, 17, 31):
+        one.reset()
+        one.prefill(prompts[b:b + 1], want_logits=False)
+        for layer in (0, 2):
+            for x, y in zip(many.read_state(b, layer), one.read_state(0, layer)):
+                assert np.array_equal(x, y), (b, layer)
