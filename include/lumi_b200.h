@@ -248,6 +248,28 @@ int32_t lumi_k_gemm_bf16_tcgen05(uint64_t a_hi, uint64_t a_lo, uint64_t w, uint6
 int32_t lumi_debug_gemm_wait_timeout(uint64_t a_hi, uint64_t w, uint64_t d, int32_t M, int32_t N, int32_t K,
                                      uint64_t wait_limit_ns, int32_t skip_unit, uint64_t status_word);
 
+/* One tensor-core product with everything that the steps' products carry (no counterpart in the reference; tests, profiling):
+ * the kernels that may take it (few_rows: the one for up to 1024 rows; pairs: pairs of CTAs from 4096 rows on; split_k: a split of K up to 128 rows),
+ * the epilogue around it, and the failure-path hook above.  Device pointers, 0 where there is none.
+ *   out = act((A W^T) * s + bias (+ D)),  s = 1 / sqrt(sum(ssq_in[row][0 .. ssq_parts)) * inv_k + eps), 1 without ssq_in.
+ * D, or with out_hi (and out_lo) the bf16 halves of out * gamma_next (of out without gamma_next), and ssq_out[row][column / 32] the sums of out^2.
+ * act: 0 none, 2 relu squared.  groups > 0: products of column blocks: group g multiplies columns [g K, (g + 1) K) of A (rows of lda) with rows
+ * [g group_rows, ...) of W; its results go to columns g out_step + n, n < out_n, of D (ldd) and out_hi / out_lo (ldo), with gate (3 relu, 4 silu:
+ * rows of W sixteen gates and sixteen ups in turn) and mul (times sigmoid(mul[row * ldmul + column])).
+ * status_word given: waits are limited to wait_limit_ns, work unit skip_unit (-1: none) is not fed, the call synchronises and answers LUMI_E_TIMEOUT. */
+typedef struct lumi_gemm_probe {
+    uint64_t a_hi, a_lo, w, d;
+    uint64_t bias, ssq_in, gamma_next, out_hi, out_lo, ssq_out, mul;
+    uint64_t status_word, wait_limit_ns;
+    int32_t M, N, K, ldd, accumulate;
+    int32_t few_rows, pairs, split_k;
+    int32_t ssq_parts, ssq_stride, act;
+    float inv_k, eps;
+    int32_t groups, group_rows, lda, out_step, out_n, gate, ldmul, ldo;
+    int32_t skip_unit;
+} lumi_gemm_probe;
+int32_t lumi_debug_gemm(const lumi_gemm_probe* probe);
+
 /* Host-side only (no device is touched, nothing is launched; no counterpart in the reference): the output-tile width and
  * the number of CTAs K is split over that the persistent kernel of lumi_k_gemm_bf16_tcgen05 and the decode / prefill steps
  * takes for a product of this shape (products of few rows have a kernel of their own: gemm_few_rows.cu).  two_planes: activations as bf16 hi + lo halves; producer: the epilogue also leaves the next RMSNorm's

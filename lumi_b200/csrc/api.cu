@@ -3005,6 +3005,33 @@ extern "C" int32_t lumi_debug_gemm_wait_timeout(uint64_t a_hi, uint64_t w, uint6
     return LUMI_OK;
 }
 
+extern "C" int32_t lumi_debug_gemm(const lumi_gemm_probe* q) {
+    if (!q || !q->a_hi || !q->w || (!q->d && !q->out_hi)) return fail(LUMI_E_INVALID, "a product needs its operands and an output");
+    KernelScratch ks;
+    if (q->split_k) LUMI_TRY(kernel_scratch(&ks));
+    GemmArgs g{(const __nv_bfloat16*)q->a_hi, (const __nv_bfloat16*)q->a_lo, (const __nv_bfloat16*)q->w, (float*)q->d, q->ldd, q->M, q->N, q->K, q->accumulate,
+               (int32_t*)q->status_word, ks.counters, ks.n_counters, ks.scratch, ks.floats};
+    g.few_rows = q->few_rows != 0;
+    g.pairs = q->pairs != 0;
+    if (q->status_word) { g.wait_limit_ns = q->wait_limit_ns; g.debug_skip_unit = q->skip_unit; }
+    g.nf.ssq_in = (const float*)q->ssq_in; g.nf.ssq_parts = q->ssq_parts; g.nf.ssq_stride = q->ssq_stride; g.nf.inv_k = q->inv_k; g.nf.eps = q->eps;
+    g.nf.gamma_next = (const float*)q->gamma_next; g.nf.out_hi = (__nv_bfloat16*)q->out_hi; g.nf.out_lo = (__nv_bfloat16*)q->out_lo;
+    g.nf.ssq_out = (float*)q->ssq_out; g.nf.act = q->act; g.nf.bias = (const float*)q->bias;
+    GemmExt ex;
+    if (q->groups > 0) {
+        ex.groups = q->groups; ex.group_rows = q->group_rows; ex.lda = q->lda; ex.out_step = q->out_step; ex.out_n = q->out_n; ex.gate = q->gate;
+        ex.mul = (const float*)q->mul; ex.ldmul = q->ldmul; ex.ldo = q->ldo;
+        g.ext = &ex;
+    }
+    LUMI_TRY(launch_gemm_tcgen05(g, nullptr));
+    if (!q->status_word) return LUMI_OK;
+    LUMI_CUDA(cudaStreamSynchronize(nullptr));
+    int32_t st = 0;
+    LUMI_CUDA(cudaMemcpy(&st, (const void*)q->status_word, sizeof(st), cudaMemcpyDeviceToHost));
+    if (st & STATUS_TIMEOUT) return fail(LUMI_E_TIMEOUT, "a bounded device-side wait expired in the tensor-core GEMM (limit %llu ns)", (unsigned long long)q->wait_limit_ns);
+    return LUMI_OK;
+}
+
 extern "C" int32_t lumi_k_row_gemm(uint64_t a_f32, uint64_t w, int32_t w_dtype, uint64_t d, int32_t M, int32_t N, int32_t K, int32_t accumulate,
                                    uint64_t stream) {
     if (!a_f32 || !w || !d || M <= 0 || N <= 0 || K <= 0 || ((a_f32 | w) & 15)) return fail(LUMI_E_INVALID, "bad argument to lumi_k_row_gemm");

@@ -275,6 +275,8 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_ahi, const __grid
     uint64_t* tmem_empty = tmem_full + 2;         // [2]
     uint64_t* drain_bar = tmem_empty + 2;         // failure path only
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain_bar + 1);
+    volatile uint32_t* gave_up = tmem_slot + 1;   // PAIR: a wait of either CTA ran out; then (first CTA) the k-blocks that either issued
+    volatile uint32_t* issued = tmem_slot + 2;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int num_kb = K / BK;
@@ -291,6 +293,7 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_ahi, const __grid
         for (int s = 0; s < S; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
         for (int i = 0; i < 2; ++i) { mbar_init(&tmem_full[i], 1); mbar_init(&tmem_empty[i], PAIR ? 8 : 4); }
         mbar_init(drain_bar, 1);
+        *gave_up = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
@@ -365,7 +368,8 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_ahi, const __grid
         if (lane == 0) {
             uint32_t kbg = 0;                    // k-blocks issued so far, over all tiles of this CTA
             for (int u = unit0; u < ntiles * splits && !timed_out; u += units_at_once) {
-                if (u == skip_unit) break;       // test hook: this unit's operands never arrive, so the waits below it run out
+                // test hook: this unit's operands (a pair: the second CTA's) never arrive, so the waits below it run out
+                if (u == skip_unit && (!PAIR || rank == 1)) break;
                 const int t = u / splits, sp = u - t * splits;
                 const Place pl = place(t);
                 const int m0 = pl.m0, n0 = pl.n0;
@@ -389,7 +393,9 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_ahi, const __grid
                     if (kbg >= pre) tma_load_2d(st + T::A_BYTES * (SPLIT ? 2 : 1), &map_w, &full_bar[s], kb * BK, n0);
                 }
             }
-            if (timed_out && rank == 0) {
+            if constexpr (PAIR) {
+                st_cluster_u32(map_to_rank(smem_u32(const_cast<uint32_t*>(issued + rank)), 0), kbg);
+            } else if (timed_out) {
                 // drain: wait (bounded) for the copies this thread issued and nobody may consume
                 for (uint32_t k = kbg > (uint32_t)S ? kbg - S : 0; k < kbg; ++k) mbar_wait(&full_bar[k % S], (k / S) & 1u, wait_ns);
             }
@@ -671,8 +677,28 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_ahi, const __grid
     }
     if (timed_out && status != nullptr) atomicOr(status, STATUS_TIMEOUT);
     tc_fence_before();
-    if constexpr (PAIR) { __syncwarp(); cluster_arrive(); cluster_wait(); }      // neither CTA's memory goes away under the other's MMAs and arrivals
-    else __syncthreads();
+    if constexpr (PAIR) {                         // neither CTA's memory goes away under the other's MMAs and arrivals
+        if (timed_out)
+            for (uint32_t r = 0; r < 2; ++r) st_cluster_u32(map_to_rank(smem_u32(const_cast<uint32_t*>(gave_up)), r), 1u);
+        __syncwarp();
+        cluster_arrive();
+        cluster_wait();
+        if (*gave_up != 0) {                      // ... nor under a copy: the first CTA, on whose barriers both CTAs' copies complete, waits (bounded) for all of them
+            if (rank == 0 && threadIdx.x == 0) {
+                const uint32_t i0 = issued[0], i1 = issued[1], lo = min(i0, i1), hi = max(i0, i1);      // at most S apart: neither gets past an unconsumed stage
+                for (uint32_t k = lo; k < hi; ++k) {          // only one CTA issued this block: the barrier expects both halves, or neither
+                    if (i0 > i1) mbar_complete_tx(&full_bar[k % S], (uint32_t)T::STAGE);
+                    else mbar_expect_tx(&full_bar[k % S], (uint32_t)T::STAGE);
+                }
+                for (uint32_t k = hi > (uint32_t)S ? hi - S : 0; k < hi; ++k) mbar_wait(&full_bar[k % S], (k / S) & 1u, wait_ns);
+            }
+            __syncwarp();
+            cluster_arrive();
+            cluster_wait();
+        }
+    } else {
+        __syncthreads();
+    }
     if (warp == 1) {
         tc_fence_after();
         if constexpr (PAIR) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(2u * ACC_COLS) : "memory");
