@@ -277,6 +277,9 @@ int32_t lumi_debug_gemm(const lumi_gemm_probe* probe);
 int32_t lumi_debug_gemm_plan(int32_t M, int32_t N, int32_t K, int32_t two_planes, int32_t producer, int32_t* width,
                              int32_t* splits);
 
+/* Host-side only: the remainder by 2 pi (in fp32) that the chunked scan takes of its running angles, of n values (tests; it has to be fmodf's). */
+int32_t lumi_debug_fmod_near(const float* x, int64_t n, float* out);
+
 /* Same contraction on CUDA cores with fp32 activations: D[M][N] = A[M][K] * W[N][K]^T (+ residual R).
  * w_dtype LUMI_DTYPE_*.  norm_gamma != 0 applies RMSNorm(gamma) to each row of A first. */
 int32_t lumi_k_gemv(uint64_t a_f32, uint64_t w, int32_t w_dtype, uint64_t d, uint64_t residual,

@@ -173,7 +173,7 @@ __device__ __forceinline__ int swz(int row, int col, int pitch) {
 
 // fmodf(x, y) for y > 0 in a few instructions: the remainder of the nearest smaller multiple is exact in one fused multiply-add, and a
 // quotient that rounding carried over a multiple is put back and the multiply-add repeated.
-__device__ __forceinline__ float fmod_near(float x, float y, float inv_y) {
+__host__ __device__ __forceinline__ float fmod_near(float x, float y, float inv_y) {
     if (!(fabsf(x) < 1e6f)) return fmodf(x, y);
     const float q = truncf(x * inv_y);
     float r = fmaf(-q, y, x);
@@ -711,3 +711,10 @@ cudaError_t launch_gather_last(const float* xr, float* x, int D, int ts, int nb,
 }
 
 }  // namespace lumi
+
+extern "C" int32_t lumi_debug_fmod_near(const float* x, int64_t n, float* out) {
+    if (!x || !out || n < 0) return lumi::fail(LUMI_E_INVALID, "null argument");
+    const float two_pi = 6.28318530717958647692f, inv = 0.15915494309189533577f;      // as the scan has them
+    for (int64_t i = 0; i < n; ++i) out[i] = lumi::fmod_near(x[i], two_pi, inv);
+    return LUMI_OK;
+}

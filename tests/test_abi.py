@@ -57,6 +57,21 @@ def test_good_config_passes_parsing():
     assert st in (0, -6), msg                # OK on a GPU box, LUMI_E_CUDA where no device exists
 
 
+def test_remainder_of_the_running_angles():
+    """The scan's own remainder by 2 pi equals fmodf bit by bit (the sign of zero apart) over the range it is taken by hand, around every kind of multiple."""
+    g = np.random.default_rng(5)
+    two_pi = np.float32(2 * np.pi)
+    near = np.float32(two_pi) * g.integers(-159_000, 159_000, size=200_000).astype(np.float32)
+    x = np.concatenate([g.uniform(-1e6, 1e6, 300_000), g.uniform(-20, 20, 300_000), np.exp(g.uniform(-90, 13, 100_000)), near,
+                        np.nextafter(near, np.float32(np.inf)), np.nextafter(near, np.float32(-np.inf)),
+                        np.float32(two_pi) * np.arange(-40, 41), [0.0, 1e6, -1e6, 3e7, 1e30, np.inf, -np.inf, np.nan, 1e-45]]).astype(np.float32)
+    out = np.empty_like(x)
+    assert lumi_b200.lib().lumi_debug_fmod_near(x.ctypes.data, x.size, out.ctypes.data) == 0
+    with np.errstate(invalid="ignore"):
+        want = np.fmod(x, two_pi)
+    assert np.array_equal(out, want, equal_nan=True)
+
+
 def test_null_arguments():
     L = lumi_b200.lib()
     assert L.lumi_model_finalize(None) == -1
