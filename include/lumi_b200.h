@@ -138,10 +138,13 @@ void    lumi_session_free(lumi_session* s);
  *                         "chunked_prefill" = minimum prompt length (default 128, 0 = never) from which bf16
  *                         models (attention layers included, unless one has a sliding window) prefill with the
  *                         chunked SSD scan (chunk 64), attention over all rows of a slice and tensor-core GEMMs
- *                         over all prompt tokens (same state to rounding).  Shorter prompts from 4 tokens on, fp32 models without
-                         attention layers and other head shapes also go a layer at a time, with the recurrence in token
-                         order in the decode step's arithmetic; with 0 every prompt goes token by token; "prefill_rows" =
- *                         token rows per pass of that path (default 131072; sets its workspace size: 41 KB per row);
+ *                         over all prompt tokens (same state to rounding).  Shorter prompts from 4 to 8 tokens on, fp32 models without
+ *                         attention layers and other head shapes also go a layer at a time, with the recurrence in token
+ *                         order in the decode step's arithmetic, and products over all rows with activations as the same
+ *                         sequences' decode steps take them (fp32; tensor-core batches of bf16 models bf16 halves); with 0
+ *                         every prompt goes token by token; "prefill_rows" =
+ *                         token rows per pass of that path (default 131072; sets its workspace size: 41 KB per row; in token
+ *                         order at most 16384, fewer where there is no room, and token by token where there is none);
  *                         (designs that list their layers take slices for every prompt of two tokens and more, unless 0);
  *                         "overlap" = minimum batch (default 0 = never) from which the tensor-core path runs two
  *                         lanes of sequences side by side on prioritised streams (measured neutral: the state

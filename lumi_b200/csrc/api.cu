@@ -1814,8 +1814,9 @@ int32_t enqueue_step(lumi_session* s, int B, bool with_head, int64_t* launches,
     StepPlan p{s, B, use_tc(s, B)};
     p.prof = prof;
     p.row_len = row_len;
-    // five to eight rows of bf16 weights: early CTAs of the next kernels take registers and shared memory from the staging CTAs (8 sequences, 64 tokens
-    // of the 48-layer base model: 140 ms with dependent launch, 127 without; fp32, 6 sequences: 122 and 126)
+    // five to eight rows of bf16 weights: early CTAs of the next kernels take registers and shared memory from the staging CTAs.  24 tokens of
+    // the 48-layer base model, with dependent launch / without, 5 to 8 sequences: 48.0 / 43.9, 49.5 / 45.0, 51.1 / 46.8, 52.0 / 47.9 ms; hybrid,
+    // 300 tokens behind: 54.4 / 50.7, 56.2 / 52.2, 58.0 / 54.5, 59.5 / 56.0; fp32, 6 sequences, 64 tokens: 122 / 126
     const bool staged_rows = !c.stacked() && s->m->wdtype == LUMI_DTYPE_BF16 && B > 4;
     // dependent launch overlaps each kernel's prologue (weight prefetch) with its predecessor; it is
     // used on the weight-streaming path, where launch gaps are the same order as the kernels
@@ -2071,9 +2072,10 @@ bool use_chunked_scan(const lumi_session* s, int T) {
 
 // Prompts a layer at a time with the recurrence in token order: what the chunked scan does not take (fp32 weights, prompts under its
 // minimum, head shapes other than its own).  The weights are read once per pass instead of once per token.  Where the line lies, on
-// the 48-layer base model (pass against decode steps): bf16, one sequence, 3 tokens about 2.2 against 1.84 ms, 4 tokens 2.22 against
-// 2.47, 32 tokens 2.85 against 19.5; fp32, one sequence, 6 tokens 3.66 against 3.26 ms, 8 tokens 3.57 against 4.32, 32 tokens 3.72
-// against 16.7; four sequences of 4 tokens 3.18 against 4.99.  fp32 passes cost their K splits and tiles of 32 rows however few the rows are.
+// the 48-layer base model (pass against decode steps): fp32 activations, bf16 weights, one sequence, 6 tokens 3.40 against 3.41 ms, 7 tokens
+// 3.41 against 3.89, two sequences of 5 3.33 against 4.17, of 4 about 3.3 against 3.40; hybrid, one sequence, 5 tokens about 3.6 against 3.33, 6
+// tokens 3.68 against 3.93; fp32 weights, one sequence, 6 tokens about 3.6 against 3.48, 8 tokens 3.65 against 4.57, three of 4 3.51 against 4.74.
+// Such passes cost their tiles of 32 rows however few the rows are.  bf16 halves (nine sequences and more): from 4 tokens on in every case measured.
 bool use_rows_prefill(const lumi_session* s, int batch, int T) {
     const Config& c = s->m->cfg;
     if (c.stacked() || s->opt_chunked_prefill <= 0 || T < 4 || s->m->n_mamba == 0 || !ssm_rows_supported(c.head_dim(), c.d_state)) return false;

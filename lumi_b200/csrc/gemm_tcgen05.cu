@@ -324,7 +324,8 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_ahi, const __grid
     const int tiles_pg = EXT ? (ex.group_rows + BN - 1) / BN : 0;       // column tiles per group
     // Tiles are numbered by blocks of kBlockRows rows, column by column within a block: a block's rows of A are read from memory once and, with
     // the weights, stay in L2 for all columns.  By columns alone, 32768 rows of 1024 as two planes, 134 MB, came from memory once per column
-    // tile: 32768 x 7360 x 1024 960 -> 771 us with single CTAs, 894 -> 735 us with pairs.
+    // tile: 32768 x 7360 x 1024 960 -> 771 us with single CTAs, 894 -> 735 us with pairs.  At longer K a block is more than L2 holds (8448: 138 MB)
+    // and still pays: 32768 rows 1024 x 5632 599 -> 485 us, 2048 x 8448 1825 -> 1458, 8448 x 2048 1919 -> 1413 (blocks of 1024 rows: 472, 1404, 1441).
     // (splits > 1: one row tile)
     constexpr int kTileRows = PAIR ? 2 * BM : BM, kBlockTiles = kBlockRows / kTileRows;
     const int tiles_all = tiles_m > 0 ? ntiles / tiles_m : 0;      // column tiles

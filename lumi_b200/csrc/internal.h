@@ -496,8 +496,7 @@ cudaError_t launch_kv_advance(int32_t* kv_pos, int b0, int nb, int by, cudaStrea
 // per-row scale; the kernel sums `ssq_parts` partial sums of x^2 per row (stride ssq_stride) and multiplies its
 // accumulator rows by 1 / sqrt(sum * inv_k + eps).  Producer side (out_hi): beside D the kernel writes
 // D * gamma_next as bf16 hi (+ lo) rows of width N and, per row, the sum of D^2 over each strip of 32 columns into
-// ssq_out[row * ssq_stride + column / 32] (independent of the tile width, so results do not depend on the row
-// count) — the next product's consumer side.  All null: plain product.
+// ssq_out[row * ssq_stride + column / 32] (independent of the tile width) — the next product's consumer side.  All null: plain product.
 struct NormFuse {
     const float* ssq_in = nullptr;
     int ssq_parts = 0;

@@ -457,6 +457,8 @@ __global__ void __launch_bounds__(256, 2) gemv_pre_kernel(const float* A, int ld
     // bf16 rows half of it stays free, the chain runs several kernels ahead of itself and their requests get in the way of the few
     // loads everyone waits for: there, and with several sequences, only behind this kernel's own wait.  64 tokens of the 48-layer base model,
     // at once / behind the wait, ms: bf16 1 sequence 43.9 / 37.0, 3 sequences 88.6 / 83.6; fp32 1 sequence 40.5 / 42.8, 3 sequences 82.8 / 80.1.
+    // 24 tokens, 1 to 4 sequences: bf16 16.3 / 13.5, 22.8 / 19.9, 32.1 / 30.8, 32.7 / 31.2; hybrid, 300 tokens behind, 17.8 / 17.0, 26.3 / 24.1, 37.5 / 35.3,
+    // 38.4 / 36.4; fp32, 2 to 4 sequences, 21.1 / 20.2, 29.1 / 28.2, 31.2 / 30.4.
     const bool late = sizeof(WT) == 2 || M > 1;
     if (!late) pdl_launch_dependents();
     if (threadIdx.x == 0) {
@@ -1505,8 +1507,9 @@ static cudaError_t gemv_launch(const GemvArgs& a, int KS, cudaStream_t st) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
     }
-    // as many CTAs as are resident together, each with several groups of rows: eight staged and normed rows cost a CTA more than
-    // a group's weights.  Without overlap, us: 8 bf16 rows x 7360 x 1024 41.1 -> 23.9, x 32000 x 1024 141 -> 56 (two weight rows per warp now as well);
+    // about as many CTAs as shared memory lets run together, each with several groups of rows: eight staged and normed rows cost a CTA more than
+    // a group's weights.  (Registers let two CTAs of the instances with two rows per warp or gated rows run on an SM, so that with four per SM
+    // their grids are up to two waves; two per SM have not been measured there.)  Without overlap, us: 8 bf16 rows x 7360 x 1024 41.1 -> 23.9, x 32000 x 1024 141 -> 56 (two weight rows per warp now as well);
     // one row x 32000 x 1024 24.6 -> 19.1; at most four CTAs of eight staged rows per SM instead of two 30.6 and 69
     const int rows_per_cta = (8 / KS) * RPW, groups = (a.N + rows_per_cta - 1) / rows_per_cta;
     const int resident = sm_count() * std::max(1, std::min(NB == 8 ? 2 : 4, (int)((200 * 1024) / smem)));

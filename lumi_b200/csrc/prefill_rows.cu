@@ -1,12 +1,13 @@
 // Prompts a layer at a time where the chunked scan does not apply: fp32 weights, short prompts, other head shapes.
 //
 // Fed token by token (inference/src/main.rs:121-125), a prompt of T tokens reads every weight T times.  Taken a layer at a
-// time it reads them once: the projections become products over all rows (`launch_row_gemm` for fp32 weights, the tensor-core
-// product for bf16 ones), and only the recurrence runs in token order (`ssm_rows_kernel`, the decode step's arithmetic with
+// time it reads them once: the projections become products over all rows (`launch_row_gemm` for fp32 activations, the tensor-core
+// product for bf16 halves), and only the recurrence runs in token order (`ssm_rows_kernel`, the decode step's arithmetic with
 // the state in registers).
 //
-// Measured on the 48-layer base model: scoring 4 x 96 tokens in fp32 125.5 -> 16.7 ms, a 32-token prompt of one sequence 16.7 -> 3.7 ms
-// in fp32 and 19.5 -> 2.9 ms in bf16.
+// Measured on the 48-layer base model: scoring 4 x 96 tokens in fp32 125.5 -> 16.7 ms, a 32-token prompt of one sequence
+// with the step behind it 4.8 ms in fp32 (token by token 16.7 without the step) and 20.9 -> 4.6 ms in bf16; twelve bf16 sequences of 100 tokens
+// (halves) 10.4 ms.
 #include "internal.h"
 
 namespace lumi {

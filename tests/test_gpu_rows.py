@@ -30,7 +30,7 @@ def same_state(rows, steps, b, layer, tol):
 
 
 # Sums of at most 512 products in two orders: 512 * 2^-24 = 3e-5 of the sum of magnitudes at the very worst, a tenth of it in practice;
-# bf16 models add the products' bf16 halves (2^-17 per factor) on one side only, because few rows take fp32 activations.
+# bf16 models of nine sequences and more round activations to two bf16 halves (2^-17 per factor) on both sides, after sums in two orders.
 TOL = {"f32": 3e-5, "bf16": 2e-4}
 
 
