@@ -19,20 +19,27 @@
 // same angle, rounding-level differences; the stored angle may differ from the sequential one by a multiple
 // of 2 pi).
 //
-// One CTA of four warps per (head, sequence), three CTAs per SM (69 KiB of shared memory, 168 registers).
-//   * Staging: the chunk's x, z, theta (64 x 32 fp32 each) and the group's raw B, C (64 x 64 fp32 each) arrive by
-//     five cp.async.bulk.tensor copies on one mbarrier (bounded wait).  The operand tiles are built IN PLACE over the
+// One CTA of four warps per (head, sequence), four CTAs per SM (54 KiB of shared memory, 128 registers).
+//   * Staging: the chunk's x, theta (64 x 32 fp32 each) and the group's raw B, C (64 x 64 fp32 each) arrive by four
+//     cp.async.bulk.tensor copies on one mbarrier (bounded wait).  The operand tiles are built IN PLACE over the
 //     raw rows, so the copies for chunk c+1 are issued when chunk c's products are done; their flight time is covered
-//     by the two other CTAs of the SM (and the per-token scalars dt, lambda, A, BCNorm scales of chunk c+1 are
-//     requested into registers at the start of chunk c).
+//     by the three other CTAs of the SM.  z and the next chunk's per-token scalars (dt, lambda, A, BCNorm scales) come by small
+//     asynchronous copies into places that are free by then.
+//   * Segments of 16 tokens, one per warp: decays are taken from segment to segment.  What later segments and the state take of token j is
+//     x_j kap_j times its decay to the end of its segment, one tile for both; Y = C~ S^_in^T walks over the segments ahead of the warp's own, each time
+//     a decay, then + G X; the segment's own block, which needs the warp's rows only, is the one place with a decay per pair of tokens.  Every factor is at
+//     most 1, whatever the decays.
 //   * Arithmetic: every operand is an fp32 value split into bf16 hi + lo; a product is three
 //     mma.sync.m16n8k16 (hi*hi + hi*lo + lo*hi, fp32 accumulate), which keeps ~16 mantissa bits per factor.
-//     Warp w owns tokens 16w..16w+15: its C~ rows stay in registers as A fragments, G's accumulators are masked,
-//     decayed and re-used in place as the A fragments of W X (no trip through shared memory), and the state S^
+//     Warp w owns tokens 16w..16w+15: its C~ rows stay in registers as A fragments, G's accumulators are
+//     re-used in place as the A fragments of G X (no trip through shared memory), and the state S^
 //     lives in accumulator registers across the chunks of a launch (warp w: 16 rows of P x 32 columns of N).
 //     Independent accumulators are interleaved so that no multiply-add waits for the one issued just before it.
 //   * The pointwise part (softplus / sigmoid / tanh / SiLU / sin / cos) uses the fast hardware forms here: their
 //     error (~1e-6) is far below the operand split's (1.5e-5) — the decode step keeps the exact forms.
+// What bounds it: instruction issue (half of the slots) and shared memory (half of its cycles) together; memory is at a fifth of its rate.  64 sequences x 2048
+// tokens, 64 heads: 4.00 ms with decays per pair of tokens throughout and three CTAs per SM, 2.85 ms by segments with four, 2.39 ms with one address per
+// tile and lane and the scalars copied ahead (15.0, 11.6 and fewer thousand warp instructions per chunk and head).
 #include "internal.h"
 #include "embed_post.cuh"
 
@@ -49,17 +56,17 @@ int32_t make_f32_map_2d(CUtensorMap* map, const void* ptr, uint64_t rows, uint64
 namespace {
 
 constexpr int LCH = 64;          // chunk length
-constexpr int TSB = 72;          // row stride (bf16 elements) of the operand tiles: 144 bytes, conflict-free fragment loads
 constexpr uint64_t kScanWaitLimitNs = 500ull * 1000 * 1000;
 
 __device__ __forceinline__ float sigmoid_ref(float x) { return __fdiv_rn(1.0f, __fadd_rn(1.0f, expf(-x))); }
 __device__ __forceinline__ float softplus_ref(float x) { return logf(__fadd_rn(expf(x), 1.0f)); }
-__device__ __forceinline__ float silu_fast(float x) { return __fdividef(x, 1.0f + __expf(-x)); }
-__device__ __forceinline__ float tanh_fast(float x) {
-    // 1 - 2 / (e^{2x} + 1): absolute error ~1e-7; the argument is clamped so e^{2x} stays finite
-    const float xc = fminf(fmaxf(x, -15.f), 15.f);
-    return 1.0f - __fdividef(2.0f, __expf(2.0f * xc) + 1.0f);
-}
+// The hardware forms without the steps around them that keep results below 2^-126 alive: a term that small is gone behind the next addition.
+__device__ __forceinline__ float ex2_ftz(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
+__device__ __forceinline__ float rcp_ftz(float x) { float y; asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
+constexpr float kLog2E = 1.44269504088896340736f;
+__device__ __forceinline__ float silu_fast(float x) { return x * rcp_ftz(1.0f + ex2_ftz(-kLog2E * x)); }
+// 1 - 2 / (e^{2x} + 1): absolute error ~1e-7; e^{2x} may be 0 or infinite
+__device__ __forceinline__ float tanh_fast(float x) { return fmaf(-2.0f, rcp_ftz(ex2_ftz(2.0f * kLog2E * x) + 1.0f), 1.0f); }
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ uint64_t globaltimer_ns() {
@@ -120,13 +127,28 @@ __device__ __forceinline__ void mma3x4(float (&d0)[4], float (&d1)[4], float (&d
     mma_bf16(d0, ah, bl0[0], bl0[1]); mma_bf16(d1, ah, bl0[2], bl0[3]); mma_bf16(d2, ah, bl1[0], bl1[1]); mma_bf16(d3, ah, bl1[2], bl1[3]);
     mma_bf16(d0, al, bh0[0], bh0[1]); mma_bf16(d1, al, bh0[2], bh0[3]); mma_bf16(d2, al, bh1[0], bh1[1]); mma_bf16(d3, al, bh1[2], bh1[3]);
 }
-__device__ __forceinline__ void ldsm_x4(uint32_t (&r)[4], const void* p) {
+__device__ __forceinline__ void ldsm_x4(uint32_t (&r)[4], uint32_t at) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_u32(p)));
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(at) : "memory");
 }
-__device__ __forceinline__ void ldsm_x4_trans(uint32_t (&r)[4], const void* p) {
+__device__ __forceinline__ void ldsm_x4_trans(uint32_t (&r)[4], uint32_t at) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_u32(p)));
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(at) : "memory");
+}
+__device__ __forceinline__ void sts32(uint32_t at, uint32_t v) { asm volatile("st.shared.b32 [%0], %1;" ::"r"(at), "r"(v) : "memory"); }
+__device__ __forceinline__ void sts128(uint32_t at, const uint32_t (&v)[4]) {
+    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]) : "memory");
+}
+__device__ __forceinline__ void cp_async4(void* dst, const float* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+// (a0, a1) * s then * g + b, two fp32 at a time
+__device__ __forceinline__ float2 norm2(float2 v, float s, float2 g, float2 b) {
+    float2 r;
+    asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %4};\n\tmul.rn.f32x2 x, x, y;\n\t"
+        "mov.b64 y, {%5, %6};\n\tmov.b64 z, {%7, %8};\n\tfma.rn.f32x2 x, x, y, z;\n\tmov.b64 {%0, %1}, x;\n\t}"
+        : "=f"(r.x), "=f"(r.y) : "f"(v.x), "f"(v.y), "f"(s), "f"(g.x), "f"(g.y), "f"(b.x), "f"(b.y));
+    return r;
 }
 // two fp32 values -> bf16x2 hi word and bf16x2 lo word (first value in the low half)
 __device__ __forceinline__ void split2(float v0, float v1, uint32_t& hi, uint32_t& lo) {
@@ -144,32 +166,38 @@ __device__ __forceinline__ void split_bf16(float v, __nv_bfloat16& hi, __nv_bflo
     lo = __float2bfloat16_rn(v - __bfloat162float(hi));
 }
 
-// Shared memory of a CTA (69 KiB: three CTAs per SM).  The five bulk tensor copies of a chunk land in rx, rth, rB, rC, rz
-// (dense boxes).  The operand tiles of the tensor-core products are then written IN PLACE over the raw rows they were
-// computed from — token i's raw B row (256 bytes) becomes B~ hi (first 128 bytes) and B~ lo (last 128 bytes) of token i,
-// the same for C, silu(x) transposed replaces the raw x rows, the gate replaces z — so no operand tile needs memory of
-// its own.  Inside a 128-byte row the eight 16-byte chunks are XOR-ed with (row % 8) so that ldmatrix and the fragment
-// stores stay free of bank conflicts without padding.
+// Shared memory of a CTA (54 KiB: four CTAs per SM).  The four bulk tensor copies of a chunk land in rx, rth, rB, rC (dense boxes).  The
+// operand tiles of the tensor-core products are then written IN PLACE over raw rows that nobody reads any more: token i's raw B row
+// (256 bytes) becomes B~ hi (first 128 bytes) and B~ lo (last 128 bytes) of token i, the same for C; silu(x) transposed replaces the raw x
+// rows and the state S^ the raw theta rows.  A warp's rows of C~ move on into its registers, and its rows of z are copied over them.
+// Inside a 128-byte row the eight 16-byte chunks are XOR-ed with a key of the row, so that ldmatrix and the stores stay free of bank
+// conflicts without padding.
 struct PfSmem {
     float rx[LCH][32];                 // raw x            -> X^T: [plane hi | lo][p = 32 rows][token, 128 bytes]
-    float rth[LCH][32];                // raw theta
+    float rth[LCH][32];                // raw theta        -> S^: [plane hi | lo][p = 32 rows][n, 128 bytes]
     float rB[LCH][64];                 // raw B (group)    -> B~: row = token, [hi 128 bytes | lo 128 bytes]
-    float rC[LCH][64];                 // raw C (group)    -> C~: same layout
-    float rz[LCH][32];                 // raw z            -> gate silu(z)
-    uint8_t St[2 * 32 * 128];          // augmented state S^: [plane hi | lo][p = 32 rows][n, 128 bytes]
+    float rC[LCH][64];                 // raw C (group)    -> C~: same layout -> z of the warp's tokens
     struct Scalars {                   // per token; the next chunk's are prepared under this one
-        float ell[LCH], eli[LCH], lam[LCH], kap[LCH], wj[LCH], dtp[LCH], rbs[LCH], rcs[LCH];
+        float dtp[LCH], rbs[LCH], rcs[LCH];      // dt pi, BCNorm scales
+        float ell[LCH], eli[LCH];      // log2 of the decay from the start of the token's segment of 16 to the token itself, and the decay
+        float lam[LCH], kap[LCH];
+        float xw[LCH];                 // kap times the decay from the token to the end of its segment
+        float seg[4];                  // decay over each segment
+        float after, pad[3];           // raw lambda of the token behind the chunk
     } sc[2];
     float seg[4][32];                  // angle sums of the four 16-token segments
     float gam[4][64];                  // this group's BCNorm weights: b gamma, b bias, c gamma, c bias
     unsigned long long bar;
 };
 
-// byte offset of bf16 element (row, col) inside a tile whose rows are `pitch` bytes apart and hold 64 bf16 (128 bytes)
-// with the 16-byte chunks XOR-ed by row % 8
-__device__ __forceinline__ int swz(int row, int col, int pitch) {
-    return row * pitch + ((((col >> 3) ^ (row & 7)) << 4) | ((col & 7) << 1));
-}
+// Element (row, col) of the B~ / C~ tiles lies at row * 256 + (((col / 8) ^ (row % 8)) << 4) + col % 8 * 2, lo plane 128 bytes on; of the X^T / S^
+// tiles (row = p) at p * 128 + (((col / 8) ^ key_of(p)) << 4) + col % 8 * 2, lo plane 4096 bytes on.  The key differs within every eight
+// consecutive rows and within every eight rows {8 a + 2 n + e : a = 0 .. 3, e = 0, 1} that pcol() makes one matrix.  Columns in steps of 16
+// (two chunks) then only flip bits of a lane's address: address ^ (step << 5).
+__device__ __forceinline__ int key_of(int p) { return (((p >> 3) ^ (p >> 1)) & 3) << 1 | (p & 1); }
+// Column c of tile nt of a product whose columns are head dims: with this order a lane's results of the four tiles are the eight head dims
+// 8 t4 .. 8 t4 + 7, one 16-byte store.
+__device__ __forceinline__ int pcol(int nt, int c) { return 8 * (c >> 1) + 2 * nt + (c & 1); }
 
 // fmodf(x, y) for y > 0 in a few instructions: the remainder of the nearest smaller multiple is exact in one fused multiply-add, and a
 // quotient that rounding carried over a multiple is put back and the multiply-add repeated.
@@ -182,7 +210,7 @@ __host__ __device__ __forceinline__ float fmod_near(float x, float y, float inv_
     return r;
 }
 
-constexpr uint32_t kChunkTxBytes = 3 * LCH * 32 * 4 + 2 * LCH * 64 * 4;
+constexpr uint32_t kChunkTxBytes = 2 * LCH * 32 * 4 + 2 * LCH * 64 * 4;
 
 // row r = b * ts + t  of the super-chunk; token ids come from prompt[(t_abs) * batch_total + b_abs]
 template <typename WT>
@@ -242,13 +270,14 @@ __global__ void gather_last_kernel(const float* __restrict__ xr, float* __restri
     for (int k = threadIdx.x; k < D; k += blockDim.x) x[(size_t)(b0 + b) * D + k] = xr[((size_t)b * ts + idx) * D + k];
 }
 
-__global__ void __launch_bounds__(128, 3)
+__global__ void __launch_bounds__(128, 4)
 ssd_prefill_kernel(const __grid_constant__ CUtensorMap map32, const __grid_constant__ CUtensorMap map64, PrefillArgs a) {
     constexpr int P = 32, N = 64, HN = 32;
-    extern __shared__ uint8_t pf_raw[];
-    PfSmem& sm = *reinterpret_cast<PfSmem*>((reinterpret_cast<uintptr_t>(pf_raw) + 1023) & ~(uintptr_t)1023);
+    extern __shared__ __align__(1024) uint8_t pf_raw[];
+    PfSmem& sm = *reinterpret_cast<PfSmem*>(pf_raw);
     const int h = blockIdx.x, b = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g4 = lane >> 2, t4 = lane & 3;               // mma fragment coordinates: row group, column pair
+    const int lm = lane >> 3, lr = lane & 7;               // ldmatrix: matrix and row that this lane addresses
     const int H = a.H, DI = H * P, BC = a.G * N, R = a.ldp;
     const int tsl = a.ts;                                   // rows per sequence in the projection / output arrays
     // tokens this sequence takes from the launch (prompts of different lengths end early; none: the state stays as it is)
@@ -277,51 +306,63 @@ ssd_prefill_kernel(const __grid_constant__ CUtensorMap map32, const __grid_const
     }
     __syncthreads();
 
-    auto issue_chunk = [&](int t0) {               // one thread: the five box copies of the chunk starting at token t0
+    auto issue_chunk = [&](int t0) {               // one thread: the four box copies of the chunk starting at token t0
         const int row0 = b * tsl + t0;
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(kChunkTxBytes) : "memory");
-        tma_load_2d(&sm.rx[0][0], &map32, bar, h * P, row0);
-        tma_load_2d(&sm.rz[0][0], &map32, bar, DI + h * P, row0);
         tma_load_2d(&sm.rth[0][0], &map32, bar, off_dt + 3 * H + h * HN, row0);
+        tma_load_2d(&sm.rx[0][0], &map32, bar, h * P, row0);
         tma_load_2d(&sm.rB[0][0], &map64, bar, off_b + grp * N, row0);
         tma_load_2d(&sm.rC[0][0], &map64, bar, off_c + grp * N, row0);
     };
-    uint8_t* const tB = reinterpret_cast<uint8_t*>(&sm.rB[0][0]);     // B~ tile (in place): pitch 256, lo plane at +128
-    uint8_t* const tC = reinterpret_cast<uint8_t*>(&sm.rC[0][0]);     // C~ tile (in place)
-    uint8_t* const tX = reinterpret_cast<uint8_t*>(&sm.rx[0][0]);     // X^T tile (in place): pitch 128, lo plane at +4096
-    uint8_t* const tS = sm.St;                                        // S^ tile: pitch 128, lo plane at +4096
+    // this lane's addresses in the operand tiles (ldmatrix reads and stores), the parts that change with the loops left out
+    const uint32_t tB = smem_u32(&sm.rB[0][0]), tC = smem_u32(&sm.rC[0][0]), tX = smem_u32(&sm.rx[0][0]), tS = smem_u32(&sm.rth[0][0]);
+    const int i0 = 16 * warp;                              // first token of this warp's segment
+    const uint32_t own = (uint32_t)(i0 * 256 + ((lane >> 2) << 4) + ((lane & 3) << 2));                        // B~ / C~ stores: columns 2 lane, 2 lane + 1
+    const uint32_t aC = tC + (uint32_t)((i0 + 8 * (lm & 1) + lr) * 256 + (((lm >> 1) ^ lr) << 4));           // C~ rows as A fragments
+    const uint32_t aB = tB + (uint32_t)((8 * (lm >> 1) + lr) * 256 + (((lm & 1) ^ lr) << 4));                 // B~ rows of a segment as B fragments
+    const int pn = pcol(lm >> 1, lr);                       // head dim of this lane's row in the two tiles 0 and 1; tiles 2 and 3: + 4, whose key differs by 4
+    const uint32_t aP = (uint32_t)(pn * 128 + (((lm & 1) ^ key_of(pn)) << 4)), aP2 = (aP + 4u * 128u) ^ 64u;
     // Per-token scalars of a chunk (model.rs:307, 314-317), by warp 0 alone: lane l takes tokens 2 l and 2 l + 1, the last lane also lambda
     // of the token behind the chunk.  Done for the next chunk while the other warps, which have more of the causal products, are still at theirs.
-    auto prepare_scalars = [&](int t0, PfSmem::Scalars& q) {
+    // Their raw values are copied (asynchronously, by the same lanes) into the places that take the results.
+    auto fetch_scalars = [&](int t0, PfSmem::Scalars& q) {
         const int nv = min(LCH, ts - t0);
-        float n_dt[2] = {0.f, 0.f}, n_lam[2] = {0.f, 0.f}, n_a[2] = {0.f, 0.f}, n_rb[2] = {0.f, 0.f}, n_rc[2] = {0.f, 0.f}, n_after = 0.f;
 #pragma unroll
-        for (int e = 0; e < 2; ++e)
-            if (2 * lane + e < nv) {
-                const size_t row = (size_t)b * tsl + t0 + 2 * lane + e;
+        for (int e = 0; e < 2; ++e) {
+            const int i = 2 * lane + e;
+            if (i < nv) {
+                const size_t row = (size_t)b * tsl + t0 + i;
                 const float* pr = a.proj + row * R + off_dt + h;
-                n_dt[e] = pr[0]; n_lam[e] = pr[H]; n_a[e] = pr[2 * H];
-                n_rb[e] = a.rb[row]; n_rc[e] = a.rc[row];
+                cp_async4(&q.dtp[i], pr); cp_async4(&q.lam[i], pr + H); cp_async4(&q.ell[i], pr + 2 * H);
+                cp_async4(&q.rbs[i], a.rb + row); cp_async4(&q.rcs[i], a.rc + row);
             }
-        if (lane == 31 && t0 + LCH < ts) n_after = a.proj[((size_t)b * tsl + t0 + LCH) * R + off_dt + H + h];
-        float dtpv[2] = {0.f, 0.f}, gl[2] = {0.f, 0.f}, lm[2] = {0.f, 0.f};
+        }
+        if (lane == 31 && t0 + LCH < ts) cp_async4(&q.after, a.proj + ((size_t)b * tsl + t0 + LCH) * R + off_dt + H + h);
+    };
+    auto prepare_scalars = [&](int t0, PfSmem::Scalars& q) {      // (this lane's copies have landed)
+        const int nv = min(LCH, ts - t0);
+        float dtpv[2] = {0.f, 0.f}, gl[2] = {0.f, 0.f}, lv[2] = {0.f, 0.f};
 #pragma unroll
-        for (int e = 0; e < 2; ++e)
-            if (2 * lane + e < nv) {
-                dtpv[e] = softplus_ref(__fadd_rn(n_dt[e], dtb));
-                float av = -softplus_ref(n_a[e]);
+        for (int e = 0; e < 2; ++e) {
+            const int i = 2 * lane + e;
+            if (i < nv) {
+                dtpv[e] = softplus_ref(__fadd_rn(q.dtp[i], dtb));
+                float av = -softplus_ref(q.ell[i]);
                 av = fminf(fmaxf(av, -1e6f), -1e-4f);
                 gl[e] = __fmul_rn(av, dtpv[e]);           // log a_t
-                lm[e] = sigmoid_ref(n_lam[e]);
+                lv[e] = sigmoid_ref(q.lam[i]);
+            } else {
+                q.rbs[i] = 0.f; q.rcs[i] = 0.f;
             }
-        const float after = t0 + LCH < ts ? sigmoid_ref(n_after) : -1.0f;      // < 0: no next token in this launch
-        const float sum = gl[0] + gl[1];                   // inclusive prefix of log a over the chunk
-        float incl = sum;
+        }
+        const float after = lane == 31 && t0 + LCH < ts ? sigmoid_ref(q.after) : -1.0f;      // < 0: no next token in this launch
+        float incl = gl[0] + gl[1];                        // inclusive prefix of log a over the segment of 16 tokens: eight lanes
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) { const float n = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= o) incl += n; }
-        const float excl = incl - sum;
-        const float l[2] = {excl + gl[0], excl + sum};
-        const float tot = __shfl_sync(0xffffffffu, l[1], 31), down = __shfl_down_sync(0xffffffffu, lm[0], 1);
+        for (int o = 1; o < 8; o <<= 1) { const float n = __shfl_up_sync(0xffffffffu, incl, o, 8); if ((lane & 7) >= o) incl += n; }
+        float excl = __shfl_up_sync(0xffffffffu, incl, 1, 8);
+        if ((lane & 7) == 0) excl = 0.f;
+        const float l[2] = {excl + gl[0], incl};
+        const float tot = __shfl_sync(0xffffffffu, incl, lane | 7), down = __shfl_down_sync(0xffffffffu, lv[0], 1);
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
             const int i = 2 * lane + e;
@@ -329,18 +370,23 @@ ssd_prefill_kernel(const __grid_constant__ CUtensorMap map32, const __grid_const
             if (i < nv) {
                 // lambda of the next token: this lane's second one, the next lane's first, or the one behind the chunk
                 float ln = -1.0f;
-                if (i + 1 < nv) ln = e == 0 ? lm[1] : down;
+                if (i + 1 < nv) ln = e == 0 ? lv[1] : down;
                 else if (nv == LCH) ln = after;                  // lane 31's last token only
-                k = ln < 0.f ? lm[e] : __fadd_rn(lm[e], __fsub_rn(1.0f, ln));
+                k = ln < 0.f ? lv[e] : __fadd_rn(lv[e], __fsub_rn(1.0f, ln));
             }
-            q.dtp[i] = dtpv[e]; q.ell[i] = l[e]; q.lam[i] = lm[e]; q.rbs[i] = n_rb[e]; q.rcs[i] = n_rc[e];
-            q.kap[i] = k;
-            q.wj[i] = __expf(tot - l[e]) * k;
-            q.eli[i] = __expf(l[e]);
+            q.dtp[i] = dtpv[e] * PI_F;
+            q.ell[i] = l[e] * kLog2E; q.eli[i] = ex2_ftz(l[e] * kLog2E);
+            q.lam[i] = lv[e]; q.kap[i] = k;
+            q.xw[i] = ex2_ftz((tot - l[e]) * kLog2E) * k;
         }
+        if ((lane & 7) == 0) q.seg[lane >> 3] = ex2_ftz(tot * kLog2E);
     };
     if (tid == 0) issue_chunk(0);
-    if (warp == 0) prepare_scalars(0, sm.sc[0]);
+    if (warp == 0) {
+        fetch_scalars(0, sm.sc[0]);
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        prepare_scalars(0, sm.sc[0]);
+    }
 
     // state S^ of this warp: rows p0 + {g4, g4 + 8}, columns n0 + 8 nt + 2 t4 + {0, 1}
     const int p0 = 16 * (warp & 1), n0 = 32 * (warp >> 1);
@@ -357,21 +403,19 @@ ssd_prefill_kernel(const __grid_constant__ CUtensorMap map32, const __grid_const
 
     __syncthreads();                                       // the first chunk's scalars are there
 
-    // this warp's block of S^ as bf16 hi + lo into the shared tile (B operand of C~ S^T in the next chunk)
-    auto store_state_tile = [&]() {
+    // S^_in = S + (1 - lam_first) x_prev (x) B~_prev   (prev_bx of the decode state, model.rs:359)
+    {
+        const float oml = __fadd_rn(__fmul_rn(sm.sc[0].lam[0], -1.0f), 1.0f);
+        const float xp0 = a.xprev[bh * P + p0 + g4] * oml, xp1 = a.xprev[bh * P + p0 + g4 + 8] * oml;
 #pragma unroll
         for (int nt = 0; nt < 4; ++nt) {
-            uint32_t hi, lo;
-            const int col = n0 + 8 * nt + 2 * t4;
-            split2(S[nt][0], S[nt][1], hi, lo);
-            *reinterpret_cast<uint32_t*>(tS + swz(p0 + g4, col, 128)) = hi;
-            *reinterpret_cast<uint32_t*>(tS + 4096 + swz(p0 + g4, col, 128)) = lo;
-            split2(S[nt][2], S[nt][3], hi, lo);
-            *reinterpret_cast<uint32_t*>(tS + swz(p0 + g4 + 8, col, 128)) = hi;
-            *reinterpret_cast<uint32_t*>(tS + 4096 + swz(p0 + g4 + 8, col, 128)) = lo;
+            const float2 bp = *reinterpret_cast<const float2*>(a.bprev + bh * N + n0 + 8 * nt + 2 * t4);
+            S[nt][0] = fmaf(xp0, bp.x, S[nt][0]); S[nt][1] = fmaf(xp0, bp.y, S[nt][1]);
+            S[nt][2] = fmaf(xp1, bp.x, S[nt][2]); S[nt][3] = fmaf(xp1, bp.y, S[nt][3]);
         }
-    };
+    }
 
+    const int ia = i0 + g4, ib = ia + 8;                   // the tokens whose results this lane holds
     uint32_t phase = 0;
     // One chunk.  FULL: all 64 tokens are valid, so every "past the end of the sequence" test folds away.
     auto do_chunk = [&](auto full_c, const int t0, const int chunk) -> bool {
@@ -380,65 +424,73 @@ ssd_prefill_kernel(const __grid_constant__ CUtensorMap map32, const __grid_const
         auto valid = [&](int i) { return FULL || i < nv; };
         const bool last_chunk = t0 + LCH >= ts;
         PfSmem::Scalars& sc = sm.sc[chunk & 1];
-        // ---- 0. the chunk's raw rows have landed (every thread waits, bounded; the next barrier makes one verdict of it)
+        // ---- 1. the chunk's raw rows have landed (every thread waits, bounded; the next barrier makes one verdict of it)
         const bool landed = mbar_wait(bar, phase, kScanWaitLimitNs);
         phase ^= 1;
-        if (chunk == 0) {
-            // S^_in = S + (1 - lam_first) x_prev (x) B~_prev   (prev_bx of the decode state, model.rs:359)
-            const float oml = __fadd_rn(__fmul_rn(sc.lam[0], -1.0f), 1.0f);
-            const float xp0 = a.xprev[bh * P + p0 + g4] * oml, xp1 = a.xprev[bh * P + p0 + g4 + 8] * oml;
+        // ---- 2. thread (lane, warp) takes column `lane` (angle pair k, head dim p) of the warp's 16 tokens: angles, rotated
+        //         B~ and C~ (one sin / cos for both), silu(x) transposed.  Every raw row of B and C is read only by the warp that owns
+        //         its token, so a row can be overwritten by its operand tile after a warp-level barrier.
+        const int k = lane, p = lane;
+        float loc[16], xs[16], run = 0.f;
+#pragma unroll
+        for (int i4 = 0; i4 < 16; i4 += 4) {
+            const float4 dp = *reinterpret_cast<const float4*>(&sc.dtp[i0 + i4]);
+            const float d4[4] = {dp.x, dp.y, dp.z, dp.w};
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int i = i0 + i4 + q;
+                const float d = d4[q] * tanh_fast(sm.rth[i][k]);             // model.rs:341-342
+                run += valid(i) ? d : 0.f;                                   // the rows behind the sequence are another one's
+                loc[i4 + q] = run;
+                xs[i4 + q] = valid(i) ? silu_fast(sm.rx[i][p]) : 0.f;        // model.rs:310
+            }
+        }
+        sm.seg[warp][k] = run;
+        if (!__syncthreads_and(landed)) return false;
+        // every warp has read its raw x and theta.  S^ over theta: this warp's block as bf16 hi + lo (B operand of C~ S^T)
+        {
+            // columns n0 + 8 nt + 2 t4: chunk n0 / 8 + nt; rows g4 and g4 + 8 of the block, whose keys differ by 2
+            const uint32_t at = tS + (uint32_t)((p0 + g4) * 128 + (((n0 >> 3) ^ key_of(p0 + g4)) << 4) + 4 * t4);
 #pragma unroll
             for (int nt = 0; nt < 4; ++nt) {
-                const float2 bp = *reinterpret_cast<const float2*>(a.bprev + bh * N + n0 + 8 * nt + 2 * t4);
-                S[nt][0] = fmaf(xp0, bp.x, S[nt][0]); S[nt][1] = fmaf(xp0, bp.y, S[nt][1]);
-                S[nt][2] = fmaf(xp1, bp.x, S[nt][2]); S[nt][3] = fmaf(xp1, bp.y, S[nt][3]);
-            }
-            store_state_tile();
-        }
-        // ---- 2. thread (lane, warp) takes column `lane` (angle pair k, head dim p) of the warp's 16 tokens: angles, rotated
-        //         B~ and C~ (one sin / cos for both), silu(x) transposed, gate.  Every raw row is read only by the warp that owns
-        //         its token, so a row can be overwritten by its operand tile after a warp-level barrier.
-        {
-            const int k = lane, i0 = 16 * warp;
-            float loc[16], run = 0.f;
-#pragma unroll
-            for (int ii = 0; ii < 16; ++ii) {
-                const float d = sc.dtp[i0 + ii] * (tanh_fast(sm.rth[i0 + ii][k]) * PI_F);      // model.rs:341-342; dtp = 0 past the end
-                run += d;
-                loc[ii] = run;
-            }
-            sm.seg[warp][k] = run;
-            // x -> silu (registers; the tile is written after every warp has read its raw x) ; z -> gate in place
-            const int p = lane;
-            float xs[16];
-#pragma unroll
-            for (int ii = 0; ii < 16; ++ii) {
-                const int i = i0 + ii;
-                xs[ii] = valid(i) ? silu_fast(sm.rx[i][p]) : 0.f;                              // model.rs:310
-                sm.rz[i][p] = valid(i) ? silu_fast(sm.rz[i][p]) : 0.f;                         // model.rs:370
-            }
-            if (!__syncthreads_and(landed)) return false;
-            // reduced mod 2 pi at every segment boundary, so sums stay small and keep their low bits
-            float base = cum;
-#pragma unroll
-            for (int s2 = 0; s2 < 4; ++s2) {
-                if (s2 == warp) base = cum;
-                cum = fmod_near(cum + sm.seg[s2][k], TWO_PI, INV_TWO_PI);
-            }
-            if (last_chunk) {                              // hand-over: x of the launch's last token (every warp has read the old one)
-#pragma unroll
-                for (int ii = 0; ii < 16; ++ii) if (i0 + ii == nv - 1) a.xprev[bh * P + p] = xs[ii];
-            }
-            // X^T tile over the raw x rows: row p, tokens i0 .. i0 + 15 (two per 32-bit word)
-#pragma unroll
-            for (int ii = 0; ii < 16; ii += 2) {
                 uint32_t hi, lo;
-                split2(xs[ii], xs[ii + 1], hi, lo);
-                *reinterpret_cast<uint32_t*>(tX + swz(p, i0 + ii, 128)) = hi;
-                *reinterpret_cast<uint32_t*>(tX + 4096 + swz(p, i0 + ii, 128)) = lo;
+                const uint32_t a0 = at ^ (uint32_t)(nt << 4), a1 = (a0 ^ 32u) + 1024u;
+                split2(S[nt][0], S[nt][1], hi, lo);
+                sts32(a0, hi);
+                sts32(a0 + 4096, lo);
+                split2(S[nt][2], S[nt][3], hi, lo);
+                sts32(a1, hi);
+                sts32(a1 + 4096, lo);
             }
-            const float bgm0 = sm.gam[0][2 * k], bgm1 = sm.gam[0][2 * k + 1], bbs0 = sm.gam[1][2 * k], bbs1 = sm.gam[1][2 * k + 1];
-            const float cgm0 = sm.gam[2][2 * k], cgm1 = sm.gam[2][2 * k + 1], cbs0 = sm.gam[3][2 * k], cbs1 = sm.gam[3][2 * k + 1];
+        }
+        if (warp == 0 && !last_chunk) fetch_scalars(t0 + LCH, sm.sc[(chunk + 1) & 1]);
+        // reduced mod 2 pi at every segment boundary, so sums stay small and keep their low bits
+        float base = cum;
+#pragma unroll
+        for (int s2 = 0; s2 < 4; ++s2) {
+            if (s2 == warp) base = cum;
+            cum = fmod_near(cum + sm.seg[s2][k], TWO_PI, INV_TWO_PI);
+        }
+        if (last_chunk) {                                  // hand-over: x of the launch's last token (every warp has read the old one)
+#pragma unroll
+            for (int ii = 0; ii < 16; ++ii) if (i0 + ii == nv - 1) a.xprev[bh * P + p] = xs[ii];
+        }
+        // X^T tile over the raw x rows: row p, tokens i0 .. i0 + 15, eight to a 16-byte chunk
+        auto store_x = [&]() {
+            const uint32_t at = tX + (uint32_t)(p * 128 + (((i0 >> 3) ^ key_of(p)) << 4));
+#pragma unroll
+            for (int i8 = 0; i8 < 16; i8 += 8) {
+                uint32_t hi[4], lo[4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) split2(xs[i8 + 2 * e], xs[i8 + 2 * e + 1], hi[e], lo[e]);
+                sts128(at ^ (uint32_t)(i8 << 1), hi);
+                sts128((at ^ (uint32_t)(i8 << 1)) + 4096, lo);
+            }
+        };
+        store_x();
+        {
+            const float2 bgm = *reinterpret_cast<const float2*>(&sm.gam[0][2 * k]), bbs = *reinterpret_cast<const float2*>(&sm.gam[1][2 * k]);
+            const float2 cgm = *reinterpret_cast<const float2*>(&sm.gam[2][2 * k]), cbs = *reinterpret_cast<const float2*>(&sm.gam[3][2 * k]);
 #pragma unroll
             for (int i4 = 0; i4 < 16; i4 += 4) {           // four tokens at a time: all lanes read the raw rows, then overwrite them
                 float2 rawb[4], rawc[4];
@@ -447,190 +499,207 @@ ssd_prefill_kernel(const __grid_constant__ CUtensorMap map32, const __grid_const
                     rawb[q] = *reinterpret_cast<const float2*>(&sm.rB[i0 + i4 + q][2 * k]);
                     rawc[q] = *reinterpret_cast<const float2*>(&sm.rC[i0 + i4 + q][2 * k]);
                 }
+                const float4 rb4 = *reinterpret_cast<const float4*>(&sc.rbs[i0 + i4]), rc4 = *reinterpret_cast<const float4*>(&sc.rcs[i0 + i4]);
+                const float rbv[4] = {rb4.x, rb4.y, rb4.z, rb4.w}, rcv[4] = {rc4.x, rc4.y, rc4.z, rc4.w};
                 __syncwarp();
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
                     const int i = i0 + i4 + q;
                     float ang = base + loc[i4 + q];
-                    ang -= TWO_PI * rintf(ang * INV_TWO_PI);                 // into [-pi, pi] for the fast sin / cos
+                    // into [-pi, pi] for the fast sin / cos; the sum with 1.5 * 2^23 rounds to a whole number
+                    ang = fmaf(-TWO_PI, fmaf(ang, INV_TWO_PI, 12582912.f) - 12582912.f, ang);
                     float b0 = 0.f, b1 = 0.f, c0 = 0.f, c1 = 0.f;
                     if (valid(i)) {
-                        const float rb = sc.rbs[i], rc = sc.rcs[i];
-                        const float nb0 = fmaf(rawb[q].x * rb, bgm0, bbs0), nb1 = fmaf(rawb[q].y * rb, bgm1, bbs1);      // model.rs:311-313
-                        const float nc0 = fmaf(rawc[q].x * rc, cgm0, cbs0), nc1 = fmaf(rawc[q].y * rc, cgm1, cbs1);
+                        const float2 nb = norm2(rawb[q], rbv[q], bgm, bbs), nc = norm2(rawc[q], rcv[q], cgm, cbs);                  // model.rs:311-313
                         float sa, ca;
                         __sincosf(ang, &sa, &ca);
-                        b0 = ca * nb0 - sa * nb1;                            // model.rs:345-348
-                        b1 = sa * nb0 + ca * nb1;
-                        c0 = ca * nc0 - sa * nc1;
-                        c1 = sa * nc0 + ca * nc1;
+                        b0 = ca * nb.x - sa * nb.y;                          // model.rs:345-348
+                        b1 = sa * nb.x + ca * nb.y;
+                        c0 = ca * nc.x - sa * nc.y;
+                        c1 = sa * nc.x + ca * nc.y;
                         if (last_chunk && i == nv - 1) {                     // hand-over: B~ of the launch's last token, in fp32
                             a.bprev[bh * N + 2 * k] = b0;
                             a.bprev[bh * N + 2 * k + 1] = b1;
                         }
                     }
                     uint32_t hi, lo;
+                    const uint32_t at = tB + (own ^ (uint32_t)(((i4 + q) & 7) << 4)) + (uint32_t)((i4 + q) * 256);      // C~ lies behind B~
                     split2(b0, b1, hi, lo);
-                    *reinterpret_cast<uint32_t*>(tB + swz(i, 2 * k, 256)) = hi;
-                    *reinterpret_cast<uint32_t*>(tB + 128 + swz(i, 2 * k, 256)) = lo;
+                    sts32(at, hi);
+                    sts32(at + 128, lo);
                     split2(c0, c1, hi, lo);
-                    *reinterpret_cast<uint32_t*>(tC + swz(i, 2 * k, 256)) = hi;
-                    *reinterpret_cast<uint32_t*>(tC + 128 + swz(i, 2 * k, 256)) = lo;
+                    sts32(at + sizeof(sm.rB), hi);
+                    sts32(at + sizeof(sm.rB) + 128, lo);
                 }
-                __syncwarp();
             }
         }
-        __syncthreads();
-        // ---- 2b. this warp's C~ rows as A fragments (hi, lo) from its own rows of the tile
+        __syncwarp();
+        // ---- 3. this warp's C~ rows as A fragments (hi, lo) from its own rows of the tile; then z of its tokens over them, token i's
+        //         32 values at row i, their 16-byte chunks XOR-ed by i % 2
         uint32_t Ch[4][4], Cl[4][4];
+#pragma unroll
+        for (int ks = 0; ks < 4; ++ks) {
+            ldsm_x4(Ch[ks], aC ^ (uint32_t)(ks << 5));
+            ldsm_x4(Cl[ks], (aC ^ (uint32_t)(ks << 5)) + 128);
+        }
+        __syncwarp();
         {
-            const int lm = lane >> 3, lr = lane & 7;
+            const float* zp = a.proj + ((size_t)b * tsl + t0 + i0 + lm) * R + DI + h * P + 4 * lr;
+            const uint32_t dst = tC + (uint32_t)((i0 + lm) * 256 + ((lr ^ (lm & 1)) << 4));
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+                if (valid(i0 + lm + 4 * r))
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + r * 1024u), "l"(zp + (size_t)(4 * r) * R) : "memory");
+        }
+        // G = C~ B~^T against the 16 tokens of segment jp, as accumulators of two 8-column tiles.
+        // Four independent accumulation chains (hi*hi, and hi*lo with lo*hi, of the two tiles), added at the end
+        auto causal_product = [&](int jp, float (&g0)[4], float (&g1)[4]) {
+            float g0b[4], g1b[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) { g0[e] = 0.f; g1[e] = 0.f; g0b[e] = 0.f; g1b[e] = 0.f; }
+            const uint32_t at = aB + (uint32_t)(jp * 4096);
 #pragma unroll
             for (int ks = 0; ks < 4; ++ks) {
-                const int row = 16 * warp + 8 * (lm & 1) + lr, col = 16 * ks + 8 * (lm >> 1);
-                ldsm_x4(Ch[ks], tC + swz(row, col, 256));
-                ldsm_x4(Cl[ks], tC + 128 + swz(row, col, 256));
+                uint32_t bh4[4], bl4[4];
+                ldsm_x4(bh4, at ^ (uint32_t)(ks << 5));
+                ldsm_x4(bl4, (at ^ (uint32_t)(ks << 5)) + 128);
+                mma_bf16(g0, Ch[ks], bh4[0], bh4[1]);
+                mma_bf16(g1, Ch[ks], bh4[2], bh4[3]);
+                mma_bf16(g0b, Ch[ks], bl4[0], bl4[1]);
+                mma_bf16(g1b, Ch[ks], bl4[2], bl4[3]);
+                mma_bf16(g0b, Cl[ks], bh4[0], bh4[1]);
+                mma_bf16(g1b, Cl[ks], bh4[2], bh4[3]);
             }
-        }
-        // ---- 3. Y2 = C~ S^_in^T, G = C~ B~^T (causal part), W = mask / decay (G) (+ D on the diagonal), Y1 = W X
-        float y1[4][4], y2[4][4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) { g0[e] += g0b[e]; g1[e] += g1b[e]; }
+        };
+        // d += W X over the 16 tokens of segment jp
+        auto add_wx = [&](float (&d)[4][4], const float (&w0)[4], const float (&w1)[4], int jp) {
+            uint32_t wh[4], wl[4], xh0[4], xl0[4], xh1[4], xl1[4];
+            split2(w0[0], w0[1], wh[0], wl[0]);
+            split2(w0[2], w0[3], wh[1], wl[1]);
+            split2(w1[0], w1[1], wh[2], wl[2]);
+            split2(w1[2], w1[3], wh[3], wl[3]);
+            const uint32_t x01 = tX + (aP ^ (uint32_t)(jp << 5)), x23 = tX + (aP2 ^ (uint32_t)(jp << 5));
+            ldsm_x4(xh0, x01);
+            ldsm_x4(xl0, x01 + 4096);
+            ldsm_x4(xh1, x23);
+            ldsm_x4(xl1, x23 + 4096);
+            mma3x4(d[0], d[1], d[2], d[3], wh, wl, xh0, xl0, xh1, xl1);
+        };
+        // ---- 4. the segment's own block, which needs this warp's rows only: W = mask / decay (G), lam_i (C~_i . B~_i) + D on the diagonal
+        float y[4][4];
 #pragma unroll
         for (int nt = 0; nt < 4; ++nt)
 #pragma unroll
-            for (int e = 0; e < 4; ++e) { y1[nt][e] = 0.f; y2[nt][e] = 0.f; }
+            for (int e = 0; e < 4; ++e) y[nt][e] = 0.f;
         {
-            // ldmatrix row address of this lane inside a [rows][TSB] tile: matrix m = lane / 8, row r = lane % 8
-            const int lm = lane >> 3, lr = lane & 7;
+            float g0[4], g1[4];
+            causal_product(warp, g0, g1);
+            const float la = sc.ell[ia], lb = sc.ell[ib], ma = sc.lam[ia], mb = sc.lam[ib];
+            // element e of tile q: row (e < 2 ? g4 : g4 + 8), column 8 q + 2 t4 + (e & 1) of the segment
 #pragma unroll
-            for (int ks = 0; ks < 4; ++ks) {
-                uint32_t sh0[4], sl0[4], sh1[4], sl1[4];   // p tiles 0, 1 and 2, 3
-                const int row = 8 * (lm >> 1) + lr, col = 16 * ks + 8 * (lm & 1);
-                ldsm_x4(sh0, tS + swz(row, col, 128));
-                ldsm_x4(sl0, tS + 4096 + swz(row, col, 128));
-                ldsm_x4(sh1, tS + swz(row + 16, col, 128));
-                ldsm_x4(sl1, tS + 4096 + swz(row + 16, col, 128));
-                mma3x4(y2[0], y2[1], y2[2], y2[3], Ch[ks], Cl[ks], sh0, sl0, sh1, sl1);
-            }
-            const int ia = 16 * warp + g4, ib = ia + 8;
-            const float ella = sc.ell[ia], ellb = sc.ell[ib];
-            for (int jp = 0; jp <= warp; ++jp) {           // token columns 16 jp .. 16 jp + 15
-                // six independent accumulation chains (hi*hi, hi*lo, lo*hi of the two 8-column tiles), added at the end
-                float g0[4] = {0.f, 0.f, 0.f, 0.f}, g1[4] = {0.f, 0.f, 0.f, 0.f};
-                float g0b[4] = {0.f, 0.f, 0.f, 0.f}, g1b[4] = {0.f, 0.f, 0.f, 0.f}, g0c[4] = {0.f, 0.f, 0.f, 0.f}, g1c[4] = {0.f, 0.f, 0.f, 0.f};
+            for (int q = 0; q < 2; ++q) {
+                const float2 lj = *reinterpret_cast<const float2*>(&sc.ell[i0 + 8 * q + 2 * t4]), kj = *reinterpret_cast<const float2*>(&sc.kap[i0 + 8 * q + 2 * t4]);
 #pragma unroll
-                for (int ks = 0; ks < 4; ++ks) {
-                    uint32_t bh4[4], bl4[4];
-                    const int row = 16 * jp + 8 * (lm >> 1) + lr, col = 16 * ks + 8 * (lm & 1);
-                    ldsm_x4(bh4, tB + swz(row, col, 256));
-                    ldsm_x4(bl4, tB + 128 + swz(row, col, 256));
-                    mma_bf16(g0, Ch[ks], bh4[0], bh4[1]);
-                    mma_bf16(g1, Ch[ks], bh4[2], bh4[3]);
-                    mma_bf16(g0b, Ch[ks], bl4[0], bl4[1]);
-                    mma_bf16(g1b, Ch[ks], bl4[2], bl4[3]);
-                    mma_bf16(g0c, Cl[ks], bh4[0], bh4[1]);
-                    mma_bf16(g1c, Cl[ks], bh4[2], bh4[3]);
-                }
-#pragma unroll
-                for (int e = 0; e < 4; ++e) { g0[e] += g0b[e] + g0c[e]; g1[e] += g1b[e] + g1c[e]; }
-                // element e of tile q: row (e < 2 ? ia : ib), column 16 jp + 8 q + 2 t4 + (e & 1)
-                float wv[2][4];
-#pragma unroll
-                for (int q = 0; q < 2; ++q)
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        const int i = (e < 2) ? ia : ib, j = 16 * jp + 8 * q + 2 * t4 + (e & 1);
-                        const float gv = q == 0 ? g0[e] : g1[e];
-                        float w = 0.f;
-                        if (j < i) w = gv * __expf(((e < 2) ? ella : ellb) - sc.ell[j]) * sc.kap[j];
-                        else if (j == i) w = fmaf(gv, sc.lam[i], dskip);          // lam_i (C~_i . B~_i) x_i + D x_i
-                        wv[q][e] = w;
-                    }
-                uint32_t wh[4], wl[4];
-                split2(wv[0][0], wv[0][1], wh[0], wl[0]);
-                split2(wv[0][2], wv[0][3], wh[1], wl[1]);
-                split2(wv[1][0], wv[1][1], wh[2], wl[2]);
-                split2(wv[1][2], wv[1][3], wh[3], wl[3]);
-                {
-                    uint32_t xh0[4], xl0[4], xh1[4], xl1[4];
-                    const int row = 8 * (lm >> 1) + lr, col = 16 * jp + 8 * (lm & 1);
-                    ldsm_x4(xh0, tX + swz(row, col, 128));
-                    ldsm_x4(xl0, tX + 4096 + swz(row, col, 128));
-                    ldsm_x4(xh1, tX + swz(row + 16, col, 128));
-                    ldsm_x4(xl1, tX + 4096 + swz(row + 16, col, 128));
-                    mma3x4(y1[0], y1[1], y1[2], y1[3], wh, wl, xh0, xl0, xh1, xl1);
+                for (int e = 0; e < 4; ++e) {
+                    const int i = (e < 2) ? g4 : g4 + 8, j = 8 * q + 2 * t4 + (e & 1);
+                    float& g = q == 0 ? g0[e] : g1[e];
+                    const float below = g * (ex2_ftz((e < 2 ? la : lb) - ((e & 1) ? lj.y : lj.x)) * ((e & 1) ? kj.y : kj.x));
+                    g = j < i ? below : j == i ? fmaf(g, e < 2 ? ma : mb, dskip) : 0.f;
                 }
             }
-            // y = Y1 + e^{l_i} Y2, gated; four lanes of a quad exchange words so that each stores 16 bytes of a row
-            const float ela = sc.eli[ia], elb = sc.eli[ib];
-            uint32_t oh[2][4], ol[2][4];                   // [row a / b][p tile]
-#pragma unroll
-            for (int nt = 0; nt < 4; ++nt) {
-                const float2 ga = *reinterpret_cast<const float2*>(&sm.rz[ia][8 * nt + 2 * t4]);
-                const float2 gb = *reinterpret_cast<const float2*>(&sm.rz[ib][8 * nt + 2 * t4]);
-                split2(fmaf(ela, y2[nt][0], y1[nt][0]) * ga.x, fmaf(ela, y2[nt][1], y1[nt][1]) * ga.y, oh[0][nt], ol[0][nt]);
-                split2(fmaf(elb, y2[nt][2], y1[nt][2]) * gb.x, fmaf(elb, y2[nt][3], y1[nt][3]) * gb.y, oh[1][nt], ol[1][nt]);
-            }
-#pragma unroll
-            for (int rr = 0; rr < 2; ++rr) {
-                const int i = rr == 0 ? ia : ib;
-                uint32_t vh[4], vl[4];
-#pragma unroll
-                for (int r = 0; r < 4; ++r) {
-                    // step r: this lane hands over its word for p tile (t4 - r) & 3 and receives, from lane (t4 + r) & 3
-                    // of its quad, that lane's word for p tile t4
-                    const int give = (t4 - r) & 3, from = (lane & ~3) | ((t4 + r) & 3);
-                    const uint32_t sh_ = give == 0 ? oh[rr][0] : give == 1 ? oh[rr][1] : give == 2 ? oh[rr][2] : oh[rr][3];
-                    const uint32_t sl_ = give == 0 ? ol[rr][0] : give == 1 ? ol[rr][1] : give == 2 ? ol[rr][2] : ol[rr][3];
-                    const uint32_t rh = __shfl_sync(0xffffffffu, sh_, from);
-                    const uint32_t rl = __shfl_sync(0xffffffffu, sl_, from);
-                    const int slot = (t4 + r) & 3;
-                    if (slot == 0) { vh[0] = rh; vl[0] = rl; } else if (slot == 1) { vh[1] = rh; vl[1] = rl; }
-                    else if (slot == 2) { vh[2] = rh; vl[2] = rl; } else { vh[3] = rh; vl[3] = rl; }
-                }
-                if (valid(i)) {
-                    const size_t o = ((size_t)b * tsl + t0 + i) * DI + h * P + 8 * t4;
-                    *reinterpret_cast<uint4*>(a.yhi + o) = make_uint4(vh[0], vh[1], vh[2], vh[3]);
-                    if (a.ylo) *reinterpret_cast<uint4*>(a.ylo + o) = make_uint4(vl[0], vl[1], vl[2], vl[3]);
-                }
-            }
+            add_wx(y, g0, g1, warp);
         }
-        if (warp == 0 && !last_chunk) prepare_scalars(t0 + LCH, sm.sc[(chunk + 1) & 1]);
-        // ---- 4. S^_out = e^{l_last} S^_in + (w x)^T B~  for this warp's 16 x 32 block; new S^ tile for the next chunk
+        // X^T again, now each token times kap and its decay to the end of its segment: what later segments and the state take of it
+#pragma unroll
+        for (int i4 = 0; i4 < 16; i4 += 4) {
+            const float4 w4 = *reinterpret_cast<const float4*>(&sc.xw[i0 + i4]);
+            xs[i4] *= w4.x; xs[i4 + 1] *= w4.y; xs[i4 + 2] *= w4.z; xs[i4 + 3] *= w4.w;
+        }
+        __syncwarp();
+        store_x();
+        __syncthreads();
+        // ---- 5. Y2 = C~ S^_in^T, then the earlier segments one by one: decay over the segment, + G X of its tokens; at the end the decay
+        //         from the start of the own segment to the token.  Every factor is at most 1.
         {
-            const float el = __expf(sc.ell[LCH - 1]);
+            float acc[4][4];
 #pragma unroll
             for (int nt = 0; nt < 4; ++nt)
 #pragma unroll
-                for (int e = 0; e < 4; ++e) S[nt][e] *= el;
-            const int lm = lane >> 3, lr = lane & 7;
+                for (int e = 0; e < 4; ++e) acc[nt][e] = 0.f;
 #pragma unroll
-            for (int ks = 0; ks < 4; ++ks) {               // tokens 16 ks .. 16 ks + 15
-                uint32_t ah[4], al[4];
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const int p = p0 + g4 + 8 * (e & 1), j = 16 * ks + 2 * t4 + 8 * (e >> 1);
-                    const float2 xh = unpack2(*reinterpret_cast<const uint32_t*>(tX + swz(p, j, 128)));
-                    const float2 xl = unpack2(*reinterpret_cast<const uint32_t*>(tX + 4096 + swz(p, j, 128)));
-                    split2((xh.x + xl.x) * sc.wj[j], (xh.y + xl.y) * sc.wj[j + 1], ah[e], al[e]);
-                }
-                {
-                    uint32_t bh0[4], bl0[4], bh1[4], bl1[4];   // state columns n0 .. n0 + 15 and n0 + 16 .. n0 + 31
-                    const int row = 16 * ks + 8 * (lm & 1) + lr, col = n0 + 8 * (lm >> 1);
-                    ldsm_x4_trans(bh0, tB + swz(row, col, 256));
-                    ldsm_x4_trans(bl0, tB + 128 + swz(row, col, 256));
-                    ldsm_x4_trans(bh1, tB + swz(row, col + 16, 256));
-                    ldsm_x4_trans(bl1, tB + 128 + swz(row, col + 16, 256));
-                    mma3x4(S[0], S[1], S[2], S[3], ah, al, bh0, bl0, bh1, bl1);
-                }
+            for (int ks = 0; ks < 4; ++ks) {
+                uint32_t sh0[4], sl0[4], sh1[4], sl1[4];   // p tiles 0, 1 and 2, 3
+                const uint32_t s01 = tS + (aP ^ (uint32_t)(ks << 5)), s23 = tS + (aP2 ^ (uint32_t)(ks << 5));
+                ldsm_x4(sh0, s01);
+                ldsm_x4(sl0, s01 + 4096);
+                ldsm_x4(sh1, s23);
+                ldsm_x4(sl1, s23 + 4096);
+                mma3x4(acc[0], acc[1], acc[2], acc[3], Ch[ks], Cl[ks], sh0, sl0, sh1, sl1);
             }
+            for (int jp = 0; jp < warp; ++jp) {            // tokens 16 jp .. 16 jp + 15
+                float g0[4], g1[4];
+                causal_product(jp, g0, g1);
+                const float f = sc.seg[jp];
+#pragma unroll
+                for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) acc[nt][e] *= f;
+                add_wx(acc, g0, g1, jp);
+            }
+            const float ela = sc.eli[ia], elb = sc.eli[ib];
+#pragma unroll
+            for (int nt = 0; nt < 4; ++nt) {
+                y[nt][0] = fmaf(ela, acc[nt][0], y[nt][0]); y[nt][1] = fmaf(ela, acc[nt][1], y[nt][1]);
+                y[nt][2] = fmaf(elb, acc[nt][2], y[nt][2]); y[nt][3] = fmaf(elb, acc[nt][3], y[nt][3]);
+            }
+        }
+        // gated by silu(z) (model.rs:370); a lane has head dims 8 t4 .. 8 t4 + 7 of its two tokens
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncwarp();
+#pragma unroll
+        for (int rr = 0; rr < 2; ++rr) {
+            const int i = rr == 0 ? ia : ib;
+            const float* const zr = &sm.rC[i][0];
+            const float4 z0 = *reinterpret_cast<const float4*>(zr + ((2 * t4) ^ (i & 1)) * 4), z1 = *reinterpret_cast<const float4*>(zr + ((2 * t4 + 1) ^ (i & 1)) * 4);
+            uint32_t vh[4], vl[4];
+            split2(y[0][2 * rr] * silu_fast(z0.x), y[0][2 * rr + 1] * silu_fast(z0.y), vh[0], vl[0]);
+            split2(y[1][2 * rr] * silu_fast(z0.z), y[1][2 * rr + 1] * silu_fast(z0.w), vh[1], vl[1]);
+            split2(y[2][2 * rr] * silu_fast(z1.x), y[2][2 * rr + 1] * silu_fast(z1.y), vh[2], vl[2]);
+            split2(y[3][2 * rr] * silu_fast(z1.z), y[3][2 * rr + 1] * silu_fast(z1.w), vh[3], vl[3]);
+            if (valid(i)) {
+                const size_t o = ((size_t)b * tsl + t0 + i) * DI + h * P + 8 * t4;
+                *reinterpret_cast<uint4*>(a.yhi + o) = make_uint4(vh[0], vh[1], vh[2], vh[3]);
+                if (a.ylo) *reinterpret_cast<uint4*>(a.ylo + o) = make_uint4(vl[0], vl[1], vl[2], vl[3]);
+            }
+        }
+        if (warp == 0 && !last_chunk) prepare_scalars(t0 + LCH, sm.sc[(chunk + 1) & 1]);
+        // ---- 6. S^ segment by segment: decay over the segment, + X^T B~ of its tokens, for this warp's 16 x 32 block
+        const int pa = p0 + 8 * (lm & 1) + lr;
+        const uint32_t aXA = tX + (uint32_t)(pa * 128 + (((lm >> 1) ^ key_of(pa)) << 4));                          // X^T rows as A fragments
+        const uint32_t aBT = tB + (uint32_t)((8 * (lm & 1) + lr) * 256 + ((((n0 >> 3) + (lm >> 1)) ^ lr) << 4));  // B~ columns n0 .. as B fragments
+#pragma unroll
+        for (int ks = 0; ks < 4; ++ks) {                   // tokens 16 ks .. 16 ks + 15
+            const float f = sc.seg[ks];
+#pragma unroll
+            for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) S[nt][e] *= f;
+            uint32_t ah[4], al[4], bh0[4], bl0[4], bh1[4], bl1[4];   // state columns n0 .. n0 + 15 and n0 + 16 .. n0 + 31
+            const uint32_t xa = aXA ^ (uint32_t)(ks << 5), bt = aBT + (uint32_t)(ks * 4096);
+            ldsm_x4(ah, xa);
+            ldsm_x4(al, xa + 4096);
+            ldsm_x4_trans(bh0, bt);
+            ldsm_x4_trans(bl0, bt + 128);
+            ldsm_x4_trans(bh1, bt ^ 32u);
+            ldsm_x4_trans(bl1, (bt ^ 32u) + 128);
+            mma3x4(S[0], S[1], S[2], S[3], ah, al, bh0, bl0, bh1, bl1);
         }
         // every operand tile and raw row of this chunk has been consumed: order these generic-proxy accesses before the copies
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncthreads();
-        if (!last_chunk) {
-            if (tid == 0) issue_chunk(t0 + LCH);
-            store_state_tile();                            // every warp has read S^_in's tile
-        }
+        if (!last_chunk && tid == 0) issue_chunk(t0 + LCH);
         return true;
     };
     bool failed = false;
@@ -686,7 +755,7 @@ cudaError_t launch_bc_stats(const PrefillArgs& a, int P, int N, cudaStream_t st)
 }
 
 cudaError_t launch_prefill_scan(const PrefillArgs& a, cudaStream_t st) {
-    const size_t smem = sizeof(PfSmem) + 1024;
+    const size_t smem = sizeof(PfSmem);
     static bool set = false;
     if (!set) {
         cudaError_t e = cudaFuncSetAttribute(ssd_prefill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
