@@ -845,6 +845,7 @@ extern "C" void lumi_session_free(lumi_session* s) {
     for (LayerState& L : s->lstate) { if (L.kv) cudaFree(L.kv); if (L.S) cudaFree(L.S); if (L.conv) cudaFree(L.conv); }
     if (s->pos_freq) cudaFree(s->pos_freq);
     if (s->want_idx) cudaFree(s->want_idx);
+    if (s->row_blocks) cudaFree(s->row_blocks);
     if (s->lat_kv) cudaFree(s->lat_kv);
     if (s->ret_seg) cudaFree(s->ret_seg);
     if (s->ctl_host) cudaFreeHost(s->ctl_host);
@@ -1272,6 +1273,13 @@ int32_t attention_block(StepPlan& p, const Layer& L) {
 
 // ---- listed layers ------------------------------------------------------------------------------------------
 // Rows of one pass: nseq sequences (slots b0 ...) x ts tokens; decode steps have ts == 1.
+// The blocks of a pass's rows that prompts of different lengths fill (GemmArgs::row_blocks); none: all rows.
+struct RowBlocks {
+    const int32_t* list = nullptr;
+    int n = 0;
+    void give(GemmArgs& g) const { g.row_blocks = list; g.n_row_blocks = n; }
+};
+
 struct RowPass {
     RowBufs* b;
     int nseq, ts, b0;
@@ -1284,6 +1292,7 @@ struct RowPass {
     // sums of squares there are per row
     const float* gamma_ready = nullptr;
     int ssq_parts = 0;
+    RowBlocks blocks;
     int rows() const { return nseq * ts; }
 };
 
@@ -1299,10 +1308,10 @@ EmbedPost embed_post_of(const lumi_session* s, const RowBufs& b, int slot0, bool
     return e;
 }
 
-// Models with experts keep the persistent kernel's single CTAs, K split by the rows up to 128 of them: a router that meets a near tie falls the
-// other way when the last bits move, and a whole expert with it.  (128 sequences, 16 steps, 32 experts: with the sums of the kernel for few
-// rows one sequence's logits moved by 0.06 of their root mean square, everything else by 1e-4; the distance from 64 bits was the same,
-// 9e-4.)  Pairs of CTAs give the same bits and could be let in; these models have not been measured with them.
+// Models with experts keep the persistent kernel (single CTAs and pairs give the same bits), K split by the rows up to 128 of them: a router that
+// meets a near tie falls the other way when the last bits move, and a whole expert with it.  (128 sequences, 16 steps, 32 experts: with the sums
+// of the kernel for few rows one sequence's logits moved by 0.06 of their root mean square, everything else by 1e-4; the distance from 64 bits
+// was the same, 9e-4.)
 bool has_experts(const lumi_session* s) {
     for (const LayerSpec& L : s->m->cfg.specs) if (L.ff.experts > 0) return true;
     return false;
@@ -1311,7 +1320,8 @@ bool has_experts(const lumi_session* s) {
 // D = act(A W^T) over `rows` rows: tensor cores from the bf16 halves, or the weight-streaming kernel from fp32 rows.  The result
 // goes to out32, or (tensor cores, out_hi given) as bf16 halves only.
 int32_t product(StepPlan& p, int rows, const DevTensor& W, const float* in32, const __nv_bfloat16* hi, const __nv_bfloat16* lo, float* out32,
-                int ldd, int act, __nv_bfloat16* out_hi = nullptr, __nv_bfloat16* out_lo = nullptr, const PostAdd& post = PostAdd()) {
+                int ldd, int act, __nv_bfloat16* out_hi = nullptr, __nv_bfloat16* out_lo = nullptr, const PostAdd& post = PostAdd(),
+                const RowBlocks& blocks = RowBlocks()) {
     lumi_session* s = p.s;
     const int N = (int)W.rows, K = (int)W.cols;
     mark(p);
@@ -1328,7 +1338,8 @@ int32_t product(StepPlan& p, int rows, const DevTensor& W, const float* in32, co
     g.nf.act = act;
     g.nf.out_hi = out_hi;
     g.nf.out_lo = s->opt_split ? out_lo : nullptr;
-    g.few_rows = g.pairs = !has_experts(s);
+    g.few_rows = !has_experts(s);
+    blocks.give(g);
     return launch_gemm_tcgen05(g, p.st_hi);
 }
 
@@ -1353,7 +1364,7 @@ int32_t product_of_x(StepPlan& p, RowPass& r, const DevTensor& W, float* out32, 
     RowBufs& b = *r.b;
     PostAdd post;
     if (r.pending != nullptr) { post.o = b.mix; post.w = r.pending; post.x_out = b.x2; post.width = p.s->m->cfg.d_model; }
-    LUMI_TRY(product(p, r.rows(), W, b.x, b.xh, b.xl, out32, ldd, act, out_hi, out_lo, post));
+    LUMI_TRY(product(p, r.rows(), W, b.x, b.xh, b.xl, out32, ldd, act, out_hi, out_lo, post, r.blocks));
     if (r.pending != nullptr) { std::swap(b.x, b.x2); r.pending = nullptr; }
     return LUMI_OK;
 }
@@ -1413,12 +1424,12 @@ int32_t post_norm_layer(StepPlan& p, RowPass& r, const Layer& L) {
     }
     p.n += n - 1;                                         // mark() counted one
     p.fam = m.kind == MIXER_DELTA ? FAM_OUT_PROJ : FAM_ATTN;
-    LUMI_TRY(product(p, rows, L.s.out, b.y32, b.ah, b.al, b.mix, ldx, 0));
+    LUMI_TRY(product(p, rows, L.s.out, b.y32, b.ah, b.al, b.mix, ldx, 0, nullptr, nullptr, PostAdd(), r.blocks));
     LUMI_TRY(add_normed(p, r, L.s.norm1));
     if (L.spec->ff.ff > 0) {
         p.fam = FAM_ATTN;
         LUMI_TRY(product_of_x(p, r, L.s.up, b.y32, (int)L.s.up.rows, 2, ah, b.al));
-        LUMI_TRY(product(p, rows, L.s.down, b.y32, b.ah, b.al, b.mix, ldx, 0));
+        LUMI_TRY(product(p, rows, L.s.down, b.y32, b.ah, b.al, b.mix, ldx, 0, nullptr, nullptr, PostAdd(), r.blocks));
         LUMI_TRY(add_normed(p, r, L.s.norm2));
     }
     return LUMI_OK;
@@ -1466,7 +1477,8 @@ int32_t norm_product(StepPlan& p, RowPass& r, const DevTensor& W, const float* g
         g.ext = &ex;
     }
     mark(p);
-    g.few_rows = g.pairs = !has_experts(s);
+    g.few_rows = !has_experts(s);
+    r.blocks.give(g);
     return launch_gemm_tcgen05(g, p.st_hi);
 }
 
@@ -1489,7 +1501,8 @@ int32_t residual_product(StepPlan& p, RowPass& r, const DevTensor& W, const floa
     g.nf.bias = bias;
     g.nf.gamma_next = gamma_next; g.nf.out_hi = b.xh; g.nf.out_lo = s->opt_split ? b.xl : nullptr;
     g.nf.ssq_out = b.ssq; g.nf.ssq_stride = b.ssq_stride;
-    g.few_rows = g.pairs = !has_experts(s);
+    g.few_rows = !has_experts(s);
+    r.blocks.give(g);
     LUMI_TRY(launch_gemm_tcgen05(g, p.st_hi));
     r.gamma_ready = gamma_next;
     r.ssq_parts = (N + 31) / 32;
@@ -1505,8 +1518,9 @@ struct GroupedProduct {
     const float* bias; const float* mul; int ldmul;
     float* out32; int ld32; __nv_bfloat16 *oh, *ol; int ldo;
 };
-int32_t grouped_product(StepPlan& p, int rows, const GroupedProduct& q) {
+int32_t grouped_product(StepPlan& p, const RowPass& r, const GroupedProduct& q) {
     lumi_session* s = p.s;
+    const int rows = r.rows();
     mark(p);
     if (!p.tc) {
         const BlockProductArgs a{q.a32, q.lda32, q.a_step, q.W->p, q.W->dtype, (int)q.W->cols, q.group_rows, q.bias, q.mul, q.ldmul, q.out32, q.ld32, q.out_step,
@@ -1523,7 +1537,8 @@ int32_t grouped_product(StepPlan& p, int rows, const GroupedProduct& q) {
     g.nf.out_hi = q.oh;
     g.nf.out_lo = s->opt_split ? q.ol : nullptr;
     g.ext = &ex;
-    g.few_rows = g.pairs = !has_experts(s);
+    g.few_rows = !has_experts(s);
+    r.blocks.give(g);
     return launch_gemm_tcgen05(g, p.st_hi);
 }
 
@@ -1583,7 +1598,7 @@ int32_t rglru_mixer(StepPlan& p, RowPass& r, const Layer& L, int li) {
     LUMI_CUDA(launch_rglru_conv(a, p.st_lo));
     const GroupedProduct q{&L.s.rg, m.blocks, 2 * bp, bs, 2 * bp, 2 * bp, b.qkv, m.channels, bs, b.bh, b.bl, L.s.rg_b, nullptr, 0, b.gates, m.blocks * 2 * bp,
                            nullptr, nullptr, 0};
-    LUMI_TRY(grouped_product(p, r.rows(), q));
+    LUMI_TRY(grouped_product(p, r, q));
     mark(p);
     int n = 0;
     LUMI_CUDA(launch_rglru_scan(a, p.st_lo, &n));
@@ -1631,12 +1646,12 @@ int32_t latent_mixer(StepPlan& p, RowPass& r, const Layer& L, int li) {
     if (!expand) {
         const GroupedProduct uk{&L.s.uk, m.heads, ls.lp, m.dim, ls.lp, ls.row, b.proj + L.s.off_q, ldp, ls.dk, b.lh, b.ll, nullptr, nullptr, 0, b.qlat, m.heads * ls.row,
                                 nullptr, nullptr, 0};
-        LUMI_TRY(grouped_product(p, rows, uk));
+        LUMI_TRY(grouped_product(p, r, uk));
         mark(p);
         LUMI_CUDA(launch_latent_attention(a, p.st_hi));
         const GroupedProduct uv{&L.s.uv, m.heads, (int)(L.s.uv.rows / m.heads), m.kv_rank, m.vdim, m.vdim, b.ctx, m.heads * ls.lp, ls.lp, b.lh, b.ll, nullptr,
                                 b.proj + L.s.off_g, ldp, b.y32, (int)L.s.out.cols, p.tc ? b.ah : nullptr, p.tc ? b.al : nullptr, (int)L.s.out.cols};
-        return grouped_product(p, rows, uv);
+        return grouped_product(p, r, uv);
     }
     // keys and values per head for a few sequences' rings at a time, then attention over them (pages of a slot lie together)
     const int ring = s->pages_per_seq * kPageTokens, hw = ls.dk_pad + ls.dv_pad, ld = m.heads * hw, chunk = latent_expand_seqs(s, m, r.nseq);
@@ -1685,6 +1700,7 @@ int32_t experts_ff(StepPlan& p, RowPass& r, const Layer& L, const float* gamma_n
         RowPass rp{&part, std::min(e.rows, rows - r0), 1, 0, nullptr, -1};
         rp.gamma_ready = r.gamma_ready;
         rp.ssq_parts = r.ssq_parts;
+        if (rp.rows() == rows) rp.blocks = r.blocks;
         LUMI_TRY(norm_product(p, rp, L.s.router, L.s.norm2, nullptr, e.logits, (int)L.s.router.rows));
         MoeArgs a{};
         a.logits = e.logits; a.ldl = (int)L.s.router.rows;
@@ -1699,6 +1715,7 @@ int32_t experts_ff(StepPlan& p, RowPass& r, const Layer& L, const float* gamma_n
             continue;
         }
         a.gh = e.gh; a.gl = s->opt_split ? e.gl : nullptr; a.y = e.y;
+        if (r.blocks.list != nullptr) { a.row_len = r.row_len; a.ts = r.ts; a.t_abs0 = r.t_abs0; a.b0 = r.b0; a.row0 = r0; }
         a.gamma_next = gamma_next; a.xh = part.xh; a.xl = s->opt_split ? part.xl : nullptr; a.ssq = part.ssq; a.ssq_stride = b.ssq_stride;
         mark(p);
         LUMI_CUDA(launch_moe_route(a, p.st_hi));
@@ -2165,10 +2182,35 @@ bool use_chunked_prefill(lumi_session* s, int batch, int T, bool scored = false)
     return use_rows_prefill(s, batch, T) && rows_workspace(s, batch, T, scored);
 }
 
+// Blocks of rows that the prompts fill, for every slice of the slice loops (in their order) of prompts of different lengths.  Behind a prompt's end a
+// slice's rectangle is padding: with lengths spread evenly up to the longest that is nearly half of all rows, and products take most of a
+// prompt's time (48 prompts of 64 to 512 tokens, 12 layers of width 1024, experts: 22.9 -> 17.2 ms).
+int32_t slice_blocks(lumi_session* s, int batch, int nb_max, int T, int TS, const int32_t* lens_host, std::vector<RowBlocks>& out) {
+    std::vector<int32_t> all;
+    for (int b0 = 0; b0 < batch; b0 += nb_max)
+        for (int t0 = 0; t0 < T; t0 += TS) {
+            const int ts = std::min(TS, T - t0);
+            const size_t first = all.size();
+            for (int q = 0; q < std::min(nb_max, batch - b0); ++q) {
+                const int n = std::max(0, std::min(ts, lens_host[b0 + q] - t0));
+                if (n == 0) continue;
+                const long r0 = (long)q * ts;
+                for (int32_t k = (int32_t)(r0 / kRowBlock); k <= (int32_t)((r0 + n - 1) / kRowBlock); ++k)
+                    if (all.size() == first || all.back() < k) all.push_back(k);
+            }
+            out.push_back(RowBlocks{nullptr, (int)(all.size() - first)});
+        }
+    if (all.size() > s->row_blocks_cap) LUMI_TRY(grow(s->row_blocks, s->row_blocks_cap, all.size()));
+    LUMI_CUDA(cudaMemcpyAsync(s->row_blocks, all.data(), sizeof(int32_t) * all.size(), cudaMemcpyHostToDevice, s->stream));
+    size_t at = 0;
+    for (RowBlocks& r : out) { r.list = s->row_blocks + at; at += r.n; }
+    return LUMI_OK;
+}
+
 // The slice loop for designs that list their layers: slices of up to slice_max tokens per sequence, each through every layer
 // with the caches and states carried from slice to slice.  Arguments as for prefill_chunked.
 int32_t prefill_listed(lumi_session* s, int batch, int T, bool with_head, float* score_out, const int32_t* lens, int slot0,
-                       const std::vector<int32_t>* want, float* want_out) {
+                       const std::vector<int32_t>* want, float* want_out, const int32_t* lens_host) {
     const Config& c = s->m->cfg;
     const int ldx = c.x_ld(), V = c.vocab;
     const int nb_max = std::min(batch, 2048);
@@ -2205,12 +2247,15 @@ int32_t prefill_listed(lumi_session* s, int batch, int T, bool with_head, float*
     }
     LUMI_TRY(ensure_latent_rows(s, b, lat_rows));
     if (want != nullptr && want->size() > s->want_cap) LUMI_TRY(grow(s->want_idx, s->want_cap, want->size()));
-    size_t wanted = 0;
+    std::vector<RowBlocks> blocks;
+    if (lens_host != nullptr) LUMI_TRY(slice_blocks(s, batch, nb_max, T, TS, lens_host, blocks));
+    size_t wanted = 0, slice = 0;
     std::vector<int32_t> local;                           // outlives the copies below (synchronised before it changes)
     for (int b0 = 0; b0 < batch; b0 += nb_max) {
         const int nb = std::min(nb_max, batch - b0);
         for (int t0 = 0; t0 < T; t0 += TS) {
             RowPass r{&b, nb, std::min(TS, T - t0), slot0 + b0, lens, t0};
+            if (!blocks.empty()) r.blocks = blocks[slice++];
             const int M = r.rows();
             StepPlan p{s, M, use_tc(s, M)};
             p.st_hi = p.st_lo = s->stream;
@@ -2271,11 +2316,11 @@ int32_t prefill_listed(lumi_session* s, int batch, int T, bool with_head, float*
 // lens (device, [batch]) != null: prompts of different lengths inside the [T][batch] rectangle (T = the longest): every sequence
 // ends in the state after its own last token, x holds the residual at that token, and padding is never looked at.
 // slot0: slot of the first sequence (designs that list their layers; 0 otherwise).  want (host, ascending prompt positions, one
-// sequence): logits of those positions go to want_out (device, [n_want][vocab]).
+// sequence): logits of those positions go to want_out (device, [n_want][vocab]).  lens_host: lens as the caller has it.
 int32_t prefill_chunked(lumi_session* s, int batch, int T, bool with_head, float* score_out = nullptr, const int32_t* lens = nullptr,
-                        int slot0 = 0, const std::vector<int32_t>* want = nullptr, float* want_out = nullptr) {
+                        int slot0 = 0, const std::vector<int32_t>* want = nullptr, float* want_out = nullptr, const int32_t* lens_host = nullptr) {
     const Config& c = s->m->cfg;
-    if (c.stacked()) return prefill_listed(s, batch, T, with_head, score_out, lens, slot0, want, want_out);
+    if (c.stacked()) return prefill_listed(s, batch, T, with_head, score_out, lens, slot0, want, want_out, lens_host);
     const int D = c.d_model, DI = c.d_inner(), R = c.in_proj_out();
     const bool hybrid = s->m->n_attn > 0;
     const PrefillPass ps = prefill_pass(s, batch, T, s->pf_pass);
@@ -2283,6 +2328,10 @@ int32_t prefill_chunked(lumi_session* s, int batch, int T, bool with_head, float
     const int KVD = hybrid ? c.kv_dim() : 0, Q = D + 2 * KVD, MLP = hybrid ? c.mlp_dim() : 0;
     const int nb_max = ps.nb, TS = ps.ts;
     LUMI_TRY(prefill_workspace(s, ps, score_out != nullptr));
+    std::vector<RowBlocks> blocks;
+    if (lens_host != nullptr && tc) LUMI_TRY(slice_blocks(s, batch, nb_max, T, TS, lens_host, blocks));
+    size_t slice = 0;
+    RowBlocks live;                                                     // the slice's
     const size_t B = s->max_batch;
     __nv_bfloat16* const hi = tc ? s->pf_hi : nullptr;
     __nv_bfloat16* const lo = tc && s->opt_split ? s->pf_lo : nullptr;
@@ -2303,6 +2352,7 @@ int32_t prefill_chunked(lumi_session* s, int batch, int T, bool with_head, float
         GemmArgs g{hi + r0 * K, lo ? lo + r0 * K : nullptr, (const __nv_bfloat16*)W.p, out, N, rows, N, K, accumulate, &s->ctl->status,
                    scan ? nullptr : s->gemm_counters, kGemmCounters, s->gemm_scratch, kGemmScratchFloats};
         g.few_rows = !scan;
+        live.give(g);
         return launch_gemm_tcgen05(g, s->stream);
     };
     for (int b0 = 0; b0 < batch; b0 += nb_max) {
@@ -2310,6 +2360,7 @@ int32_t prefill_chunked(lumi_session* s, int batch, int T, bool with_head, float
         for (int t0 = 0; t0 < T; t0 += TS) {
             const int ts = std::min(TS, T - t0);
             const int M = nb * ts;
+            if (!blocks.empty()) live = blocks[slice++];
             LUMI_CUDA(launch_prefill_embed(s->m->embedding.p, s->m->embedding.dtype, s->prompt_dev, s->pf_x, D, c.vocab, M, ts, t0, b0,
                                            batch, s->ctl, s->stream, lens));
             s->launches += 1;
@@ -2510,7 +2561,7 @@ extern "C" int32_t lumi_prefill_ragged(lumi_session* s, const uint32_t* tokens, 
     if (chunked) s->ctl_host->prompt_pos = longest;
     LUMI_TRY(push_ctl(s));
     if (chunked) {
-        LUMI_TRY(prefill_chunked(s, batch, longest, false, nullptr, s->row_len));
+        LUMI_TRY(prefill_chunked(s, batch, longest, false, nullptr, s->row_len, 0, nullptr, nullptr, lengths));
     } else {
         const bool mega = s->opt_mega;
         s->opt_mega = 0;
@@ -3015,6 +3066,7 @@ extern "C" int32_t lumi_debug_gemm(const lumi_gemm_probe* q) {
                (int32_t*)q->status_word, ks.counters, ks.n_counters, ks.scratch, ks.floats};
     g.few_rows = q->few_rows != 0;
     g.pairs = q->pairs != 0;
+    g.row_blocks = (const int32_t*)q->row_blocks; g.n_row_blocks = q->n_row_blocks;
     if (q->status_word) { g.wait_limit_ns = q->wait_limit_ns; g.debug_skip_unit = q->skip_unit; }
     g.nf.ssq_in = (const float*)q->ssq_in; g.nf.ssq_parts = q->ssq_parts; g.nf.ssq_stride = q->ssq_stride; g.nf.inv_k = q->inv_k; g.nf.eps = q->eps;
     g.nf.gamma_next = (const float*)q->gamma_next; g.nf.out_hi = (__nv_bfloat16*)q->out_hi; g.nf.out_lo = (__nv_bfloat16*)q->out_lo;

@@ -25,6 +25,7 @@ int32_t gemm_tcgen05_init();
 
 namespace {
 
+static_assert(kRowBlock == 32, "a row block is what an epilogue warp owns");
 constexpr int BM = 128;
 constexpr int kSmemBudget = 196608;          // bytes of pipeline stages
 constexpr int kMaxSplits = 4;                // K split over at most this many CTAs
@@ -263,7 +264,7 @@ __global__ void __launch_bounds__(192, 1)
 gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_ahi, const __grid_constant__ CUtensorMap map_alo,
                        const __grid_constant__ CUtensorMap map_w, float* D, int ldd, int M, int N, int K,
                        int accumulate, int tiles_m, int ntiles, int splits, int32_t* tile_counters, float* scratch, int32_t* status,
-                       uint64_t wait_ns, int skip_unit, NormFuse nf, GemmExt ex) {
+                       uint64_t wait_ns, int skip_unit, NormFuse nf, GemmExt ex, const int32_t* __restrict__ row_blocks, int n_blocks) {
     using T = Tile<BN, SPLIT, 1, PAIR>;
     constexpr int S = T::STAGES;
     const int rank = PAIR ? (int)(blockIdx.x & 1) : 0, unit0 = PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x, units_at_once = PAIR ? (int)(gridDim.x >> 1) : (int)gridDim.x;
@@ -351,6 +352,12 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_ahi, const __grid
         return p;
     };
     const bool by_rows = EXT && ex.tiles != nullptr;      // the tiles are known only behind the dependency wait
+    // Row blocks given: a row tile is four (a pair: eight) blocks of kRowBlock rows from anywhere in A, one per epilogue warp, and m0 counts
+    // gathered rows.  Blocks past the last one read as zeros and are not stored.
+    auto block_row = [&](int m) {
+        const int i = m / kRowBlock;
+        return i < n_blocks ? __ldg(row_blocks + i) * kRowBlock : M;
+    };
     if (!PAIR && !by_rows && warp == 0 && lane == 0 && (int)blockIdx.x < ntiles * splits && (int)blockIdx.x != skip_unit) {
         const int t = blockIdx.x / splits, sp = blockIdx.x - t * splits;
         const int n0 = place(t).n0;
@@ -375,11 +382,30 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_ahi, const __grid
                 const Place pl = place(t);
                 const int m0 = pl.m0, n0 = pl.n0;
                 const int kb0 = sp * num_kb / splits, kb1 = (sp + 1) * num_kb / splits;
+                int blk[BM / kRowBlock];
+                if (row_blocks != nullptr)
+#pragma unroll
+                    for (int j = 0; j < BM / kRowBlock; ++j) blk[j] = block_row(m0 + j * kRowBlock);
                 for (int kb = kb0; kb < kb1; ++kb, ++kbg) {
                     const int s = kbg % S;
                     const uint32_t ph = (kbg / S) & 1u;
                     if (!mbar_wait(&empty_bar[s], ph ^ 1u, wait_ns)) { timed_out = true; break; }
                     uint8_t* st = base + s * T::STAGE;
+                    if (row_blocks != nullptr) {
+                        const uint32_t bar = PAIR ? map_to_rank(smem_u32(&full_bar[s]), 0) : smem_u32(&full_bar[s]);
+                        if (PAIR ? rank == 0 : kbg >= pre) mbar_expect_tx(&full_bar[s], (PAIR ? 2u : 1u) * (uint32_t)T::STAGE);
+                        auto load = [&](void* dst, const CUtensorMap* map, int x, int y) {
+                            if constexpr (PAIR) tma_load_2d_pair(dst, map, bar, x, y);
+                            else tma_load_2d(dst, map, &full_bar[s], x, y);
+                        };
+#pragma unroll
+                        for (int j = 0; j < BM / kRowBlock; ++j) {
+                            load(st + j * kRowBlock * BK * 2, &map_ahi, pl.k0 + kb * BK, blk[j]);
+                            if (SPLIT) load(st + T::A_BYTES + j * kRowBlock * BK * 2, &map_alo, pl.k0 + kb * BK, blk[j]);
+                        }
+                        if (PAIR || kbg >= pre) load(st + T::A_BYTES * (SPLIT ? 2 : 1), &map_w, kb * BK, n0 + (PAIR ? rank * (BN / 2) : 0));
+                        continue;
+                    }
                     if constexpr (PAIR) {        // both CTAs' copies complete on the first one's barrier
                         const uint32_t bar = map_to_rank(smem_u32(&full_bar[s]), 0);
                         if (rank == 0) mbar_expect_tx(&full_bar[s], 2u * (uint32_t)T::STAGE);
@@ -459,9 +485,10 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_ahi, const __grid
             // sums of squares arrive as `ssq_parts` partial sums per row (one per 32 columns of x, added in column order,
             // so the result does not depend on any tile shape) and the scale multiplies the accumulator below.
             // Read while the tensor core still works on this tile.
+            const int row = row_blocks != nullptr ? block_row(m0 + q * 32) + lane : m0 + q * 32 + lane;
             float rs = 1.0f;
-            if (nf.ssq_in != nullptr && m0 + q * 32 + lane < M) {
-                const float* pp = nf.ssq_in + (size_t)(m0 + q * 32 + lane) * nf.ssq_stride;
+            if (nf.ssq_in != nullptr && row < M) {
+                const float* pp = nf.ssq_in + (size_t)row * nf.ssq_stride;
                 float t = 0.f;
                 int pz = 0;
                 if ((nf.ssq_stride & 3) == 0) {
@@ -510,7 +537,6 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_ahi, const __grid
                 last = __shfl_sync(0xffffffffu, last, 0);
                 if (last) {
                     __threadfence();
-                    const int row = m0 + row_l;
                     const int nlim = min(N, n0 + BN);
                     if (row < M) {
                         // 16 columns at a time: the residual and every split's partial are requested together, added in
@@ -587,7 +613,6 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_ahi, const __grid
                 }
                 continue;
             }
-            const int row = m0 + q * 32 + lane;
             if constexpr (EXT) {
 #pragma unroll 1
                 for (int cb = 0; cb < BN / 32; ++cb) {
@@ -750,17 +775,20 @@ int sm_count_gemm() {
     return n;
 }
 
+// Rows that the row tiles cover.
+int tiled_rows(const GemmArgs& a) { return a.row_blocks != nullptr ? a.n_row_blocks * kRowBlock : a.M; }
+
 template <int BN, bool SPLIT, bool EXT = false, bool PAIR = false>
 int32_t launch_persistent(const GemmArgs& a, int splits, cudaStream_t st) {
     using T = Tile<BN, SPLIT, 1, PAIR>;
     CUtensorMap mh, ml, mw;
-    const int lda = EXT ? a.ext->lda : a.K;
-    LUMI_TRY(make_map(&mh, a.a_hi, a.M, lda, BM));
-    LUMI_TRY(make_map(&ml, SPLIT ? a.a_lo : a.a_hi, a.M, lda, BM));
+    const int lda = EXT ? a.ext->lda : a.K, box = a.row_blocks != nullptr ? kRowBlock : BM;
+    LUMI_TRY(make_map(&mh, a.a_hi, a.M, lda, box));
+    LUMI_TRY(make_map(&ml, SPLIT ? a.a_lo : a.a_hi, a.M, lda, box));
     LUMI_TRY(make_map(&mw, a.w, a.N, a.K, PAIR ? BN / 2 : BN));
     auto kern = gemm_persistent_kernel<BN, SPLIT, EXT, PAIR>;
     LUMI_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, T::SMEM));
-    const int tiles_m = (a.M + (PAIR ? 2 * BM : BM) - 1) / (PAIR ? 2 * BM : BM);
+    const int tiles_m = (tiled_rows(a) + (PAIR ? 2 * BM : BM) - 1) / (PAIR ? 2 * BM : BM);
     const int tiles_n = EXT ? (a.ext->group_rows + BN - 1) / BN * (a.ext->tiles != nullptr ? 1 : a.ext->groups) : (a.N + BN - 1) / BN;
     const int ntiles = (EXT && a.ext->tiles != nullptr ? a.ext->max_tiles : tiles_m) * tiles_n;      // by rows: as many as there can be
     const int units = ntiles * splits;
@@ -781,7 +809,7 @@ int32_t launch_persistent(const GemmArgs& a, int splits, cudaStream_t st) {
         ++cfg.numAttrs;
     }
     LUMI_CUDA(cudaLaunchKernelEx(&cfg, kern, mh, ml, mw, a.d, a.ldd, a.M, a.N, a.K, a.accumulate, tiles_m, ntiles, splits, a.tile_counters,
-                                 a.scratch, a.status_word, a.wait_limit_ns ? a.wait_limit_ns : kWaitLimitNs, a.debug_skip_unit, a.nf, EXT ? *a.ext : GemmExt()));
+                                 a.scratch, a.status_word, a.wait_limit_ns ? a.wait_limit_ns : kWaitLimitNs, a.debug_skip_unit, a.nf, EXT ? *a.ext : GemmExt(), a.row_blocks, a.n_row_blocks));
     return LUMI_OK;
 }
 
@@ -844,11 +872,12 @@ int32_t gemm_tcgen05_init() {
 // (measured at 64 x 1024 x 2048: 19.1 us against 23.2 us, +12.6 % tokens per second on the 64-sequence decode; wide split
 // tiles lost more in the fix-up than they gained).
 // LUMI_GEMM_SPLITK=1 turns splitting off.
+static bool width_counts(const GemmArgs& a);
 static void pick_tile(const GemmArgs& a, int* width, int* splits) {
     static const int widths[] = {256, 224, 208, 192, 160, 128, 96, 64, 32};
     static const int env_splits = getenv("LUMI_GEMM_SPLITK") ? atoi(getenv("LUMI_GEMM_SPLITK")) : kMaxSplits;
     const int max_splits = env_splits < 1 ? 1 : (env_splits > kMaxSplits ? kMaxSplits : env_splits);
-    const long tiles_m = (a.M + BM - 1) / BM;
+    const long tiles_m = ((width_counts(a) ? a.M : tiled_rows(a)) + BM - 1) / BM;
     const int num_kb = a.K / BK;
     const long sms = sm_count_gemm();
     int best = 256;
@@ -862,7 +891,7 @@ static void pick_tile(const GemmArgs& a, int* width, int* splits) {
     }
     *width = best;
     *splits = 1;
-    if (max_splits < 2 || tiles_m > 1 || a.tile_counters == nullptr || a.scratch == nullptr) return;   // one row tile only: 256 rows measured 3 % slower split
+    if (max_splits < 2 || tiles_m > 1 || a.row_blocks != nullptr || a.tile_counters == nullptr || a.scratch == nullptr) return;   // one row tile only: 256 rows measured 3 % slower split
     const long a_kb = a.a_lo != nullptr ? 32 : 16;                   // KiB of activations per k-block of a 128-row tile
     const long unsplit = best_rounds * num_kb * (a_kb + best / 8);   // KiB through one CTA
     long best_split = -1;
@@ -882,7 +911,32 @@ void gemm_tcgen05_plan(const GemmArgs& a, int* width, int* splits) { pick_tile(a
 // Products that gemm_few_rows.cu takes.
 static bool few_rows(const GemmArgs& a) {
     static const bool on = !(getenv("LUMI_FEW_ROWS") && atoi(getenv("LUMI_FEW_ROWS")) == 0);      // 0: tuning aid
-    return on && a.few_rows && (a.ext == nullptr || a.ext->tiles == nullptr) && gemm_few_rows_takes(a);
+    return on && a.few_rows && a.row_blocks == nullptr && (a.ext == nullptr || a.ext->tiles == nullptr) && gemm_few_rows_takes(a);
+}
+
+// A strip of columns that a tile's end cuts (widths of 208) rounds the scaled sum once more before the bias is added, so the width shows in the last bit
+// of a product with both a folded norm and a bias.  Such products keep the width that all of their rows have with single CTAs: a prompt among others of other
+// lengths, and models with experts above all, get the same bits as ever.
+static bool width_counts(const GemmArgs& a) { return a.ext == nullptr && a.nf.ssq_in != nullptr && a.nf.bias != nullptr; }
+
+// Tile width for pairs of CTAs (256-row tiles, half as many workers), or 0 where single CTAs take the product.  Widths whose half is a multiple
+// of 32: 208 was 15 % slower than single CTAs of that width.  Measured with blocked tiles, pair / single, microseconds: 4096 rows 7360 x 1024
+// 104.5 / 115.6, 1024 x 2048 33.5 / 33.7, 6208 x 1024 89 / 101; 32768 rows 735 / 771, 173 / 189, 625 / 720, 8192 x 2048 1403 / 1497; below 4096 rows
+// half as many, twice as high tiles leave more of the last round idle (2048 rows 1024 x 2048 23.6 / 22.1).  The results are the same bits as
+// single CTAs', at every width of either (but see above).
+static int pair_width(const GemmArgs& a) {
+    static const bool on = !(getenv("LUMI_GEMM_PAIR") && atoi(getenv("LUMI_GEMM_PAIR")) == 0);      // 0: tuning aid
+    if (!on || !a.pairs || a.a_lo == nullptr || tiled_rows(a) < kPairMinRows || width_counts(a)) return 0;
+    const long tiles_m = (tiled_rows(a) + 2 * BM - 1) / (2 * BM), workers = sm_count_gemm() / 2;
+    const int groups = a.ext != nullptr ? a.ext->groups : 1, cols = a.N / groups;
+    int best = 0;
+    long best_cost = -1;
+    for (int w : {256, 192, 128}) {
+        if (a.ext != nullptr && w == 192) continue;       // tiles of groups: widths of which groups are whole multiples or close to it
+        const long tiles = tiles_m * groups * ((cols + w - 1) / w), cost = (tiles + workers - 1) / workers * (w + 32);
+        if (best_cost < 0 || cost < best_cost) { best = w; best_cost = cost; }
+    }
+    return best;
 }
 
 // Products in groups and gated results.
@@ -895,7 +949,15 @@ static int32_t launch_ext(const GemmArgs& a, cudaStream_t st) {
         return fail(LUMI_E_INVALID, "tcgen05 GEMM in groups: %d groups of %d rows of W, N %d, rows of A of %d elements", e.groups, e.group_rows, a.N, e.lda);
     LUMI_TRY(gemm_tcgen05_init());
     if (few_rows(a)) return launch_gemm_few_rows(a, st);
-    const long tiles_m = by_rows ? e.max_tiles : (a.M + BM - 1) / BM;
+    const bool split = a.a_lo != nullptr;
+    if (!by_rows) {
+        switch (pair_width(a)) {
+            case 256: return launch_persistent<256, true, true, true>(a, 1, st);
+            case 128: return launch_persistent<128, true, true, true>(a, 1, st);
+            default: break;
+        }
+    }
+    const long tiles_m = by_rows ? e.max_tiles : (tiled_rows(a) + BM - 1) / BM;
     int best = 256;
     long best_cost = -1;
     for (int w : {256, 128, 64, 32}) {
@@ -904,29 +966,10 @@ static int32_t launch_ext(const GemmArgs& a, cudaStream_t st) {
         const long cost = rounds * (w + 32);
         if (best_cost < 0 || cost < best_cost) { best = w; best_cost = cost; }
     }
-    const bool split = a.a_lo != nullptr;
 #define LUMI_EXT_CASE(W) if (best == W) return split ? launch_persistent<W, true, true>(a, 1, st) : launch_persistent<W, false, true>(a, 1, st);
     LUMI_EXT_CASE(256) LUMI_EXT_CASE(128) LUMI_EXT_CASE(64) LUMI_EXT_CASE(32)
 #undef LUMI_EXT_CASE
     return LUMI_OK;
-}
-
-// Tile width for pairs of CTAs (256-row tiles, half as many workers), or 0 where single CTAs take the product.  Widths whose half is a multiple
-// of 32: 208 was 15 % slower than single CTAs of that width.  Measured with blocked tiles, pair / single, microseconds: 4096 rows 7360 x 1024
-// 104.5 / 115.6, 1024 x 2048 33.5 / 33.7, 6208 x 1024 89 / 101; 32768 rows 735 / 771, 173 / 189, 625 / 720, 8192 x 2048 1403 / 1497; below 4096 rows
-// half as many, twice as high tiles leave more of the last round idle (2048 rows 1024 x 2048 23.6 / 22.1).  The results are the same bits as
-// single CTAs', at every width of either.
-static int pair_width(const GemmArgs& a) {
-    static const bool on = !(getenv("LUMI_GEMM_PAIR") && atoi(getenv("LUMI_GEMM_PAIR")) == 0);      // 0: tuning aid
-    if (!on || !a.pairs || a.a_lo == nullptr || a.M < kPairMinRows) return 0;
-    const long tiles_m = (a.M + 2 * BM - 1) / (2 * BM), workers = sm_count_gemm() / 2;
-    int best = 0;
-    long best_cost = -1;
-    for (int w : {256, 192, 128}) {
-        const long tiles = tiles_m * ((a.N + w - 1) / w), cost = (tiles + workers - 1) / workers * (w + 32);
-        if (best_cost < 0 || cost < best_cost) { best = w; best_cost = cost; }
-    }
-    return best;
 }
 
 int32_t launch_gemm_tcgen05(const GemmArgs& a, cudaStream_t st) {
@@ -934,6 +977,16 @@ int32_t launch_gemm_tcgen05(const GemmArgs& a, cudaStream_t st) {
         return fail(LUMI_E_UNSUPPORTED, "tcgen05 GEMM needs K %% 64 == 0 (M %d N %d K %d)", a.M, a.N, a.K);
     if ((reinterpret_cast<uintptr_t>(a.a_hi) | reinterpret_cast<uintptr_t>(a.w) | reinterpret_cast<uintptr_t>(a.a_lo)) & 15)
         return fail(LUMI_E_INVALID, "tcgen05 GEMM operands must be 16-byte aligned");
+    if (a.row_blocks != nullptr) {
+        // below, every row is taken: few rows have kernels and splits of K of their own, and a list that leaves little out saves little
+        if (a.n_row_blocks < 0) return fail(LUMI_E_INVALID, "tcgen05 GEMM: %d row blocks", a.n_row_blocks);
+        if (a.M <= kFewRowsMax || (long)a.n_row_blocks * kRowBlock * 16 > (long)a.M * 15 || (a.ext != nullptr && a.ext->tiles != nullptr)) {
+            GemmArgs all = a;
+            all.row_blocks = nullptr;
+            return launch_gemm_tcgen05(all, st);
+        }
+        if (a.n_row_blocks == 0) return LUMI_OK;
+    }
     if (a.ext != nullptr) return launch_ext(a, st);
     LUMI_TRY(gemm_tcgen05_init());
     const bool split = a.a_lo != nullptr;

@@ -337,6 +337,7 @@ struct lumi_session {
     int slice_max = 0;                 // most tokens of a sequence per pass (what the ring leaves beside the widest window)
     double* pos_freq = nullptr;        // [d_model / 2] frequencies of the position vectors
     int32_t* want_idx = nullptr; size_t want_cap = 0;
+    int32_t* row_blocks = nullptr; size_t row_blocks_cap = 0;       // rows that prompts of different lengths have, slice by slice
     // activations
     float *x = nullptr, *proj = nullptr, *y32 = nullptr, *logits = nullptr;
     __nv_bfloat16 *act_hi = nullptr, *act_lo = nullptr;
@@ -527,6 +528,7 @@ struct GemmExt {
     int ldo = 0;
 };
 
+constexpr int kRowBlock = 32;            // rows of a block of GemmArgs::row_blocks
 struct GemmArgs {
     const __nv_bfloat16 *a_hi, *a_lo;   // [M][K]
     const __nv_bfloat16* w;             // [N][K]
@@ -546,6 +548,10 @@ struct GemmArgs {
     // order of the sums, depend on the rows (as the persistent kernel's do where it is given counters, up to 128 rows).  pairs: pairs of CTAs, whose
     // results are the same bits as single ones'.
     bool few_rows = false, pairs = true;
+    // Prompts of different lengths: only these blocks of kRowBlock rows of A and D (device, ascending, numbers of blocks) are computed; what the others
+    // of D hold stays.  Same bits as without the list.
+    const int32_t* row_blocks = nullptr;
+    int n_row_blocks = 0;
 };
 int32_t launch_gemm_tcgen05(const GemmArgs& a, cudaStream_t st);   // returns LUMI_* status
 constexpr int kFewRowsMax = 1024;                                   // rows up to which gemm_few_rows.cu may take a product
@@ -790,6 +796,9 @@ struct MoeArgs {
     float* h32; const void *w_up, *w_down; int w_dtype, act;
     // what the next product takes (tensor-core path): x * gamma_next as halves and its sum of squares
     const float* gamma_next; __nv_bfloat16 *xh, *xl; float* ssq; int ssq_stride;
+    // prompts of different lengths (null otherwise): row r is token (row0 + r) % ts of the sequence in slot b0 + (row0 + r) / ts, whose
+    // prompt goes on to row_len; rows behind it are left out
+    const int32_t* row_len; int ts, t_abs0, b0, row0;
 };
 size_t moe_plan_ints(int rows, int top, int E_max);
 int moe_max_tiles(int rows, int top, int E);

@@ -54,6 +54,13 @@ __device__ __forceinline__ void next_largest(const float* z, int E, float pz, in
     if (bi >= E) bi = E - 1;                              // (only if scores are not numbers)
 }
 
+// Whether a row is part of a prompt (rows behind a shorter one are left out: their logits and residuals are not kept up).
+__device__ __forceinline__ bool row_lives(const MoeArgs& a, int row) {
+    if (a.row_len == nullptr) return true;
+    const int r = a.row0 + row;
+    return r % a.ts < a.row_len[a.b0 + r / a.ts] - a.t_abs0;
+}
+
 __global__ void __launch_bounds__(256) moe_route_kernel(MoeArgs a) {
     __shared__ int last;
     __shared__ int sums[2][256];
@@ -62,7 +69,7 @@ __global__ void __launch_bounds__(256) moe_route_kernel(MoeArgs a) {
     const Plan p = plan_of(a);
     pdl_release();
     pdl_sync();
-    if (row < a.rows) {
+    if (row < a.rows && row_lives(a, row)) {
         const float* z = a.logits + (size_t)row * a.ldl;
         float pz = 0.f;
         int pi = -1;
@@ -142,6 +149,7 @@ __global__ void __launch_bounds__(128) moe_gather_kernel(MoeArgs a) {
     const Plan p = plan_of(a);
     pdl_release();
     pdl_sync();
+    if (!row_lives(a, row)) return;
     const float4* x = reinterpret_cast<const float4*>(a.x + (size_t)row * a.ldx);
     float s = 0.f;
     for (int c = tid; c < n4; c += 128) { const float4 v = x[c]; s = fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, fmaf(v.w, v.w, s)))); }
@@ -164,6 +172,7 @@ __global__ void __launch_bounds__(128) moe_combine_kernel(MoeArgs a) {
     const Plan p = plan_of(a);
     pdl_release();
     pdl_sync();
+    if (!row_lives(a, row)) return;
     float4* x = reinterpret_cast<float4*>(a.x + (size_t)row * a.ldx);
     float s = 0.f;
     for (int c = tid; c < n4; c += 128) {
