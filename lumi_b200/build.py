@@ -16,7 +16,7 @@ LIBDIR = os.path.join(HERE, "lib")
 LIB = os.path.join(LIBDIR, "liblumi_b200.so")
 CLI = os.path.join(LIBDIR, "lumi-infer-b200")
 
-SOURCES = ["api.cu", "kernels.cu", "gemm_tcgen05.cu", "gemm_few_rows.cu", "attention.cu", "decode_b1.cu", "block_static.cu", "prefill_ssd.cu", "prefill_rows.cu", "safetensors.cpp",
+SOURCES = ["api.cu", "kernels.cu", "gemm_tcgen05.cu", "gemm_few_rows.cu", "gemm_rows_f32.cu", "attention.cu", "decode_b1.cu", "block_static.cu", "prefill_ssd.cu", "prefill_rows.cu", "safetensors.cpp",
            "architectures.cpp", "sublayer.cu", "delta_rule.cu", "window_attention.cu", "block_product.cu", "retention.cu", "rglru.cu", "latent_attention.cu",
            "moe.cu"]
 HEADERS = ["internal.h", "json_min.h", "rows.cuh", "tf32.cuh", "tcgen05.cuh", "embed_post.cuh", os.path.join("..", "..", "include", "lumi_b200.h")]

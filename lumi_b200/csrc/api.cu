@@ -2089,15 +2089,15 @@ bool use_chunked_scan(const lumi_session* s, int T) {
 
 // Prompts a layer at a time with the recurrence in token order: what the chunked scan does not take (fp32 weights, prompts under its
 // minimum, head shapes other than its own).  The weights are read once per pass instead of once per token.  Where the line lies, on
-// the 48-layer base model (pass against decode steps): fp32 activations, bf16 weights, one sequence, 6 tokens 3.40 against 3.41 ms, 7 tokens
-// 3.41 against 3.89, two sequences of 5 3.33 against 4.17, of 4 about 3.3 against 3.40; hybrid, one sequence, 5 tokens about 3.6 against 3.33, 6
-// tokens 3.68 against 3.93; fp32 weights, one sequence, 6 tokens about 3.6 against 3.48, 8 tokens 3.65 against 4.57, three of 4 3.51 against 4.74.
+// the 48-layer base model (pass against decode steps): fp32 activations, bf16 weights, one sequence, 4 tokens 2.6 against 2.36 ms, 5 tokens
+// 2.65 against 2.87, two sequences of 4 2.6 against 3.43; hybrid, one sequence, 4 tokens 2.85 against 2.72, 5 tokens 2.87 against 3.34;
+// fp32 weights, one sequence, 5 tokens 2.95 against 2.96, 6 tokens 3.0 against 3.47, two of 4 2.95 against 3.43.
 // Such passes cost their tiles of 32 rows however few the rows are.  bf16 halves (nine sequences and more): from 4 tokens on in every case measured.
 bool use_rows_prefill(const lumi_session* s, int batch, int T) {
     const Config& c = s->m->cfg;
     if (c.stacked() || s->opt_chunked_prefill <= 0 || T < 4 || s->m->n_mamba == 0 || !ssm_rows_supported(c.head_dim(), c.d_state)) return false;
-    if (s->m->wdtype == LUMI_DTYPE_F32 && T < 8 && (long)batch * T < 12) return false;
-    if (s->m->wdtype == LUMI_DTYPE_BF16 && !use_tc(s, batch) && T < 6 && (long)batch * T < 10) return false;
+    if (s->m->wdtype == LUMI_DTYPE_F32 && T < 6 && (long)batch * T < 8) return false;
+    if (s->m->wdtype == LUMI_DTYPE_BF16 && !use_tc(s, batch) && T < 5 && (long)batch * T < 8) return false;
     if (s->m->wdtype == LUMI_DTYPE_F32) return s->m->n_attn == 0 && row_gemm_supported(c.d_model) && row_gemm_supported(c.d_inner());
     if (s->opt_gemm == 1 || !use_tc(s, 9)) return false;
     for (const Layer& L : s->m->layers) if (L.is_attn && L.window > 0) return false;       // as for the chunked scan below
@@ -2346,7 +2346,7 @@ int32_t prefill_chunked(lumi_session* s, int batch, int T, bool with_head, float
     auto product = [&](int K, const DevTensor& W, float* out, int rows, int N, int accumulate, size_t r0 = 0) -> int32_t {
         if (!tc) {
             LUMI_CUDA(launch_row_gemm(RowGemmArgs{y + r0 * K, K, W.p, W.dtype, out, N, rows, N, K, accumulate, s->gemm_counters, kGemmCounters, s->gemm_scratch,
-                                                  2 * kGemmScratchFloats}, s->stream));
+                                                  2 * kGemmScratchFloats, &s->ctl->status}, s->stream));
             return LUMI_OK;
         }
         GemmArgs g{hi + r0 * K, lo ? lo + r0 * K : nullptr, (const __nv_bfloat16*)W.p, out, N, rows, N, K, accumulate, &s->ctl->status,

@@ -622,6 +622,7 @@ struct RowGemmArgs {
     int accumulate;
     int32_t* counters; int n_counters;
     float* scratch; size_t scratch_floats;
+    int32_t* status;                     // takes STATUS_TIMEOUT (may be null)
 };
 bool row_gemm_supported(int K);
 cudaError_t launch_row_gemm(const RowGemmArgs& g, cudaStream_t st);

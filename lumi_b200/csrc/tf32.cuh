@@ -7,7 +7,7 @@ namespace lumi {
 struct Tf2 { uint32_t hi, lo; };
 __device__ __forceinline__ Tf2 split_tf32(float x) {
     Tf2 r;
-    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r.hi) : "f"(x));
+    r.hi = (__float_as_uint(x) + 0x1000u) & 0xffffe000u;
     r.lo = __float_as_uint(x - __uint_as_float(r.hi));
     return r;
 }
