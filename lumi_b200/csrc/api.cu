@@ -1825,6 +1825,12 @@ static int pdl_gemm_max() {
     return v;
 }
 
+// Programmatic dependent launch while it lives: of the CUDA-core kernels, of the tensor-core products.
+struct DependentLaunch {
+    DependentLaunch(bool rows, bool gemm) { set_launch_pdl(rows); set_launch_pdl_gemm(gemm); }
+    ~DependentLaunch() { set_launch_pdl(false); set_launch_pdl_gemm(false); }
+};
+
 int32_t enqueue_step(lumi_session* s, int B, bool with_head, int64_t* launches,
                      std::vector<std::pair<int, cudaEvent_t>>* prof = nullptr, const int32_t* row_len = nullptr) {
     const Config& c = s->m->cfg;
@@ -1837,10 +1843,10 @@ int32_t enqueue_step(lumi_session* s, int B, bool with_head, int64_t* launches,
     const bool staged_rows = !c.stacked() && s->m->wdtype == LUMI_DTYPE_BF16 && B > 4;
     // dependent launch overlaps each kernel's prologue (weight prefetch) with its predecessor; it is
     // used on the weight-streaming path, where launch gaps are the same order as the kernels
-    struct PdlScope { PdlScope(bool on) { set_launch_pdl(on); } ~PdlScope() { set_launch_pdl(false); } } pdl_scope(s->opt_pdl && prof == nullptr && (p.tc ? pdl_tc_max() > 0 && B <= pdl_tc_max() : !staged_rows));
+    const bool rows_early = s->opt_pdl && prof == nullptr && (p.tc ? pdl_tc_max() > 0 && B <= pdl_tc_max() : !staged_rows);
     // the tensor-core GEMMs themselves: dependent launch up to LUMI_PDL_GEMM rows (their barrier / TMEM set-up then runs under the
     // tail of the state step; unlike an early state step this takes nothing from a running GEMM)
-    struct PdlGemmScope { PdlGemmScope(bool on) { set_launch_pdl_gemm(on); } ~PdlGemmScope() { set_launch_pdl_gemm(false); } } pdl_gemm_scope(s->opt_pdl && prof == nullptr && p.tc && B <= pdl_gemm_max());
+    const DependentLaunch dependent(rows_early, s->opt_pdl && prof == nullptr && p.tc && B <= pdl_gemm_max());
     p.st_hi = p.st_lo = s->stream;
     mark(p);
     LUMI_CUDA(launch_embed(s->m->embedding.p, s->m->embedding.dtype, s->tok_cur, s->x, B, c.x_ld(), c.vocab, s->ctl, s->stream, row_len,
@@ -2262,6 +2268,10 @@ int32_t prefill_listed(lumi_session* s, int batch, int T, bool with_head, float*
             mark(p);
             LUMI_CUDA(launch_prefill_embed(s->m->embedding.p, s->m->embedding.dtype, s->prompt_dev, b.x, ldx, V, M, r.ts, t0, b0, batch, s->ctl,
                                            s->stream, lens, embed_post_of(s, b, slot0 + b0, p.tc)));
+            // Slices of few rows are a chain of short kernels, as steps are: dependent launch as there.  The embedding kernel above is launched in order, so
+            // what the slice before left (states, caches, positions) is complete for kernels that read it ahead of their own wait.
+            // One sequence's 77 tokens in portions of 23, 12 layers: 6.4 -> 5.7 ms.
+            const DependentLaunch dependent(s->opt_pdl && M <= pdl_tc_max(), s->opt_pdl && p.tc && M <= pdl_gemm_max());
             float* const stream = b.x;
             for (const Layer& L : s->m->layers) LUMI_TRY(listed_layer(p, r, L));
             LUMI_TRY(settle(p, r, stream));
