@@ -168,6 +168,46 @@ __global__ void __launch_bounds__(256) norm_split_kernel(const float* x, const f
     }
 }
 
+// The same for many rows, one warp each: a CTA per row is a chain of load, barrier and store with eight rows in flight on an SM, and at 3.4 TB/s waited
+// for memory most of the time.  The sum is taken as above (256 partial sums, the trees of eight warps, these in order), so its bits are the same; the row
+// is read again for the result (from L1), four elements per lane.  32768 rows of 1024: 80 -> 49 us.
+__global__ void __launch_bounds__(256) norm_split_rows_kernel(const float* __restrict__ x, const float* __restrict__ gamma, __nv_bfloat16* hi, __nv_bfloat16* lo,
+                                                              int rows, int D, float eps, float* ssq, int ssq_stride) {
+    const int b = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    pdl_launch_dependents();
+    pdl_wait();
+    if (b >= rows) return;
+    const float* xr = x + (size_t)b * D;
+    float s[8];
+#pragma unroll
+    for (int w = 0; w < 8; ++w) s[w] = 0.f;
+    for (int i = 0; i < D; i += 256)
+#pragma unroll
+        for (int w = 0; w < 8; ++w) {
+            const int k = i + 32 * w + lane;
+            if (k < D) s[w] = fmaf(xr[k], xr[k], s[w]);
+        }
+    float t = 0.f;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) t += warp_sum(s[w]);
+    float r = 1.0f;
+    if (ssq != nullptr) { if (lane == 0) ssq[(size_t)b * ssq_stride] = t; }
+    else r = rms_scale(t, D, eps);
+    for (int i = 4 * lane; i < D; i += 128) {
+        const float4 v = *reinterpret_cast<const float4*>(xr + i), g = __ldg(reinterpret_cast<const float4*>(gamma + i));
+        float w[4] = {v.x, v.y, v.z, v.w};
+        const float gg[4] = {g.x, g.y, g.z, g.w};
+        __nv_bfloat16 h[4], l[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            w[e] = __fmul_rn(ssq != nullptr ? w[e] : __fmul_rn(w[e], r), gg[e]);
+            split_bf16(w[e], h[e], l[e]);
+        }
+        *reinterpret_cast<uint2*>(hi + (size_t)b * D + i) = *reinterpret_cast<const uint2*>(h);
+        if (lo) *reinterpret_cast<uint2*>(lo + (size_t)b * D + i) = *reinterpret_cast<const uint2*>(l);
+    }
+}
+
 // ---- weight-streaming GEMV for small batches ---------------------------------------------------------
 // D[m][n] = sum_k A'[m][k] W[n][k] (+ R[m][n]),  A' = RMSNorm(A; gamma) when gamma != null.
 //
@@ -1486,6 +1526,9 @@ cudaError_t launch_embed(const void* emb, int dtype, const uint32_t* tok_cur, fl
 
 cudaError_t launch_norm_split(const float* x, const float* gamma, __nv_bfloat16* hi, __nv_bfloat16* lo, int B, int D,
                               float eps, cudaStream_t st, float* ssq, int ssq_stride) {
+    const uintptr_t at = reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(gamma) | reinterpret_cast<uintptr_t>(hi) | reinterpret_cast<uintptr_t>(lo);
+    if (B >= 2048 && gamma != nullptr && (D & 3) == 0 && (at & 15) == 0)
+        return launch_k(norm_split_rows_kernel, dim3((B + 7) / 8), dim3(256), 0, st, x, gamma, hi, lo, B, D, eps, ssq, ssq_stride);
     return launch_k(norm_split_kernel, dim3(B), dim3(256), 0, st, x, gamma, hi, lo, D, eps, ssq, ssq_stride);
 }
 
