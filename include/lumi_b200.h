@@ -271,7 +271,7 @@ typedef struct lumi_gemm_probe {
     int32_t groups, group_rows, lda, out_step, out_n, gate, ldmul, ldo;
     int32_t skip_unit;
     uint64_t row_blocks;      /* device int32: blocks of 32 rows to compute, or 0 for all rows */
-    int32_t n_row_blocks, reserved;
+    int32_t n_row_blocks, ordered;   /* ordered: few_rows in the order of sums of single CTAs */
 } lumi_gemm_probe;
 int32_t lumi_debug_gemm(const lumi_gemm_probe* probe);
 

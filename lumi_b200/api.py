@@ -49,7 +49,7 @@ class GemmProbe(C.Structure):
                 + [(n, C.c_int32) for n in ("M", "N", "K", "ldd", "accumulate", "few_rows", "pairs", "split_k", "ssq_parts", "ssq_stride", "act")]
                 + [("inv_k", C.c_float), ("eps", C.c_float)]
                 + [(n, C.c_int32) for n in ("groups", "group_rows", "lda", "out_step", "out_n", "gate", "ldmul", "ldo", "skip_unit")]
-                + [("row_blocks", C.c_uint64), ("n_row_blocks", C.c_int32), ("reserved", C.c_int32)])
+                + [("row_blocks", C.c_uint64), ("n_row_blocks", C.c_int32), ("ordered", C.c_int32)])
 
 
 class Stats(C.Structure):

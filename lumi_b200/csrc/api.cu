@@ -1308,7 +1308,8 @@ EmbedPost embed_post_of(const lumi_session* s, const RowBufs& b, int slot0, bool
     return e;
 }
 
-// Models with experts keep the persistent kernel (single CTAs and pairs give the same bits), K split by the rows up to 128 of them: a router that
+// Models with experts keep the order of sums of the persistent kernel's single CTAs, K split by the rows up to 128 of them (pairs give the same bits, the
+// kernel for few rows in its ordered form too): a router that
 // meets a near tie falls the other way when the last bits move, and a whole expert with it.  (128 sequences, 16 steps, 32 experts: with the sums
 // of the kernel for few rows one sequence's logits moved by 0.06 of their root mean square, everything else by 1e-4; the distance from 64 bits
 // was the same, 9e-4.)
@@ -1338,7 +1339,8 @@ int32_t product(StepPlan& p, int rows, const DevTensor& W, const float* in32, co
     g.nf.act = act;
     g.nf.out_hi = out_hi;
     g.nf.out_lo = s->opt_split ? out_lo : nullptr;
-    g.few_rows = !has_experts(s);
+    g.few_rows = true;
+    g.ordered = has_experts(s);
     blocks.give(g);
     return launch_gemm_tcgen05(g, p.st_hi);
 }
@@ -1477,7 +1479,8 @@ int32_t norm_product(StepPlan& p, RowPass& r, const DevTensor& W, const float* g
         g.ext = &ex;
     }
     mark(p);
-    g.few_rows = !has_experts(s);
+    g.few_rows = true;
+    g.ordered = has_experts(s);
     r.blocks.give(g);
     return launch_gemm_tcgen05(g, p.st_hi);
 }
@@ -1501,7 +1504,8 @@ int32_t residual_product(StepPlan& p, RowPass& r, const DevTensor& W, const floa
     g.nf.bias = bias;
     g.nf.gamma_next = gamma_next; g.nf.out_hi = b.xh; g.nf.out_lo = s->opt_split ? b.xl : nullptr;
     g.nf.ssq_out = b.ssq; g.nf.ssq_stride = b.ssq_stride;
-    g.few_rows = !has_experts(s);
+    g.few_rows = true;
+    g.ordered = has_experts(s);
     r.blocks.give(g);
     LUMI_TRY(launch_gemm_tcgen05(g, p.st_hi));
     r.gamma_ready = gamma_next;
@@ -1537,7 +1541,8 @@ int32_t grouped_product(StepPlan& p, const RowPass& r, const GroupedProduct& q) 
     g.nf.out_hi = q.oh;
     g.nf.out_lo = s->opt_split ? q.ol : nullptr;
     g.ext = &ex;
-    g.few_rows = !has_experts(s);
+    g.few_rows = true;
+    g.ordered = has_experts(s);
     r.blocks.give(g);
     return launch_gemm_tcgen05(g, p.st_hi);
 }
@@ -3076,6 +3081,7 @@ extern "C" int32_t lumi_debug_gemm(const lumi_gemm_probe* q) {
                (int32_t*)q->status_word, ks.counters, ks.n_counters, ks.scratch, ks.floats};
     g.few_rows = q->few_rows != 0;
     g.pairs = q->pairs != 0;
+    g.ordered = q->ordered != 0;
     g.row_blocks = (const int32_t*)q->row_blocks; g.n_row_blocks = q->n_row_blocks;
     if (q->status_word) { g.wait_limit_ns = q->wait_limit_ns; g.debug_skip_unit = q->skip_unit; }
     g.nf.ssq_in = (const float*)q->ssq_in; g.nf.ssq_parts = q->ssq_parts; g.nf.ssq_stride = q->ssq_stride; g.nf.inv_k = q->inv_k; g.nf.eps = q->eps;

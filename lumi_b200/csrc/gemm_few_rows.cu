@@ -8,6 +8,9 @@
 // partials of its share of the rows, adds them in split order (the result does not depend on timing) and finishes these rows, lanes
 // along the output columns, so that residual, result and halves are read and written in whole lines.
 //
+// ORDERED: in the persistent kernel's order, for models whose results must not move by a bit with the kernel: hi and lo go into the same columns, one after
+// the other for every k-block, K is split as it is there, and sums of squares are taken as its threads take them.
+//
 // What bounds it: the latency of one round of copies and of the reduction; at many weights (the head, 2048-wide layers) their stream.
 // Measured on the 48-layer base model: 16 steps of 64 sequences 31.3 -> 24.5 ms.
 #include "internal.h"
@@ -47,12 +50,13 @@ struct FewRowsShape {
 };
 
 // Warp 0: copies.  Warp 1: TMEM, MMA.  Warps 2, 3: the rows' scales.  Warps 4 - 7: accumulators to the owners of the rows.  All: finish.
-template <int NB, bool SPLIT, bool EXT>
+template <int NB, bool SPLIT, bool EXT, bool ORDERED>
 __global__ void __launch_bounds__(kThreads, 2)
 gemm_few_rows_kernel(const __grid_constant__ CUtensorMap map_hi, const __grid_constant__ CUtensorMap map_lo, const __grid_constant__ CUtensorMap map_w,
                      float* D, FewRowsShape sh, int splits, int32_t* status, uint64_t wait_ns, int skip_unit, NormFuse nf, GemmExt ex) {
     constexpr int A_BYTES = NB * BK * 2, STAGE = kWBytes + A_BYTES * (SPLIT ? 2 : 1);
-    constexpr uint32_t COLS = SPLIT ? 2 * NB : NB;
+    constexpr bool APART = SPLIT && !ORDERED;                           // hi and lo in columns of their own
+    constexpr uint32_t COLS = APART ? 2 * NB : NB;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     // partial results: behind the stages, since another CTA's arrive while this one still multiplies; without a cluster they reuse the stages
@@ -132,6 +136,10 @@ gemm_few_rows_kernel(const __grid_constant__ CUtensorMap map_hi, const __grid_co
 #pragma unroll
                 for (int k = 0; k < BK / 16; ++k)
                     umma_bf16(tmem, make_smem_desc(w + k * 32), make_smem_desc(act + k * 32), idesc, (i > 0 || k > 0) ? 1u : 0u);
+                if constexpr (SPLIT && ORDERED) {
+#pragma unroll
+                    for (int k = 0; k < BK / 16; ++k) umma_bf16(tmem, make_smem_desc(w + k * 32), make_smem_desc(act + A_BYTES + k * 32), idesc, 1u);
+                }
                 umma_commit(&tl.empty[s]);
                 if (++s == S) { s = 0; ph ^= 1u; }
             }
@@ -204,7 +212,7 @@ gemm_few_rows_kernel(const __grid_constant__ CUtensorMap map_hi, const __grid_co
                 if (m0 + cb * 32 >= sh.M) break;
                 uint32_t hi[32];
                 tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(cb * 32), hi);
-                if (SPLIT) {
+                if (APART) {
                     uint32_t lo[32];
                     tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(NB + cb * 32), lo);
 #pragma unroll
@@ -250,6 +258,10 @@ gemm_few_rows_kernel(const __grid_constant__ CUtensorMap map_hi, const __grid_co
             const float4 o = r0 == warp ? old[j] : old4(row);
             const float rs = tl.rs[r];
             float v[4] = {fmaf(acc.x, rs, o.x), fmaf(acc.y, rs, o.y), fmaf(acc.z, rs, o.z), fmaf(acc.w, rs, o.w)};
+            if constexpr (ORDERED && EXT) {                             // there the scaled sum is rounded before the bias is added
+                v[0] = __fadd_rn(__fmul_rn(acc.x, rs), o.x); v[1] = __fadd_rn(__fmul_rn(acc.y, rs), o.y);
+                v[2] = __fadd_rn(__fmul_rn(acc.z, rs), o.z); v[3] = __fadd_rn(__fmul_rn(acc.w, rs), o.w);
+            }
             if constexpr (EXT) {
                 int col = nl;
                 const int lim = ex.out_n;
@@ -317,9 +329,19 @@ gemm_few_rows_kernel(const __grid_constant__ CUtensorMap map_hi, const __grid_co
                         if (nf.out_lo != nullptr) *reinterpret_cast<uint2*>(nf.out_lo + oo) = *reinterpret_cast<const uint2*>(l);
                     }
                     if (nf.ssq_out != nullptr) {                        // sums of squares of strips of 32 columns: eight lanes
-                        float q = in ? fmaf(v[0], v[0], fmaf(v[1], v[1], fmaf(v[2], v[2], v[3] * v[3]))) : 0.f;
+                        float q = 0.f;
+                        if constexpr (ORDERED) {                        // (N % 32 == 0: whole strips) column after column, as one thread of the persistent kernel
 #pragma unroll
-                        for (int x = 1; x < 8; x <<= 1) q += __shfl_xor_sync(0xffffffffu, q, x);
+                            for (int x = 0; x < 8; ++x) {
+                                const float t = splits > 1 ? fmaf(v[2], v[2], fmaf(v[3], v[3], fmaf(v[0], v[0], fmaf(v[1], v[1], q))))
+                                                           : fmaf(v[0], v[0], fmaf(v[1], v[1], fmaf(v[2], v[2], fmaf(v[3], v[3], q))));
+                                q = __shfl_sync(0xffffffffu, t, (lane & ~7) | x);
+                            }
+                        } else {
+                            q = in ? fmaf(v[0], v[0], fmaf(v[1], v[1], fmaf(v[2], v[2], v[3] * v[3]))) : 0.f;
+#pragma unroll
+                            for (int x = 1; x < 8; x <<= 1) q += __shfl_xor_sync(0xffffffffu, q, x);
+                        }
                         if ((lane & 7) == 0 && in) nf.ssq_out[(size_t)row * nf.ssq_stride + (nl >> 5)] = q;
                     }
                 }
@@ -351,7 +373,8 @@ FewRowsPlan few_rows_plan(const GemmArgs& a) {
     const int num_kb = a.K / BK, stage = kWBytes + p.nb * BK * 2 * (a.a_lo != nullptr ? 2 : 1);
     const long whole = (long)p.tiles * p.row_tiles;       // CTAs with K in one piece
     p.splits = 1;
-    while (p.splits < kMaxCluster && num_kb >= 4 * p.splits && whole * 2 * p.splits <= (p.splits == 4 ? sms() / 2 : sms())) p.splits *= 2;
+    if (a.ordered) p.splits = gemm_persistent_splits(a);
+    else while (p.splits < kMaxCluster && num_kb >= 4 * p.splits && whole * 2 * p.splits <= (p.splits == 4 ? sms() / 2 : sms())) p.splits *= 2;
     const int part = p.splits > 1 ? p.nb * kWRows * 4 : 0;
     const int budget = (whole * p.splits > sms() ? 112 : 220) * 1024 - part - kTailBytes - 1024;      // more CTAs than SMs: two share one
     p.stages = std::max(2, std::min({kMaxStages, budget / stage, (num_kb + p.splits - 1) / p.splits}));
@@ -359,14 +382,14 @@ FewRowsPlan few_rows_plan(const GemmArgs& a) {
     return p;
 }
 
-template <int NB, bool SPLIT, bool EXT>
+template <int NB, bool SPLIT, bool EXT, bool ORDERED>
 int32_t launch_t(const GemmArgs& a, const FewRowsPlan& p, cudaStream_t st) {
     CUtensorMap mh, ml, mw;
     const int lda = EXT ? a.ext->lda : a.K;
     LUMI_TRY(make_bf16_operand_map(&mh, a.a_hi, a.M, lda, NB));
     LUMI_TRY(make_bf16_operand_map(&ml, SPLIT ? a.a_lo : a.a_hi, a.M, lda, NB));
     LUMI_TRY(make_bf16_operand_map(&mw, a.w, a.N, a.K, kWRows));
-    auto kern = gemm_few_rows_kernel<NB, SPLIT, EXT>;
+    auto kern = gemm_few_rows_kernel<NB, SPLIT, EXT, ORDERED>;
     LUMI_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, p.smem));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(p.tiles * p.splits, p.row_tiles);
@@ -394,7 +417,14 @@ int32_t launch_t(const GemmArgs& a, const FewRowsPlan& p, cudaStream_t st) {
 // one, microseconds: 64 rows 7360 x 1024 11.6 / 12.9, 1024 x 2048 7.8 / 12.4, 32000 x 1024 22.1 / 25.3, 2048 x 5632 14.6 / 21.5; 128 rows 1024 x
 // 2048 10.4 / 14.5, 2048 x 5632 19.3 / 25.9, 8192 x 2048 19.8 / 20.6, but in one piece 32000 x 2048 40.3 / 36.6, 11264 x 2048 28.6 / 25.4; 256
 // rows 1024 x 2048 12.3 / 18.7, 2048 x 5632 21.0 / 43.6, but in one piece 8192 x 2048 23.9 / 22.8; 512 rows 1024 x 2048 13.2 / 19.1.
+// In the persistent kernel's order (measured on a model of width 2048 with 128 rows and of width 1024 with 23): up to 64 rows always, up to 128 where K
+// is shared there.
 bool gemm_few_rows_takes(const GemmArgs& a) {
+    if (a.ordered) {
+        // a strip cut by a tile's end adds a bias differently (width_counts in gemm_tcgen05.cu), and takes its sum of squares by single elements
+        if (a.M > 128 || (a.ext == nullptr && (a.N % 32 != 0 || (a.nf.ssq_in != nullptr && a.nf.bias != nullptr) || (a.ldd & 3) != 0))) return false;
+        return a.M <= 64 || gemm_persistent_splits(a) > 1;
+    }
     return a.M <= 64 || (a.M <= kFewRowsMax && few_rows_plan(a).splits > 1);
 }
 
@@ -404,8 +434,10 @@ int32_t launch_gemm_few_rows(const GemmArgs& a, cudaStream_t st) {
     const bool split = a.a_lo != nullptr;
 #define LUMI_FEW(NB_) \
     if (p.nb == NB_) { \
-        if (a.ext != nullptr) return split ? launch_t<NB_, true, true>(a, p, st) : launch_t<NB_, false, true>(a, p, st); \
-        return split ? launch_t<NB_, true, false>(a, p, st) : launch_t<NB_, false, false>(a, p, st); \
+        if (a.ordered && a.ext != nullptr) return split ? launch_t<NB_, true, true, true>(a, p, st) : launch_t<NB_, false, true, true>(a, p, st); \
+        if (a.ordered) return split ? launch_t<NB_, true, false, true>(a, p, st) : launch_t<NB_, false, false, true>(a, p, st); \
+        if (a.ext != nullptr) return split ? launch_t<NB_, true, true, false>(a, p, st) : launch_t<NB_, false, true, false>(a, p, st); \
+        return split ? launch_t<NB_, true, false, false>(a, p, st) : launch_t<NB_, false, false, false>(a, p, st); \
     }
     LUMI_FEW(32) LUMI_FEW(64) LUMI_FEW(128)
 #undef LUMI_FEW

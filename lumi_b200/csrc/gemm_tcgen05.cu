@@ -908,6 +908,13 @@ static void pick_tile(const GemmArgs& a, int* width, int* splits) {
 // The tile width and K split launch_gemm_tcgen05 would take for these arguments (host-side choice only; nothing is launched).
 void gemm_tcgen05_plan(const GemmArgs& a, int* width, int* splits) { pick_tile(a, width, splits); }
 
+int gemm_persistent_splits(const GemmArgs& a) {
+    if (a.ext != nullptr) return 1;
+    int width = 0, splits = 1;
+    pick_tile(a, &width, &splits);
+    return splits;
+}
+
 // Products that gemm_few_rows.cu takes.
 static bool few_rows(const GemmArgs& a) {
     static const bool on = !(getenv("LUMI_FEW_ROWS") && atoi(getenv("LUMI_FEW_ROWS")) == 0);      // 0: tuning aid

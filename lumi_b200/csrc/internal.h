@@ -547,7 +547,8 @@ struct GemmArgs {
     // Besides the persistent kernel's single CTAs, which kernels may take the product.  few_rows: gemm_few_rows.cu, whose K shares, and with them the
     // order of the sums, depend on the rows (as the persistent kernel's do where it is given counters, up to 128 rows).  pairs: pairs of CTAs, whose
     // results are the same bits as single ones'.
-    bool few_rows = false, pairs = true;
+    // ordered: gemm_few_rows.cu only with the persistent kernel's order of sums, for the same bits.
+    bool few_rows = false, pairs = true, ordered = false;
     // Prompts of different lengths: only these blocks of kRowBlock rows of A and D (device, ascending, numbers of blocks) are computed; what the others
     // of D hold stays.  Same bits as without the list.
     const int32_t* row_blocks = nullptr;
@@ -556,6 +557,7 @@ struct GemmArgs {
 int32_t launch_gemm_tcgen05(const GemmArgs& a, cudaStream_t st);   // returns LUMI_* status
 constexpr int kFewRowsMax = 1024;                                   // rows up to which gemm_few_rows.cu may take a product
 bool gemm_few_rows_takes(const GemmArgs& a);
+int gemm_persistent_splits(const GemmArgs& a);                      // CTAs that share K in the persistent kernel
 int32_t launch_gemm_few_rows(const GemmArgs& a, cudaStream_t st);   // for launch_gemm_tcgen05
 void gemm_tcgen05_plan(const GemmArgs& a, int* width, int* splits);     // the tile width and K split that launch would take
 int32_t gemm_tcgen05_init();                                        // resolves the driver entry point
