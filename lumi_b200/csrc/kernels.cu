@@ -865,8 +865,10 @@ struct SsmSmem {
 // WPH warps share one head: each owns P / WPH consecutive state rows.  WPH = 1 at large batch (a
 // warp streams a whole 8 KiB tile); WPH = 4 at small batch, where the tile compute of one warp
 // would otherwise sit on the critical path of the token.
+// `ahead` (WPH = 1; 0: off): while the predecessor still works, each warp also asks L2 for the tile of the warp that many blocks
+// on, so that blocks which have no room beside the predecessor find their state in L2 when they start.
 template <int P, int N, int WPH, int MINB>
-__global__ void __launch_bounds__(256, MINB) ssm_step_kernel(SsmArgs a) {
+__global__ void __launch_bounds__(256, MINB) ssm_step_kernel(SsmArgs a, int ahead) {
     __shared__ SsmSmem<P, N> sm_all[8];
     __shared__ float red[2][8];
     constexpr int CG = N / 4;              // lanes sharing one state row
@@ -909,6 +911,13 @@ __global__ void __launch_bounds__(256, MINB) ssm_step_kernel(SsmArgs a) {
         bpq = reinterpret_cast<const float4*>(a.bprev + bh * N)[c];
 #pragma unroll
         for (int j = 0; j < (HN + 31) / 32; ++j) cu_old[j] = (lane + 32 * j < HN) ? a.cum[bh * HN + lane + 32 * j] : 0.f;
+    }
+    if (WPH == 1 && ahead > 0 && lane == 0) {
+        const int to = blockIdx.y * gridDim.x + blockIdx.x + ahead;
+        const int tb = to / gridDim.x, th = (to - tb * gridDim.x) * hpb + hl;
+        if (tb < gridDim.y && th < H)
+            asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;"
+                         ::"l"(a.h + ((size_t)tb * H + th) * (P * N)), "n"(P * N * 4) : "memory");
     }
     // parameters of the layer and the factor of the previous token: not produced by the predecessor either
     const int hh = active ? h : H - 1;
@@ -1556,7 +1565,7 @@ cudaError_t launch_norm_split(const float* x, const float* gamma, __nv_bfloat16*
     return launch_k(norm_split_kernel, dim3(B), dim3(256), 0, st, x, gamma, hi, lo, D, eps, ssq, ssq_stride);
 }
 
-static int sm_count() {
+int sm_count() {
     static int n = 0;
     if (n == 0) {
         int dev = 0;
@@ -1738,7 +1747,12 @@ static cudaError_t ssm_variant(const SsmArgs& a, cudaStream_t st) {
     int hpb = 8 / WPH;
     if (hpb > a.H) hpb = a.H;
     dim3 grid((a.H + hpb - 1) / hpb, a.B);
-    return launch_k(ssm_step_kernel<P, N, WPH, MINB>, grid, dim3(hpb * WPH * 32), 0, st, a);
+    // Tiles asked for one block per SM ahead.  Base model, 16 steps, 64 / 128 / 300 sequences: 25.0 / 42.3 / 74.3 -> 24.6 / 40.7 /
+    // 73.7 ms (two blocks per SM, the number that is resident: 25.0 / 40.8 / 74.8; four: 25.0 / 42.8 / 80.3, they crowd out states in
+    // use).  With more blocks the stream is steady and the requests get in its way: 512 / 800 sequences 111.6 / 170.7 -> 112.3 /
+    // 172.3 ms; the line lies between 2400 blocks (gain) and 4096 (loss).
+    const int ahead = (long)grid.x * grid.y <= 20L * sm_count() ? sm_count() : 0;
+    return launch_k(ssm_step_kernel<P, N, WPH, MINB>, grid, dim3(hpb * WPH * 32), 0, st, a, ahead);
 }
 
 // LUMI_SSM_VARIANT (tuning aid): warps per head x minimum resident blocks per SM for the
@@ -1758,7 +1772,7 @@ static cudaError_t ssm_launch(const SsmArgs& a, cudaStream_t st) {
             if (hpb_env < 0) { const char* e = getenv("LUMI_SSM_HPB"); hpb_env = e ? atoi(e) : 1; }
             int hpb = a.H < hpb_env ? a.H : hpb_env;
             dim3 grid((a.H + hpb - 1) / hpb, a.B);
-            return launch_k(ssm_step_kernel<P, N, 4, 3>, grid, dim3(hpb * 4 * 32), 0, st, a);
+            return launch_k(ssm_step_kernel<P, N, 4, 3>, grid, dim3(hpb * 4 * 32), 0, st, a, 0);
         }
     }
     if constexpr (P == 32 && N == 64) {

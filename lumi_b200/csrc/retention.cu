@@ -51,9 +51,10 @@ __device__ __forceinline__ bool state_wait(uint64_t* bar) {
 // CTA = (head, sequence).  Thread (rg, cg) holds rows rg, rg + RG, ... (VPT of them at most) of four neighbouring columns.
 // VPT = 0: the state stays in global memory (heads beyond shared memory).  VPT = -1: the state lies in shared memory, in kParts parts of
 // `pr` rows (a multiple of RG) that bulk copies bring and take back: while one part is worked on, the others are on their way.
+// `ahead` (VPT = -1; 0: off): a block also asks L2 for the state of the block that many on, which has no room on an SM yet.
 constexpr int kParts = 4;
 template <int NT, int VPT>
-__global__ void __launch_bounds__(NT) retention_step_kernel(RetentionArgs a, int cwl, int part_rows) {
+__global__ void __launch_bounds__(NT) retention_step_kernel(RetentionArgs a, int cwl, int part_rows, int ahead) {
     extern __shared__ __align__(128) float dyn[];
     __shared__ __align__(8) uint64_t bars[kParts];
     float* sm = dyn + (VPT < 0 ? (size_t)a.dk * a.dvp : 0);
@@ -86,7 +87,10 @@ __global__ void __launch_bounds__(NT) retention_step_kernel(RetentionArgs a, int
     };
     pdl_release();
     // the state belongs to the step before this one, which has ended: read ahead of the predecessor's results
-    if (VPT < 0 && a.row_len == nullptr && tid == 0) request();
+    if (VPT < 0 && a.row_len == nullptr && tid == 0) {
+        request();
+        if (ahead > 0 && sl * a.H + h + ahead < (int)(gridDim.x * gridDim.y)) l2_prefetch(S + (size_t)ahead * dk * c4n, (uint32_t)dk * dvp * 4u);
+    }
     float4 s[VPT > 0 ? VPT : 1];
     if constexpr (VPT > 0) {
 #pragma unroll
@@ -432,7 +436,9 @@ cudaError_t step_launch(const RetentionArgs& a, int cwl, cudaStream_t st) {
         if (e != cudaSuccess) return e;
     }
     const int RG = NT >> cwl, part_rows = ((a.dk + kParts - 1) / kParts + RG - 1) / RG * RG;
-    return launch_rows(kern, dim3(a.H, a.nseq), NT, smem, st, a, cwl, part_rows);
+    // one block per SM ahead, as in ssm_variant: the same line, the same reason
+    const int ahead = VPT < 0 && (long)a.H * a.nseq <= 20L * sm_count() ? sm_count() : 0;
+    return launch_rows(kern, dim3(a.H, a.nseq), NT, smem, st, a, cwl, part_rows, ahead);
 }
 
 // columns per CTA (nw warp pairs of 8 ntw each): as many as the value dimension has and shared memory takes, fewer where the heads

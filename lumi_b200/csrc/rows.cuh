@@ -4,8 +4,15 @@
 
 namespace lumi {
 
+int sm_count();                                            // of the current device (kernels.cu)
+
 __device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_sync() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// Whole 16-byte pieces of global memory on their way to L2; nothing waits for them.
+__device__ __forceinline__ void l2_prefetch(const void* p, uint32_t bytes) {
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
+}
 
 __device__ __forceinline__ float warp_total(float v) {
 #pragma unroll
