@@ -135,8 +135,19 @@ __global__ void __launch_bounds__(kThreads, 1) row_gemm_kernel(const __grid_cons
     const int g0 = blockIdx.z * groups_per_split, g1 = min(groups, g0 + groups_per_split);
     const int kb0 = g0 * kGroupBlocks, kb1 = min(blocks, g1 * kGroupBlocks);
 
-    // a wait that expired in an earlier launch: no new work
-    if (__syncthreads_or(g.status != nullptr && (*reinterpret_cast<volatile int32_t*>(g.status) & STATUS_TIMEOUT))) return;
+    const bool split = gridDim.z > 1;
+    const int tile = blockIdx.y * gridDim.x + blockIdx.x;
+    // K split: every CTA of a tile arrives at its counter, also one that has nothing to add, and the last one leaves it at zero for the next product
+    auto arrive = [&]() {
+        const bool is_last = atomicAdd(g.counters + tile, 1) == (int)gridDim.z - 1;
+        if (is_last) g.counters[tile] = 0;
+        return is_last;
+    };
+    // a wait that expired in an earlier launch, or in an earlier CTA of this one: no new work
+    if (__syncthreads_or(g.status != nullptr && (*reinterpret_cast<volatile int32_t*>(g.status) & STATUS_TIMEOUT))) {
+        if (split && threadIdx.x == 0) arrive();
+        return;
+    }
     if (threadIdx.x == 0) {
         for (int i = 0; i < kStages; ++i) { mbar_init(&full[i], kLoadWarps + (T::PW == 1 ? 1 : 0)); mbar_init(&empty[i], 1); }
         for (int i = 0; i < kAccs; ++i) { mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], kSumWarps); }
@@ -156,11 +167,12 @@ __global__ void __launch_bounds__(kThreads, 1) row_gemm_kernel(const __grid_cons
     tc_fence_after();
     const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(tmem_slot);
     bool timed_out = false;
+    auto wait = [&](uint64_t* bar, uint32_t parity) { return mbar_wait(bar, parity, g.wait_ns); };
 
     if (warp < kLoadWarps) {
         // a k-block arrives in one piece (rows and K past the end as zeros); once it is in registers the next one is on its way
         uint8_t* const raw = base + T::RAWS;
-        const bool issues = threadIdx.x == 0;
+        const bool issues = threadIdx.x == 0 && tile + (int)(blockIdx.z * gridDim.x * gridDim.y) >= g.skip_units;
         int requested = 0;
         auto request = [&](int kb) {
             ++requested;
@@ -170,7 +182,7 @@ __global__ void __launch_bounds__(kThreads, 1) row_gemm_kernel(const __grid_cons
         };
         auto request_w = [&](int kb) {                                    // bf16 weights need no splitting
             const int it = kb - kb0, s = it % kStages;
-            if (!mbar_wait(&empty[s], (uint32_t)((it / kStages) & 1) ^ 1u)) return false;
+            if (!wait(&empty[s], (uint32_t)((it / kStages) & 1) ^ 1u)) return false;
             mbar_expect_tx(&full[s], (uint32_t)T::W_PLANE);
             tma_load_2d(base + s * T::STAGE, &map_w, &full[s], kb * BK, n0);
             return true;
@@ -182,7 +194,7 @@ __global__ void __launch_bounds__(kThreads, 1) row_gemm_kernel(const __grid_cons
         }
         for (int kb = kb0; kb < kb1; ++kb) {
             const int it = kb - kb0, s = it % kStages;
-            if (!mbar_wait(raw_full, (uint32_t)(it & 1))) timed_out = true;
+            if (!wait(raw_full, (uint32_t)(it & 1))) timed_out = true;
             if (__any_sync(0xffffffffu, timed_out)) { timed_out = true; break; }
             Pieces<T::PW == 3 ? kWRows : 16> w;
             Pieces<NB> a;
@@ -191,10 +203,10 @@ __global__ void __launch_bounds__(kThreads, 1) row_gemm_kernel(const __grid_cons
             __syncwarp();
             if (lane == 0) mbar_arrive(raw_empty);
             if (issues && kb + 1 < kb1) {
-                if (mbar_wait(raw_empty, (uint32_t)(it & 1))) request(kb + 1);
+                if (wait(raw_empty, (uint32_t)(it & 1))) request(kb + 1);
                 else timed_out = true;
             }
-            if (!mbar_wait(&empty[s], (uint32_t)((it / kStages) & 1) ^ 1u)) timed_out = true;
+            if (!wait(&empty[s], (uint32_t)((it / kStages) & 1) ^ 1u)) timed_out = true;
             if (__any_sync(0xffffffffu, timed_out)) { timed_out = true; break; }
             uint8_t* const st = base + s * T::STAGE;
             if constexpr (T::PW == 3) w.store(st, T::W_PLANE, threadIdx.x);
@@ -211,9 +223,9 @@ __global__ void __launch_bounds__(kThreads, 1) row_gemm_kernel(const __grid_cons
             }
         }
         if (timed_out && issues) {                                        // let the copies land (bounded) that nobody may wait for
-            mbar_wait(raw_full, (uint32_t)((requested - 1) & 1));
+            wait(raw_full, (uint32_t)((requested - 1) & 1));
             if constexpr (T::PW == 1)
-                for (int k = max(kb0, w_next - kStages); k < w_next; ++k) mbar_wait(&full[(k - kb0) % kStages], (uint32_t)(((k - kb0) / kStages) & 1));
+                for (int k = max(kb0, w_next - kStages); k < w_next; ++k) wait(&full[(k - kb0) % kStages], (uint32_t)(((k - kb0) / kStages) & 1));
         }
     } else if (warp == kLoadWarps) {
         if (lane == 0) {
@@ -222,9 +234,9 @@ __global__ void __launch_bounds__(kThreads, 1) row_gemm_kernel(const __grid_cons
             int step = 0;                                                 // kAccK of K each
             for (int kb = kb0; kb < kb1 && !timed_out; ++kb) {
                 const int it = kb - kb0, s = it % kStages, grp = it / kGroupBlocks, first = it % kGroupBlocks == 0;
-                if (!mbar_wait(&full[s], (uint32_t)((it / kStages) & 1))) { timed_out = true; break; }
+                if (!wait(&full[s], (uint32_t)((it / kStages) & 1))) { timed_out = true; break; }
                 const uint32_t small = tmem + (uint32_t)((kAccs + 2 * (grp & 1)) * NB);
-                if (first && !mbar_wait(&small_empty[grp & 1], (uint32_t)((grp / 2) & 1) ^ 1u)) { timed_out = true; break; }
+                if (first && !wait(&small_empty[grp & 1], (uint32_t)((grp / 2) & 1) ^ 1u)) { timed_out = true; break; }
                 tc_fence_after();
                 const uint32_t w = smem_u32(base + s * T::STAGE), a = w + T::PW * T::W_PLANE;
 #pragma unroll
@@ -232,7 +244,7 @@ __global__ void __launch_bounds__(kThreads, 1) row_gemm_kernel(const __grid_cons
                     const int acc = step % kAccs;
                     const bool fresh = k % (kAccK / 16) == 0, done = (k + 1) % (kAccK / 16) == 0;
                     if (fresh) {
-                        if (!mbar_wait(&acc_empty[acc], (uint32_t)((step / kAccs) & 1) ^ 1u)) { timed_out = true; break; }
+                        if (!wait(&acc_empty[acc], (uint32_t)((step / kAccs) & 1) ^ 1u)) { timed_out = true; break; }
                         tc_fence_after();
                     }
                     auto wd = [&](int p) { return make_smem_desc(w + p * T::W_PLANE + k * 32); };
@@ -252,15 +264,13 @@ __global__ void __launch_bounds__(kThreads, 1) row_gemm_kernel(const __grid_cons
             }
             if (timed_out) {                                              // let every MMA issued so far finish (bounded) before TMEM is freed
                 umma_commit(drain);
-                mbar_wait(drain, 0);
+                wait(drain, 0);
             }
         }
     } else {
         const int q = warp & 3, half = (warp - kFirstSum) >> 2;          // TMEM lane quarter, half of the columns
         const uint32_t lanes = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(half * CW);
         const int n = n0 + q * 32 + lane, mc = m0 + half * CW, tid = threadIdx.x - 32 * kFirstSum;
-        const bool split = gridDim.z > 1;
-        const int tile = blockIdx.y * gridDim.x + blockIdx.x;
         float* const total = reinterpret_cast<float*>(base + T::TOTALS) + tid;             // 256 apart
         float* const parts = g.scratch + (size_t)tile * groups * kWRows * NB + tid;        // K split: the groups' sums
         const int cols = n < g.N ? max(0, min(CW, g.M - mc)) : 0;                          // of this thread that exist
@@ -293,7 +303,7 @@ __global__ void __launch_bounds__(kThreads, 1) row_gemm_kernel(const __grid_cons
 #pragma unroll 1
                 for (int t = 0; t < steps; ++t, ++step) {
                     const int acc = step % kAccs;
-                    if (!mbar_wait(&acc_full[acc], (uint32_t)((step / kAccs) & 1))) timed_out = true;
+                    if (!wait(&acc_full[acc], (uint32_t)((step / kAccs) & 1))) timed_out = true;
                     timed_out = __any_sync(0xffffffffu, timed_out);
                     if (timed_out) break;
                     tc_fence_after();
@@ -309,7 +319,7 @@ __global__ void __launch_bounds__(kThreads, 1) row_gemm_kernel(const __grid_cons
                 for (int j = 0; j < CW / 2; ++j) sum[j] = add2(sum[j], unit[j]);
             }
             if (timed_out) break;
-            if (!mbar_wait(&small_full[gi & 1], (uint32_t)((gi / 2) & 1))) timed_out = true;
+            if (!wait(&small_full[gi & 1], (uint32_t)((gi / 2) & 1))) timed_out = true;
             timed_out = __any_sync(0xffffffffu, timed_out);
             if (timed_out) break;
             tc_fence_after();
@@ -342,14 +352,21 @@ __global__ void __launch_bounds__(kThreads, 1) row_gemm_kernel(const __grid_cons
                 }
             }
         }
+        // a wait ran out: what is missing is no number, in the result or in the partial sums
+        if (timed_out) {
+            const float nan = __int_as_float(0x7fffffff), v[8] = {nan, nan, nan, nan, nan, nan, nan, nan};
+            if (split)
+                for (int gr = g0; gr < g1; ++gr)
+                    for (int j = 0; j < CW; ++j) parts[(size_t)gr * kWRows * NB + j * 256] = nan;
+            else
+#pragma unroll 1
+                for (int c = 0; c < CW; c += 8) put8(c, v);
+        }
         if (split) {
-            // the last CTA of the tile to arrive adds the groups as above (a CTA whose wait ran out arrives too: the status says so)
+            // the last CTA of the tile to arrive adds the groups as above
             __threadfence();
             asm volatile("bar.sync 1, 256;" ::: "memory");
-            if (tid == 0) {
-                *last = atomicAdd(g.counters + tile, 1) == (int)gridDim.z - 1;
-                if (*last) g.counters[tile] = 0;                          // ready for the next product
-            }
+            if (tid == 0) *last = arrive();
             asm volatile("bar.sync 1, 256;" ::: "memory");
             if (*last) {
                 __threadfence();
@@ -389,7 +406,8 @@ int sms() {
 }
 
 template <int NB, typename WT>
-cudaError_t launch_t(const RowGemmArgs& g, dim3 grid, int per, cudaStream_t st) {
+cudaError_t launch_t(RowGemmArgs g, dim3 grid, int per, cudaStream_t st) {
+    if (g.wait_ns == 0) g.wait_ns = kWaitLimitNs;
     using T = RowsTile<NB, WT>;
     CUtensorMap ma, mw;
     if (make_f32_map_2d(&ma, g.A, (uint64_t)g.M, (uint64_t)g.K, (uint64_t)g.lda * 4, BK, NB) != LUMI_OK) return cudaErrorInvalidValue;

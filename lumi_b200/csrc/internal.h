@@ -614,8 +614,8 @@ cudaError_t launch_bc_stats(const PrefillArgs& a, int P, int N, cudaStream_t st)
 // prompt length.  y32 (may be null): [nb * ts][heads * P] fp32 beside or in place of yhi / ylo.
 bool ssm_rows_supported(int P, int N);
 cudaError_t launch_ssm_rows(const PrefillArgs& a, int P, int N, float* y32, cudaStream_t st);
-// D[M][N] (+)= A[M][K] W[N][K]^T in fp32 on the CUDA cores, for many rows (prefill_rows.cu).  K % 16 == 0, lda % 4 == 0, 16-byte aligned operands.  counters (zeroed
-// ints, left zeroed) and scratch serve the split of K.
+// D[M][N] (+)= A[M][K] W[N][K]^T with fp32 activations, for many rows (gemm_rows_f32.cu).  K % 16 == 0, lda % 4 == 0, 16-byte aligned operands.  counters (zeroed
+// ints, left zeroed, also after a wait that ran out) and scratch serve the split of K.
 struct RowGemmArgs {
     const float* A; int lda;
     const void* W; int w_dtype;          // LUMI_DTYPE_*
@@ -625,6 +625,8 @@ struct RowGemmArgs {
     int32_t* counters; int n_counters;
     float* scratch; size_t scratch_floats;
     int32_t* status;                     // takes STATUS_TIMEOUT (may be null)
+    uint64_t wait_ns = 0;                // limit of every wait, 0: the usual one
+    int skip_units = 0;                  // test hook: the operands of this many CTAs (x, then y, then z) never arrive
 };
 bool row_gemm_supported(int K);
 cudaError_t launch_row_gemm(const RowGemmArgs& g, cudaStream_t st);
