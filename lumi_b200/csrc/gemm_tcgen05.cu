@@ -62,8 +62,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_ahi, const __grid_constant__
     const int n0 = blockIdx.x * BN, m0 = blockIdx.y * BM;
     const int num_kb = K / BK;
 
-    // a wait that expired in an earlier CTA of this launch: do not start new work
-    if (status != nullptr && (*reinterpret_cast<volatile int32_t*>(status) & STATUS_TIMEOUT)) return;
+    // a wait that expired in an earlier CTA of this launch: do not start new work (one verdict for all threads: the word may change while they look)
+    if (__syncthreads_or(status != nullptr && (*reinterpret_cast<volatile int32_t*>(status) & STATUS_TIMEOUT))) return;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < S; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }

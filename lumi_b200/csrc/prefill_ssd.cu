@@ -292,8 +292,8 @@ ssd_prefill_kernel(const __grid_constant__ CUtensorMap map32, const __grid_const
     const float dskip = a.dskip[h], dtb = a.dtb[h];
     uint64_t* bar = reinterpret_cast<uint64_t*>(&sm.bar);
 
-    // a wait that expired in an earlier CTA of this launch: do not start new work
-    if (a.status != nullptr && (*reinterpret_cast<volatile int32_t*>(a.status) & STATUS_TIMEOUT)) return;
+    // a wait that expired in an earlier CTA of this launch: do not start new work (one verdict for all threads: the word may change while they look)
+    if (__syncthreads_or(a.status != nullptr && (*reinterpret_cast<volatile int32_t*>(a.status) & STATUS_TIMEOUT))) return;
 
     if (tid == 0) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(bar)));
