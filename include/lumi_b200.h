@@ -292,15 +292,15 @@ int32_t lumi_k_gemv(uint64_t a_f32, uint64_t w, int32_t w_dtype, uint64_t d, uin
 
 /* The same product for many rows (prompts a layer at a time): D[M][N] (+)= A[M][K] * W[N][K]^T to the precision of fp32 multiply-adds, on the
  * tensor cores; K % 16 == 0, rows of A 16-byte aligned.  The order of a sum depends on K alone, so a row's results are the same bits alone and among
- * others.  Should one of the kernel's bounded waits run out, the results it concerns are no numbers. */
+ * others.  Infinities and numbers of any size give what multiply-adds give. */
 int32_t lumi_k_row_gemm(uint64_t a_f32, uint64_t w, int32_t w_dtype, uint64_t d, int32_t M, int32_t N, int32_t K,
                         int32_t accumulate, uint64_t stream);
 
-/* Failure-path test hook of that product: every device-side wait limited to wait_limit_ns, the operands of the first skip_units CTAs (tiles of weight rows,
- * then of prompt rows, then shares of K) never requested, so that their waits run out.  status_word: a zeroed device int32, or 0 for none.  Returns
- * LUMI_E_TIMEOUT when a wait gave up and there is a status word; further calls work.  Synchronises the default stream. */
+/* Failure-path test hook of that product: the operands of the first skip_units CTAs (tiles of weight rows, then of prompt rows, then shares of K) are never
+ * requested, so that their waits run out (after half a second).  status_word: a zeroed device int32, or 0 for none.  Returns LUMI_E_TIMEOUT when a wait gave
+ * up and there is a status word; further calls work.  Synchronises the default stream. */
 int32_t lumi_debug_row_gemm_wait_timeout(uint64_t a_f32, uint64_t w, int32_t w_dtype, uint64_t d, int32_t M, int32_t N, int32_t K,
-                                         uint64_t wait_limit_ns, int32_t skip_units, uint64_t status_word);
+                                         int32_t skip_units, uint64_t status_word);
 
 /* The fused Mamba-3 state step alone (inference/src/model.rs:301-370 after in_proj, before
  * out_proj): proj[B][ldp] holds in_proj's output rows; h[B][H][P][N], x_prev[B][H][P],

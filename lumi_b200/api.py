@@ -96,7 +96,7 @@ def lib():
         L.lumi_k_gemm_bf16_tcgen05.argtypes = [u64, u64, u64, u64, i32, i32, i32, i32, i32, u64]
         L.lumi_k_gemv.argtypes = [u64, u64, i32, u64, u64, u64, i32, i32, i32, u64]
         L.lumi_k_row_gemm.argtypes = [u64, u64, i32, u64, i32, i32, i32, i32, u64]
-        L.lumi_debug_row_gemm_wait_timeout.argtypes = [u64, u64, i32, u64, i32, i32, i32, u64, i32, u64]
+        L.lumi_debug_row_gemm_wait_timeout.argtypes = [u64, u64, i32, u64, i32, i32, i32, i32, u64]
         L.lumi_k_ssm_step.argtypes = [u64, i32] + [u64] * 11 + [i32] * 5 + [u64]
         L.lumi_debug_gemm_wait_timeout.argtypes = [u64, u64, u64, i32, i32, i32, u64, i32, u64]
         L.lumi_debug_gemm.argtypes = [C.POINTER(GemmProbe)]

@@ -3120,30 +3120,30 @@ extern "C" int32_t lumi_debug_gemm(const lumi_gemm_probe* q) {
     return LUMI_OK;
 }
 
-static int32_t row_product(uint64_t a_f32, uint64_t w, int32_t w_dtype, uint64_t d, int32_t M, int32_t N, int32_t K, int32_t accumulate, int32_t* status, uint64_t wait_ns,
+static int32_t row_product(uint64_t a_f32, uint64_t w, int32_t w_dtype, uint64_t d, int32_t M, int32_t N, int32_t K, int32_t accumulate, int32_t* status,
                            int32_t skip_units, cudaStream_t stream) {
     if (!a_f32 || !w || !d || M <= 0 || N <= 0 || K <= 0 || ((a_f32 | w) & 15)) return fail(LUMI_E_INVALID, "bad argument to a product of rows");
     if (!row_gemm_supported(K)) return fail(LUMI_E_UNSUPPORTED, "a product of rows needs K %% 16 == 0");
     KernelScratch ks;
     LUMI_TRY(kernel_scratch(&ks));
     LUMI_CUDA(launch_row_gemm(RowGemmArgs{(const float*)a_f32, K, (const void*)w, w_dtype, (float*)d, N, M, N, K, accumulate, ks.counters, ks.n_counters, ks.scratch,
-                                          ks.floats, status, wait_ns, skip_units}, stream));
+                                          ks.floats, status, skip_units}, stream));
     return LUMI_OK;
 }
 
 extern "C" int32_t lumi_k_row_gemm(uint64_t a_f32, uint64_t w, int32_t w_dtype, uint64_t d, int32_t M, int32_t N, int32_t K, int32_t accumulate,
                                    uint64_t stream) {
-    return row_product(a_f32, w, w_dtype, d, M, N, K, accumulate, nullptr, 0, 0, (cudaStream_t)stream);
+    return row_product(a_f32, w, w_dtype, d, M, N, K, accumulate, nullptr, 0, (cudaStream_t)stream);
 }
 
-extern "C" int32_t lumi_debug_row_gemm_wait_timeout(uint64_t a_f32, uint64_t w, int32_t w_dtype, uint64_t d, int32_t M, int32_t N, int32_t K, uint64_t wait_limit_ns,
+extern "C" int32_t lumi_debug_row_gemm_wait_timeout(uint64_t a_f32, uint64_t w, int32_t w_dtype, uint64_t d, int32_t M, int32_t N, int32_t K,
                                                     int32_t skip_units, uint64_t status_word) {
-    if (wait_limit_ns == 0 || skip_units < 0) return fail(LUMI_E_INVALID, "bad argument to lumi_debug_row_gemm_wait_timeout");
-    LUMI_TRY(row_product(a_f32, w, w_dtype, d, M, N, K, 0, (int32_t*)status_word, wait_limit_ns, skip_units, nullptr));
+    if (skip_units < 0) return fail(LUMI_E_INVALID, "bad argument to lumi_debug_row_gemm_wait_timeout");
+    LUMI_TRY(row_product(a_f32, w, w_dtype, d, M, N, K, 0, (int32_t*)status_word, skip_units, nullptr));
     LUMI_CUDA(cudaStreamSynchronize(nullptr));
     int32_t st = 0;
     if (status_word) LUMI_CUDA(cudaMemcpy(&st, (const void*)status_word, sizeof(st), cudaMemcpyDeviceToHost));
-    if (st & STATUS_TIMEOUT) return fail(LUMI_E_TIMEOUT, "a bounded device-side wait expired in the product of rows (limit %llu ns)", (unsigned long long)wait_limit_ns);
+    if (st & STATUS_TIMEOUT) return fail(LUMI_E_TIMEOUT, "a bounded device-side wait expired in the product of rows");
     return LUMI_OK;
 }
 

@@ -52,6 +52,12 @@ struct RowsTile {
 // pairs of fp32 numbers
 __device__ __forceinline__ uint64_t pair2(uint32_t a, uint32_t b) { uint64_t d; asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(a), "r"(b)); return d; }
 __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) { uint64_t d; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
+// a - b as one multiply-add by -1 (as a + (-b) the halves of b needed their signs turned first)
+__device__ __forceinline__ uint64_t minus2(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(b), "l"(0xbf800000bf800000ull), "l"(a));
+    return d;
+}
 __device__ __forceinline__ float first_of(uint64_t d) { return __uint_as_float((uint32_t)d); }
 __device__ __forceinline__ float second_of(uint64_t d) { return __uint_as_float((uint32_t)(d >> 32)); }
 
@@ -79,7 +85,7 @@ __device__ __forceinline__ void tmem_pairs(uint32_t taddr, uint64_t (&v)[CW / 2]
 
 // Four consecutive elements into their planes.  x = hi + mid + lo exactly: hi the nearest bf16, mid the upper eight bits of what is left, lo the eight behind
 // them.  (Nearest for the first, so that mid has either sign and the products left out do not all have the sign of theirs.)  What is infinite, or
-// above bf16's largest number (3.39e38), makes the results of its row no numbers.
+// above bf16's largest number (3.39e38), has planes that are no numbers: such sums are taken again (plain_result).
 __device__ __forceinline__ void store_planes(const float4& a, uint8_t* at, int plane) {
     uint64_t r[2] = {pair2(__float_as_uint(a.x), __float_as_uint(a.y)), pair2(__float_as_uint(a.z), __float_as_uint(a.w))};
     uint32_t w[3][2];
@@ -87,11 +93,10 @@ __device__ __forceinline__ void store_planes(const float4& a, uint8_t* at, int p
     for (int e = 0; e < 2; ++e) {
         const __nv_bfloat162 h = __floats2bfloat162_rn(first_of(r[e]), second_of(r[e]));
         w[0][e] = *reinterpret_cast<const uint32_t*>(&h);
-        // x - h as x + (-h): the two halves widened with their signs turned
-        r[e] = add2(r[e], pair2((w[0][e] << 16) ^ 0x80000000u, (w[0][e] & 0xffff0000u) ^ 0x80000000u));
+        r[e] = minus2(r[e], pair2(w[0][e] << 16, w[0][e] & 0xffff0000u));                  // the two halves, widened
         const uint32_t m0 = (uint32_t)r[e], m1 = (uint32_t)(r[e] >> 32);
         w[1][e] = __byte_perm(m0, m1, 0x7632);
-        r[e] = add2(r[e], pair2((m0 & 0xffff0000u) ^ 0x80000000u, (m1 & 0xffff0000u) ^ 0x80000000u));
+        r[e] = minus2(r[e], pair2(m0 & 0xffff0000u, m1 & 0xffff0000u));
         w[2][e] = __byte_perm((uint32_t)r[e], (uint32_t)(r[e] >> 32), 0x7632);
     }
 #pragma unroll
@@ -117,6 +122,38 @@ struct Pieces {
         }
     }
 };
+
+// One result by fp32 multiply-adds: chains of 16, eight to a unit, four units to a group, the groups in order.  For sums of planes that are not finite: an infinite
+// operand has planes that are no numbers, one above bf16's largest number an infinite one, though the result may be infinite or finite.
+template <typename WT>
+__device__ __forceinline__ float plain_result(const float* a, const WT* w, int K) {
+    float total = 0.f;
+    for (int k0 = 0; k0 < K && total == total; k0 += 512) {             // (no number stays none)
+        float group = 0.f;
+        for (int k1 = k0; k1 < min(K, k0 + 512); k1 += 128) {
+            float unit = 0.f;
+            for (int k = k1; k < min(K, k1 + 128); k += 16) {
+                float chain = 0.f;
+#pragma unroll
+                for (int e = 0; e < 16; e += 4) {
+                    const float4 x = *reinterpret_cast<const float4*>(a + k + e);
+                    float4 y;
+                    if constexpr (sizeof(WT) == 4) {
+                        y = *reinterpret_cast<const float4*>(w + k + e);
+                    } else {
+                        const uint2 v = *reinterpret_cast<const uint2*>(w + k + e);
+                        y = make_float4(__uint_as_float(v.x << 16), __uint_as_float(v.x & 0xffff0000u), __uint_as_float(v.y << 16), __uint_as_float(v.y & 0xffff0000u));
+                    }
+                    chain = fmaf(x.w, y.w, fmaf(x.z, y.z, fmaf(x.y, y.y, fmaf(x.x, y.x, chain))));
+                }
+                unit += chain;
+            }
+            group += unit;
+        }
+        total += group;
+    }
+    return total;
+}
 
 template <int NB, typename WT>
 __global__ void __launch_bounds__(kThreads, 1) row_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, RowGemmArgs g, int groups_per_split) {
@@ -167,12 +204,11 @@ __global__ void __launch_bounds__(kThreads, 1) row_gemm_kernel(const __grid_cons
     tc_fence_after();
     const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(tmem_slot);
     bool timed_out = false;
-    auto wait = [&](uint64_t* bar, uint32_t parity) { return mbar_wait(bar, parity, g.wait_ns); };
 
     if (warp < kLoadWarps) {
         // a k-block arrives in one piece (rows and K past the end as zeros); once it is in registers the next one is on its way
         uint8_t* const raw = base + T::RAWS;
-        const bool issues = threadIdx.x == 0 && tile + (int)(blockIdx.z * gridDim.x * gridDim.y) >= g.skip_units;
+        const bool issues = threadIdx.x == 0;
         int requested = 0;
         auto request = [&](int kb) {
             ++requested;
@@ -182,19 +218,19 @@ __global__ void __launch_bounds__(kThreads, 1) row_gemm_kernel(const __grid_cons
         };
         auto request_w = [&](int kb) {                                    // bf16 weights need no splitting
             const int it = kb - kb0, s = it % kStages;
-            if (!wait(&empty[s], (uint32_t)((it / kStages) & 1) ^ 1u)) return false;
+            if (!mbar_wait(&empty[s], (uint32_t)((it / kStages) & 1) ^ 1u)) return false;
             mbar_expect_tx(&full[s], (uint32_t)T::W_PLANE);
             tma_load_2d(base + s * T::STAGE, &map_w, &full[s], kb * BK, n0);
             return true;
         };
         int w_next = kb0;                                                 // (this thread) the next block of bf16 weights to be requested
-        if (issues) {
+        if (issues && tile + (int)(blockIdx.z * gridDim.x * gridDim.y) >= g.skip_units) {      // (test hook: nothing is asked for, and every wait runs out)
             request(kb0);
             if constexpr (T::PW == 1) for (; w_next < min(kb1, kb0 + kStages); ++w_next) request_w(w_next);
         }
         for (int kb = kb0; kb < kb1; ++kb) {
             const int it = kb - kb0, s = it % kStages;
-            if (!wait(raw_full, (uint32_t)(it & 1))) timed_out = true;
+            if (!mbar_wait(raw_full, (uint32_t)(it & 1))) timed_out = true;
             if (__any_sync(0xffffffffu, timed_out)) { timed_out = true; break; }
             Pieces<T::PW == 3 ? kWRows : 16> w;
             Pieces<NB> a;
@@ -203,10 +239,10 @@ __global__ void __launch_bounds__(kThreads, 1) row_gemm_kernel(const __grid_cons
             __syncwarp();
             if (lane == 0) mbar_arrive(raw_empty);
             if (issues && kb + 1 < kb1) {
-                if (wait(raw_empty, (uint32_t)(it & 1))) request(kb + 1);
+                if (mbar_wait(raw_empty, (uint32_t)(it & 1))) request(kb + 1);
                 else timed_out = true;
             }
-            if (!wait(&empty[s], (uint32_t)((it / kStages) & 1) ^ 1u)) timed_out = true;
+            if (!mbar_wait(&empty[s], (uint32_t)((it / kStages) & 1) ^ 1u)) timed_out = true;
             if (__any_sync(0xffffffffu, timed_out)) { timed_out = true; break; }
             uint8_t* const st = base + s * T::STAGE;
             if constexpr (T::PW == 3) w.store(st, T::W_PLANE, threadIdx.x);
@@ -223,9 +259,9 @@ __global__ void __launch_bounds__(kThreads, 1) row_gemm_kernel(const __grid_cons
             }
         }
         if (timed_out && issues) {                                        // let the copies land (bounded) that nobody may wait for
-            wait(raw_full, (uint32_t)((requested - 1) & 1));
+            mbar_wait(raw_full, (uint32_t)((requested - 1) & 1));
             if constexpr (T::PW == 1)
-                for (int k = max(kb0, w_next - kStages); k < w_next; ++k) wait(&full[(k - kb0) % kStages], (uint32_t)(((k - kb0) / kStages) & 1));
+                for (int k = max(kb0, w_next - kStages); k < w_next; ++k) mbar_wait(&full[(k - kb0) % kStages], (uint32_t)(((k - kb0) / kStages) & 1));
         }
     } else if (warp == kLoadWarps) {
         if (lane == 0) {
@@ -234,9 +270,9 @@ __global__ void __launch_bounds__(kThreads, 1) row_gemm_kernel(const __grid_cons
             int step = 0;                                                 // kAccK of K each
             for (int kb = kb0; kb < kb1 && !timed_out; ++kb) {
                 const int it = kb - kb0, s = it % kStages, grp = it / kGroupBlocks, first = it % kGroupBlocks == 0;
-                if (!wait(&full[s], (uint32_t)((it / kStages) & 1))) { timed_out = true; break; }
+                if (!mbar_wait(&full[s], (uint32_t)((it / kStages) & 1))) { timed_out = true; break; }
                 const uint32_t small = tmem + (uint32_t)((kAccs + 2 * (grp & 1)) * NB);
-                if (first && !wait(&small_empty[grp & 1], (uint32_t)((grp / 2) & 1) ^ 1u)) { timed_out = true; break; }
+                if (first && !mbar_wait(&small_empty[grp & 1], (uint32_t)((grp / 2) & 1) ^ 1u)) { timed_out = true; break; }
                 tc_fence_after();
                 const uint32_t w = smem_u32(base + s * T::STAGE), a = w + T::PW * T::W_PLANE;
 #pragma unroll
@@ -244,7 +280,7 @@ __global__ void __launch_bounds__(kThreads, 1) row_gemm_kernel(const __grid_cons
                     const int acc = step % kAccs;
                     const bool fresh = k % (kAccK / 16) == 0, done = (k + 1) % (kAccK / 16) == 0;
                     if (fresh) {
-                        if (!wait(&acc_empty[acc], (uint32_t)((step / kAccs) & 1) ^ 1u)) { timed_out = true; break; }
+                        if (!mbar_wait(&acc_empty[acc], (uint32_t)((step / kAccs) & 1) ^ 1u)) { timed_out = true; break; }
                         tc_fence_after();
                     }
                     auto wd = [&](int p) { return make_smem_desc(w + p * T::W_PLANE + k * 32); };
@@ -264,7 +300,7 @@ __global__ void __launch_bounds__(kThreads, 1) row_gemm_kernel(const __grid_cons
             }
             if (timed_out) {                                              // let every MMA issued so far finish (bounded) before TMEM is freed
                 umma_commit(drain);
-                wait(drain, 0);
+                mbar_wait(drain, 0);
             }
         }
     } else {
@@ -275,17 +311,27 @@ __global__ void __launch_bounds__(kThreads, 1) row_gemm_kernel(const __grid_cons
         float* const parts = g.scratch + (size_t)tile * groups * kWRows * NB + tid;        // K split: the groups' sums
         const int cols = n < g.N ? max(0, min(CW, g.M - mc)) : 0;                          // of this thread that exist
         float* const out = g.D + (size_t)mc * g.ldd + n;
+        uint32_t again = 0;                                                                // columns whose sums are not finite: taken again below
         auto put8 = [&](int c, const float (&v)[8]) {                                      // columns c .. c + 7
             float old[8];
             if (cols >= c + 8) {
 #pragma unroll
                 for (int j = 0; j < 8; ++j) old[j] = g.accumulate ? out[(size_t)(c + j) * g.ldd] : 0.f;
 #pragma unroll
-                for (int j = 0; j < 8; ++j) out[(size_t)(c + j) * g.ldd] = g.accumulate ? old[j] + v[j] : v[j];
+                for (int j = 0; j < 8; ++j) {
+                    const bool finite = v[j] - v[j] == 0.f;
+                    if (!finite) again |= 1u << (c + j);
+                    out[(size_t)(c + j) * g.ldd] = !finite ? old[j] : g.accumulate ? old[j] + v[j] : v[j];
+                }
             } else {
 #pragma unroll
                 for (int j = 0; j < 8; ++j)
-                    if (c + j < cols) out[(size_t)(c + j) * g.ldd] = g.accumulate ? out[(size_t)(c + j) * g.ldd] + v[j] : v[j];
+                    if (c + j < cols) {
+                        const float o = g.accumulate ? out[(size_t)(c + j) * g.ldd] : 0.f;
+                        const bool finite = v[j] - v[j] == 0.f;
+                        if (!finite) again |= 1u << (c + j);
+                        out[(size_t)(c + j) * g.ldd] = !finite ? o : g.accumulate ? o + v[j] : v[j];
+                    }
             }
         };
         int step = 0;
@@ -303,7 +349,7 @@ __global__ void __launch_bounds__(kThreads, 1) row_gemm_kernel(const __grid_cons
 #pragma unroll 1
                 for (int t = 0; t < steps; ++t, ++step) {
                     const int acc = step % kAccs;
-                    if (!wait(&acc_full[acc], (uint32_t)((step / kAccs) & 1))) timed_out = true;
+                    if (!mbar_wait(&acc_full[acc], (uint32_t)((step / kAccs) & 1))) timed_out = true;
                     timed_out = __any_sync(0xffffffffu, timed_out);
                     if (timed_out) break;
                     tc_fence_after();
@@ -319,7 +365,7 @@ __global__ void __launch_bounds__(kThreads, 1) row_gemm_kernel(const __grid_cons
                 for (int j = 0; j < CW / 2; ++j) sum[j] = add2(sum[j], unit[j]);
             }
             if (timed_out) break;
-            if (!wait(&small_full[gi & 1], (uint32_t)((gi / 2) & 1))) timed_out = true;
+            if (!mbar_wait(&small_full[gi & 1], (uint32_t)((gi / 2) & 1))) timed_out = true;
             timed_out = __any_sync(0xffffffffu, timed_out);
             if (timed_out) break;
             tc_fence_after();
@@ -339,52 +385,53 @@ __global__ void __launch_bounds__(kThreads, 1) row_gemm_kernel(const __grid_cons
             if (split) {
 #pragma unroll
                 for (int j = 0; j < CW; ++j) parts[(size_t)gr * kWRows * NB + j * 256] = grp[j];
-            } else if (gr + 1 < g1) {
-#pragma unroll
-                for (int j = 0; j < CW; ++j) total[j * 256] = gr == 0 ? grp[j] : total[j * 256] + grp[j];
             } else {
 #pragma unroll
-                for (int c = 0; c < CW; c += 8) {
-                    float v[8];
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) v[j] = gr == 0 ? grp[c + j] : total[(c + j) * 256] + grp[c + j];
-                    put8(c, v);
-                }
+                for (int j = 0; j < CW; ++j) total[j * 256] = gr == 0 ? grp[j] : total[j * 256] + grp[j];
             }
         }
-        // a wait ran out: what is missing is no number, in the result or in the partial sums
-        if (timed_out) {
-            const float nan = __int_as_float(0x7fffffff), v[8] = {nan, nan, nan, nan, nan, nan, nan, nan};
-            if (split)
-                for (int gr = g0; gr < g1; ++gr)
-                    for (int j = 0; j < CW; ++j) parts[(size_t)gr * kWRows * NB + j * 256] = nan;
-            else
+        // a wait ran out: what is missing is no number, so that plain multiply-adds put it right where the last CTA of the tile still comes to it
+        if (timed_out)
 #pragma unroll 1
-                for (int c = 0; c < CW; c += 8) put8(c, v);
-        }
+            for (int j = 0; j < CW; ++j) {
+                if (!split) total[j * 256] = __int_as_float(0x7fffffff);
+                else
+                    for (int gr = g0; gr < g1; ++gr) parts[(size_t)gr * kWRows * NB + j * 256] = __int_as_float(0x7fffffff);
+            }
+        bool puts = true;
         if (split) {
             // the last CTA of the tile to arrive adds the groups as above
             __threadfence();
             asm volatile("bar.sync 1, 256;" ::: "memory");
             if (tid == 0) *last = arrive();
             asm volatile("bar.sync 1, 256;" ::: "memory");
-            if (*last) {
-                __threadfence();
+            puts = *last;
+            __threadfence();
+        }
+        if (puts)
 #pragma unroll
-                for (int c = 0; c < CW; c += 8) {
-                    float v[8];
+            for (int c = 0; c < CW; c += 8) {
+                float v[8];
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) v[j] = __ldcg(parts + (c + j) * 256);
-                    for (int z = 1; z < groups; ++z) {
-                        float u[8];
+                for (int j = 0; j < 8; ++j) v[j] = split ? __ldcg(parts + (c + j) * 256) : total[(c + j) * 256];
+                for (int z = 1; split && z < groups; z += 4) {                             // four groups' loads in flight
+                    float u[4][8];
 #pragma unroll
-                        for (int j = 0; j < 8; ++j) u[j] = __ldcg(parts + (size_t)z * kWRows * NB + (c + j) * 256);
+                    for (int i = 0; i < 4; ++i)
 #pragma unroll
-                        for (int j = 0; j < 8; ++j) v[j] += u[j];
-                    }
-                    put8(c, v);
+                        for (int j = 0; j < 8; ++j) u[i][j] = z + i < groups ? __ldcg(parts + (size_t)(z + i) * kWRows * NB + (c + j) * 256) : 0.f;
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) v[j] += u[i][j];
                 }
+                put8(c, v);
             }
+        for (; again != 0; again &= again - 1) {
+            const int c = __ffs(again) - 1;
+            float* const at = out + (size_t)c * g.ldd;
+            const float x = plain_result(g.A + (size_t)(mc + c) * g.lda, static_cast<const WT*>(g.W) + (size_t)n * g.K, g.K);
+            *at = g.accumulate ? *at + x : x;
         }
     }
     if (timed_out && g.status != nullptr) atomicOr(g.status, STATUS_TIMEOUT);
@@ -406,8 +453,7 @@ int sms() {
 }
 
 template <int NB, typename WT>
-cudaError_t launch_t(RowGemmArgs g, dim3 grid, int per, cudaStream_t st) {
-    if (g.wait_ns == 0) g.wait_ns = kWaitLimitNs;
+cudaError_t launch_t(const RowGemmArgs& g, dim3 grid, int per, cudaStream_t st) {
     using T = RowsTile<NB, WT>;
     CUtensorMap ma, mw;
     if (make_f32_map_2d(&ma, g.A, (uint64_t)g.M, (uint64_t)g.K, (uint64_t)g.lda * 4, BK, NB) != LUMI_OK) return cudaErrorInvalidValue;

@@ -625,7 +625,6 @@ struct RowGemmArgs {
     int32_t* counters; int n_counters;
     float* scratch; size_t scratch_floats;
     int32_t* status;                     // takes STATUS_TIMEOUT (may be null)
-    uint64_t wait_ns = 0;                // limit of every wait, 0: the usual one
     int skip_units = 0;                  // test hook: the operands of this many CTAs (x, then y, then z) never arrive
 };
 bool row_gemm_supported(int K);

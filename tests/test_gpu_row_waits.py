@@ -12,7 +12,7 @@ def run(a, w, d, skip, status):
     import torch
     torch.cuda.synchronize()
     return lumi_b200.lib().lumi_debug_row_gemm_wait_timeout(a.data_ptr(), w.data_ptr(), int(w.dtype == torch.bfloat16), d.data_ptr(), a.shape[0], w.shape[0], a.shape[1],
-                                                            2_000_000, skip, status.data_ptr() if status is not None else 0)
+                                                            skip, status.data_ptr() if status is not None else 0)
 
 
 # one tile; K in one piece over several tiles; K over three CTAs per tile and 228 CTAs: with 148 that are not fed, a tile's last share begins after the
@@ -41,14 +41,15 @@ def test_the_next_product_is_right(M, N, K, skip, wdt):
 
 
 @pytest.mark.parametrize("M,N,K,skip", CASES)
-def test_no_result_of_a_lost_wait_looks_like_one(M, N, K, skip):
-    """Without a status word: what the kernel could not compute is no number, the rest has its usual bits."""
+def test_a_lost_wait_costs_time_and_no_result(M, N, K, skip):
+    """Without a status word every CTA goes on, and what the tensor core did not deliver is summed by multiply-adds: the bound of the ordinary product."""
     import torch
     a, w = operands(M, N, K)
     want = product(a, w)
-    product(-2 * a, w)
+    ref = a.double() @ w.double().T
+    product(-2 * a, w)                                        # partial sums of another product in the scratch memory
     d = torch.full((M, N), 7.0, device="cuda")
     assert run(a, w, d, skip, None) == 0
-    assert bool((torch.isnan(d) | (d == want)).all())
+    assert (d.double() - ref).abs().max() < 2e-6 * ref.abs().max()
     product(-2 * a, w)
     assert torch.equal(product(a, w), want)
