@@ -5,19 +5,22 @@
 // products of planes the six that reach fp32's last bit are taken (hi hi, hi mid, mid hi, mid mid, hi lo, lo hi: what is left out is 2^-24 of a
 // product).  Products of bf16 numbers are exact; what the tensor core loses is in its sums, which it cuts off instead of rounding: 1e-6 over K =
 // 1024 in one accumulator, 4e-8 over 32.  So the hi hi products go 32 of K at a time into an empty accumulator, which eight warps take out and add up in
-// fp32; the other five, 2^-8 of the size and with them their error, stay in two accumulators for 256 of K.
-// The order of a sum is fixed by K alone: four accumulators to a unit of 128 of K, two units and the small products to a group of 256, the groups
-// in order, wherever K is split and however many rows there are; a row's results are the same bits alone and among others.  Error against 64 bits (root mean
-// square, of the results'), K = 128 / 1024 / 2816: 6.4e-8 / 8.0e-8 / 9.5e-8; the fp32 multiply-adds that did this before came to 8.8e-8 / 10.1e-8 / 11.0e-8.
-// (16 of K at a time: 6.3e-8 / 8.0e-8 / 9.0e-8, 5 - 10 % slower; 64: 7.6e-8 / 9.0e-8 / 9.9e-8, not faster.)
+// fp32; the other five, 2^-8 of the size and with them their error, stay in two accumulators for 256 of K.  What was cut off has the sign of the sum, so
+// it adds up where operands have one sign; its average is put back (with_cut).
+// The order of a sum is fixed by K alone: two accumulators to a k-block of 64, four k-blocks and the small products to a group of 256, two groups to a
+// pair, the pairs in order, wherever K is split and however many rows there are; a row's results are the same bits alone and among others.  Error
+// against 64 bits (root mean square, of the results'), K = 128 / 1024 / 2048 / 2816, beside the fp32 multiply-adds that did this before: operands of both signs
+// 5.6 / 7.3 / 7.9 / 8.4e-8 (8.8 / 10.1 / 10.6 / 11.0), of one sign 4.8 / 4.7 / 4.8 / 5.2e-8 (4.8 / 4.7 / 4.7 / 5.1), with a mean of two deviations 3.9 / 3.7 / 4.3 / 5.2e-8
+// (4.2 / 3.9 / 4.2 / 5.1).  (Groups of 256 one by one and nothing put back: 6.4 / 8.0 / 8.9 / 9.5, 6.3 / 6.2 / 6.4 / 6.9, 4.5 / 4.3 / 5.0 / 5.7e-8.)
 //
 // The weights take the 128-row side of the MMA, NB rows of the prompt the other; products with two planes of the same weights go as one MMA of twice the
 // width.  Warps 0 - 6: a k-block, copied densely to shared memory ahead of time, to registers and split into planes as the MMA reads them (K-major, 128-byte
 // swizzle; bf16 weights are copied straight to their plane).  Warp 7: TMEM, MMA.  Warps 8 - 15: accumulators, sums, results.
 // What bounds it: the splitting (15 pieces of four elements per thread and k-block of 64, 1600 of 2700 cycles), then the MMAs (16 per k-block of 100 cycles,
-// operand reads).  Measured against packed fp32 multiply-adds on the CUDA cores, microseconds: fp32 weights 384 x 7360 x 1024 184 -> 98, 384 x 1024 x 2048
-// 135 -> 41, 384 x 32000 x 1024 700 -> 328, 960 x 7360 x 1024 407 -> 185, 32 x 7360 x 1024 35 -> 29, 32 x 1024 x 2048 21 -> 21; bf16 weights 384 x 7360 x
-// 1024 184 -> 74, 32 x 7360 x 1024 33 -> 25.  Scores of 4 x 96 tokens, 48 layers in fp32: 16.6 -> 10.1 ms; a bf16 prompt of 100 tokens 10.0 -> 6.1 ms.
+// operand reads).  At the cap of 128 registers the 64-row tiles spill 92 bytes a thread (76 with bf16 weights), the held group above all.  Launches back to back, weights
+// from memory, against packed fp32 multiply-adds on the CUDA cores, microseconds: fp32 weights 384 x 7360 x 1024 177 -> 84, 384 x 1024 x 2048 129 -> 31, 384 x
+// 32000 x 1024 692 -> 309, 960 x 7360 x 1024 401 -> 167, 32 x 7360 x 1024 30 -> 21, 32 x 1024 x 2048 15 -> 16; bf16 weights 384 x 7360 x 1024 175 -> 60, 32 x
+// 7360 x 1024 27 -> 16.  Scores of 4 x 96 tokens, 48 layers in fp32: 16.6 -> 10.1 ms; a bf16 prompt of 100 tokens 10.0 -> 6.1 ms.
 #include "internal.h"
 #include "tcgen05.cuh"
 
@@ -60,6 +63,14 @@ __device__ __forceinline__ uint64_t minus2(uint64_t a, uint64_t b) {
 }
 __device__ __forceinline__ float first_of(uint64_t d) { return __uint_as_float((uint32_t)d); }
 __device__ __forceinline__ float second_of(uint64_t d) { return __uint_as_float((uint32_t)(d >> 32)); }
+
+// What joins a group's sum h of hi hi products, with what the tensor core cut off of them: half a last place of every sum of 32 on the average, always toward
+// zero, which in a group of such sums is about half a last place of h.  0.4 of one is put back (0.5 serves sums near a power of two, 0.3 those with a
+// mantissa near 1.6).  Sums whose last three bits are zero have lost nothing as a rule (whole numbers, rows with a single entry) and stay exact.
+__device__ __forceinline__ uint32_t with_cut(float h, float small) {
+    const uint32_t b = __float_as_uint(h);
+    return __float_as_uint(fmaf(__uint_as_float(b & 0xff800000u), (b & 7u) != 0 ? 0.4f * 1.1920929e-7f : 0.f, small));
+}
 
 // CW columns of this warp's 32 lanes of TMEM, in pairs
 template <int CW>
@@ -334,20 +345,19 @@ __global__ void __launch_bounds__(kThreads, 1) row_gemm_kernel(const __grid_cons
                     }
             }
         };
+        float held[CW];                                                                    // an even group's sum, until its neighbour's is there
         int step = 0;
         for (int gr = g0; gr < g1 && !timed_out; ++gr) {
             const int gi = gr - g0, kbe = min(blocks, (gr + 1) * kGroupBlocks);
-            uint64_t sum[CW / 2];
+            uint64_t sum[CW / 2], unit[CW / 2];                                            // unit: the last k-block's, not yet in sum
 #pragma unroll
-            for (int j = 0; j < CW / 2; ++j) sum[j] = 0;
+            for (int j = 0; j < CW / 2; ++j) sum[j] = unit[j] = 0;
 #pragma unroll 1
-            for (int kb = gr * kGroupBlocks; kb < kbe && !timed_out; kb += 2) {            // a unit
-                uint64_t unit[CW / 2];
+            for (int kb = gr * kGroupBlocks; kb < kbe && !timed_out; ++kb) {
 #pragma unroll
-                for (int j = 0; j < CW / 2; ++j) unit[j] = 0;
-                const int steps = min(2, kbe - kb) * (BK / kAccK);
-#pragma unroll 1
-                for (int t = 0; t < steps; ++t, ++step) {
+                for (int j = 0; j < CW / 2; ++j) sum[j] = add2(sum[j], unit[j]);
+#pragma unroll
+                for (int t = 0; t < BK / kAccK; ++t, ++step) {
                     const int acc = step % kAccs;
                     if (!mbar_wait(&acc_full[acc], (uint32_t)((step / kAccs) & 1))) timed_out = true;
                     timed_out = __any_sync(0xffffffffu, timed_out);
@@ -359,22 +369,24 @@ __global__ void __launch_bounds__(kThreads, 1) row_gemm_kernel(const __grid_cons
                     __syncwarp();
                     if (lane == 0) mbar_arrive(&acc_empty[acc]);
 #pragma unroll
-                    for (int j = 0; j < CW / 2; ++j) unit[j] = add2(unit[j], v[j]);
+                    for (int j = 0; j < CW / 2; ++j) unit[j] = t == 0 ? v[j] : add2(unit[j], v[j]);
                 }
-#pragma unroll
-                for (int j = 0; j < CW / 2; ++j) sum[j] = add2(sum[j], unit[j]);
             }
             if (timed_out) break;
             if (!mbar_wait(&small_full[gi & 1], (uint32_t)((gi / 2) & 1))) timed_out = true;
             timed_out = __any_sync(0xffffffffu, timed_out);
             if (timed_out) break;
             tc_fence_after();
-            {
-                uint64_t v[CW / 2], u[CW / 2];
-                tmem_pairs<CW>(lanes + (uint32_t)((kAccs + 2 * (gi & 1)) * NB), v);
-                tmem_pairs<CW>(lanes + (uint32_t)((kAccs + 2 * (gi & 1) + 1) * NB), u);
 #pragma unroll
-                for (int j = 0; j < CW / 2; ++j) sum[j] = add2(sum[j], add2(v[j], u[j]));
+            for (int c = 0; c < CW / 2; c += 8) {                                          // sixteen columns at a time
+                uint64_t v[8], u[8];
+                tmem_pairs<16>(lanes + (uint32_t)((kAccs + 2 * (gi & 1)) * NB + 2 * c), v);
+                tmem_pairs<16>(lanes + (uint32_t)((kAccs + 2 * (gi & 1) + 1) * NB + 2 * c), u);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    const uint64_t s = add2(v[j], u[j]), h = add2(sum[c + j], unit[c + j]);
+                    sum[c + j] = add2(sum[c + j], add2(unit[c + j], pair2(with_cut(first_of(h), first_of(s)), with_cut(second_of(h), second_of(s)))));
+                }
             }
             tc_fence_before();
             __syncwarp();
@@ -385,9 +397,15 @@ __global__ void __launch_bounds__(kThreads, 1) row_gemm_kernel(const __grid_cons
             if (split) {
 #pragma unroll
                 for (int j = 0; j < CW; ++j) parts[(size_t)gr * kWRows * NB + j * 256] = grp[j];
+            } else if (gr % 2 == 0 && gr + 1 < g1) {
+#pragma unroll
+                for (int j = 0; j < CW; ++j) held[j] = grp[j];
             } else {
 #pragma unroll
-                for (int j = 0; j < CW; ++j) total[j * 256] = gr == 0 ? grp[j] : total[j * 256] + grp[j];
+                for (int j = 0; j < CW; ++j) {
+                    const float two = gr % 2 == 0 ? grp[j] : held[j] + grp[j];
+                    total[j * 256] = gr < 2 ? two : total[j * 256] + two;
+                }
             }
         }
         // a wait ran out: what is missing is no number, so that plain multiply-adds put it right where the last CTA of the tile still comes to it
@@ -413,17 +431,17 @@ __global__ void __launch_bounds__(kThreads, 1) row_gemm_kernel(const __grid_cons
             for (int c = 0; c < CW; c += 8) {
                 float v[8];
 #pragma unroll
-                for (int j = 0; j < 8; ++j) v[j] = split ? __ldcg(parts + (c + j) * 256) : total[(c + j) * 256];
-                for (int z = 1; split && z < groups; z += 4) {                             // four groups' loads in flight
+                for (int j = 0; j < 8; ++j) if (!split) v[j] = total[(c + j) * 256];
+                for (int z = 0; split && z < groups; z += 4) {                             // four groups' loads in flight
                     float u[4][8];
 #pragma unroll
                     for (int i = 0; i < 4; ++i)
 #pragma unroll
                         for (int j = 0; j < 8; ++j) u[i][j] = z + i < groups ? __ldcg(parts + (size_t)(z + i) * kWRows * NB + (c + j) * 256) : 0.f;
 #pragma unroll
-                    for (int i = 0; i < 4; ++i)
+                    for (int i = 0; i < 4; i += 2)
 #pragma unroll
-                        for (int j = 0; j < 8; ++j) v[j] += u[i][j];
+                        for (int j = 0; j < 8; ++j) v[j] = z + i == 0 ? u[i][j] + u[i + 1][j] : v[j] + (u[i][j] + u[i + 1][j]);
                 }
                 put8(c, v);
             }
