@@ -171,7 +171,7 @@ __global__ void __launch_bounds__(256) norm_split_kernel(const float* x, const f
 // The same for many rows, one warp each: a CTA per row is a chain of load, barrier and store with eight rows in flight on an SM, and at 3.4 TB/s waited
 // for memory most of the time.  The sum is taken as above (256 partial sums, the trees of eight warps, these in order), so its bits are the same; the row
 // is read again for the result (from L1), four elements per lane.  32768 rows of 1024: 80 -> 49 us.
-__global__ void __launch_bounds__(256) norm_split_rows_kernel(const float* __restrict__ x, const float* __restrict__ gamma, __nv_bfloat16* hi, __nv_bfloat16* lo,
+__global__ void __launch_bounds__(256) norm_split_rows_kernel(const float* x, const float* __restrict__ gamma, __nv_bfloat16* __restrict__ hi, __nv_bfloat16* __restrict__ lo,
                                                               int rows, int D, float eps, float* ssq, int ssq_stride) {
     const int b = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     pdl_launch_dependents();
@@ -197,7 +197,7 @@ __global__ void __launch_bounds__(256) norm_split_rows_kernel(const float* __res
         const float4 v = *reinterpret_cast<const float4*>(xr + i), g = __ldg(reinterpret_cast<const float4*>(gamma + i));
         float w[4] = {v.x, v.y, v.z, v.w};
         const float gg[4] = {g.x, g.y, g.z, g.w};
-        __nv_bfloat16 h[4], l[4];
+        __align__(8) __nv_bfloat16 h[4], l[4];
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
             w[e] = __fmul_rn(ssq != nullptr ? w[e] : __fmul_rn(w[e], r), gg[e]);
