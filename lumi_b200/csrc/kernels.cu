@@ -29,32 +29,6 @@ namespace {
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
-#ifdef LUMI_TIMELINE
-// debugging aid (not compiled by default): per-kernel time stamps of a few CTAs
-__device__ unsigned long long g_tl[65536 * 10];
-__device__ unsigned g_tl_n;
-__device__ __forceinline__ unsigned long long tl_now() { unsigned long long t; asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t)); return t; }
-__device__ __forceinline__ bool tl_on() { return threadIdx.x == 0 && (blockIdx.x == 0 || blockIdx.x == gridDim.x / 2 || blockIdx.x == gridDim.x - 1) && blockIdx.y == 0; }
-__device__ __forceinline__ void tl_rec(int kind, const unsigned long long (&m)[6], unsigned long long cend) {
-    unsigned i = atomicAdd(&g_tl_n, 1u);
-    if (i < 65536u) {
-        unsigned smid; asm volatile("mov.u32 %0, %%smid;" : "=r"(smid));
-        g_tl[i * 10] = kind; g_tl[i * 10 + 1] = blockIdx.x; g_tl[i * 10 + 2] = smid;
-        for (int j = 0; j < 6; ++j) g_tl[i * 10 + 3 + j] = m[j];
-        g_tl[i * 10 + 9] = cend;
-    }
-}
-// slot 0: start (global ns); slots 1..4: SM cycle counter at the marks; slot 5: global ns at the wait's end
-#define TL_T0 unsigned long long tlm[6] = {tl_now(), 0, 0, 0, 0, 0};
-#define TL_T1 tlm[5] = tl_now(); tlm[1] = clock64();
-#define TL_MARK(i) tlm[i] = clock64();
-#define TL_END(kind) if (tl_on()) { tl_rec(kind, tlm, clock64()); }
-#else
-#define TL_T0
-#define TL_T1
-#define TL_MARK(i)
-#define TL_END(kind)
-#endif
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -492,7 +466,6 @@ __global__ void __launch_bounds__(256, 2) gemv_pre_kernel(const float* A, int ld
     const uint32_t row_bytes = (uint32_t)K * (uint32_t)sizeof(WT);
     unsigned char* wrows = reinterpret_cast<unsigned char*>(xs + (size_t)NB * K);
 
-    TL_T0
     // When the next kernel may come.  At once, where one sequence's fp32 rows fill the shared memory and hold the kernels after it off; with
     // bf16 rows half of it stays free, the chain runs several kernels ahead of itself and their requests get in the way of the few
     // loads everyone waits for: there, and with several sequences, only behind this kernel's own wait.  64 tokens of the 48-layer base model,
@@ -557,7 +530,6 @@ __global__ void __launch_bounds__(256, 2) gemv_pre_kernel(const float* A, int ld
     }
     pdl_wait();
     if (late) pdl_launch_dependents();
-    TL_T1
 
     // residuals of the rows whose stores this lane owns (register rows, first shared-memory group)
     float rres_r[NB], rres_s[NB];
@@ -640,7 +612,6 @@ __global__ void __launch_bounds__(256, 2) gemv_pre_kernel(const float* A, int ld
                 }
             }
         }
-        TL_MARK(2)
     } else {
         for (int i = threadIdx.x; i < NB * K4; i += 256) {
             int b = i / K4, k4 = i - b * K4;
@@ -649,7 +620,6 @@ __global__ void __launch_bounds__(256, 2) gemv_pre_kernel(const float* A, int ld
             reinterpret_cast<float4*>(xs)[i] = v;
         }
         __syncthreads();
-        TL_MARK(2)
         if (post.o != nullptr) {
 #pragma unroll
             for (int b = 0; b < NB; ++b) {
@@ -758,7 +728,6 @@ __global__ void __launch_bounds__(256, 2) gemv_pre_kernel(const float* A, int ld
             }
         }
     }
-    TL_MARK(3)
     bool timed_out = false;
     for (int j0 = warp; j0 < ns && !timed_out; j0 += 8 * GR) {
         if (j0 != warp) {            // later groups (rare): their residuals are fetched here
@@ -787,7 +756,6 @@ __global__ void __launch_bounds__(256, 2) gemv_pre_kernel(const float* A, int ld
             if (timed_out) break;
         }
         if (timed_out) break;
-        if (j0 == warp) { TL_MARK(4) }
         const int ng = min(GR, (ns - j0 + 7) / 8);      // valid rows of this group
         // one straight-line body per row count, so that no branch sits between the loads and their use
         auto body = [&](auto ngc) {
@@ -849,7 +817,6 @@ __global__ void __launch_bounds__(256, 2) gemv_pre_kernel(const float* A, int ld
             }
         }
     }
-    TL_END(K == 1024 ? 1 : 3)
 }
 
 // ---- fused Mamba-3 decode step ---------------------------------------------------------------------
@@ -889,7 +856,6 @@ __global__ void __launch_bounds__(256, MINB) ssm_step_kernel(SsmArgs a, int ahea
     const size_t bh = (size_t)b * H + (active ? h : H - 1);
     const int c = lane % CG, r0 = lane / CG;
 
-    TL_T0
     pdl_launch_dependents();
     // prompts of different lengths: a sequence whose prompt has ended keeps its state until the others are done
     // (prompt_pos was advanced by the previous step, which has finished: see below)
@@ -937,7 +903,6 @@ __global__ void __launch_bounds__(256, MINB) ssm_step_kernel(SsmArgs a, int ahea
 #pragma unroll
     for (int j = 0; j < ROWS_PL; ++j) v_xp[j] = a.xprev[bh * P + min(sub * ROWS + lane + 32 * j, P - 1)];
     pdl_wait();
-    TL_T1
 
     const float* pr = a.proj + (size_t)b * a.ldp;
     const float* Bp = pr + 2 * DI;
@@ -1021,7 +986,6 @@ __global__ void __launch_bounds__(256, MINB) ssm_step_kernel(SsmArgs a, int ahea
     sc = warp_sum(sc);
     if (lane == 0) { red[0][warp] = sb; red[1][warp] = sc; }
     __syncthreads();       // also orders every warp's reads of bprev / cum / xprev above before the writes below
-    TL_MARK(2)
     if (!active) return;
     float tb = 0.f, tc = 0.f;
     for (int w = 0; w < nwarp; ++w) { tb += red[0][w]; tc += red[1][w]; }
@@ -1058,7 +1022,6 @@ __global__ void __launch_bounds__(256, MINB) ssm_step_kernel(SsmArgs a, int ahea
     }
     __syncwarp();
 
-    TL_MARK(3)
     const float4 bq = reinterpret_cast<const float4*>(sm.bt)[c];
     const float4 cq = reinterpret_cast<const float4*>(sm.ct)[c];
 #pragma unroll 1
@@ -1090,7 +1053,6 @@ __global__ void __launch_bounds__(256, MINB) ssm_step_kernel(SsmArgs a, int ahea
         }
     }
     __syncwarp();
-    TL_MARK(4)
     for (int p = lane; p < ROWS; p += 32) {
         const int row = prow0 + p;
         float xv = sm.xa[row];
@@ -1108,7 +1070,6 @@ __global__ void __launch_bounds__(256, MINB) ssm_step_kernel(SsmArgs a, int ahea
     }
     if (sub == 0)
         for (int s2 = lane; s2 < N; s2 += 32) a.bprev[bh * N + s2] = sm.bt[s2];
-    TL_END(2)
 }
 
 // h <- h_init broadcast over head_dim (model.rs:744-748); factors and angles <- 0 (:751-752)
