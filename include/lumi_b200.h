@@ -349,6 +349,10 @@ int32_t lumi_k_window_attention(uint64_t proj, int32_t ldp, const int32_t* off, 
 int32_t lumi_k_norm_add(uint64_t x, uint64_t o, uint64_t w, uint64_t y, uint64_t hi, uint64_t lo, int32_t rows, int32_t width, int32_t ld,
                         float eps, uint64_t stream);
 
+/* The gate of an attention block's MLP alone (inference/src/model.rs:550-552): rows of gu hold `width` gates, then `width` ups; sigmoid(gate) * up goes to
+ * out32 [rows][width] and / or hi (and lo) as bf16 halves (0: none).  width % 8 == 0, ld % 4 == 0, 16-byte aligned pointers. */
+int32_t lumi_k_gate_mul(uint64_t gu, int32_t ld, uint64_t out32, uint64_t hi, uint64_t lo, int32_t rows, int32_t width, uint64_t stream);
+
 /* One Mamba block (RMSNorm -> in_proj -> state step -> out_proj + residual, inference/src/model.rs:296-375
  * in arithmetic) WITHOUT any allocation.  This entry point has no counterpart in the reference.
  *

@@ -3251,3 +3251,10 @@ extern "C" int32_t lumi_k_norm_add(uint64_t x, uint64_t o, uint64_t w, uint64_t 
     LUMI_CUDA(launch_row_norm(a, (cudaStream_t)stream));
     return LUMI_OK;
 }
+
+extern "C" int32_t lumi_k_gate_mul(uint64_t gu, int32_t ld, uint64_t out32, uint64_t hi, uint64_t lo, int32_t rows, int32_t width, uint64_t stream) {
+    if (!gu || (!out32 && !hi) || rows <= 0 || width <= 0 || (width % 8) || ld < 2 * width || (ld % 4) || ((gu | out32 | hi | lo) & 15))
+        return fail(LUMI_E_INVALID, "bad argument to lumi_k_gate_mul");
+    LUMI_CUDA(launch_gate_mul((const float*)gu, ld, (float*)out32, (__nv_bfloat16*)hi, (__nv_bfloat16*)lo, rows, width, (cudaStream_t)stream));
+    return LUMI_OK;
+}

@@ -1,5 +1,6 @@
 """GPU: the gate of an attention block's MLP takes two quads per thread, in prompts and in steps, at widths that fill its blocks or not;
-the state step asks for states one block per SM ahead, over heads that do not fill their last block.
+results of the state step where it asks for states one block per SM ahead, over heads that do not fill their last block (the requests
+themselves change no result; the gate's own values: test_gpu_gate_values.py).
 
 Bound: the benchmark definition's 2e-2 of the largest logit for bf16 weights (the cache of keys and values is bf16)."""
 import numpy as np
