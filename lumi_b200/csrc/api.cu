@@ -1317,6 +1317,10 @@ bool has_experts(const lumi_session* s) {
     for (const LayerSpec& L : s->m->cfg.specs) if (L.ff.experts > 0) return true;
     return false;
 }
+bool has_delta(const lumi_session* s) {
+    for (const LayerSpec& L : s->m->cfg.specs) if (L.mixer.kind == MIXER_DELTA) return true;
+    return false;
+}
 
 // D = act(A W^T) over `rows` rows: tensor cores from the bf16 halves, or the weight-streaming kernel from fp32 rows.  The result
 // goes to out32, or (tensor cores, out_hi given) as bf16 halves only.
@@ -2275,8 +2279,12 @@ int32_t prefill_listed(lumi_session* s, int batch, int T, bool with_head, float*
                                            s->stream, lens, embed_post_of(s, b, slot0 + b0, p.tc)));
             // Slices of few rows are a chain of short kernels, as steps are: dependent launch as there.  The embedding kernel above is launched in order, so
             // what the slice before left (states, caches, positions) is complete for kernels that read it ahead of their own wait.
-            // One sequence's 77 tokens in portions of 23, 12 layers: 6.4 -> 5.7 ms.
-            const DependentLaunch dependent(s->opt_pdl && M <= pdl_tc_max(), s->opt_pdl && p.tc && M <= pdl_gemm_max());
+            // One sequence, 12 layers of width 1024, Zozonex / Zutazen, off -> on, ms: 2 tokens 0.58 -> 0.50 / 0.80 -> 0.70, 4 tokens 0.76 -> 0.71 / 0.95 -> 0.88, 16
+            // tokens 0.82 -> 0.68 / 1.34 -> 1.17, 64 tokens 0.85 -> 0.75 / 1.49 -> 1.35, 128 tokens 1.05 -> 0.93 / 1.51 -> 1.34; products alone 256 tokens 1.34 -> 1.27 /
+            // 1.66 -> 1.52, 1024 tokens 3.16 -> 3.07 / 2.21 -> 2.05.  Not where five to eight rows go through the streaming kernels past delta-rule steps, whose
+            // shared memory then keeps the kernel behind them from its SMs: 5 tokens 0.94 -> 1.02, 8 tokens 1.11 -> 1.25 (without such layers 1.22 -> 1.16, 1.41 -> 1.33).
+            const bool rows_early = s->opt_pdl && M <= pdl_tc_max() && (p.tc || M <= 4 || !has_delta(s));
+            const DependentLaunch dependent(rows_early, s->opt_pdl && p.tc && M <= pdl_gemm_max());
             float* const stream = b.x;
             for (const Layer& L : s->m->layers) LUMI_TRY(listed_layer(p, r, L));
             LUMI_TRY(settle(p, r, stream));
