@@ -144,7 +144,7 @@ __global__ void __launch_bounds__(256) norm_split_kernel(const float* x, const f
 
 // The same for many rows, one warp each: a CTA per row is a chain of load, barrier and store with eight rows in flight on an SM, and at 3.4 TB/s waited
 // for memory most of the time.  The sum is taken as above (256 partial sums, the trees of eight warps, these in order), so its bits are the same; the row
-// is read again for the result (from L1), four elements per lane.  32768 rows of 1024: 80 -> 49 us.
+// is read again for the result (from L1), four elements per lane.  32768 rows of 1024: 76 -> 49 us.
 __global__ void __launch_bounds__(256) norm_split_rows_kernel(const float* x, const float* __restrict__ gamma, __nv_bfloat16* __restrict__ hi, __nv_bfloat16* __restrict__ lo,
                                                               int rows, int D, float eps, float* ssq, int ssq_stride) {
     const int b = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
@@ -1521,7 +1521,10 @@ cudaError_t launch_embed(const void* emb, int dtype, const uint32_t* tok_cur, fl
 cudaError_t launch_norm_split(const float* x, const float* gamma, __nv_bfloat16* hi, __nv_bfloat16* lo, int B, int D,
                               float eps, cudaStream_t st, float* ssq, int ssq_stride) {
     const uintptr_t at = reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(gamma) | reinterpret_cast<uintptr_t>(hi) | reinterpret_cast<uintptr_t>(lo);
-    if (B >= 2048 && gamma != nullptr && (D & 3) == 0 && (at & 15) == 0)
+    // CTA / warp per row, us.  Width 512: 1024 rows 3.7 / 3.4, 16384 rows 32 / 11; 1024: 1536 rows 5.6 / 6.4, 2048 rows 6.4 / 6.4, 4096 rows 10.1 / 7.7, 16384 rows
+    // 37 / 24; 1536: 1536 rows 8.1 / 8.6, 2048 rows 8.9 / 8.7, 32768 rows 126 / 80; 2048: 2048 rows 9.2 / 12.0, 8192 rows 29.5 / 29.6, 32768 rows 116 / 122 (a row is
+    // a longer chain for its warp, and eight of them no longer stay in L1).
+    if (B >= 2048 && D <= 1536 && gamma != nullptr && (D & 3) == 0 && (at & 15) == 0)
         return launch_k(norm_split_rows_kernel, dim3((B + 7) / 8), dim3(256), 0, st, x, gamma, hi, lo, B, D, eps, ssq, ssq_stride);
     return launch_k(norm_split_kernel, dim3(B), dim3(256), 0, st, x, gamma, hi, lo, D, eps, ssq, ssq_stride);
 }
@@ -1708,10 +1711,10 @@ static cudaError_t ssm_variant(const SsmArgs& a, cudaStream_t st) {
     int hpb = 8 / WPH;
     if (hpb > a.H) hpb = a.H;
     dim3 grid((a.H + hpb - 1) / hpb, a.B);
-    // Tiles asked for one block per SM ahead.  Base model, 16 steps, 64 / 128 / 300 sequences: 25.0 / 42.3 / 74.3 -> 24.6 / 40.7 /
-    // 73.7 ms (two blocks per SM, the number that is resident: 25.0 / 40.8 / 74.8; four: 25.0 / 42.8 / 80.3, they crowd out states in
-    // use).  With more blocks the stream is steady and the requests get in its way: 512 / 800 sequences 111.6 / 170.7 -> 112.3 /
-    // 172.3 ms; the line lies between 2400 blocks (gain) and 4096 (loss).
+    // Tiles asked for one block per SM ahead.  Base model, 16 steps, without / with: 64 sequences 23.6 / 23.3 ms, 128 sequences 40.7 / 39.0, 200 to 400
+    // sequences the same (two blocks per SM, the number that is resident, and four gave less: four crowd out states in use).  With more blocks the stream is
+    // steady and the requests get in its way: 512 / 800 sequences 105.7 / 162.1 -> 107.7 / 163.7 ms; the line lies between 3200 blocks (no change) and
+    // 4096 (loss).
     const int ahead = (long)grid.x * grid.y <= 20L * sm_count() ? sm_count() : 0;
     return launch_k(ssm_step_kernel<P, N, WPH, MINB>, grid, dim3(hpb * WPH * 32), 0, st, a, ahead);
 }
