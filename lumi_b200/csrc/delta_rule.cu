@@ -446,7 +446,7 @@ __global__ void __launch_bounds__(256) delta_prep_pairs_kernel(DeltaArgs a, int 
     const float* cw = (is_v ? a.conv_v : (is_k ? a.conv_k : a.conv_q)) + (size_t)ch0 * TAPS;
     const size_t oo = is_v ? (size_t)2 * a.G * dk4 + (size_t)head * a.dvp : (size_t)un * dk4;
     const int channels = 2 * Cq + a.H * a.dv;
-    const float q_scale = __frcp_rn(__fsqrt_rn((float)a.dk));
+    const float root = __fsqrt_rn((float)a.dk), q_scale = __frcp_rn(root);
     for (int c0 = 0; c0 < d; c0 += 64 * NP) {             // value heads may be wider than the key heads NP was chosen for
         float2 wt[NP][TAPS], x[NP][TAPS];                 // x[.][(t - tb + j) % TAPS]: input of token t - (TAPS - 1) + j
         auto chan = [&](int i) { return c0 + 2 * lane + 64 * i; };
@@ -500,7 +500,10 @@ __global__ void __launch_bounds__(256) delta_prep_pairs_kernel(DeltaArgs a, int 
                 }
                 if (!is_v) {
                     float r = __frcp_rn(__fsqrt_rn(warp_total(s) + a.unit_eps));
-                    if (!is_k) r *= q_scale;
+                    if (!is_k) {                          // r / root, the product put right by what it left
+                        const float quot = r * q_scale;
+                        r = fmaf(fmaf(-quot, root, r), q_scale, quot);
+                    }
 #pragma unroll
                     for (int i = 0; i < NP; ++i) { v[i].x *= r; v[i].y *= r; }
                 }

@@ -775,7 +775,7 @@ cudaError_t launch_prefill_scan(const PrefillArgs& a, cudaStream_t st) {
         set = true;
     }
     const int rows = a.nb * a.ts;
-    // the projection rows as a 2-D fp32 tensor [rows][ldp]; boxes of 64 tokens x 32 columns (x, z, theta) and x 64 (B, C)
+    // the projection rows as a 2-D fp32 tensor [rows][ldp]; boxes of 64 tokens x 32 columns (x, theta) and x 64 (B, C)
     CUtensorMap m32, m64;
     if (make_f32_map_2d(&m32, a.proj, (uint64_t)rows, (uint64_t)a.ldp, (uint64_t)a.ldp * 4, 32, LCH) != LUMI_OK ||
         make_f32_map_2d(&m64, a.proj, (uint64_t)rows, (uint64_t)a.ldp, (uint64_t)a.ldp * 4, 64, LCH) != LUMI_OK)
