@@ -436,8 +436,11 @@ cudaError_t step_launch(const RetentionArgs& a, int cwl, cudaStream_t st) {
         if (e != cudaSuccess) return e;
     }
     const int RG = NT >> cwl, part_rows = ((a.dk + kParts - 1) / kParts + RG - 1) / RG * RG;
-    // one block per SM ahead, as in ssm_variant: the same line, the same reason
-    const int ahead = VPT < 0 && (long)a.H * a.nseq <= 20L * sm_count() ? sm_count() : 0;
+    // One block per SM ahead, where there are more blocks than the SMs hold at once.  Steps of six layers, without / with: heads of (128, 128), three blocks per SM,
+    // 5 / 10 / 20 / 40 blocks per SM 0.377 / 0.566 / 0.797 / 1.348 -> 0.368 / 0.556 / 0.780 / 1.300 ms; of (64, 128), six per SM, 15 / 40 per SM 0.536 / 0.820 ->
+    // 0.531 / 0.812, but 5 per SM, all of them there already, 0.282 -> 0.285.
+    const long resident = std::min<long>(2048 / NT, 228 * 1024 / (smem + 1024));
+    const int ahead = VPT < 0 && (long)a.H * a.nseq > resident * sm_count() ? sm_count() : 0;
     return launch_rows(kern, dim3(a.H, a.nseq), NT, smem, st, a, cwl, part_rows, ahead);
 }
 
