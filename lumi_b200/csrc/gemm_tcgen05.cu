@@ -875,6 +875,29 @@ int32_t gemm_tcgen05_init() {
     return LUMI_OK;
 }
 
+static bool width_counts(const GemmArgs& a);
+struct TileChoice { int width; long cost, rounds; };
+// The tile width of the least cost, with K in one piece: rounds of tiles times (width + 32: the part of a tile's time that does not shrink).
+static TileChoice tile_choice(const GemmArgs& a) {
+    static const int plain[] = {256, 224, 208, 192, 160, 128, 96, 64, 32}, ext[] = {256, 128, 64, 32};
+    const bool by_rows = a.ext != nullptr && a.ext->tiles != nullptr;
+    const int groups = a.ext != nullptr && !by_rows ? a.ext->groups : 1, cols = a.ext != nullptr ? a.ext->group_rows : a.N;
+    auto rounds_of = [&](long rows, int w) {
+        const long tiles = (by_rows ? a.ext->max_tiles : (rows + BM - 1) / BM) * groups * ((cols + w - 1) / w);
+        return (tiles + sm_count_gemm() - 1) / sm_count_gemm();
+    };
+    TileChoice best{256, -1, 1};
+    for (int i = 0; i < (a.ext != nullptr ? 4 : 9); ++i) {
+        const int w = a.ext != nullptr ? ext[i] : plain[i];
+        if (a.ext == nullptr && a.nf.out_hi != nullptr && (w % 32) != 0) continue;       // the folded norm's partial sums are per 32 aligned columns
+        const long rounds = rounds_of(width_counts(a) ? a.M : tiled_rows(a), w), cost = rounds * (w + 32);
+        if (best.cost < 0 || cost < best.cost) best = TileChoice{w, cost, rounds};
+    }
+    best.rounds = rounds_of(tiled_rows(a), best.width);
+    best.cost = best.rounds * (best.width + 32);
+    return best;
+}
+
 // Tile width of the persistent kernel: the GPU works in rounds of one tile per SM, a round costs about its tile's
 // width, so take the width with the least rounds x width (7360 columns x 16 row tiles: 208 -> 4 rounds of 576 tiles,
 // against 4 rounds of 464 tiles at 256).  Ties go to the wider tile (less operand traffic per flop).
@@ -887,28 +910,18 @@ int32_t gemm_tcgen05_init() {
 // (measured at 64 x 1024 x 2048: 19.1 us against 23.2 us, +12.6 % tokens per second on the 64-sequence decode; wide split
 // tiles lost more in the fix-up than they gained).
 // LUMI_GEMM_SPLITK=1 turns splitting off.
-static bool width_counts(const GemmArgs& a);
 static void pick_tile(const GemmArgs& a, int* width, int* splits) {
-    static const int widths[] = {256, 224, 208, 192, 160, 128, 96, 64, 32};
     static const int env_splits = getenv("LUMI_GEMM_SPLITK") ? atoi(getenv("LUMI_GEMM_SPLITK")) : kMaxSplits;
     const int max_splits = env_splits < 1 ? 1 : (env_splits > kMaxSplits ? kMaxSplits : env_splits);
     const long tiles_m = ((width_counts(a) ? a.M : tiled_rows(a)) + BM - 1) / BM;
     const int num_kb = a.K / BK;
     const long sms = sm_count_gemm();
-    int best = 256;
-    long best_cost = -1, best_rounds = 1;
-    for (int w : widths) {
-        if (a.nf.out_hi != nullptr && (w % 32) != 0) continue;       // the folded norm's partial sums are per 32 aligned columns
-        const long tiles = tiles_m * ((a.N + w - 1) / w);
-        const long rounds = (tiles + sms - 1) / sms;
-        const long cost = rounds * (w + 32);                         // + 32: the part of a tile's time that does not shrink
-        if (best_cost < 0 || cost < best_cost) { best = w; best_cost = cost; best_rounds = rounds; }
-    }
-    *width = best;
+    const TileChoice one = tile_choice(a);
+    *width = one.width;
     *splits = 1;
     if (max_splits < 2 || tiles_m > 1 || a.row_blocks != nullptr || a.tile_counters == nullptr || a.scratch == nullptr) return;   // one row tile only: 256 rows measured 3 % slower split
     const long a_kb = a.a_lo != nullptr ? 32 : 16;                   // KiB of activations per k-block of a 128-row tile
-    const long unsplit = best_rounds * num_kb * (a_kb + best / 8);   // KiB through one CTA
+    const long unsplit = one.rounds * num_kb * (a_kb + one.width / 8);       // KiB through one CTA
     long best_split = -1;
     for (int w : {64, 32}) {
         const long tiles = tiles_m * ((a.N + w - 1) / w);
@@ -979,15 +992,7 @@ static int32_t launch_ext(const GemmArgs& a, cudaStream_t st) {
             default: break;
         }
     }
-    const long tiles_m = by_rows ? e.max_tiles : (tiled_rows(a) + BM - 1) / BM;
-    int best = 256;
-    long best_cost = -1;
-    for (int w : {256, 128, 64, 32}) {
-        const long tiles = tiles_m * ((e.group_rows + w - 1) / w) * (by_rows ? 1 : e.groups);
-        const long rounds = (tiles + sm_count_gemm() - 1) / sm_count_gemm();
-        const long cost = rounds * (w + 32);
-        if (best_cost < 0 || cost < best_cost) { best = w; best_cost = cost; }
-    }
+    const int best = tile_choice(a).width;
 #define LUMI_EXT_CASE(W) if (best == W) return split ? launch_persistent<W, true, true>(a, 1, st) : launch_persistent<W, false, true>(a, 1, st);
     LUMI_EXT_CASE(256) LUMI_EXT_CASE(128) LUMI_EXT_CASE(64) LUMI_EXT_CASE(32)
 #undef LUMI_EXT_CASE
@@ -1000,13 +1005,16 @@ int32_t launch_gemm_tcgen05(const GemmArgs& a, cudaStream_t st) {
     if ((reinterpret_cast<uintptr_t>(a.a_hi) | reinterpret_cast<uintptr_t>(a.w) | reinterpret_cast<uintptr_t>(a.a_lo)) & 15)
         return fail(LUMI_E_INVALID, "tcgen05 GEMM operands must be 16-byte aligned");
     if (a.row_blocks != nullptr) {
-        // below, every row is taken: few rows have kernels and splits of K of their own, and a list that leaves little out saves little
+        // Every row is taken where few rows have kernels and splits of K of their own, where the list leaves next to nothing out, and, above 3 / 4 of the
+        // rows, where single CTAs would come to no fewer rounds: four copies of 32 rows are then slower than one of 128.  All rows / a list, us: 2048 x 1024 x
+        // 2048, one round either way, 15 / 16 of the rows 23.7 / 25.4, 3 / 4 23.7 / 24.7, half 23.7 / 23.6; 2048 x 7360 x 1024, 15 / 16 62.6 / 53.8, 3 / 4 62.6 /
+        // 51.0; pairs 8192 x 7360 x 1024 198 / 185 and 198 / 152, 8192 x 1024 x 2048 56.2 / 55.7 and 56.2 / 49.2.
         if (a.n_row_blocks < 0) return fail(LUMI_E_INVALID, "tcgen05 GEMM: %d row blocks", a.n_row_blocks);
-        if (a.M <= kFewRowsMax || (long)a.n_row_blocks * kRowBlock * 16 > (long)a.M * 15 || (a.ext != nullptr && a.ext->tiles != nullptr)) {
-            GemmArgs all = a;
-            all.row_blocks = nullptr;
+        GemmArgs all = a;
+        all.row_blocks = nullptr;
+        if (a.M <= kFewRowsMax || (long)a.n_row_blocks * kRowBlock * 16 > (long)a.M * 15 || (a.ext != nullptr && a.ext->tiles != nullptr) ||
+            ((long)a.n_row_blocks * kRowBlock * 4 > (long)a.M * 3 && pair_width(a) == 0 && tile_choice(a).cost >= tile_choice(all).cost))
             return launch_gemm_tcgen05(all, st);
-        }
         if (a.n_row_blocks == 0) return LUMI_OK;
     }
     if (a.ext != nullptr) return launch_ext(a, st);
