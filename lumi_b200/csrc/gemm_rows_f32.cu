@@ -17,7 +17,7 @@
 // width.  Warps 0 - 6: a k-block, copied densely to shared memory ahead of time, to registers and split into planes as the MMA reads them (K-major, 128-byte
 // swizzle; bf16 weights are copied straight to their plane).  Warp 7: TMEM, MMA.  Warps 8 - 15: accumulators, sums, results.
 // What bounds it: the splitting (15 pieces of four elements per thread and k-block of 64, 1600 of 2700 cycles), then the MMAs (16 per k-block of 100 cycles,
-// operand reads).  At the cap of 128 registers the 64-row tiles load 88 bytes of spills a thread (76 with bf16 weights), the held group above all.  Launches back to back, weights
+// operand reads).  At the cap of 128 registers the 64-row tiles load 76 bytes of spills a thread, the held group above all.  Launches back to back, weights
 // from memory, against packed fp32 multiply-adds on the CUDA cores, microseconds: fp32 weights 384 x 7360 x 1024 177 -> 84, 384 x 1024 x 2048 129 -> 31, 384 x
 // 32000 x 1024 692 -> 309, 960 x 7360 x 1024 401 -> 167, 32 x 7360 x 1024 30 -> 21, 32 x 1024 x 2048 15 -> 16; bf16 weights 384 x 7360 x 1024 175 -> 60, 32 x
 // 7360 x 1024 27 -> 16.  Scores of 4 x 96 tokens, 48 layers in fp32: 16.6 -> 10.1 ms; a bf16 prompt of 100 tokens 10.0 -> 6.1 ms.
@@ -139,7 +139,7 @@ struct Pieces {
 template <typename WT>
 __device__ __forceinline__ float plain_result(const float* a, const WT* w, int K) {
     float total = 0.f;
-    for (int k0 = 0; k0 < K && total == total; k0 += 512) {             // (no number stays none)
+    for (int k0 = 0; k0 < K; k0 += 512) {
         float group = 0.f;
         for (int k1 = k0; k1 < min(K, k0 + 512); k1 += 128) {
             float unit = 0.f;
@@ -157,6 +157,7 @@ __device__ __forceinline__ float plain_result(const float* a, const WT* w, int K
                     }
                     chain = fmaf(x.w, y.w, fmaf(x.z, y.z, fmaf(x.y, y.y, fmaf(x.x, y.x, chain))));
                 }
+                if (chain != chain) return chain;                       // no number stays none: rows without numbers cost little
                 unit += chain;
             }
             group += unit;

@@ -9,15 +9,17 @@ INF = float("inf")
 BIG = 3.4e38                                                  # rounds to infinity in bf16
 
 
-def check(a, w, touched):
+def check(a, w, touched, prev=None):
     import torch
     want = a.double() @ w.double().T                          # nothing overflows 64 bits: the infinities are those of the operands
-    got = product(a, w).double()
+    want = want if prev is None else want + prev.double()
+    got = product(a, w, prev).double()
     assert torch.equal(torch.isnan(got), torch.isnan(want))
     assert torch.equal(got[want.isinf()], want[want.isinf()])
     fin = want.isfinite()
     size = a.double().abs().nan_to_num(0, 0, 0) @ w.double().abs().nan_to_num(0, 0, 0).T
     bound = (2 + (32 + a.shape[1] / 32) / 2) * 2.0 ** -23 * size      # as for finite operands of any size
+    bound += 0 if prev is None else 2.0 ** -24 * want.abs()
     assert bool(((got - want).abs()[fin] <= bound[fin]).all())
     assert bool(fin.any()) and bool((want.isinf() | (want.abs() > 1e30))[touched].any())
 
@@ -32,7 +34,9 @@ def test_activations(M, N, K, wdt):
     w[0, 3] = 0                                               # infinity times zero
     if M > 40:
         a[37, 1], a[37, 200] = INF, -INF                      # no number for most columns
-    check(a, w, torch.arange(M, device="cuda") % (M - 1) <= 1)
+    touched = torch.arange(M, device="cuda") % (M - 1) <= 1
+    check(a, w, touched)
+    check(a, w, touched, torch.randn((M, N), device="cuda"))  # added to what is there
 
 
 @pytest.mark.parametrize("wdt", ["f32", "bf16"])
