@@ -19,7 +19,7 @@
 // same angle, rounding-level differences; the stored angle may differ from the sequential one by a multiple
 // of 2 pi).
 //
-// One CTA of four warps per (head, sequence), four CTAs per SM (54 KiB of shared memory, 128 registers).
+// One CTA of four warps per (head, sequence), four CTAs per SM (54 KiB of shared memory, 128 registers, 24 bytes of spills).
 //   * Staging: the chunk's x, theta (64 x 32 fp32 each) and the group's raw B, C (64 x 64 fp32 each) arrive by four
 //     cp.async.bulk.tensor copies on one mbarrier (bounded wait).  The operand tiles are built IN PLACE over the
 //     raw rows, so the copies for chunk c+1 are issued when chunk c's products are done; their flight time is covered
