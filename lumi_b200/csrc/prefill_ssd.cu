@@ -27,9 +27,10 @@
 //     asynchronous copies into places that are free by then.
 //   * Segments of 16 tokens, one per warp: decays are taken from segment to segment.  What later segments and the state take of token j is
 //     x_j kap_j times its decay to the end of its segment, one tile for both; Y = C~ S^_in^T walks over the segments ahead of the warp's own, each time
-//     a decay, then + G X; the segment's own block, which needs the warp's rows only, is the one place with a decay per pair of tokens.  Every factor is at
-//     most 1, whatever the decays: logarithms are summed anew behind a token whose decay is 0 in fp32 (a sum with -1e6 in it leaves nothing of the
-//     -0.02 behind it), so sums stay above 16 x -126 in powers of two, and differences that rounding turns positive count as 0.
+//     a decay, then + G X; the segment's own block, which needs the warp's rows only, is the one place with a decay per pair of tokens.  A logarithm counts as
+//     -88 at least, where the decay is 0 in fp32: behind the -1e6 of a clamped decay a sum would have nothing left of the -0.02 of the tokens that follow. So sums
+//     stay above 16 x -88: a factor behind one such token is right to 2^-16 of itself, as the split of operands below, behind fifteen to 2^-11, and at most
+//     1 but for that.
 //   * Arithmetic: every operand is an fp32 value split into bf16 hi + lo; a product is three
 //     mma.sync.m16n8k16 (hi*hi + hi*lo + lo*hi, fp32 accumulate), which keeps ~16 mantissa bits per factor.
 //     Warp w owns tokens 16w..16w+15: its C~ rows stay in registers as A fragments, G's accumulators are
@@ -177,10 +178,9 @@ struct PfSmem {
     float rC[LCH][64];                 // raw C (group)    -> C~: same layout -> z of the warp's tokens
     struct Scalars {                   // per token; the next chunk's are prepared under this one
         float dtp[LCH], rbs[LCH], rcs[LCH];      // dt pi, BCNorm scales
-        float ell[LCH], eli[LCH];      // log2 of the decay from the start of the token's segment of 16 (or from `start`) to the token itself, and the decay
+        float ell[LCH], eli[LCH];      // log2 of the decay from the start of the token's segment of 16 to the token itself, and the decay
         float lam[LCH], kap[LCH];
         float xw[LCH];                 // kap times the decay from the token to the end of its segment
-        int start[LCH];                // the last token of the segment, up to this one, that let nothing through of what came before it; -1: none
         float seg[4];                  // decay over each segment
         float after, pad[3];           // raw lambda of the token behind the chunk
     } sc[2];
@@ -341,7 +341,6 @@ ssd_prefill_kernel(const __grid_constant__ CUtensorMap map32, const __grid_const
     auto prepare_scalars = [&](int t0, PfSmem::Scalars& q) {      // (this lane's copies have landed)
         const int nv = min(LCH, ts - t0);
         float dtpv[2] = {0.f, 0.f}, gl[2] = {0.f, 0.f}, lv[2] = {0.f, 0.f};
-        bool none[2] = {false, false};                     // nothing is left behind this token's decay (2^-126 and less is 0 below)
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
             const int i = 2 * lane + e;
@@ -349,30 +348,19 @@ ssd_prefill_kernel(const __grid_constant__ CUtensorMap map32, const __grid_const
                 dtpv[e] = softplus_ref(__fadd_rn(q.dtp[i], dtb));
                 float av = -softplus_ref(q.ell[i]);
                 av = fminf(fmaxf(av, -1e6f), -1e-4f);
-                gl[e] = __fmul_rn(av, dtpv[e]);           // log a_t
-                none[e] = gl[e] * kLog2E < -126.f;
+                gl[e] = fmaxf(__fmul_rn(av, dtpv[e]), -88.f);      // log a_t; e^-88 < 2^-126 is 0 below
                 lv[e] = sigmoid_ref(q.lam[i]);
             } else {
                 q.rbs[i] = 0.f; q.rcs[i] = 0.f;
             }
         }
         const float after = lane == 31 && t0 + LCH < ts ? sigmoid_ref(q.after) : -1.0f;      // < 0: no next token in this launch
-        // Inclusive prefix of log a over the segment of 16 tokens (eight lanes).  It begins anew behind a token that lets nothing through: a sum that held
-        // such a term would have lost the bits of the decays behind it.
-        const int t0s = 2 * (lane & 7);
-        int from = none[1] ? t0s + 1 : none[0] ? t0s : -1;                   // the last such token so far
-        float incl = none[1] ? 0.f : none[0] ? gl[1] : gl[0] + gl[1];
+        float incl = gl[0] + gl[1];                        // inclusive prefix of log a over the segment of 16 tokens: eight lanes
 #pragma unroll
-        for (int o = 1; o < 8; o <<= 1) {
-            const float n = __shfl_up_sync(0xffffffffu, incl, o, 8);
-            const int f = __shfl_up_sync(0xffffffffu, from, o, 8);
-            if ((lane & 7) >= o && from < 0) { incl += n; from = f; }
-        }
+        for (int o = 1; o < 8; o <<= 1) { const float n = __shfl_up_sync(0xffffffffu, incl, o, 8); if ((lane & 7) >= o) incl += n; }
         float excl = __shfl_up_sync(0xffffffffu, incl, 1, 8);
-        int before = __shfl_up_sync(0xffffffffu, from, 1, 8);
-        if ((lane & 7) == 0) { excl = 0.f; before = -1; }
-        const float l[2] = {none[0] ? 0.f : excl + gl[0], incl};
-        const int start[2] = {none[0] ? t0s : before, from}, last = __shfl_sync(0xffffffffu, from, lane | 7);
+        if ((lane & 7) == 0) excl = 0.f;
+        const float l[2] = {excl + gl[0], incl};
         const float tot = __shfl_sync(0xffffffffu, incl, lane | 7), down = __shfl_down_sync(0xffffffffu, lv[0], 1);
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
@@ -386,11 +374,11 @@ ssd_prefill_kernel(const __grid_constant__ CUtensorMap map32, const __grid_const
                 k = ln < 0.f ? lv[e] : __fadd_rn(lv[e], __fsub_rn(1.0f, ln));
             }
             q.dtp[i] = dtpv[e] * PI_F;
-            q.ell[i] = l[e] * kLog2E; q.eli[i] = start[e] < 0 ? ex2_ftz(l[e] * kLog2E) : 0.f;
-            q.lam[i] = lv[e]; q.kap[i] = k; q.start[i] = start[e];
-            q.xw[i] = t0s + e >= last ? ex2_ftz(fminf(tot - l[e], 0.f) * kLog2E) * k : 0.f;
+            q.ell[i] = l[e] * kLog2E; q.eli[i] = ex2_ftz(l[e] * kLog2E);
+            q.lam[i] = lv[e]; q.kap[i] = k;
+            q.xw[i] = ex2_ftz((tot - l[e]) * kLog2E) * k;
         }
-        if ((lane & 7) == 0) q.seg[lane >> 3] = last < 0 ? ex2_ftz(tot * kLog2E) : 0.f;
+        if ((lane & 7) == 0) q.seg[lane >> 3] = ex2_ftz(tot * kLog2E);
     };
     if (tid == 0) issue_chunk(0);
     if (warp == 0) {
@@ -608,7 +596,6 @@ ssd_prefill_kernel(const __grid_constant__ CUtensorMap map32, const __grid_const
             float g0[4], g1[4];
             causal_product(warp, g0, g1);
             const float la = sc.ell[ia], lb = sc.ell[ib], ma = sc.lam[ia], mb = sc.lam[ib];
-            const int sa = sc.start[ia], sb = sc.start[ib];
             // element e of tile q: row (e < 2 ? g4 : g4 + 8), column 8 q + 2 t4 + (e & 1) of the segment
 #pragma unroll
             for (int q = 0; q < 2; ++q) {
@@ -617,8 +604,8 @@ ssd_prefill_kernel(const __grid_constant__ CUtensorMap map32, const __grid_const
                 for (int e = 0; e < 4; ++e) {
                     const int i = (e < 2) ? g4 : g4 + 8, j = 8 * q + 2 * t4 + (e & 1);
                     float& g = q == 0 ? g0[e] : g1[e];
-                    const float below = g * (ex2_ftz(fminf((e < 2 ? la : lb) - ((e & 1) ? lj.y : lj.x), 0.f)) * ((e & 1) ? kj.y : kj.x));
-                    g = j < i ? (j >= (e < 2 ? sa : sb) ? below : 0.f) : j == i ? fmaf(g, e < 2 ? ma : mb, dskip) : 0.f;
+                    const float below = g * (ex2_ftz((e < 2 ? la : lb) - ((e & 1) ? lj.y : lj.x)) * ((e & 1) ? kj.y : kj.x));
+                    g = j < i ? below : j == i ? fmaf(g, e < 2 ? ma : mb, dskip) : 0.f;
                 }
             }
             add_wx(y, g0, g1, warp);

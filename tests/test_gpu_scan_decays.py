@@ -38,8 +38,8 @@ def test_decays_behind_a_total_one(places, strong):
                                                            yhi.data_ptr(), ylo.data_ptr(), scratch.data_ptr(), 1, T, H, G, 0))
     torch.cuda.synchronize()
     got = (yhi.double() + ylo.double()).cpu().numpy()
-    # as in the test of the edges: 2^-14 of the sum of a result's terms, which is up to about 12 times the largest result here; a decay taken from sums of
-    # at most 16 x 126 is off by 2^-14 of itself, two roundings of 2^-13 / 2 each, where every token of a segment is just short of total, and by 2^-18 else
+    # as in the test of the edges: 2^-14 of the sum of a result's terms, which is up to about 12 times the largest result here; logarithms count as -88 at
+    # least, so behind the up to three strong tokens of a segment here a decay is off by 2^-15 of itself (four roundings of sums up to 264, 2^-17 each)
     assert np.abs(got - want).max() <= 12 * 2.0 ** -14 * np.abs(want).max()
     off = dev[3].cpu().numpy()[0].astype(np.float64) - cum
     off -= 2 * np.pi * np.rint(off / (2 * np.pi))
