@@ -2481,6 +2481,9 @@ int32_t prefill_chunked(lumi_session* s, int batch, int T, bool with_head, float
 int32_t check_status(lumi_session* s) {
     const int st = s->ctl_host->status;
     if (st & STATUS_TIMEOUT) {
+        // CTAs whose wait ran out, or that found the status set, have not arrived at the counters of a split of K: the next products find zeros again.  (Arrivals
+        // by the persistent kernel itself cost its products of 64 to 600 rows 2 - 3 %.)
+        LUMI_CUDA(cudaMemset(s->gemm_counters, 0, sizeof(int32_t) * 2 * kGemmCounters));
         unsigned words[8] = {0};
         if (s->b1_grid_ctl) cudaMemcpy(words, s->b1_grid_ctl, sizeof(words), cudaMemcpyDeviceToHost);
         return fail(LUMI_E_TIMEOUT, "a bounded device-side wait expired (tensor-core GEMM or persistent decode kernel; barrier words %u %u %u %u %u %u abort %u diag 0x%x)",
@@ -3124,6 +3127,7 @@ extern "C" int32_t lumi_debug_gemm(const lumi_gemm_probe* q) {
     LUMI_CUDA(cudaStreamSynchronize(nullptr));
     int32_t st = 0;
     LUMI_CUDA(cudaMemcpy(&st, (const void*)q->status_word, sizeof(st), cudaMemcpyDeviceToHost));
+    if ((st & STATUS_TIMEOUT) && ks.counters != nullptr) LUMI_CUDA(cudaMemset(ks.counters, 0, sizeof(int32_t) * ks.n_counters));      // as check_status does
     if (st & STATUS_TIMEOUT) return fail(LUMI_E_TIMEOUT, "a bounded device-side wait expired in the tensor-core GEMM (limit %llu ns)", (unsigned long long)q->wait_limit_ns);
     return LUMI_OK;
 }

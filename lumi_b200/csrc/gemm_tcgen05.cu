@@ -285,24 +285,9 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_ahi, const __grid
     // A successor launched with programmatic dependent launch may become resident now and run the part of its
     // prologue that does not depend on this kernel (the state step requests its state tiles there).
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    // K split: each of a tile's splits arrives at the counter of every row quarter, also one that has nothing to add, and the last leaves it at zero
-    auto arrive = [&](int t, int quarter) {
-        const bool is_last = atomicAdd(tile_counters + t * 4 + quarter, 1) == splits - 1;
-        if (is_last) atomicExch(tile_counters + t * 4 + quarter, 0);             // ready for the next launch
-        return is_last;
-    };
-    // a wait that ran out before: no new work (one verdict for all threads: the word may change while they look)
-    if (__syncthreads_or(status != nullptr && (*reinterpret_cast<volatile int32_t*>(status) & STATUS_TIMEOUT))) {
-        if constexpr (PAIR) {
-            ntiles = 0;                           // the cluster's barriers are taken
-        } else {
-            if (splits > 1) {
-                asm volatile("griddepcontrol.wait;" ::: "memory");               // the predecessor may be counting there
-                if (warp >= 2 && lane == 0)
-                    for (int u = unit0; u < ntiles * splits; u += units_at_once) arrive(u / splits, warp & 3);
-            }
-            return;
-        }
+    if (status != nullptr && (*reinterpret_cast<volatile int32_t*>(status) & STATUS_TIMEOUT)) {
+        if constexpr (PAIR) ntiles = 0;           // no work, but the cluster's barriers are taken
+        else return;
     }
 
     if (threadIdx.x == 0) {
@@ -519,11 +504,7 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_ahi, const __grid
             }
             if (!mbar_wait(&tmem_full[as], aph, wait_ns)) timed_out = true;
             timed_out = __any_sync(0xffffffffu, timed_out);     // tcgen05.ld below is warp-collective
-            if (timed_out) {
-                if (splits > 1 && lane == 0)
-                    for (int r = u; r < ntiles * splits; r += units_at_once) arrive(r / splits, q);
-                break;
-            }
+            if (timed_out) break;
             tc_fence_after();
             const int acc_in = accumulate;
             if (splits > 1) {
@@ -548,7 +529,11 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_ahi, const __grid
                 __threadfence();
                 __syncwarp();
                 int last = 0;
-                if (lane == 0) last = arrive(t, q);
+                if (lane == 0) {
+                    const int32_t old = atomicAdd(tile_counters + t * 4 + q, 1);
+                    last = old == splits - 1;
+                    if (last) atomicExch(tile_counters + t * 4 + q, 0);          // ready for the next launch
+                }
                 last = __shfl_sync(0xffffffffu, last, 0);
                 if (last) {
                     __threadfence();

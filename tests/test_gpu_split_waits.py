@@ -1,4 +1,4 @@
-"""GPU: a product with K split whose wait ran out leaves its tile counters at zero: the next product with another split is right.  (It does not write a tile
+"""GPU: after a product with K split whose wait ran out the call leaves the tile counters at zero: the next product with another split is right.  (It does not write a tile
 whose counter is beyond its own number of splits; with the same number, partial sums that arrive in time hide the fault.)"""
 import ctypes as C
 
